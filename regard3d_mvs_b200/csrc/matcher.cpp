@@ -424,7 +424,6 @@ struct Match {
   std::vector<uint64_t> tile_cells;  // host copy (ranged: counted on the device)
   std::vector<int> tile_maxnum;
   std::vector<int> tile_width;  // ranged: label width of the kernel shape chosen for the tile
-  std::vector<int> tile_over32;  // ranged: pixels with more than 32 labels
   bool ranged = false;
   // device outputs of the SGM stage
   float* tile_disp = nullptr;
@@ -684,14 +683,12 @@ bool finalize_layout(Match& M, int W, int H_, int partner_w, const r3dgpu_stereo
   M.tile_cells.resize(n);
   M.tile_maxnum.resize(n);
   M.tile_width.assign(n, 0);
-  M.tile_over32.assign(n, 0);
   for (size_t i = 0; i < n; ++i) {
     const Tile& t = M.layout.tiles[i];
     if (M.ranged) {
       const int* st = M.h_stats + i * kTileStats;
       M.tile_cells[i] = M.h_count[i];
       M.tile_maxnum[i] = st[0];
-      M.tile_over32[i] = st[1];
       M.tile_width[i] = sgm_ranged_width_for(st, static_cast<int64_t>(t.w) * t.h);
     } else {
       M.tile_cells[i] = static_cast<uint64_t>(t.w) * static_cast<uint64_t>(t.h) * static_cast<uint64_t>(M.m.nd);
@@ -816,35 +813,20 @@ void plan_path_waves(const std::vector<std::pair<int, int>>& tiles, const std::v
     const Match& M = *matches[mt.first];
     const Tile& T = M.layout.tiles[mt.second];
     const int64_t px = static_cast<int64_t>(T.w) * T.h;
-    const SgmPathShape sh = ranged ? sgm_path_ranged_shape(M.tile_over32[mt.second], px) : sgm_path_shape(M.m.nd);
+    const SgmPathShape sh = ranged ? sgm_path_ranged_shape(static_cast<int64_t>(M.tile_cells[mt.second]), px)
+                                   : sgm_path_shape(M.m.nd);
     es.push_back(Entry{mt.first, mt.second, sh, static_cast<int64_t>(M.tile_cells[mt.second]), px,
                        M.m.diagonal_lr ? static_cast<int64_t>(T.h) * (T.w + M.m.nd) : 0, T.h,
                        M.tile_maxnum[mt.second]});
   }
   // Waves keep byte terms when every match of the group allows them (all
-  // P2 <= 255); otherwise u16 sums only. Ranged groups take byte terms when
-  // all their tiles fit one wave with them (10 bytes per cell held against
-  // 3): a single hierarchical pair's level runs about twice as fast, while
-  // a large batch level split into more waves measured no faster beside the
-  // single-level track. R3DGPU_RANGED_TERMS=0 or 1 forces either.
+  // P2 <= 255); otherwise u16 sums. R3DGPU_RANGED_TERMS=0 keeps u16 sums on
+  // ranged groups (tests of that mode).
   bool terms = true;
   for (const auto& mt : tiles) terms = terms && matches[mt.first]->m.term_u8 != 0;
   if (ranged && terms) {
     const char* rt = std::getenv("R3DGPU_RANGED_TERMS");
-    if (rt != nullptr && *rt != '\0') {
-      terms = std::atoi(rt) == 1;
-    } else {
-      int64_t c = 0, p = 0, k = 0, r = 0;
-      int mx = 16;
-      for (const Entry& e : es) {
-        c += e.cells;
-        p += e.px;
-        k += e.keys;
-        r += e.rows;
-        mx = std::max(mx, e.maxnum);
-      }
-      terms = sgm_path_ranged_buffers(c, p, k, r, mx, sms, true).total <= cap_bytes;
-    }
+    if (rt != nullptr && *rt != '\0') terms = std::atoi(rt) == 1;
   }
   auto bytes = [&](int64_t cells, int64_t px, int64_t keys, int64_t rows, int maxnum) -> size_t {
     return ranged ? sgm_path_ranged_buffers(cells, px, keys, rows, maxnum, sms, terms).total
@@ -1911,9 +1893,7 @@ r3dgpu_status r3dgpu_sgm_cost_volume_host(const r3dgpu_view_u16* left, const r3d
       SgmMatch* dm = A.alloc<SgmMatch>(1);
       R3D_CUDA(cudaMemcpyAsync(dm, hm, sizeof(SgmMatch), cudaMemcpyHostToDevice, s));
       const int64_t px = static_cast<int64_t>(wl) * h;
-      int over32 = 0;
-      for (int64_t i = 0; i < px; ++i) over32 += ranges_num[i] > 32 ? 1 : 0;
-      const SgmPathShape sh = sgm_path_ranged_shape(over32, px);
+      const SgmPathShape sh = sgm_path_ranged_shape(static_cast<int64_t>(cells), px);
       SgmPathJob* hj = W.pinned.alloc<SgmPathJob>(1);
       *hj = SgmPathJob{};
       hj->w = wl;

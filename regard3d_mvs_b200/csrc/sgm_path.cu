@@ -41,6 +41,7 @@ using sgm_simd::group_umin;
 using sgm_simd::kSent2;
 constexpr float kInfF = __builtin_huge_valf();
 constexpr int kPathThreads = 256;
+constexpr int kPathCounters = 256;  // block counters of a wave's launches (one each)
 
 inline size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
 
@@ -107,8 +108,10 @@ constexpr int kCostStage = 2048;  // staged partner codes per warp at most (sgm_
 // width + labels - 1), so that narrow waves run more CTAs per SM.
 R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
     sgm_path_cost_kernel(const SgmMatch* R3D_RESTRICT matches, const SgmPathJob* R3D_RESTRICT jobs, int njobs,
-                         int64_t rows, uint8_t* R3D_RESTRICT cost, int stage_words, uint16_t* R3D_RESTRICT ints) {
+                         int64_t rows, uint8_t* R3D_RESTRICT cost, int stage_words, uint16_t* R3D_RESTRICT ints,
+                         int* R3D_RESTRICT counters) {
   R3D_DYNAMIC_SMEM(smem);
+  if (blockIdx.x == 0 && threadIdx.x < kPathCounters) counters[threadIdx.x] = 0;
   const int lane = static_cast<int>(threadIdx.x & 31u), warp = static_cast<int>(threadIdx.x >> 5);
   const int wpb = static_cast<int>(blockDim.x) >> 5;
   uint64_t* stage = reinterpret_cast<uint64_t*>(smem) + static_cast<size_t>(warp) * stage_words;
@@ -198,16 +201,66 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
 // last pass forms S = L_8 + 7 C + sum T_r (at most 8 (255 + 255) < 2^16, so
 // the sum modulo 2^16 is the plain sum) and takes the winner-takes-all.
 enum PassMode { kFirst = 0, kAccumulate = 1, kLast = 2, kTerm = 3, kLastTerm = 4 };
-constexpr int kTermArrays = 7;
-// The passes of one launch: n directions, chain blocks of pass q numbered
-// from start[q] (start[n] = all blocks), slot = its term array.
+constexpr int kTermArrays = 7;    // of the full-range passes (the last pass adds its own path)
+constexpr int kRangedTerms = 8;   // of the ranged passes (summed per pixel)
+constexpr int kMaxPasses = 8;
+// The passes of one launch: n directions (slot = its term array), their
+// number per chain class, and the chain blocks of all of them together. The
+// blocks are numbered tile after tile, within a tile direction after
+// direction: the directions of a tile run close together, so that its costs
+// are read from DRAM about once and from L2 after that.
 struct PassSet {
   int n;
   uint32_t one;  // 1 (see fma_add)
-  int cls[kTermArrays], dx[kTermArrays], dy[kTermArrays], slot[kTermArrays];
-  int64_t start[kTermArrays + 1];
+  int cls[kMaxPasses], dx[kMaxPasses], dy[kMaxPasses], slot[kMaxPasses];
+  int per_class[kPathClasses];
+  int64_t total;
+  int* next;  // the next block to hand out after one per resident warp (zeroed with the wave)
 };
-constexpr int kPathStages = 4;  // ring stages of the ranged passes
+
+// The block a warp takes after its current one: warps take one each to begin
+// with, then the next free one, since blocks differ in length (diagonals, wide
+// ranges): a fixed stride left a second round half empty.
+R3D_DEVICE int64_t next_block(const PassSet& ps, int64_t nwarps) {
+  uint32_t n = 0;
+  if (r3dsimt::lane_id() == 0) n = static_cast<uint32_t>(atomicAdd(ps.next, 1));
+  return nwarps + static_cast<int64_t>(r3dsimt::shfl(n, 0));
+}
+
+// Tile j, direction and chain block (returned: the block's number within its
+// tile and direction, of CPW chains) of block gblk of the launch.
+template <int CPW>
+R3D_DEVICE int64_t locate_block(const SgmPathJob* jobs, int njobs, const PassSet& ps, int64_t gblk, int& j, int& cls,
+                                int& dx, int& dy, int& slot) {
+  const int64_t n0 = ps.per_class[0], n1 = ps.per_class[1], n2 = ps.per_class[2];
+  auto key = [n0, n1, n2](const SgmPathJob& q) { return n0 * q.blk[0] + n1 * q.blk[1] + n2 * q.blk[2]; };
+  j = find_job(jobs, njobs, gblk, key);
+  const SgmPathJob& job = jobs[j];
+  int64_t blk = gblk - key(job);
+  cls = ps.cls[0];
+  dx = ps.dx[0];
+  dy = ps.dy[0];
+  slot = ps.slot[0];
+  bool found = false;
+#pragma unroll
+  for (int q = 0; q < kMaxPasses; ++q) {  // static indices only: no local copy of ps
+    if (q < ps.n && !found) {
+      const int c = ps.cls[q];
+      const int chains = c == 0 ? job.h : (c == 1 ? job.w : job.w + job.h - 1);
+      const int nb = (chains + CPW - 1) / CPW;
+      if (blk < nb) {
+        found = true;
+        cls = c;
+        dx = ps.dx[q];
+        dy = ps.dy[q];
+        slot = ps.slot[q];
+      } else {
+        blk -= nb;
+      }
+    }
+  }
+  return blk;
+}
 
 // Per-halfword a + b modulo 2^16.
 R3D_DEVICE uint32_t add2(uint32_t a, uint32_t b, bool no_carry) { return no_carry ? a + b : r3dsimt::vadd2(a, b); }
@@ -321,25 +374,12 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN((PathRing<G, K, MODE>::kThreads), (PathRin
   unsigned char* const ring_sum = ring + CPW * Ring::ND + gi * 2 * Ring::ND + 2 * e0;
   unsigned char* const ring_term = ring + CPW * Ring::ND + gi * Ring::ND + e0;  // + r * CPW * ND
   unsigned char* const ring_int = ring + Ring::kPlaneBytes + lane * 4;
-  const int64_t total_blocks = ps.start[ps.n];
   const uint32_t one = ps.one;
-  for (int64_t gblk = static_cast<int64_t>(blockIdx.x) * wpb + (threadIdx.x >> 5); gblk < total_blocks;
-       gblk += nwarps) {
+  for (int64_t gblk = static_cast<int64_t>(blockIdx.x) * wpb + (threadIdx.x >> 5); gblk < ps.total;
+       gblk = next_block(ps, nwarps)) {
     if (cancelled(cancel)) break;
-    // The pass of the block (static indices only: no local copy of ps).
-    int cls = ps.cls[0], dx = ps.dx[0], dy = ps.dy[0], tslot = ps.slot[0];
-    int64_t blk = gblk;
-#pragma unroll
-    for (int q = 1; q < kTermArrays; ++q) {
-      if (q < ps.n && gblk >= ps.start[q]) {
-        cls = ps.cls[q];
-        dx = ps.dx[q];
-        dy = ps.dy[q];
-        tslot = ps.slot[q];
-        blk = gblk - ps.start[q];
-      }
-    }
-    const int j = find_job(jobs, njobs, blk, [cls](const SgmPathJob& q) { return q.blk[cls]; });
+    int j, cls, dx, dy, tslot;
+    const int64_t blk = locate_block<CPW>(jobs, njobs, ps, gblk, j, cls, dx, dy, tslot);
     const SgmPathJob& job = jobs[j];
     const SgmMatch& m = matches[job.match];
     if (job.match != lut_match) {  // the same for the whole warp (one chain block)
@@ -353,7 +393,7 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN((PathRing<G, K, MODE>::kThreads), (PathRin
     const uint32_t p1x2 = static_cast<uint32_t>(m.p1) * 0x10001u;
     const bool no_carry = m.sum_no_carry != 0;
     int sx, sy, len;
-    chain_geometry(cls, dx, dy, w, job.h, (blk - job.blk[cls]) * CPW + gi, sx, sy, len);
+    chain_geometry(cls, dx, dy, w, job.h, blk * CPW + gi, sx, sy, len);
     int maxlen = len;
 #pragma unroll
     for (int o = G; o < 32; o <<= 1) maxlen = r3dsimt::imax(maxlen, static_cast<int>(r3dsimt::shfl_xor(maxlen, o)));
@@ -708,7 +748,50 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN((PathRing<G, K, MODE>::kThreads), (PathRin
 }
 
 // ---------------------------------------------------------------- acceptance
-// stereo_matcher.cpp:474-523 with lo = 0, num = nd for every pixel.
+// stereo_matcher.cpp:474-523: validity, the rejection of a minimum on the edge
+// of a reduced range (:501-503), the diagonal left-right check (`shift` is the
+// row's key offset), uniqueness, subpixel fit and confidence of one pixel.
+struct Winner {
+  int best;                    // label of the first minimum
+  uint32_t bcost, sec, sm, sp;  // S there, second best, S at best -+ 1
+};
+R3D_DEVICE void accept_pixel(const SgmMatch& m, const SgmPathJob& job, int x, int y, int lo, int num, const Winner& v,
+                             const uint32_t* rkeys, int shift, float& d, float& cf) {
+  const int bx = job.x0 + x, by = job.y0 + y;
+  const RowInterval rv = m.pv[by];
+  const int jb = v.best - lo;
+  const int xr = bx - m.dmin - v.best;
+  bool ok = xr >= rv.first && xr <= rv.last;
+  if ((jb == 0 && lo > 0) || (jb == num - 1 && lo + num < m.nd)) ok = false;
+  if (ok && m.diagonal_lr) {
+    const uint32_t key = rkeys[job.rk_off + static_cast<int64_t>(y) * (job.w + m.nd) + (x - v.best + shift)];
+    const int rb = key == 0xFFFFFFFFu ? 0xFFFF : static_cast<int>(key & 0xFFFFu) - x + v.best;
+    const int diff = rb - v.best;
+    if ((diff < 0 ? -diff : diff) > m.lr_max_diff) ok = false;
+  }
+  const float best_cost = static_cast<float>(v.bcost);
+  if (ok && m.uniqueness > 0.0F && v.sec != 0xFFFFu &&
+      best_cost > __fmul_rn(__fsub_rn(1.0F, m.uniqueness), static_cast<float>(v.sec)))
+    ok = false;
+  if (!ok) return;
+  float delta = 0.0F;
+  if (jb > 0 && jb < num - 1)
+    delta = sgm_simd::subpixel_delta(m.subpixel, static_cast<float>(v.sm), best_cost, static_cast<float>(v.sp));
+  d = __fadd_rn(static_cast<float>(m.dmin + v.best), delta);
+  if (m.confidence)
+    cf = (v.sec != 0xFFFFu && v.sec > 0u) ? __fsub_rn(1.0F, __fdiv_rn(best_cost, static_cast<float>(v.sec))) : 0.0F;
+}
+
+R3D_DEVICE int4 pack_winner(const Winner& v) {
+  return make_int4(static_cast<int>(static_cast<uint32_t>(v.best) | (v.bcost << 16)),
+                   static_cast<int>(v.sec | (v.sm << 16)), static_cast<int>(v.sp), 0);
+}
+R3D_DEVICE Winner unpack_winner(int4 in) {
+  return Winner{in.x & 0xFFFF, static_cast<uint32_t>(in.x) >> 16, static_cast<uint32_t>(in.y) & 0xFFFFu,
+                static_cast<uint32_t>(in.y) >> 16, static_cast<uint32_t>(in.z)};
+}
+
+// Full range: lo = 0, num = nd for every pixel.
 R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
     sgm_path_accept_kernel(const SgmMatch* R3D_RESTRICT matches, const SgmPathJob* R3D_RESTRICT jobs, int njobs,
                            int64_t pixels, const int4* R3D_RESTRICT info, const uint32_t* R3D_RESTRICT rkeys) {
@@ -720,38 +803,10 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
     const int nd = m.nd, w = job.w;
     const int p = static_cast<int>(i - job.px_off);
     const int y = p / w, x = p - (p / w) * w;
-    const int bx = job.x0 + x, by = job.y0 + y;
-    const RowInterval lv = m.bv[by];
+    const RowInterval lv = m.bv[job.y0 + y];
     float d = kInfF, cf = 0.0F;
-    if (bx >= lv.first && bx <= lv.last) {
-      const int4 in = info[i];
-      const int best = in.x & 0xFFFF;
-      const uint32_t bcost = static_cast<uint32_t>(in.x) >> 16;
-      const uint32_t sec = static_cast<uint32_t>(in.y) & 0xFFFFu;
-      const uint32_t sm = static_cast<uint32_t>(in.y) >> 16;
-      const uint32_t sp = static_cast<uint32_t>(in.z);
-      const RowInterval rv = m.pv[by];
-      const int xr = bx - m.dmin - best;
-      bool ok = xr >= rv.first && xr <= rv.last;
-      if (ok && m.diagonal_lr) {
-        const uint32_t key = rkeys[job.rk_off + static_cast<int64_t>(y) * (w + nd) + (x - best + nd - 1)];
-        const int rb = key == 0xFFFFFFFFu ? 0xFFFF : static_cast<int>(key & 0xFFFFu) - x + best;
-        const int diff = rb - best;
-        if ((diff < 0 ? -diff : diff) > m.lr_max_diff) ok = false;
-      }
-      const float best_cost = static_cast<float>(bcost);
-      if (ok && m.uniqueness > 0.0F && sec != 0xFFFFu &&
-          best_cost > __fmul_rn(__fsub_rn(1.0F, m.uniqueness), static_cast<float>(sec)))
-        ok = false;
-      if (ok) {
-        float delta = 0.0F;
-        if (best > 0 && best < nd - 1)
-          delta = sgm_simd::subpixel_delta(m.subpixel, static_cast<float>(sm), best_cost, static_cast<float>(sp));
-        d = __fadd_rn(static_cast<float>(m.dmin + best), delta);
-        if (m.confidence)
-          cf = (sec != 0xFFFFu && sec > 0u) ? __fsub_rn(1.0F, __fdiv_rn(best_cost, static_cast<float>(sec))) : 0.0F;
-      }
-    }
+    if (job.x0 + x >= lv.first && job.x0 + x <= lv.last)
+      accept_pixel(m, job, x, y, 0, nd, unpack_winner(info[i]), rkeys, nd - 1, d, cf);
     job.disp[p] = d;
     if (job.conf != nullptr) job.conf[p] = cf;
     if (p == 0) *job.cells = static_cast<unsigned long long>(w) * static_cast<unsigned long long>(job.h) * nd;
@@ -760,16 +815,34 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
 
 // ================================================================ ranged tiles
 // Per-pixel label ranges (lo, num; num a multiple of 16): the same passes on
-// costs and sums packed per tile (pixel after pixel, num labels each).
+// costs, terms and sums packed per tile, pixel after pixel, in units of 16
+// labels. Within a unit the labels are interleaved so that a 32-bit word of
+// the passes holds labels k and k + 8: the neighbours d -+ 1 of word k are
+// then words k -+ 1, without byte permutes. Byte planes (costs, terms) store
+// the bytes of word j = 0..3 of a unit as labels 2 j, 2 j + 1, 2 j + 8, 2 j + 9
+// (one mask or permute unpacks a word, one multiply-add packs two); sums
+// store word k = 0..7 as the halves of labels k and k + 8.
 
-// Per wave row: the in-row exclusive prefix of num (the pixel's cell offset
-// before its row start is added), the range and the base intensity of every
-// pixel as one 16-byte record {offset, lo | num << 16, intensity, 0}; the
-// row's label total and its right-WTA shift max(lo + num - 1 - x).
+// Record of a pixel: x = cell offset / 16 within its tile | min(units, 31)
+// << 27 (a tile has fewer than 2^31 labels; 31 stands for 31 or more, looked
+// up in the ranges), y = lo | base intensity << 16.
+constexpr int kRecShift = 27;
+constexpr uint32_t kRecOffset = (1u << kRecShift) - 1u, kRecWide = 31u;
+
+// Units of the pixel at (x, y) of the tile with record r.
+R3D_DEVICE int rec_units(const uint2& r, const SgmMatch& m, const SgmPathJob& job, int x, int y) {
+  const uint32_t n = r.x >> kRecShift;
+  if (n != kRecWide) return static_cast<int>(n);
+  return m.rnum[static_cast<int64_t>(job.y0 + y) * m.r_stride + job.x0 + x] >> 4;
+}
+
+// Per wave row: the row's label total and its right-WTA shift max(lo + num -
+// 1 - x).
 R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
     sgm_path_ranged_rows_kernel(const SgmMatch* R3D_RESTRICT matches, const SgmPathJob* R3D_RESTRICT jobs, int njobs,
-                                int64_t rows, int4* R3D_RESTRICT rec, int* R3D_RESTRICT rowsum,
-                                int* R3D_RESTRICT rowshift) {
+                                int64_t rows, int* R3D_RESTRICT rowsum, int* R3D_RESTRICT rowshift,
+                                int* R3D_RESTRICT counters) {
+  if (blockIdx.x == 0 && threadIdx.x < kPathCounters) counters[threadIdx.x] = 0;
   const int lane = static_cast<int>(threadIdx.x & 31u);
   const int wpb = static_cast<int>(blockDim.x) >> 5;
   const int64_t nwarps = static_cast<int64_t>(gridDim.x) * wpb;
@@ -777,34 +850,20 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
     const int j = find_job(jobs, njobs, r, [](const SgmPathJob& q) { return q.row_off; });
     const SgmPathJob& job = jobs[j];
     const SgmMatch& m = matches[job.match];
-    const int y = static_cast<int>(r - job.row_off), by = job.y0 + y, w = job.w;
-    int run = 0, shift = -0x7FFFFFFF;
-    for (int xb = 0; xb < w; xb += 32) {
-      const int x = xb + lane;
-      int lo = 0, num = 0, iv = 0;
-      if (x < w) {
-        const int64_t ri = static_cast<int64_t>(by) * m.r_stride + job.x0 + x;
-        lo = m.rlo[ri];
-        num = m.rnum[ri];
-        iv = m.base[static_cast<int64_t>(by) * m.base_stride + job.x0 + x];
-        shift = r3dsimt::imax(shift, lo + num - 1 - x);
-      }
-      int incl = num;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = static_cast<int>(r3dsimt::shfl(static_cast<uint32_t>(incl), lane >= o ? lane - o : lane));
-        if (lane >= o) incl += v;
-      }
-      if (x < w)
-        rec[job.px_off + static_cast<int64_t>(y) * w + x] =
-            make_int4(run + incl - num, lo | (num << 16), iv, 0);
-      run += static_cast<int>(r3dsimt::shfl(static_cast<uint32_t>(incl), 31));
+    const int64_t row = static_cast<int64_t>(job.y0 + static_cast<int>(r - job.row_off)) * m.r_stride + job.x0;
+    int sum = 0, shift = -0x7FFFFFFF;
+    for (int x = lane; x < job.w; x += 32) {
+      const int num = m.rnum[row + x];
+      sum += num;
+      shift = r3dsimt::imax(shift, m.rlo[row + x] + num - 1 - x);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+    for (int o = 16; o > 0; o >>= 1) {
+      sum += static_cast<int>(r3dsimt::shfl_xor(static_cast<uint32_t>(sum), o));
       shift = r3dsimt::imax(shift, static_cast<int>(r3dsimt::shfl_xor(static_cast<uint32_t>(shift), o)));
+    }
     if (lane == 0) {
-      rowsum[r] = run;
+      rowsum[r] = sum;
       rowshift[r] = shift;
     }
   }
@@ -836,147 +895,160 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
   }
 }
 
-// Per pixel: the final cell offset (row start added) and the u8 costs of its
-// num labels, C(p, lo + j) of stereo_matcher.cpp:305-353.
+// Per wave row, one warp: every pixel's record and the u8 costs of its num
+// labels, C(p, lo + j) of stereo_matcher.cpp:305-353.
 R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
     sgm_path_ranged_cost_kernel(const SgmMatch* R3D_RESTRICT matches, const SgmPathJob* R3D_RESTRICT jobs, int njobs,
-                                int64_t pixels, int4* R3D_RESTRICT rec, const int* R3D_RESTRICT rowstart,
+                                int64_t rows, uint2* R3D_RESTRICT rec, const int* R3D_RESTRICT rowstart,
                                 uint8_t* R3D_RESTRICT cost) {
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < pixels; i += stride) {
-    const int j = find_job(jobs, njobs, i, [](const SgmPathJob& q) { return q.px_off; });
+  const int lane = static_cast<int>(threadIdx.x & 31u);
+  const int wpb = static_cast<int>(blockDim.x) >> 5;
+  const int64_t nwarps = static_cast<int64_t>(gridDim.x) * wpb;
+  for (int64_t r = static_cast<int64_t>(blockIdx.x) * wpb + (threadIdx.x >> 5); r < rows; r += nwarps) {
+    const int j = find_job(jobs, njobs, r, [](const SgmPathJob& q) { return q.row_off; });
     const SgmPathJob& job = jobs[j];
     const SgmMatch& m = matches[job.match];
-    const int p = static_cast<int>(i - job.px_off);
-    const int y = p / job.w, x = p - y * job.w;
-    int4 rc = rec[i];
-    rc.x += rowstart[job.row_off + y];
-    rec[i] = rc;
-    const int lo = rc.y & 0xFFFF, num = static_cast<int>(static_cast<uint32_t>(rc.y) >> 16);
-    const int bx = job.x0 + x, by = job.y0 + y;
+    const int y = static_cast<int>(r - job.row_off), by = job.y0 + y, w = job.w;
     const RowInterval lv = m.bv[by], rv = m.pv[by];
-    const bool inside = bx >= lv.first && bx <= lv.last;
-    const uint64_t cl = inside ? m.cbase[static_cast<int64_t>(by) * m.cb_stride + bx] : 0;
+    const uint64_t* lrow = m.cbase + static_cast<int64_t>(by) * m.cb_stride;
     const uint64_t* crow = m.cpart + static_cast<int64_t>(by) * m.cp_stride;
+    const uint16_t* irow = m.base + static_cast<int64_t>(by) * m.base_stride;
+    const uint16_t* lorow = m.rlo + static_cast<int64_t>(by) * m.r_stride;
+    const uint16_t* numrow = m.rnum + static_cast<int64_t>(by) * m.r_stride;
     const int safe = rv.first > 0 ? rv.first : 0;
     const uint32_t inv = static_cast<uint32_t>(m.invalid_cost);
-    uint8_t* out = cost + job.cell_off + rc.x;
-    for (int c = 0; c < num; c += 16) {
-      uint32_t q[4] = {0, 0, 0, 0};
-      if (inside) {
-        const int xr0 = bx - m.dmin - lo - c;
+    int run = rowstart[r] >> 4;
+    for (int xb = 0; xb < w; xb += 32) {
+      const int x = xb + lane, bx = job.x0 + x;
+      const int lo = x < w ? lorow[bx] : 0, nu = x < w ? numrow[bx] >> 4 : 0;
+      int incl = nu;
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
-          const int xr = xr0 - k;
-          const bool ok = xr >= rv.first && xr <= rv.last;
-          const uint64_t cr = crow[ok ? xr : safe];
-          const uint32_t v = ok ? static_cast<uint32_t>(r3dsimt::popc64(cl ^ cr)) : inv;
-          q[k >> 2] |= v << (8 * (k & 3));
-        }
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = static_cast<int>(r3dsimt::shfl(static_cast<uint32_t>(incl), lane >= o ? lane - o : lane));
+        if (lane >= o) incl += v;
       }
-      *reinterpret_cast<uint4*>(out + c) = make_uint4(q[0], q[1], q[2], q[3]);
+      const int off = run + incl - nu;
+      run += static_cast<int>(r3dsimt::shfl(static_cast<uint32_t>(incl), 31));
+      if (x < w)
+        rec[job.px_off + static_cast<int64_t>(y) * w + x] =
+            make_uint2(static_cast<uint32_t>(off) | (r3dsimt::umin(static_cast<uint32_t>(nu), kRecWide) << kRecShift),
+                       static_cast<uint32_t>(lo) | (static_cast<uint32_t>(irow[bx]) << 16));
+      const bool inside = x < w && bx >= lv.first && bx <= lv.last;
+      const uint64_t cl = inside ? lrow[bx] : 0;
+      uint8_t* out = cost + job.cell_off + static_cast<int64_t>(off) * 16;
+      for (int u = 0; u < nu; ++u) {
+        uint32_t q[4] = {0, 0, 0, 0};
+        const int xr0 = bx - m.dmin - lo - 16 * u;  // right column of the unit's label 0
+        if (inside && xr0 <= rv.last && xr0 - 15 >= rv.first) {
+          // Every label reads a valid right column: the two popcounts of each
+          // Census XOR packed separately (each byte at most 32, no carries).
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int l[4] = {2 * k, 2 * k + 1, 2 * k + 8, 2 * k + 9};
+            uint32_t a = 0, b = 0;
+#pragma unroll
+            for (int i = 3; i >= 0; --i) {
+              const uint64_t d = cl ^ crow[xr0 - l[i]];
+              a = a * 256u + static_cast<uint32_t>(r3dsimt::popc(static_cast<uint32_t>(d)));
+              b = b * 256u + static_cast<uint32_t>(r3dsimt::popc(static_cast<uint32_t>(d >> 32)));
+            }
+            q[k] = a + b;
+          }
+        } else if (inside) {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            const int xr = xr0 - k;
+            const bool ok = xr >= rv.first && xr <= rv.last;
+            const uint64_t cr = crow[ok ? xr : safe];
+            const uint32_t v = ok ? static_cast<uint32_t>(r3dsimt::popc64(cl ^ cr)) : inv;
+            q[(k & 7) >> 1] |= v << (8 * ((k & 1) + 2 * (k >> 3)));
+          }
+        }
+        *reinterpret_cast<uint4*>(out + 16 * u) = make_uint4(q[0], q[1], q[2], q[3]);
+      }
     }
   }
 }
 
-// Labels of a chain's predecessor vector kept in shared memory (u32 words of
-// two labels); wider vectors continue in the chain's global overflow. A
-// buffer holds a sentinel word before the vector (index -1) and one after it
-// (index nw, written with the vector), so that a vector of at most
-// kRangedSmemWords words is read at a clamped index without bounds checks.
-// The buffers of a warp's chains are kRangedSmemStride words apart (odd, so
-// that the chains of a warp start in different banks).
-constexpr int kRangedSmemWords = 32;
-// Ranged pass CTAs have 4 warps: about 15 KB of shared memory per warp
-// (ring, records, predecessor buffers), so that three CTAs fit an SM.
-constexpr int kRangedThreads = 128;
-constexpr int kRangedSmemStride = kRangedSmemWords + 3;
+// Passes over ranged tiles: one lane walks one chain, 32 chains per warp, pixel
+// by pixel in step. A pixel's labels are taken CH = 2 K at a time (chunks of
+// K / 8 units): one chunk for most pixels, more for wider ones.
+//
+// The predecessor vector stays in registers as long as every lane's next
+// pixel has exactly CH labels in the same range as its last one (70 to 89 % of
+// the steps of smooth disparities): such a step is the plain recurrence on K
+// words, with no realignment, no shuffle and no shared-memory vector. When the
+// warp's next step is not of that kind, the lanes write their vectors in
+// label order into their own buffers (up to kVecLabels labels in shared
+// memory, wider ones in global memory that the L1 holds), and the step reads
+// its predecessor labels at its range's shift there, sentinels around them.
+// Everything is private to a lane: no barrier, no warp-wide minimum.
+//
+// One lane per chain against the lane group of the full-range passes: most
+// ranges are one or two units, so a group would idle on the narrow pixels and
+// pay shuffles for every minimum and neighbour. One warp per CTA: the shared
+// memory of an SM is split as finely as the ring allows.
+constexpr int kRangedThreads = 32;
 
-// Ring of the ranged passes: D stages of chunk 0's bytes (kPlanes bytes per
-// label: cost, plus the u16 sum or the seven byte terms) and 2 D record slots.
-template <int G, int K, int MODE>
+// Per warp: the ring of D pixels' first chunks (16-byte pieces, [piece][lane]),
+// pixel records, two predecessor buffers per lane (odd stride in words: the
+// same word of all lanes lies in distinct banks) and the match's P2 table.
+template <int K, int MODE>
 struct RangedRing {
-  static constexpr int CH = 2 * G * K;  // labels per chunk
-  static constexpr int CPW = 32 / G;
-  // Two stages for the passes that stage several planes (the accumulate
-  // pass: cost and sum; the byte-term last pass: eight planes), four for
-  // the one-plane passes: less shared memory per warp, more warps per SM.
-  static constexpr int D = MODE == kLastTerm || MODE == kAccumulate ? 2 : kPathStages;
-  static constexpr int kPlanes = MODE == kAccumulate ? 3 : (MODE == kLastTerm ? 1 + kTermArrays : 1);
-  static constexpr int kDataStage = CPW * kPlanes * CH;
-  static constexpr int kData = D * kDataStage;
-  static constexpr int kRec = 2 * D * 32 * 16;  // one record slot per lane and stage
-  static constexpr int kPrev = CPW * 2 * kRangedSmemStride * 4;
-  static constexpr int kLut = 512;  // the warp's copy of its match's P2 table
-  static constexpr int kWarpBytes = kData + kRec + kPrev + kLut;
+  static constexpr int CH = 2 * K;    // labels per chunk
+  static constexpr int UF = K / 8;    // units per chunk
+  static constexpr int D = 4;
+  static constexpr int NR = 2 * D;    // record slots (a power of two)
+  static constexpr int kPieces = UF * (MODE == kAccumulate ? 3 : 1);
+  static constexpr int kStageBytes = kPieces * 512;
+  static constexpr int kData = D * kStageBytes;
+  static constexpr int kRec = NR * 32 * 8;
+  static constexpr int kVecLabels = 32;          // labels of a vector in shared memory
+  static constexpr int kPadWords = (CH + 2) / 2;  // sentinels before and after a vector
+  static constexpr int kVecStep = kVecLabels / 2 + kPadWords;  // from buffer 0 to buffer 1
+  static constexpr int kVecStride = (2 * kVecStep + kPadWords + 1) | 1;
+  static constexpr int kVec = 32 * kVecStride * 4;
+  static constexpr int kWarpBytes = kData + kRec + kVec + 512;
   static constexpr int kBlockBytes = (kRangedThreads / 32) * kWarpBytes;
 };
 
-template <int G, int K, int MODE>
+template <int K, int MODE>
 R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
     sgm_path_ranged_kernel(const SgmMatch* R3D_RESTRICT matches, const SgmPathJob* R3D_RESTRICT jobs, int njobs,
-                           const PassSet ps, const int4* R3D_RESTRICT rec, const uint8_t* R3D_RESTRICT cost,
-                           uint16_t* sum, uint8_t* terms, int64_t tstride, uint32_t* ovf, int64_t ovf_words,
+                           const PassSet ps, const uint2* R3D_RESTRICT rec, const uint8_t* R3D_RESTRICT cost,
+                           uint16_t* sum, uint8_t* terms, int64_t tstride, uint32_t* ovf, int ovf_words,
                            const int* cancel) {
   // Modes: kFirst / kAccumulate write or add u16 sums; kTerm writes the
-  // pass's byte terms; kLastTerm writes S = L_8 + 7 C + sum of the seven
-  // terms as the u16 sum (read by the per-pixel winner-takes-all).
-  using R = RangedRing<G, K, MODE>;
-  constexpr int CPW = R::CPW, U = K / 4, CH = R::CH, D = R::D;
-  constexpr bool kReadsSum = MODE == kAccumulate;
+  // pass's byte terms (all eight directions in one launch).
+  using R = RangedRing<K, MODE>;
+  constexpr int CH = R::CH, UF = R::UF, D = R::D, NR = R::NR, NS = R::kVecLabels, PAD = R::kPadWords;
   R3D_DYNAMIC_SMEM(smem);
   const int lane = static_cast<int>(threadIdx.x & 31u), warp = static_cast<int>(threadIdx.x >> 5);
-  const int gi = lane / G, t = lane % G;
-  const int e0 = 2 * t * K;  // first label of the lane within a chunk
   const int wpb = static_cast<int>(blockDim.x) >> 5;
   const int64_t nwarps = static_cast<int64_t>(gridDim.x) * wpb;
-  unsigned char* wb = smem + static_cast<size_t>(warp) * R::kWarpBytes;
-  int4* recs = reinterpret_cast<int4*>(wb + R::kData);
-  // Buffer b of this lane's chain: words (b * CPW + gi) * kRangedSmemStride onwards.
-  uint32_t* prevw = reinterpret_cast<uint32_t*>(wb + R::kData + R::kRec) + gi * kRangedSmemStride;
-  uint16_t* const lut = reinterpret_cast<uint16_t*>(wb + R::kData + R::kRec + R::kPrev);
-  int lut_match = -1;
-  uint32_t* ovfc = ovf + (static_cast<int64_t>(blockIdx.x) * wpb * CPW + warp * CPW + gi) * 2 * ovf_words;
-  auto stage_cost = [&](int st) -> unsigned char* { return wb + st * R::kDataStage + gi * CH + e0; };
-  auto stage_sum = [&](int st) -> unsigned char* {
-    return wb + st * R::kDataStage + CPW * CH + gi * 2 * CH + 2 * e0;
-  };
-  auto stage_term = [&](int st, int r) -> unsigned char* {
-    return wb + st * R::kDataStage + (1 + r) * CPW * CH + gi * CH + e0;
-  };
-  // Word idx (labels 2 idx, 2 idx + 1) of buffer b of the predecessor vector
-  // (nw words long): two sentinels outside it.
-  // The shared-memory word is read unconditionally (at a wrapped, in-bounds
-  // index); only the rare words of wide vectors go to the overflow.
-  auto qword = [&](int b, int idx, int nw) -> uint32_t {
-    const uint32_t* vec = prevw + b * CPW * kRangedSmemStride + 1;
-    if (nw <= kRangedSmemWords) return vec[r3dsimt::imax(r3dsimt::imin(idx, nw), -1)];
-    uint32_t v = vec[idx & (kRangedSmemWords - 1)];
-    if (idx >= kRangedSmemWords && idx < nw) v = ovfc[b * ovf_words + (idx - kRangedSmemWords)];
-    return (idx < 0 || idx >= nw) ? kSent2 : v;
-  };
-  auto put_word = [&](int b, int idx, uint32_t v) {
-    if (idx < kRangedSmemWords) prevw[b * CPW * kRangedSmemStride + 1 + idx] = v;
-    else ovfc[b * ovf_words + (idx - kRangedSmemWords)] = v;
-  };
-  const int64_t total_blocks = ps.start[ps.n];
-  const uint32_t one = ps.one;
-  for (int64_t gblk = static_cast<int64_t>(blockIdx.x) * wpb + warp; gblk < total_blocks; gblk += nwarps) {
-    if (cancelled(cancel)) break;
-    // The pass of the block (static indices only: no local copy of ps).
-    int cls = ps.cls[0], dx = ps.dx[0], dy = ps.dy[0], tslot = ps.slot[0];
-    int64_t blk = gblk;
-#pragma unroll
-    for (int q = 1; q < kTermArrays; ++q) {
-      if (q < ps.n && gblk >= ps.start[q]) {
-        cls = ps.cls[q];
-        dx = ps.dx[q];
-        dy = ps.dy[q];
-        tslot = ps.slot[q];
-        blk = gblk - ps.start[q];
-      }
+  unsigned char* const wb = smem + static_cast<size_t>(warp) * R::kWarpBytes;
+  unsigned char* const data = wb + lane * 16;
+  uint2* const recs = reinterpret_cast<uint2*>(wb + R::kData) + lane;  // slot q at recs[32 q]
+  // Buffer b of the lane: words -PAD .. NS / 2 + PAD - 1 around vec + b * kVecStep.
+  uint32_t* const vec = reinterpret_cast<uint32_t*>(wb + R::kData + R::kRec) + lane * R::kVecStride + PAD;
+  uint16_t* const lut = reinterpret_cast<uint16_t*>(wb + R::kData + R::kRec + R::kVec);
+  // The lane's buffers of wide vectors: word q (from -PAD on) of buffer b at
+  // wide[(b * ovf_words + q) * 32].
+  uint32_t* const wide =
+      ovf + ((static_cast<int64_t>(blockIdx.x) * wpb + warp) * 2 * ovf_words + PAD) * 32 + lane;
+  if (ovf_words > 0) {
+    for (int k = 1; k <= PAD; ++k) {
+      wide[-32 * k] = kSent2;
+      wide[(ovf_words - k) * 32] = kSent2;
     }
-    const int j = find_job(jobs, njobs, blk, [cls](const SgmPathJob& q) { return q.blk[cls]; });
+  }
+  int lut_match = -1;
+  const uint32_t one = ps.one;
+  for (int64_t gblk = static_cast<int64_t>(blockIdx.x) * wpb + warp; gblk < ps.total;
+       gblk = next_block(ps, nwarps)) {
+    if (cancelled(cancel)) break;
+    int j, cls, dx, dy, tslot;
+    const int64_t blk = locate_block<32>(jobs, njobs, ps, gblk, j, cls, dx, dy, tslot);
     const SgmPathJob& job = jobs[j];
     const SgmMatch& m = matches[job.match];
     if (job.match != lut_match) {  // the same for the whole warp (one chain block)
@@ -990,217 +1062,309 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
     const uint32_t p1x2 = static_cast<uint32_t>(m.p1) * 0x10001u;
     const bool no_carry = m.sum_no_carry != 0;
     int sx, sy, len;
-    chain_geometry(cls, dx, dy, w, job.h, (blk - job.blk[cls]) * CPW + gi, sx, sy, len);
+    chain_geometry(cls, dx, dy, w, job.h, blk * 32 + lane, sx, sy, len);
     int maxlen = len;
 #pragma unroll
-    for (int o = G; o < 32; o <<= 1) maxlen = r3dsimt::imax(maxlen, static_cast<int>(r3dsimt::shfl_xor(maxlen, o)));
-    const uint8_t* cbase = cost + job.cell_off;
-    uint16_t* sbase = sum + job.cell_off;
-    uint8_t* tbase = terms + job.cell_off;
-    const int4* rbase = rec + job.px_off;
-    auto pix = [&](int i) -> int { return (sy + i * dy) * w + sx + i * dx; };
-    auto issue_rec = [&](int i) {
-      if (i < len) r3dsimt::cp_async16(&recs[(i & (2 * D - 1)) * 32 + lane], rbase + pix(i));
-    };
-    auto issue_data = [&](int i, int4 r) {
-      if (i >= len) return;
-      const int off = r.x, num = static_cast<int>(static_cast<uint32_t>(r.y) >> 16);
-      const int st = i & (D - 1);
+    for (int o = 1; o < 32; o <<= 1) maxlen = r3dsimt::imax(maxlen, static_cast<int>(r3dsimt::shfl_xor(maxlen, o)));
+    const uint8_t* const cbase = cost + job.cell_off;
+    uint16_t* const sbase = sum + job.cell_off;
+    uint8_t* const tout = terms + job.cell_off + tslot * tstride;
+    const int dpx = dy * w + dx;
+    const uint2* rp = rec + job.px_off + static_cast<int64_t>(sy) * w + sx;  // record of the next pixel to request
+    auto units_of = [&](const uint2& r, int i) { return rec_units(r, m, job, sx + i * dx, sy + i * dy); };
+    // Chunk of the pixel with `left` units from unit `at` on into ring slot st.
+    auto issue_chunk = [&](int st, int at, int left) {
+      unsigned char* dst = data + st * R::kStageBytes;
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (e0 + 8 * u < num) {
-          r3dsimt::cp_async8(stage_cost(st) + 8 * u, cbase + off + e0 + 8 * u);
-          if constexpr (kReadsSum) r3dsimt::cp_async16(stage_sum(st) + 16 * u, sbase + off + e0 + 8 * u);
-          if constexpr (MODE == kLastTerm) {
-#pragma unroll
-            for (int r = 0; r < kTermArrays; ++r)
-              r3dsimt::cp_async8(stage_term(st, r) + 8 * u, tbase + r * tstride + off + e0 + 8 * u);
+      for (int u = 0; u < UF; ++u) {
+        if (u == 0 || left > u) {
+          const int64_t off = static_cast<int64_t>(at + u) * 16;
+          r3dsimt::cp_async16(dst + u * 512, cbase + off);
+          if constexpr (MODE == kAccumulate) {
+            r3dsimt::cp_async16(dst + (UF + 2 * u) * 512, sbase + off);
+            r3dsimt::cp_async16(dst + (UF + 2 * u + 1) * 512, sbase + off + 8);
           }
         }
       }
     };
-    // The leading sentinels of both buffers (read from the second pixel on,
-    // after the first step's warp barrier).
-    if (t == 0) {
-      prevw[0] = kSent2;
-      prevw[CPW * kRangedSmemStride] = kSent2;
-    }
-    // Records of the first 2 D - 1 pixels now, the first D - 1 pixels' data in flight.
+    // Pixel i + D - 1's first chunk into slot st, pixel i + 2 D - 1's record;
+    // one group. (Records: requested D steps before the data, so landed.)
+    auto issue = [&](int i, int st) {
+      if (i + D - 1 < len) {
+        const uint2 r = recs[((i + D - 1) & (NR - 1)) * 32];
+        issue_chunk(st, static_cast<int>(r.x & kRecOffset), static_cast<int>(r.x >> kRecShift));
+      }
+      if (i + 2 * D - 1 < len) r3dsimt::cp_async8(&recs[((i + 2 * D - 1) & (NR - 1)) * 32], rp);
+      rp += dpx;
+      r3dsimt::cp_async_commit();
+    };
 #pragma unroll
-    for (int k = 0; k < 2 * D - 1; ++k)
-      if (k < len) recs[k * 32 + lane] = rbase[pix(k)];
+    for (int k = 0; k < 2 * D - 1; ++k) {
+      if (k < len) recs[k * 32] = *rp;
+      rp += dpx;
+    }
 #pragma unroll
     for (int k = 0; k < D - 1; ++k) {
-      issue_data(k, recs[k * 32 + lane]);
+      if (k < len) {
+        const uint2 r = recs[k * 32];
+        issue_chunk(k, static_cast<int>(r.x & kRecOffset), static_cast<int>(r.x >> kRecShift));
+      }
       r3dsimt::cp_async_commit();
     }
-    uint32_t pmin = 0, lutv = 0;
+    uint2 rc = make_uint2(0, 0);  // this pixel's record
+    if (len > 0) rc = recs[0];
+    // The predecessor's range, its minimum over labels in both halves,
+    // negated, and the clamp min L(q) + P2. A zero clamp makes the first
+    // pixel's best term 0 whatever the predecessor words hold: T = 0, L = C.
     int lo_q = 0, num_q = 0;
-    for (int i = 0; i < maxlen; ++i) {
-      const bool on = i < len;
-      // One wait per step: the group of step i - D + 1 (this pixel's data)
-      // and the older one holding record i + D - 1 are complete when at most
-      // the D - 2 most recent groups are still in flight. The slots refilled
-      // here (record and data of the previous pixel) are no longer read.
-      r3dsimt::cp_async_wait<D - 2>();
-      const int4 rc = recs[(i & (2 * D - 1)) * 32 + lane];
-      const int4 rn = recs[((i + D - 1) & (2 * D - 1)) * 32 + lane];
-      issue_rec(i + 2 * D - 1);
-      issue_data(i + D - 1, rn);
-      r3dsimt::cp_async_commit();
-      const int off = rc.x, lo = rc.y & 0xFFFF, icur = rc.z;
-      const int num = on ? static_cast<int>(static_cast<uint32_t>(rc.y) >> 16) : 0;
-      // Chunks of this pixel's range: the same for the chain's G lanes (one
-      // pixel), and the chunk loop holds no warp-wide operation.
-      const int nchw = (num + CH - 1) / CH;
-      const int sh = lo - lo_q, nwq = num_q >> 1;
-      const int cur = i & 1, prv = cur ^ 1;
-      uint32_t pen2 = 0, negmp = 0;
-      if (i > 0) {
-        const uint32_t pen = pmin + lutv;
-        pen2 = pen | (pen << 16);
-        negmp = 0u - (pmin | (pmin << 16));
+    uint32_t pen2 = 0, negmp = 0;
+    uint32_t prev[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) prev[k] = 0;
+    bool single = static_cast<int>(rc.x >> kRecShift) == UF;  // this pixel is one full chunk
+    bool fast = r3dsimt::ballot(len > 0 && !single) == 0;
+    bool clean = false;  // the buffers hold sentinels outside what this chain wrote
+    int high = 0;        // labels of the longest vector written
+    auto make_clean = [&]() {
+      if (clean) return;
+      for (int k = -PAD; k < R::kVecStride - PAD; ++k) vec[k] = kSent2;
+      clean = true;
+    };
+    // From the best terms of a chunk (its bytes in ring slot st, its cells
+    // from unit `at` on): T = best - min L(q), L = C + T, and the outputs.
+    uint32_t out[K], pm;
+    auto finish = [&](const uint32_t (&best)[K], int st, int at, bool on, bool upper) {
+      const unsigned char* src = data + st * R::kStageBytes;
+      uint32_t c2[K], tr[K];
+#pragma unroll
+      for (int u = 0; u < UF; ++u) {
+        const uint4 v = *reinterpret_cast<const uint4*>(src + u * 512);
+        const uint32_t cw[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          c2[8 * u + 2 * k] = cw[k] & 0x00FF00FFu;
+          c2[8 * u + 2 * k + 1] = r3dsimt::perm(cw[k], 0u, 0x4341u);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        tr[k] = fma_add(best[k], one, negmp);
+        out[k] = fma_add(tr[k], one, c2[k]);
+        if (k >= 8 && !upper) out[k] = kSent2;
       }
       {
-        // The next step's P2, loaded one step ahead from the next pixel's
-        // record (landed: it was issued 2 D - 1 steps ahead). Past the end of
-        // the chain that record slot holds an older or an unwritten record,
-        // so the table index is clamped to the table.
-        const int dn = recs[((i + 1) & (2 * D - 1)) * 32 + lane].z - icur;
-        const uint32_t di = static_cast<uint32_t>(dn < 0 ? -dn : dn) >> 8;
-        lutv = lut[di < 255u ? di : 255u];
+        constexpr int N3 = (K + 2) / 3;
+        uint32_t t3[N3];
+#pragma unroll
+        for (int k = 0; k < N3; ++k)
+          t3[k] = r3dsimt::vmin3(out[3 * k], out[3 * k + 1 < K ? 3 * k + 1 : 3 * k], out[3 * k + 2 < K ? 3 * k + 2 : 3 * k]);
+#pragma unroll
+        for (int k = 0; k < N3; k += 2) pm = r3dsimt::vmin3(pm, t3[k], t3[k + 1 < N3 ? k + 1 : k]);
       }
-      uint32_t pm = kSent2;
-      for (int c = 0; c < nchw; ++c) {
-        const int j0 = c * CH + e0;
-        bool uv[U];
+      if (!on) return;
 #pragma unroll
-        for (int u = 0; u < U; ++u) uv[u] = j0 + 8 * u < num;
-        uint2 craw[U];
-        uint4 sraw[U];
-        uint32_t tsum[K];  // kLastTerm: sum of the seven byte terms per label pair
-#pragma unroll
-        for (int k = 0; k < K; ++k) tsum[k] = 0;
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          craw[u] = make_uint2(0, 0);
-          sraw[u] = make_uint4(0, 0, 0, 0);
-          if (uv[u]) {
-            if (c == 0) {
-              const int st = i & (D - 1);
-              craw[u] = *reinterpret_cast<const uint2*>(stage_cost(st) + 8 * u);
-              if constexpr (kReadsSum) sraw[u] = *reinterpret_cast<const uint4*>(stage_sum(st) + 16 * u);
-            } else {
-              craw[u] = *reinterpret_cast<const uint2*>(cbase + off + j0 + 8 * u);
-              if constexpr (kReadsSum)
-                sraw[u] = r3dsimt::ld_stream(reinterpret_cast<const uint4*>(sbase + off + j0 + 8 * u));
-            }
-            if constexpr (MODE == kLastTerm) {
-#pragma unroll
-              for (int r = 0; r < kTermArrays; ++r) {
-                const uint2 tw = c == 0 ? *reinterpret_cast<const uint2*>(stage_term(i & (D - 1), r) + 8 * u)
-                                        : *reinterpret_cast<const uint2*>(tbase + r * tstride + off + j0 + 8 * u);
-                tsum[4 * u + 0] = fma_add(r3dsimt::perm(tw.x, 0u, 0x4140u), one, tsum[4 * u + 0]);
-                tsum[4 * u + 1] = fma_add(r3dsimt::perm(tw.x, 0u, 0x4342u), one, tsum[4 * u + 1]);
-                tsum[4 * u + 2] = fma_add(r3dsimt::perm(tw.y, 0u, 0x4140u), one, tsum[4 * u + 2]);
-                tsum[4 * u + 3] = fma_add(r3dsimt::perm(tw.y, 0u, 0x4342u), one, tsum[4 * u + 3]);
-              }
-            }
-          }
-        }
-        uint32_t c2[K];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          c2[4 * u + 0] = r3dsimt::perm(craw[u].x, 0u, 0x4140u);
-          c2[4 * u + 1] = r3dsimt::perm(craw[u].x, 0u, 0x4342u);
-          c2[4 * u + 2] = r3dsimt::perm(craw[u].y, 0u, 0x4140u);
-          c2[4 * u + 3] = r3dsimt::perm(craw[u].y, 0u, 0x4342u);
-        }
-        uint32_t out[K], tr[K];
-        if (i == 0) {
-#pragma unroll
-          for (int k = 0; k < K; ++k) {
-            tr[k] = 0;
-            out[k] = c2[k];
-          }
+      for (int u = 0; u < UF; ++u) {
+        if (u > 0 && !upper) continue;
+        const int64_t off = static_cast<int64_t>(at + u) * 16;
+        const int q = 8 * u;
+        if constexpr (MODE == kTerm) {
+          r3dsimt::st_stream(reinterpret_cast<uint4*>(tout + off),
+                             make_uint4(tr[q] + 256u * tr[q + 1], tr[q + 2] + 256u * tr[q + 3],
+                                        tr[q + 4] + 256u * tr[q + 5], tr[q + 6] + 256u * tr[q + 7]));
         } else {
-          // Predecessor labels j0 + sh - 2 .. j0 + sh + 2 K + 1 (its own
-          // indexing), sentinels outside its range, realigned by one label
-          // when the shift is odd.
-          const int b = j0 + sh - 2;
-          const int f = b >> 1;
-          uint32_t qw[K + 3];
+          uint32_t v[8];
 #pragma unroll
-          for (int k = 0; k < K + 3; ++k) qw[k] = qword(prv, f + k, nwq);
-          uint32_t wv[K + 2];
-          if (b & 1) {
+          for (int k = 0; k < 8; ++k) v[k] = out[q + k];
+          if constexpr (MODE == kAccumulate) {
 #pragma unroll
-            for (int k = 0; k < K + 2; ++k) wv[k] = r3dsimt::perm(qw[k], qw[k + 1], 0x5432u);
-          } else {
-#pragma unroll
-            for (int k = 0; k < K + 2; ++k) wv[k] = qw[k];
+            for (int k = 0; k < 8; k += 4) {
+              const uint4 t = *reinterpret_cast<const uint4*>(src + (UF + 2 * u + k / 4) * 512);
+              v[k] = add2(t.x, v[k], no_carry);
+              v[k + 1] = add2(t.y, v[k + 1], no_carry);
+              v[k + 2] = add2(t.z, v[k + 2], no_carry);
+              v[k + 3] = add2(t.w, v[k + 3], no_carry);
+            }
           }
-          uint32_t mprev = r3dsimt::perm(wv[0], wv[1], 0x5432u);
-#pragma unroll
-          for (int k = 0; k < K; ++k) {
-            const uint32_t mnext = r3dsimt::perm(wv[k + 1], wv[k + 2], 0x5432u);
-            const uint32_t nb = r3dsimt::vmin2(mprev, mnext);
-            const uint32_t best = r3dsimt::vmin2(wv[k + 1], r3dsimt::vaddmin2(nb, p1x2, pen2));
-            tr[k] = fma_add(best, one, negmp);
-            out[k] = fma_add(tr[k], one, c2[k]);
-            mprev = mnext;
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-          if (!uv[k / 4]) out[k] = kSent2;
-          pm = r3dsimt::vmin2(pm, out[k]);
-          if (uv[k / 4]) put_word(cur, (j0 >> 1) + k, out[k]);
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (!uv[u]) continue;
-          if constexpr (MODE == kTerm) {
-            r3dsimt::st_stream8(reinterpret_cast<uint2*>(tbase + tslot * tstride + off + j0 + 8 * u),
-                                make_uint2(r3dsimt::perm(tr[4 * u], tr[4 * u + 1], 0x6420u),
-                                           r3dsimt::perm(tr[4 * u + 2], tr[4 * u + 3], 0x6420u)));
-            continue;
-          }
-          uint4 v;
-          if constexpr (MODE == kFirst) {
-            v = make_uint4(out[4 * u], out[4 * u + 1], out[4 * u + 2], out[4 * u + 3]);
-          } else if constexpr (MODE == kLastTerm) {
-            v = make_uint4(out[4 * u] + 7u * c2[4 * u] + tsum[4 * u],
-                           out[4 * u + 1] + 7u * c2[4 * u + 1] + tsum[4 * u + 1],
-                           out[4 * u + 2] + 7u * c2[4 * u + 2] + tsum[4 * u + 2],
-                           out[4 * u + 3] + 7u * c2[4 * u + 3] + tsum[4 * u + 3]);
-          } else {
-            v = make_uint4(add2(sraw[u].x, out[4 * u], no_carry), add2(sraw[u].y, out[4 * u + 1], no_carry),
-                           add2(sraw[u].z, out[4 * u + 2], no_carry), add2(sraw[u].w, out[4 * u + 3], no_carry));
-          }
-          r3dsimt::st_stream(reinterpret_cast<uint4*>(sbase + off + j0 + 8 * u), v);
+          uint4* dst = reinterpret_cast<uint4*>(sbase + off);
+          r3dsimt::st_stream(dst, make_uint4(v[0], v[1], v[2], v[3]));
+          r3dsimt::st_stream(dst + 1, make_uint4(v[4], v[5], v[6], v[7]));
         }
       }
-      pmin = group_umin<G>(r3dsimt::umin(pm & 0xFFFFu, pm >> 16));
-      // The trailing sentinel of the vector just written.
-      if (t == 0 && (num >> 1) <= kRangedSmemWords) prevw[cur * CPW * kRangedSmemStride + 1 + (num >> 1)] = kSent2;
-      r3dsimt::syncwarp();
-      if (on) {
-        lo_q = lo;
-        num_q = num;
+    };
+    // Chunk c of pixel i (n units) into the lane's buffer of the pixel.
+    auto store_vec = [&](int i, int c, int n, bool upper) {
+      uint32_t nat[K];
+#pragma unroll
+      for (int u = 0; u < UF; ++u) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          nat[8 * u + k] = r3dsimt::perm(out[8 * u + 2 * k], out[8 * u + 2 * k + 1], 0x5410u);
+          nat[8 * u + 4 + k] = r3dsimt::perm(out[8 * u + 2 * k], out[8 * u + 2 * k + 1], 0x7632u);
+        }
       }
+      const bool last = (c + 1) * UF >= n;
+      const int end = 8 * n - c * K;  // word after the vector, from the chunk's first word
+      if (16 * n <= NS) {
+        uint32_t* v = vec + (i & 1) * R::kVecStep + c * K;
+#pragma unroll
+        for (int k = 0; k < K; ++k) v[k] = nat[k];
+        if (last) {
+          // Sentinels after the vector where a longer one was written before.
+          if (n < high) {
+#pragma unroll
+            for (int k = 0; k < PAD; ++k) v[end + k] = kSent2;
+          }
+          high = r3dsimt::imax(high, n);
+        }
+      } else {
+        uint32_t* v = wide + ((i & 1) * ovf_words + c * K) * 32;
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+          if (k < 8 || upper) v[k * 32] = nat[k];
+        if (last) {
+#pragma unroll
+          for (int k = 0; k < PAD; ++k) v[(end + k) * 32] = kSent2;
+        }
+      }
+    };
+    // best = min(L(q, d), L(q, d -+ 1) + P1, min L(q) + P2); clamping first
+    // leaves one 3-way minimum per word. From the lane's buffer of pixel i -
+    // 1, for the labels of chunk c at lo.
+    auto best_from_memory = [&](uint32_t (&best)[K], int i, int c, int lo) {
+      // Predecessor labels b - 1 .. b + CH (its own indexing).
+      int b = c * CH + lo - lo_q;
+      b = r3dsimt::imax(r3dsimt::imin(b, num_q + 1), -(CH + 1));
+      // pr[k]: labels b - 1 + 2 k, b + 2 k, from the words holding them.
+      const int f = (b - 1) >> 1;
+      const uint32_t par = 16u * (static_cast<uint32_t>(b - 1) & 1u);
+      uint32_t wd[K + 2], pr[K + 1];
+      if (num_q <= NS) {
+        const uint32_t* vq = vec + ((i & 1) ^ 1) * R::kVecStep + f;
+#pragma unroll
+        for (int k = 0; k < K + 2; ++k) wd[k] = vq[k];
+      } else {
+        const uint32_t* oq = wide + (((i & 1) ^ 1) * ovf_words + f) * 32;
+#pragma unroll
+        for (int k = 0; k < K + 2; ++k) wd[k] = oq[k * 32];
+      }
+#pragma unroll
+      for (int k = 0; k < K + 1; ++k) pr[k] = r3dsimt::funnel_r(wd[k], wd[k + 1], par);
+#pragma unroll
+      for (int u = 0; u < UF; ++u) {
+        uint32_t cl[10], s[10];
+#pragma unroll
+        for (int k = 0; k < 10; ++k) {
+          cl[k] = r3dsimt::vmin2(
+              r3dsimt::perm(pr[8 * u + (k >> 1)], pr[8 * u + (k >> 1) + 4], (k & 1) ? 0x7632u : 0x5410u), pen2);
+          s[k] = fma_add(cl[k], one, p1x2);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) best[8 * u + k] = r3dsimt::vmin3(cl[k + 1], s[k], s[k + 2]);
+      }
+    };
+    for (int i = 0; i < maxlen; ++i) {
+      const int st = i & (D - 1), st_in = (i + D - 1) & (D - 1);  // slots of this pixel and of the one issued now
+      const bool on = i < len;
+      const int at = static_cast<int>(rc.x & kRecOffset);
+      const int lo = static_cast<int>(rc.y & 0xFFFFu);
+      uint2 rn = rc;  // the next pixel's record
+      if (i + 1 < len) rn = recs[((i + 1) & (NR - 1)) * 32];
+      const bool single_n = static_cast<int>(rn.x >> kRecShift) == UF;
+      const bool okn = i + 1 >= len || (single && single_n && ((rn.y ^ rc.y) & 0xFFFFu) == 0);
+      const bool fast_next = r3dsimt::ballot(!okn) == 0;
+      pm = kSent2;
+      uint32_t best[K];
+      int n = UF;
+      if (fast) {
+        issue(i, st_in);
+        r3dsimt::cp_async_wait<D - 1>();
+        uint32_t cl[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) cl[k] = r3dsimt::vmin2(prev[k], pen2);
+#pragma unroll
+        for (int u = 0; u < UF; ++u) {
+          // Words -1 and 8 of the unit: labels (16 u - 1, 16 u + 7) and (16 u + 8, 16 u + 16).
+          uint32_t s[10];
+          s[0] = fma_add(r3dsimt::perm(u > 0 ? cl[8 * (u > 0 ? u - 1 : 0) + 7] : pen2, cl[8 * u + 7], 0x5432u), one, p1x2);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) s[1 + k] = fma_add(cl[8 * u + k], one, p1x2);
+          s[9] = fma_add(r3dsimt::perm(cl[8 * u], u + 1 < UF ? cl[8 * (u + 1 < UF ? u + 1 : 0)] : pen2, 0x5432u), one,
+                         p1x2);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) best[8 * u + k] = r3dsimt::vmin3(cl[8 * u + k], s[k], s[2 + k]);
+        }
+        finish(best, st, at, on, true);
+        if (!fast_next) {
+          make_clean();
+          if (on) store_vec(i, 0, n, true);
+        }
+      } else {
+        make_clean();
+        n = on ? units_of(rc, i) : 1;
+        const bool multi = r3dsimt::ballot(n > UF) != 0;
+        if (!multi) {
+          issue(i, st_in);
+          r3dsimt::cp_async_wait<D - 1>();
+          best_from_memory(best, i, 0, lo);
+          finish(best, st, at, on, n > 1);
+          if (!fast_next && on) store_vec(i, 0, n, n > 1);
+        } else {
+          // A lane's pixel has more chunks: they pass through this pixel's
+          // slot and the free one, each requested while the one before it
+          // is worked on; the next pixel is issued after them.
+          int sa = st, sb = st_in;
+          if (n > UF) issue_chunk(sb, at + UF, n - UF);
+          r3dsimt::cp_async_commit();
+          r3dsimt::cp_async_wait<D - 1>();
+          for (int c = 0; r3dsimt::ballot(c * UF < n) != 0; ++c) {
+            const bool have = c * UF < n, upper = n - c * UF > 1;
+            if (have) {
+              best_from_memory(best, i, c, lo);
+              finish(best, sa, at + c * UF, on, upper);
+              if (on) store_vec(i, c, n, upper);
+            }
+            // Slot sa is free: the chunk after the one in slot sb.
+            if ((c + 2) * UF < n) issue_chunk(sa, at + (c + 2) * UF, n - (c + 2) * UF);
+            r3dsimt::cp_async_commit();
+            r3dsimt::cp_async_wait<1>();
+            const int t = sa;
+            sa = sb;
+            sb = t;
+          }
+          issue(i, st_in);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < K; ++k) prev[k] = out[k];
+      {
+        const uint32_t mp = r3dsimt::vmin2(pm, r3dsimt::perm(pm, pm, 0x1032u));
+        const int dn = static_cast<int>(rn.y >> 16) - static_cast<int>(rc.y >> 16);
+        pen2 = mp + lut[(dn < 0 ? -dn : dn) >> 8] * 0x10001u;
+        negmp = 0u - mp;
+      }
+      lo_q = lo;
+      num_q = 16 * n;
+      rc = rn;
+      single = single_n;
+      fast = fast_next;
     }
     r3dsimt::cp_async_wait<0>();
-    r3dsimt::syncwarp();
   }
 }
 
-// Per pixel: winner-takes-all over the total sums (sgm_kernels.cpp:332-358;
-// first minimum, second best outside +-1, S at kb -+ 1 within the range),
-// the optional volume copy and the right-view keys of the diagonal check.
+// Per pixel: the total sums (S = 8 C + the eight byte terms with TERMS, the
+// stored u16 sums without), winner-takes-all (sgm_kernels.cpp:332-358; first
+// minimum, second best outside +-1, S at kb -+ 1 within the range) and, without the diagonal check, the acceptance rules; with it the right-view
+// keys and the pixel's record for the acceptance kernel. Also the optional
+// volume copy. Summing here instead of in the eighth path pass keeps that pass
+// as short as the others (in one launch with them: the chains of one direction
+// alone leave most of the SMs idle on a single pair) and saves the stored sum:
+// 11 bytes per cell against 12.
+template <bool TERMS>
 R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
     sgm_path_ranged_wta_kernel(const SgmMatch* R3D_RESTRICT matches, const SgmPathJob* R3D_RESTRICT jobs, int njobs,
-                               int64_t pixels, const int4* R3D_RESTRICT rec, const uint16_t* R3D_RESTRICT sum,
+                               int64_t pixels, const uint2* R3D_RESTRICT rec, const uint8_t* R3D_RESTRICT cost,
+                               const uint16_t* R3D_RESTRICT sum, const uint8_t* R3D_RESTRICT terms, int64_t tstride,
                                const int* R3D_RESTRICT rowshift, int4* R3D_RESTRICT info, uint32_t* rkeys) {
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < pixels; i += stride) {
@@ -1209,49 +1373,110 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
     const SgmMatch& m = matches[job.match];
     const int p = static_cast<int>(i - job.px_off);
     const int y = p / job.w, x = p - y * job.w;
-    const int4 rc = rec[i];
-    const int lo = rc.y & 0xFFFF, num = static_cast<int>(static_cast<uint32_t>(rc.y) >> 16);
-    const uint16_t* sp16 = sum + job.cell_off + rc.x;
-    uint32_t kmin = 0xFFFFFFFFu;
-    for (int c = 0; c < num; c += 8) {
-      const uint4 v = *reinterpret_cast<const uint4*>(sp16 + c);
-      const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
+    const uint2 rc = rec[i];
+    const int lo = static_cast<int>(rc.y & 0xFFFFu), nu = rec_units(rc, m, job, x, y), num = 16 * nu;
+    const int64_t off = static_cast<int64_t>(rc.x & kRecOffset) * 16;
+    const uint8_t* cp = cost + job.cell_off + off;
+    const uint8_t* tp = terms + job.cell_off + off;
+    const uint4* sp4 = reinterpret_cast<const uint4*>(sum + job.cell_off + off);
+    // Word k of a unit holds labels k and k + 8.
+    auto unit = [&](int u, uint32_t (&wv)[8]) {
+      if constexpr (TERMS) {
+        uint4 t[1 + kRangedTerms];
+        t[0] = *reinterpret_cast<const uint4*>(cp + 16 * u);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint32_t e = static_cast<uint32_t>(c + 2 * k);
-        kmin = r3dsimt::umin(kmin, r3dsimt::umin(((wv[k] & 0xFFFFu) << 16) | e, (wv[k] & 0xFFFF0000u) | (e + 1)));
+        for (int r = 0; r < kRangedTerms; ++r)
+          t[1 + r] = r3dsimt::ld_stream(reinterpret_cast<const uint4*>(tp + r * tstride + 16 * u));
+#pragma unroll
+        for (int r = 0; r <= kRangedTerms; ++r) {
+          const uint32_t tw[4] = {t[r].x, t[r].y, t[r].z, t[r].w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const uint32_t a = tw[k] & 0x00FF00FFu, b = r3dsimt::perm(tw[k], 0u, 0x4341u);
+            wv[2 * k] = r == 0 ? 8u * a : wv[2 * k] + a;
+            wv[2 * k + 1] = r == 0 ? 8u * b : wv[2 * k + 1] + b;
+          }
+        }
+        return;
       }
-      if (job.volume != nullptr) *reinterpret_cast<uint4*>(job.volume + rc.x + c) = v;
+      const uint4 a = sp4[2 * u], b = sp4[2 * u + 1];
+      wv[0] = a.x;
+      wv[1] = a.y;
+      wv[2] = a.z;
+      wv[3] = a.w;
+      wv[4] = b.x;
+      wv[5] = b.y;
+      wv[6] = b.z;
+      wv[7] = b.w;
+    };
+    uint32_t wv[8];
+    uint32_t kmin = 0xFFFFFFFFu;
+    for (int u = nu - 1; u >= 0; --u) {  // ends with unit 0 in wv: the only one of most pixels
+      unit(u, wv);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const uint32_t e = static_cast<uint32_t>(16 * u + k);
+        kmin = r3dsimt::umin(kmin, r3dsimt::umin((wv[k] << 16) | e, (wv[k] & 0xFFFF0000u) | (e + 8)));
+      }
+      if (job.volume != nullptr) {
+        uint16_t* vol = job.volume + off + 16 * u;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          vol[k] = static_cast<uint16_t>(wv[k] & 0xFFFFu);
+          vol[k + 8] = static_cast<uint16_t>(wv[k] >> 16);
+        }
+      }
     }
     const int kb = static_cast<int>(kmin & 0xFFFFu);
-    const uint32_t bcost = kmin >> 16;
-    uint32_t sec = 0xFFFFu;
-    for (int e = 0; e < num; ++e)
-      if (e + 1 < kb || e > kb + 1) sec = r3dsimt::umin(sec, sp16[e]);
     const int km = kb > 0 ? kb - 1 : 0;
     const int kp = kb + 1 < num ? kb + 1 : (num > 0 ? num - 1 : 0);
-    const uint32_t sm = sp16[km], spv = sp16[kp];
-    info[i] = make_int4(static_cast<int>(static_cast<uint32_t>(lo + kb) | (bcost << 16)),
-                        static_cast<int>(sec | (sm << 16)), static_cast<int>(spv), 0);
-    if (m.diagonal_lr) {
-      const RowInterval lv = m.bv[job.y0 + y];
-      const int bx = job.x0 + x;
-      if (bx >= lv.first && bx <= lv.last) {
-        uint32_t* keys = rkeys + job.rk_off + static_cast<int64_t>(y) * (job.w + m.nd);
-        const int base = x - lo + rowshift[job.row_off + y];
-        for (int e = 0; e < num; ++e)
-          atomicMin(keys + (base - e), (static_cast<uint32_t>(sp16[e]) << 16) | static_cast<uint32_t>(x));
+    uint32_t sec = 0xFFFFu, sm = 0, spv = 0;
+    for (int u = 0; u < nu; ++u) {
+      if (u > 0) unit(u, wv);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          const int e = 16 * u + k + 8 * hf;
+          const uint32_t v = hf != 0 ? wv[k] >> 16 : wv[k] & 0xFFFFu;
+          if (e + 1 < kb || e > kb + 1) sec = r3dsimt::umin(sec, v);
+          if (e == km) sm = v;
+          if (e == kp) spv = v;
+        }
       }
     }
+    const Winner win{lo + kb, kmin >> 16, sec, sm, spv};
+    const RowInterval lv = m.bv[job.y0 + y];
+    const bool inside = job.x0 + x >= lv.first && job.x0 + x <= lv.last;
+    if (m.diagonal_lr) {
+      info[i] = pack_winner(win);
+      if (inside) {
+        uint32_t* keys = rkeys + job.rk_off + static_cast<int64_t>(y) * (job.w + m.nd);
+        const int base = x - lo + rowshift[job.row_off + y];
+        for (int u = 0; u < nu; ++u) {
+          unit(u, wv);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const int e = 16 * u + k;
+            atomicMin(keys + (base - e), (wv[k] << 16) | static_cast<uint32_t>(x));
+            atomicMin(keys + (base - e - 8), (wv[k] & 0xFFFF0000u) | static_cast<uint32_t>(x));
+          }
+        }
+      }
+      continue;
+    }
+    float d = kInfF, cf = 0.0F;
+    if (inside) accept_pixel(m, job, x, y, lo, num, win, rkeys, 0, d, cf);
+    job.disp[p] = d;
+    if (job.conf != nullptr) job.conf[p] = cf;
   }
 }
 
-// Acceptance rules with per-pixel ranges (stereo_matcher.cpp:474-523): as
-// the full-range kernel's, plus the rejection of a minimum on the edge of a
-// reduced range (:501-503).
+// Acceptance of the pixels of matches with the diagonal check (their keys
+// are complete after the kernel above).
 R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
     sgm_path_ranged_accept_kernel(const SgmMatch* R3D_RESTRICT matches, const SgmPathJob* R3D_RESTRICT jobs,
-                                  int njobs, int64_t pixels, const int4* R3D_RESTRICT rec,
+                                  int njobs, int64_t pixels, const uint2* R3D_RESTRICT rec,
                                   const int4* R3D_RESTRICT info, const uint32_t* R3D_RESTRICT rkeys,
                                   const int* R3D_RESTRICT rowshift) {
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -1259,45 +1484,15 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
     const int j = find_job(jobs, njobs, i, [](const SgmPathJob& q) { return q.px_off; });
     const SgmPathJob& job = jobs[j];
     const SgmMatch& m = matches[job.match];
-    const int w = job.w;
+    if (!m.diagonal_lr) continue;
     const int p = static_cast<int>(i - job.px_off);
-    const int y = p / w, x = p - y * w;
-    const int bx = job.x0 + x, by = job.y0 + y;
-    const RowInterval lv = m.bv[by];
+    const int y = p / job.w, x = p - y * job.w;
+    const RowInterval lv = m.bv[job.y0 + y];
     float d = kInfF, cf = 0.0F;
-    if (bx >= lv.first && bx <= lv.last) {
-      const int4 in = info[i];
-      const int4 rc = rec[i];
-      const int lo = rc.y & 0xFFFF, num = static_cast<int>(static_cast<uint32_t>(rc.y) >> 16);
-      const int best = in.x & 0xFFFF;
-      const uint32_t bcost = static_cast<uint32_t>(in.x) >> 16;
-      const uint32_t sec = static_cast<uint32_t>(in.y) & 0xFFFFu;
-      const uint32_t sm = static_cast<uint32_t>(in.y) >> 16;
-      const uint32_t sp = static_cast<uint32_t>(in.z);
-      const int jb = best - lo;
-      const RowInterval rv = m.pv[by];
-      const int xr = bx - m.dmin - best;
-      bool ok = xr >= rv.first && xr <= rv.last;
-      if ((jb == 0 && lo > 0) || (jb == num - 1 && lo + num < m.nd)) ok = false;
-      if (ok && m.diagonal_lr) {
-        const uint32_t key =
-            rkeys[job.rk_off + static_cast<int64_t>(y) * (w + m.nd) + (x - best + rowshift[job.row_off + y])];
-        const int rb = key == 0xFFFFFFFFu ? 0xFFFF : static_cast<int>(key & 0xFFFFu) - x + best;
-        const int diff = rb - best;
-        if ((diff < 0 ? -diff : diff) > m.lr_max_diff) ok = false;
-      }
-      const float best_cost = static_cast<float>(bcost);
-      if (ok && m.uniqueness > 0.0F && sec != 0xFFFFu &&
-          best_cost > __fmul_rn(__fsub_rn(1.0F, m.uniqueness), static_cast<float>(sec)))
-        ok = false;
-      if (ok) {
-        float delta = 0.0F;
-        if (jb > 0 && jb < num - 1)
-          delta = sgm_simd::subpixel_delta(m.subpixel, static_cast<float>(sm), best_cost, static_cast<float>(sp));
-        d = __fadd_rn(static_cast<float>(m.dmin + best), delta);
-        if (m.confidence)
-          cf = (sec != 0xFFFFu && sec > 0u) ? __fsub_rn(1.0F, __fdiv_rn(best_cost, static_cast<float>(sec))) : 0.0F;
-      }
+    if (job.x0 + x >= lv.first && job.x0 + x <= lv.last) {
+      const uint2 rc = rec[i];
+      accept_pixel(m, job, x, y, static_cast<int>(rc.y & 0xFFFFu), 16 * rec_units(rc, m, job, x, y),
+                   unpack_winner(info[i]), rkeys, rowshift[job.row_off + y], d, cf);
     }
     job.disp[p] = d;
     if (job.conf != nullptr) job.conf[p] = cf;
@@ -1349,7 +1544,7 @@ void launch_pass(const PassSet& ps, const SgmMatch* dm, const SgmPathJob* jobs, 
     R3D_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     configured[dev] = 1;
   }
-  const int64_t nb = ps.start[ps.n];
+  const int64_t nb = ps.total;
   constexpr int threads = PathRing<G, K, MODE>::kThreads;
   R3D_LAUNCH(k, dim3(resident_grid(k, sms, nb, threads / 32, smem, threads)), dim3(threads), smem, s, dm, jobs, njobs,
              ps, cost, sum, terms, tstride, info, rkeys, ints, cancel);
@@ -1363,29 +1558,28 @@ void launch_pass(const PassSet& ps, const SgmMatch* dm, const SgmPathJob* jobs, 
   }
 }
 
-// Passes q of kPasses in `qs` (count n) as one PassSet.
-PassSet pass_set(const SgmPathSegment& g, const int* qs, int n) {
+// Passes q of kPasses in `qs` (count n) as one PassSet with the block counter `next`.
+PassSet pass_set(const SgmPathSegment& g, const int* qs, int n, int* next) {
   PassSet ps{};
   ps.one = 1;
-  int64_t start = 0;
+  ps.n = n;
+  ps.next = next;
   for (int i = 0; i < n; ++i) {
     const Pass& p = kPasses[qs[i]];
-    ps.cls[ps.n] = p.cls;
-    ps.dx[ps.n] = p.dx;
-    ps.dy[ps.n] = p.dy;
-    ps.slot[ps.n] = qs[i];
-    ps.start[ps.n] = start;
-    start += g.blocks[p.cls];
-    ++ps.n;
+    ps.cls[i] = p.cls;
+    ps.dx[i] = p.dx;
+    ps.dy[i] = p.dy;
+    ps.slot[i] = i;
+    ++ps.per_class[p.cls];
+    ps.total += g.blocks[p.cls];
   }
-  ps.start[ps.n] = start;
   return ps;
 }
 
 template <int G, int K>
 void launch_passes(const SgmMatch* dm, const SgmPathJob* jobs, const SgmPathSegment& g, const uint8_t* cost,
                    uint16_t* sum, uint8_t* terms, int64_t tstride, int4* info, uint32_t* rkeys, const uint16_t* ints,
-                   int sms, cudaStream_t s, const int* cancel) {
+                   int sms, cudaStream_t s, const int* cancel, int* counters) {
   for (int q = 0; q < 8; ++q)
     if (g.blocks[kPasses[q].cls] <= 0) return;  // no pixels: every class has chains otherwise
   if (terms != nullptr) {
@@ -1396,20 +1590,20 @@ void launch_passes(const SgmMatch* dm, const SgmPathJob* jobs, const SgmPathSegm
     // Segments whose matches fill every label unit take the kernels without
     // the per-unit validity selects.
     if (g.full != 0) {
-      launch_pass<G, K, kTerm, true>(pass_set(g, qs, kTermArrays), dm, jobs, g.count, cost, sum, terms, tstride, info,
+      launch_pass<G, K, kTerm, true>(pass_set(g, qs, kTermArrays, counters), dm, jobs, g.count, cost, sum, terms, tstride, info,
                                      rkeys, ints, sms, s, g, cancel);
-      launch_pass<G, K, kLastTerm, true>(pass_set(g, &last, 1), dm, jobs, g.count, cost, sum, terms, tstride, info,
+      launch_pass<G, K, kLastTerm, true>(pass_set(g, &last, 1, counters + 1), dm, jobs, g.count, cost, sum, terms, tstride, info,
                                          rkeys, ints, sms, s, g, cancel);
     } else {
-      launch_pass<G, K, kTerm>(pass_set(g, qs, kTermArrays), dm, jobs, g.count, cost, sum, terms, tstride, info,
+      launch_pass<G, K, kTerm>(pass_set(g, qs, kTermArrays, counters), dm, jobs, g.count, cost, sum, terms, tstride, info,
                                rkeys, ints, sms, s, g, cancel);
-      launch_pass<G, K, kLastTerm>(pass_set(g, &last, 1), dm, jobs, g.count, cost, sum, terms, tstride, info, rkeys,
+      launch_pass<G, K, kLastTerm>(pass_set(g, &last, 1, counters + 1), dm, jobs, g.count, cost, sum, terms, tstride, info, rkeys,
                                    ints, sms, s, g, cancel);
     }
     return;
   }
   for (int q = 0; q < 8; ++q) {
-    const PassSet ps = pass_set(g, &q, 1);
+    const PassSet ps = pass_set(g, &q, 1, counters + q);
     if (q == 0)
       launch_pass<G, K, kFirst>(ps, dm, jobs, g.count, cost, sum, terms, tstride, info, rkeys, ints, sms, s, g,
                                 cancel);
@@ -1500,6 +1694,8 @@ SgmPathBuffers sgm_path_buffers(int64_t cells, int64_t pixels, int64_t keys, boo
   // pass kernels copy the aligned 4-byte word holding a pixel's intensity.
   b.ints = o;
   o += align256(static_cast<size_t>(pixels) * 2 + 16);
+  b.counters = o;
+  o += align256(sizeof(int) * kPathCounters);
   b.total = o;
   return b;
 }
@@ -1513,6 +1709,8 @@ void launch_sgm_path_wave(const SgmMatch* dm, const SgmPathWave& wave, int sms, 
   int4* info = reinterpret_cast<int4*>(wave.buffer + B.info);
   uint32_t* rkeys = reinterpret_cast<uint32_t*>(wave.buffer + B.rkeys);
   uint16_t* ints = reinterpret_cast<uint16_t*>(wave.buffer + B.ints);
+  int* counters = reinterpret_cast<int*>(wave.buffer + B.counters);
+  if (8 * wave.nsegs > kPathCounters) fail(R3DGPU_EINVAL, "stereo: too many path kernel shapes in a wave");
   if (wave.keys > 0) R3D_CUDA(cudaMemsetAsync(rkeys, 0xFF, static_cast<size_t>(wave.keys) * 4, s));
   {
     constexpr size_t max_smem = static_cast<size_t>(kPathThreads / 32) * kCostStage * 8;
@@ -1528,7 +1726,7 @@ void launch_sgm_path_wave(const SgmMatch* dm, const SgmPathWave& wave, int sms, 
     const size_t smem = static_cast<size_t>(kPathThreads / 32) * words * 8;
     R3D_LAUNCH(sgm_path_cost_kernel,
                dim3(resident_grid(sgm_path_cost_kernel, sms, wave.rows, kPathThreads / 32, smem)),
-               dim3(kPathThreads), smem, s, dm, wave.jobs, wave.njobs, wave.rows, cost, words, ints);
+               dim3(kPathThreads), smem, s, dm, wave.jobs, wave.njobs, wave.rows, cost, words, ints, counters);
     launched("sgm_path_cost_kernel");
   }
   for (int q = 0; q < wave.nsegs; ++q) {
@@ -1537,7 +1735,8 @@ void launch_sgm_path_wave(const SgmMatch* dm, const SgmPathWave& wave, int sms, 
     bool done = false;
 #define R3D_SHAPE(gg, kk)                                                                                     \
   if (!done && g.shape.g_ == gg && g.shape.k_ == kk) {                                                        \
-    launch_passes<gg, kk>(dm, jobs, g, cost, sum, terms, B.term_stride, info, rkeys, ints, sms, s, wave.cancel); \
+    launch_passes<gg, kk>(dm, jobs, g, cost, sum, terms, B.term_stride, info, rkeys, ints, sms, s, wave.cancel, \
+                          counters + 8 * q);                                                                  \
     done = true;                                                                                              \
   }
     R3D_PATH_SHAPES(R3D_SHAPE)
@@ -1553,16 +1752,16 @@ void launch_sgm_path_wave(const SgmMatch* dm, const SgmPathWave& wave, int sms, 
 namespace {
 
 // Largest number of resident CTAs per SM any ranged pass kernel is launched
-// with (the overflow has one slot per resident chain).
-constexpr int kRangedMaxPerSm = 6;
+// with (the overflow has one slot per resident warp).
+constexpr int kRangedMaxPerSm = 24;
 
-template <int G, int K, int MODE>
-void launch_ranged_pass(const PassSet& ps, const SgmMatch* dm, const SgmPathJob* jobs, int njobs, const int4* rec,
+template <int K, int MODE>
+void launch_ranged_pass(const PassSet& ps, const SgmMatch* dm, const SgmPathJob* jobs, int njobs, const uint2* rec,
                         const uint8_t* cost, uint16_t* sum, uint8_t* terms, int64_t tstride, uint32_t* ovf,
-                        int64_t ovf_words, int sms, cudaStream_t s, const SgmPathSegment& seg, const int* cancel) {
+                        int ovf_words, int sms, cudaStream_t s, const SgmPathSegment& seg, const int* cancel) {
   const cudaEvent_t ev0 = profile_on() ? profile_mark(s) : nullptr;
-  auto* k = sgm_path_ranged_kernel<G, K, MODE>;
-  constexpr size_t smem = RangedRing<G, K, MODE>::kBlockBytes;
+  auto* k = sgm_path_ranged_kernel<K, MODE>;
+  constexpr size_t smem = RangedRing<K, MODE>::kBlockBytes;
   static thread_local int configured[64] = {};
   int dev = 0;
   R3D_CUDA(cudaGetDevice(&dev));
@@ -1570,49 +1769,45 @@ void launch_ranged_pass(const PassSet& ps, const SgmMatch* dm, const SgmPathJob*
     R3D_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     configured[dev] = 1;
   }
-  const int64_t nb = ps.start[ps.n];
-  int grid = resident_grid(k, sms, nb, kRangedThreads / 32, smem, kRangedThreads);
+  int grid = resident_grid(k, sms, ps.total, kRangedThreads / 32, smem, kRangedThreads);
   grid = grid < sms * kRangedMaxPerSm ? grid : sms * kRangedMaxPerSm;
   R3D_LAUNCH(k, dim3(grid), dim3(kRangedThreads), smem, s, dm, jobs, njobs, ps, rec, cost, sum, terms, tstride, ovf,
              ovf_words, cancel);
   launched("sgm_path_ranged_kernel");
   if (ev0 != nullptr) {
     char shape[32];
-    std::snprintf(shape, sizeof(shape), "%dx%d/mode%d", G, K, MODE);
-    // Per pixel and pass also the 16-byte record (range and cell offset).
+    std::snprintf(shape, sizeof(shape), "1x%d/mode%d", K, MODE);
+    // Per pixel and pass also the 8-byte record (range and cell offset).
     const uint64_t n = static_cast<uint64_t>(ps.n);
-    const uint64_t alg = MODE == kLastTerm ? (1 + kTermArrays + 2) * static_cast<uint64_t>(seg.cells)
-                                           : pass_bytes(MODE, true, seg);
     profile_pass(ev0, profile_mark(s), "sgm_path_ranged_kernel", shape, n * static_cast<uint64_t>(seg.cells),
-                 n * static_cast<uint64_t>(seg.pixels), n * (alg + 16 * static_cast<uint64_t>(seg.pixels)));
+                 n * static_cast<uint64_t>(seg.pixels), n * (pass_bytes(MODE, true, seg) + 8 * static_cast<uint64_t>(seg.pixels)));
   }
 }
 
-template <int G, int K>
-void launch_ranged_passes(const SgmMatch* dm, const SgmPathJob* jobs, const SgmPathSegment& g, const int4* rec,
+// The ranged passes' order: the long chains (rows, columns) before the
+// diagonals of the same tile, so that a launch ends on short blocks.
+constexpr int kRangedOrder[8] = {0, 7, 1, 4, 2, 3, 5, 6};
+
+template <int K>
+void launch_ranged_passes(const SgmMatch* dm, const SgmPathJob* jobs, const SgmPathSegment& g, const uint2* rec,
                           const uint8_t* cost, uint16_t* sum, uint8_t* terms, int64_t tstride, uint32_t* ovf,
-                          int64_t ovf_words, int sms, cudaStream_t s, const int* cancel) {
+                          int ovf_words, int sms, cudaStream_t s, const int* cancel, int* counters) {
   for (int q = 0; q < 8; ++q)
     if (g.blocks[kPasses[q].cls] <= 0) return;  // no pixels: every class has chains otherwise
   if (terms != nullptr) {
-    // Byte terms: the seven term passes in one launch, then the last pass
-    // (the total sum).
-    const int qs[kTermArrays] = {0, 1, 2, 3, 4, 5, 6};
-    const int last = 7;
-    launch_ranged_pass<G, K, kTerm>(pass_set(g, qs, kTermArrays), dm, jobs, g.count, rec, cost, sum, terms, tstride,
-                                    ovf, ovf_words, sms, s, g, cancel);
-    launch_ranged_pass<G, K, kLastTerm>(pass_set(g, &last, 1), dm, jobs, g.count, rec, cost, sum, terms, tstride, ovf,
-                                        ovf_words, sms, s, g, cancel);
+    // Byte terms: all eight directions in one launch.
+    launch_ranged_pass<K, kTerm>(pass_set(g, kRangedOrder, kRangedTerms, counters), dm, jobs, g.count, rec, cost, sum,
+                                 terms, tstride, ovf, ovf_words, sms, s, g, cancel);
     return;
   }
   for (int q = 0; q < 8; ++q) {
-    const PassSet ps = pass_set(g, &q, 1);
+    const PassSet ps = pass_set(g, kRangedOrder + q, 1, counters + q);
     if (q == 0)
-      launch_ranged_pass<G, K, kFirst>(ps, dm, jobs, g.count, rec, cost, sum, terms, tstride, ovf, ovf_words, sms, s,
-                                       g, cancel);
+      launch_ranged_pass<K, kFirst>(ps, dm, jobs, g.count, rec, cost, sum, terms, tstride, ovf, ovf_words, sms, s, g,
+                                    cancel);
     else
-      launch_ranged_pass<G, K, kAccumulate>(ps, dm, jobs, g.count, rec, cost, sum, terms, tstride, ovf, ovf_words, sms,
-                                            s, g, cancel);
+      launch_ranged_pass<K, kAccumulate>(ps, dm, jobs, g.count, rec, cost, sum, terms, tstride, ovf, ovf_words, sms, s,
+                                         g, cancel);
   }
 }
 
@@ -1623,33 +1818,44 @@ bool sgm_path_ranged_enabled() {
   return e == nullptr || std::strcmp(e, "path") == 0;
 }
 
-SgmPathShape sgm_path_ranged_shape(int over32, int64_t pixels) {
-  // 32-label chunks unless more than a tenth of the tile's pixels need two.
-  return static_cast<int64_t>(over32) * 10 > pixels ? SgmPathShape{4, 8} : SgmPathShape{2, 8};
+SgmPathShape sgm_path_ranged_shape(int64_t cells, int64_t pixels) {
+  // Items of 32 labels where the pixels average more than one and a half units.
+  return cells > 24 * pixels ? SgmPathShape{1, 16} : SgmPathShape{1, 8};
 }
 
 SgmPathBuffers sgm_path_ranged_buffers(int64_t cells, int64_t pixels, int64_t keys, int64_t rows, int maxnum,
                                        int sms, bool terms) {
-  SgmPathBuffers b = sgm_path_buffers(cells, pixels, keys, false);
-  size_t o = b.total;
-  // Byte terms of the ranged passes come in addition to the u16 sum (which
-  // the last pass writes for the per-pixel winner-takes-all).
-  b.terms = o;
+  SgmPathBuffers b{};
+  size_t o = 0;
+  b.cost = o;
+  o += align256(static_cast<size_t>(cells));
+  // Eight byte-term arrays, or the u16 sums.
+  b.sum = b.terms = o;
   b.term_stride = terms ? static_cast<int64_t>(align256(static_cast<size_t>(cells))) : 0;
-  o += static_cast<size_t>(kTermArrays) * static_cast<size_t>(b.term_stride);
+  o += terms ? static_cast<size_t>(kRangedTerms) * static_cast<size_t>(b.term_stride)
+             : align256(static_cast<size_t>(cells) * 2);
+  // Winners and right-view keys: only for matches with the diagonal check.
+  b.info = o;
+  if (keys > 0) o += align256(static_cast<size_t>(pixels) * 16);
+  b.rkeys = o;
+  o += align256(static_cast<size_t>(keys) * 4);
+  b.counters = o;
+  o += align256(sizeof(int) * kPathCounters);
   b.rec = o;
-  o += align256(static_cast<size_t>(pixels) * 16);
+  o += align256(static_cast<size_t>(pixels) * 8);
   b.rowsum = o;
   o += align256(static_cast<size_t>(rows) * 4);
   b.rowstart = o;
   o += align256(static_cast<size_t>(rows) * 4);
   b.rowshift = o;
   o += align256(static_cast<size_t>(rows) * 4);
-  b.overflow_words = maxnum > 2 * kRangedSmemWords ? (maxnum - 2 * kRangedSmemWords + 1) / 2 : 0;
+  // Words of a wide vector's buffer (none where every vector fits shared
+  // memory), with the sentinels around it, for both item sizes.
+  b.overflow_words = maxnum > RangedRing<8, kTerm>::kVecLabels ? maxnum / 2 + 2 * RangedRing<16, kTerm>::kPadWords + 2 : 0;
   b.overflow = o;
-  // One slot (two buffers) per resident chain: at most 16 chains per warp.
-  const int64_t slots = static_cast<int64_t>(sms) * kRangedMaxPerSm * (kPathThreads / 32) * 16;
-  o += align256(static_cast<size_t>(slots) * 2 * static_cast<size_t>(b.overflow_words) * 4);
+  // One slot (two buffers for each of 32 lanes) per resident warp.
+  const int64_t slots = static_cast<int64_t>(sms) * kRangedMaxPerSm * (kRangedThreads / 32);
+  o += align256(static_cast<size_t>(slots) * 64 * static_cast<size_t>(b.overflow_words) * 4);
   b.total = o;
   return b;
 }
@@ -1663,44 +1869,47 @@ void launch_sgm_path_ranged_wave(const SgmMatch* dm, const SgmPathRangedWave& wa
   uint8_t* terms = wave.terms != 0 ? wave.buffer + B.terms : nullptr;
   int4* info = reinterpret_cast<int4*>(wave.buffer + B.info);
   uint32_t* rkeys = reinterpret_cast<uint32_t*>(wave.buffer + B.rkeys);
-  int4* rec = reinterpret_cast<int4*>(wave.buffer + B.rec);
+  uint2* rec = reinterpret_cast<uint2*>(wave.buffer + B.rec);
   int* rowsum = reinterpret_cast<int*>(wave.buffer + B.rowsum);
   int* rowstart = reinterpret_cast<int*>(wave.buffer + B.rowstart);
   int* rowshift = reinterpret_cast<int*>(wave.buffer + B.rowshift);
   uint32_t* ovf = reinterpret_cast<uint32_t*>(wave.buffer + B.overflow);
+  int* counters = reinterpret_cast<int*>(wave.buffer + B.counters);
   if (wave.keys > 0) R3D_CUDA(cudaMemsetAsync(rkeys, 0xFF, static_cast<size_t>(wave.keys) * 4, s));
   R3D_LAUNCH(sgm_path_ranged_rows_kernel,
              dim3(resident_grid(sgm_path_ranged_rows_kernel, sms, wave.rows, kPathThreads / 32)), dim3(kPathThreads),
-             0, s, dm, wave.jobs, wave.njobs, wave.rows, rec, rowsum, rowshift);
+             0, s, dm, wave.jobs, wave.njobs, wave.rows, rowsum, rowshift, counters);
   launched("sgm_path_ranged_rows_kernel");
   R3D_LAUNCH(sgm_path_ranged_rowstart_kernel,
              dim3(resident_grid(sgm_path_ranged_rowstart_kernel, sms, wave.njobs, kPathThreads / 32)),
              dim3(kPathThreads), 0, s, wave.jobs, wave.njobs, rowsum, rowstart);
   launched("sgm_path_ranged_rowstart_kernel");
   R3D_LAUNCH(sgm_path_ranged_cost_kernel,
-             dim3(resident_grid(sgm_path_ranged_cost_kernel, sms, wave.pixels, kPathThreads)), dim3(kPathThreads), 0,
-             s, dm, wave.jobs, wave.njobs, wave.pixels, rec, rowstart, cost);
+             dim3(resident_grid(sgm_path_ranged_cost_kernel, sms, wave.rows, kPathThreads / 32)), dim3(kPathThreads),
+             0, s, dm, wave.jobs, wave.njobs, wave.rows, rec, rowstart, cost);
   launched("sgm_path_ranged_cost_kernel");
   for (int q = 0; q < wave.nsegs; ++q) {
     const SgmPathSegment& g = wave.segs[q];
     const SgmPathJob* jobs = wave.jobs + g.first;
-    if (g.shape.g_ == 2 && g.shape.k_ == 8)
-      launch_ranged_passes<2, 8>(dm, jobs, g, rec, cost, sum, terms, B.term_stride, ovf, B.overflow_words, sms, s,
-                                 wave.cancel);
-    else if (g.shape.g_ == 4 && g.shape.k_ == 8)
-      launch_ranged_passes<4, 8>(dm, jobs, g, rec, cost, sum, terms, B.term_stride, ovf, B.overflow_words, sms, s,
-                                 wave.cancel);
+    if (g.shape.k_ == 8)
+      launch_ranged_passes<8>(dm, jobs, g, rec, cost, sum, terms, B.term_stride, ovf, B.overflow_words, sms, s,
+                              wave.cancel, counters + 8 * q);
+    else if (g.shape.k_ == 16)
+      launch_ranged_passes<16>(dm, jobs, g, rec, cost, sum, terms, B.term_stride, ovf, B.overflow_words, sms, s,
+                               wave.cancel, counters + 8 * q);
     else
       fail(R3DGPU_EINVAL, "stereo: bad ranged path kernel shape");
   }
-  R3D_LAUNCH(sgm_path_ranged_wta_kernel,
-             dim3(resident_grid(sgm_path_ranged_wta_kernel, sms, wave.pixels, kPathThreads)), dim3(kPathThreads), 0,
-             s, dm, wave.jobs, wave.njobs, wave.pixels, rec, sum, rowshift, info, rkeys);
+  auto* wta = terms != nullptr ? sgm_path_ranged_wta_kernel<true> : sgm_path_ranged_wta_kernel<false>;
+  R3D_LAUNCH(wta, dim3(resident_grid(wta, sms, wave.pixels, kPathThreads)), dim3(kPathThreads), 0, s, dm, wave.jobs,
+             wave.njobs, wave.pixels, rec, cost, sum, terms, B.term_stride, rowshift, info, rkeys);
   launched("sgm_path_ranged_wta_kernel");
-  R3D_LAUNCH(sgm_path_ranged_accept_kernel,
-             dim3(resident_grid(sgm_path_ranged_accept_kernel, sms, wave.pixels, kPathThreads)), dim3(kPathThreads),
-             0, s, dm, wave.jobs, wave.njobs, wave.pixels, rec, info, rkeys, rowshift);
-  launched("sgm_path_ranged_accept_kernel");
+  if (wave.keys > 0) {  // matches with the diagonal left-right check
+    R3D_LAUNCH(sgm_path_ranged_accept_kernel,
+               dim3(resident_grid(sgm_path_ranged_accept_kernel, sms, wave.pixels, kPathThreads)), dim3(kPathThreads),
+               0, s, dm, wave.jobs, wave.njobs, wave.pixels, rec, info, rkeys, rowshift);
+    launched("sgm_path_ranged_accept_kernel");
+  }
 }
 
 }  // namespace r3dgpu

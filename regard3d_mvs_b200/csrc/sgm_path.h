@@ -48,14 +48,15 @@ SgmPathShape sgm_path_shape(int nd);
 inline bool sgm_path_fits(int w, int nd) { return w + nd - 1 <= 2048; }
 inline int64_t sgm_path_chains(int cls, int w, int h) { return cls == 0 ? h : (cls == 1 ? w : w + h - 1); }
 
-// Device buffers of a wave (bytes, 256-byte aligned pieces). Byte terms:
-// seven arrays of term_stride bytes from `terms` on (full-range waves keep
-// them in place of the u16 sum volume, ranged waves beside it).
+// Device buffers of a wave (bytes, 256-byte aligned pieces). Byte terms, in
+// place of the u16 sum volume: arrays of term_stride bytes from `terms` on
+// (seven of full-range waves, eight of ranged ones).
 struct SgmPathBuffers {
   size_t cost, sum, terms, info, rkeys, ints, total;  // ints: full-range waves, the tiles' intensities
+  size_t counters;                                    // block counters of the pass launches
   int64_t term_stride;
   size_t rec, rowsum, rowstart, rowshift, overflow;  // ranged waves only
-  int64_t overflow_words;                            // per chain buffer
+  int overflow_words;                                // per wide vector's buffer
 };
 SgmPathBuffers sgm_path_buffers(int64_t cells, int64_t pixels, int64_t keys, bool terms);
 
@@ -96,11 +97,10 @@ void launch_sgm_path_wave(const SgmMatch* dm, const SgmPathWave& wave, int sms, 
 bool sgm_path_enabled();
 
 // ---- Ranged tiles (per-pixel label ranges lo, num) through the chain passes.
-// Sums and costs are packed per tile (each pixel's num labels, row-major);
-// chunk 0 of a chain's predecessor vector (64 labels) stays in shared memory,
-// labels beyond it of the rare wide pixels in a per-chain overflow in global
-// memory. Shapes: (2, 8) = 32 labels per chunk, (4, 8) = 64.
-SgmPathShape sgm_path_ranged_shape(int over32, int64_t pixels);
+// Sums, costs and terms are packed per tile (each pixel's num labels,
+// row-major). One lane per chain; shapes (1, 8) = items of 16 labels, (1, 16)
+// = items of 32, by the tile's mean label count.
+SgmPathShape sgm_path_ranged_shape(int64_t cells, int64_t pixels);
 struct SgmPathRangedWave {
   const SgmPathJob* jobs;
   int njobs;
