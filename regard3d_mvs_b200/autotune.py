@@ -35,8 +35,7 @@ from .types import CDisparityMap, CPair, CProfile, CSynthParams, CViewU8, CViewU
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 FULL_SHAPES = ((8, 4), (8, 8), (16, 4), (8, 12), (16, 6), (16, 8), (8, 16), (16, 12), (32, 8), (32, 12))
-PATH_SHAPES = ((2, 16), (4, 8), (4, 12), (4, 16), (8, 8), (8, 12), (8, 16), (16, 8), (16, 12), (16, 16), (32, 8),
-               (32, 12))
+PATH_SHAPES = ((2, 16), (4, 8), (4, 16), (8, 8), (8, 16), (16, 8), (16, 16), (32, 8), (32, 16))
 FULL_ND = (384, 256, 192, 128, 64)
 ROWS = (64, 48, 32, 24, 16)
 ND_CHOICES = (64, 128, 192, 256, 384)

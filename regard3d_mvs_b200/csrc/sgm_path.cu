@@ -10,20 +10,20 @@
 // the diagonal ones. This file runs them that way:
 //
 //   cost kernel     u8 costs of every cell of the wave (written once);
-//   8 path passes   one launch per direction (and kernel shape); G lanes walk
-//                   one chain, K label pairs per lane, 32 / G chains per warp,
-//                   the predecessor vector in registers (its d -+ 1 neighbours
-//                   across lanes by shuffle), the next pixel's costs and sums
-//                   loaded while the current one is computed. The first pass
-//                   writes the sum volume, the next six add to it, the last
-//                   adds its path and takes the winner-takes-all records;
-//   accept kernel   the acceptance rules, subpixel fit and confidence per
-//                   pixel, into the tile's disparity and confidence.
+//   8 path passes   G lanes walk one chain, K label pairs per lane, 32 / G
+//                   chains per warp, the predecessor vector in registers, the
+//                   next pixels' costs streaming into a shared-memory ring.
+//                   Each writes its path's byte terms, all eight in one launch
+//                   (or, with a P2 above 255, adds to u16 sums, one launch each);
+//   winner kernel   total sums, winner-takes-all, acceptance rules, subpixel
+//                   fit and confidence per pixel, into the tile's disparity
+//                   and confidence.
 //
 // No CTA barrier is on the chain's critical path and every tile spreads over
 // as many SMs as it has chains, so one small pair fills the GPU as well as a
-// batch does. HBM traffic per aggregated cell: 1 B cost write, 8 x 1 B cost
-// reads, 2 B + 6 x 4 B + 2 B sum traffic.
+// batch does. Bytes per aggregated cell with terms: 1 cost write, 8 cost
+// reads (about 1 from DRAM: a tile's directions run close together), 8 term
+// writes, 9 reads.
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -41,6 +41,7 @@ using sgm_simd::group_umin;
 using sgm_simd::kSent2;
 constexpr float kInfF = __builtin_huge_valf();
 constexpr int kPathThreads = 256;
+constexpr int kPathMaxLabels = 768;  // more go to the one-CTA-per-tile kernels
 constexpr int kPathCounters = 256;  // block counters of a wave's launches (one each)
 
 inline size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
@@ -103,6 +104,10 @@ R3D_DEVICE void chain_geometry(int cls, int dx, int dy, int w, int h, int64_t c,
 // x0 + w - 1 - dmin) are staged in the warp's shared memory, then the lanes
 // take 32 consecutive pixels and write 32 labels (one sector) at a time.
 constexpr int kCostStage = 2048;  // staged partner codes per warp at most (sgm_path_fits: w + nd - 1 <= 2048)
+
+// Label of byte i of word w of a run of 16-label units (the byte order of
+// unpack_unit).
+R3D_DEVICE int unit_label(int w, int i) { return 16 * (w >> 2) + 2 * (w & 3) + (i & 1) + 8 * (i >> 1); }
 
 // `stage_words` (<= kCostStage): the widest staged row of the wave (tile
 // width + labels - 1), so that narrow waves run more CTAs per SM.
@@ -167,7 +172,7 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
                 uint32_t lo = 0, hi = 0;
 #pragma unroll
                 for (int i = 3; i >= 0; --i) {
-                  const uint64_t d = cl ^ stage[base - 4 * w4 - i];
+                  const uint64_t d = cl ^ stage[base - unit_label(w4, i)];
                   lo = lo * 256u + static_cast<uint32_t>(r3dsimt::popc(static_cast<uint32_t>(d)));
                   hi = hi * 256u + static_cast<uint32_t>(r3dsimt::popc(static_cast<uint32_t>(d >> 32)));
                 }
@@ -181,7 +186,7 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
                 const int xr = xr_first - k;
                 const bool ok = xr >= rv.first && xr <= rv.last;
                 const uint32_t v = ok ? static_cast<uint32_t>(r3dsimt::popc64(cl ^ stage[base - k])) : inv;
-                q[k >> 2] |= v << (8 * (k & 3));
+                q[4 * (k >> 4) + ((k & 7) >> 1)] |= v << (8 * ((k & 1) + 2 * ((k >> 3) & 1)));
               }
             }
           }
@@ -194,15 +199,13 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
 }
 
 // ---------------------------------------------------------------- passes
-// Pass modes. With u16 sums (any penalties): the first pass writes the sum
-// volume, the next six add to it, the last adds its path and takes the
-// winner-takes-all. With byte terms (every P2 <= 255): passes 1..7 write
-// their path's term T_r = L_r - C (in [0, P2]) as one byte per cell, and the
-// last pass forms S = L_8 + 7 C + sum T_r (at most 8 (255 + 255) < 2^16, so
-// the sum modulo 2^16 is the plain sum) and takes the winner-takes-all.
-enum PassMode { kFirst = 0, kAccumulate = 1, kLast = 2, kTerm = 3, kLastTerm = 4 };
-constexpr int kTermArrays = 7;    // of the full-range passes (the last pass adds its own path)
-constexpr int kRangedTerms = 8;   // of the ranged passes (summed per pixel)
+// Pass modes. With byte terms (every P2 <= 255) every direction writes its
+// path's term T_r = L_r - C (in [0, P2]) as one byte per cell, and the
+// per-pixel kernel forms S = 8 C + sum T_r (at most 8 (255 + 255) < 2^16, so
+// the sum modulo 2^16 is the plain sum). With u16 sums (any penalties) the
+// first pass writes the sum volume and the next seven add to it.
+enum PassMode { kFirst = 0, kAccumulate = 1, kTerm = 3 };
+constexpr int kTermArrays = 8;
 constexpr int kMaxPasses = 8;
 // The passes of one launch: n directions (slot = its term array), their
 // number per chain class, and the chain blocks of all of them together. The
@@ -266,96 +269,136 @@ R3D_DEVICE int64_t locate_block(const SgmPathJob* jobs, int njobs, const PassSet
 R3D_DEVICE uint32_t add2(uint32_t a, uint32_t b, bool no_carry) { return no_carry ? a + b : r3dsimt::vadd2(a, b); }
 
 // a * one + b with one = 1 at run time: an integer multiply-add, which the
-// FMA pipe executes, in place of an add on the ALU pipe (the pass kernels'
-// packed min, byte permutes and adds keep the ALU pipe the busier one).
+// FMA pipe executes, in place of an add on the ALU pipe (packed minima, masks
+// and byte permutes keep the ALU pipe the busier one: 64 lanes per clock each).
 R3D_DEVICE uint32_t fma_add(uint32_t a, uint32_t one, uint32_t b) { return a * one + b; }
 
-// v[j] for a runtime j in [0, K): a tree of K - 1 selects on the bits of j
-// (a register array cannot be indexed at run time without local memory).
-template <int N>
-R3D_DEVICE void pick_level(uint32_t* t, bool hi) {
+// Labels of a vector are kept in units of 16: word k = 0..7 of a unit holds
+// labels k and k + 8, so that the neighbours d -+ 1 of a word are the words
+// next to it. Byte planes (costs, terms) store word j = 0..3 of a unit as the
+// bytes of labels 2 j, 2 j + 1, 2 j + 8, 2 j + 9: one mask or permute unpacks a
+// word of two labels, one multiply-add packs two of them.
+R3D_DEVICE void unpack_unit(const uint4& v, uint32_t* c2) {
+  const uint32_t cw[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-  for (int k = 0; 2 * k < N; ++k) t[k] = (2 * k + 1 < N && hi) ? t[2 * k + 1] : t[2 * k];
+  for (int k = 0; k < 4; ++k) {
+    c2[2 * k] = cw[k] & 0x00FF00FFu;
+    c2[2 * k + 1] = r3dsimt::perm(cw[k], 0u, 0x4341u);
+  }
 }
-template <int K>
-R3D_DEVICE uint32_t pick(const uint32_t (&v)[K], int j) {
-  static_assert(K >= 2 && K <= 16, "pick: 2..16 words");
-  constexpr int n1 = (K + 1) / 2, n2 = (n1 + 1) / 2, n3 = (n2 + 1) / 2;
-  uint32_t t[K];
-#pragma unroll
-  for (int k = 0; k < K; ++k) t[k] = v[k];
-  pick_level<K>(t, (j & 1) != 0);
-  if constexpr (n1 > 1) pick_level<n1>(t, (j & 2) != 0);
-  if constexpr (n2 > 1) pick_level<n2>(t, (j & 4) != 0);
-  if constexpr (n3 > 1) pick_level<n3>(t, (j & 8) != 0);
-  return t[0];
+R3D_DEVICE uint4 pack_unit(const uint32_t* tr) {
+  return make_uint4(tr[0] + 256u * tr[1], tr[2] + 256u * tr[3], tr[4] + 256u * tr[5], tr[6] + 256u * tr[7]);
 }
 
-// Per-warp shared-memory ring of the pass kernels: Stages stages, each with
-// one pixel per chain of the bytes the pass reads (Planes bytes per label:
-// the cost, plus the u16 sum or the seven byte terms).
-// The term passes read one byte per label and keep 8 stages in flight (their
-// step is short, so 3 stages ahead left them waiting on DRAM).
-// The last pass with byte terms stages eight byte planes per pixel: two
-// stages (its step is long, one pixel ahead covers the DRAM latency).
-template <int MODE>
-struct PathMode {
-  static constexpr int kPlanes = MODE == kAccumulate || MODE == kLast ? 3 : (MODE == kLastTerm ? 1 + kTermArrays : 1);
-  static constexpr int kStages = MODE == kLastTerm ? 2 : (MODE == kTerm ? 8 : 4);
-};
-// A stage ends with one 4-byte word per lane: the aligned word of the
-// intensities that holds its chain's pixel (every lane copies its own, since
-// a cp.async wait covers only the waiting thread's copies).
-// CTA size and resident CTAs per SM: 4-warp CTAs for the byte-term last
-// pass (its eight-plane ring) and the 16-word term passes (92 registers),
-// so that CTAs pack an SM's registers and shared memory finely (the 12-word
-// term passes measured 12-19 % slower that way than in two 8-warp CTAs).
+// best = min(L(q, d), L(q, d -+ 1) + P1, min L(q) + P2) for N words whose
+// labels cl are already clamped to min L(q) + P2 (one 3-way minimum per word
+// is left); `below` and `above` hold the clamped labels before the first unit
+// (in the high half) and after the last (in the low half).
+template <int N>
+R3D_DEVICE void best_terms(const uint32_t (&cl)[N], uint32_t below, uint32_t above, uint32_t one, uint32_t p1x2,
+                           uint32_t (&best)[N]) {
+#pragma unroll
+  for (int u = 0; u < N / 8; ++u) {
+    // Words -1 and 8 of the unit: labels (16 u - 1, 16 u + 7) and (16 u + 8, 16 u + 16).
+    uint32_t s[10];
+    s[0] = fma_add(r3dsimt::perm(u > 0 ? cl[u > 0 ? 8 * u - 1 : 0] : below, cl[8 * u + 7], 0x5432u), one, p1x2);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s[1 + k] = fma_add(cl[8 * u + k], one, p1x2);
+    s[9] = fma_add(r3dsimt::perm(cl[8 * u], 8 * u + 8 < N ? cl[8 * u + 8 < N ? 8 * u + 8 : 0] : above, 0x5432u), one, p1x2);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) best[8 * u + k] = r3dsimt::vmin3(cl[8 * u + k], s[k], s[2 + k]);
+  }
+}
+
+// Per-halfword minimum of N words.
+template <int N>
+R3D_DEVICE uint32_t min_words(const uint32_t (&v)[N]) {
+  constexpr int N3 = (N + 2) / 3;
+  uint32_t t3[N3];
+#pragma unroll
+  for (int k = 0; k < N3; ++k)
+    t3[k] = r3dsimt::vmin3(v[3 * k], v[3 * k + 1 < N ? 3 * k + 1 : 3 * k], v[3 * k + 2 < N ? 3 * k + 2 : 3 * k]);
+  uint32_t m = t3[0];
+#pragma unroll
+  for (int k = 1; k < N3; k += 2) m = r3dsimt::vmin3(m, t3[k], t3[k + 1 < N3 ? k + 1 : k]);
+  return m;
+}
+
+// The eight words of unit u of a pixel's total sums, from its cost and term
+// bytes (TERMS) or its stored u16 sums.
+template <bool TERMS>
+R3D_DEVICE void sum_unit(const uint8_t* cp, const uint8_t* tp, int64_t tstride, const uint16_t* sp, int u,
+                         uint32_t (&wv)[8]) {
+  if constexpr (TERMS) {
+    uint4 t[1 + kTermArrays];
+    t[0] = r3dsimt::ld_stream(reinterpret_cast<const uint4*>(cp + 16 * u));
+#pragma unroll
+    for (int r = 0; r < kTermArrays; ++r)
+      t[1 + r] = r3dsimt::ld_stream(reinterpret_cast<const uint4*>(tp + r * tstride + 16 * u));
+#pragma unroll
+    for (int r = 0; r <= kTermArrays; ++r) {
+      uint32_t c2[8];
+      unpack_unit(t[r], c2);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) wv[k] = r == 0 ? 8u * c2[k] : wv[k] + c2[k];
+    }
+  } else {
+    const uint4* sp4 = reinterpret_cast<const uint4*>(sp);
+    const uint4 a = sp4[2 * u], b = sp4[2 * u + 1];
+    wv[0] = a.x;
+    wv[1] = a.y;
+    wv[2] = a.z;
+    wv[3] = a.w;
+    wv[4] = b.x;
+    wv[5] = b.y;
+    wv[6] = b.z;
+    wv[7] = b.w;
+  }
+}
+// Unit u's sums in label order.
+R3D_DEVICE void store_unit(uint16_t* vol, const uint32_t (&wv)[8]) {
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    vol[k] = static_cast<uint16_t>(wv[k] & 0xFFFFu);
+    vol[k + 8] = static_cast<uint16_t>(wv[k] >> 16);
+  }
+}
+
+// Per-warp shared-memory ring of the full-range passes: Stages stages, each
+// with one pixel per chain of the bytes the pass reads (the cost, and the u16
+// sum of the adding passes), then one 4-byte word per lane: the aligned word
+// of the intensities that holds its chain's pixel (every lane copies its own,
+// since a cp.async wait covers only the waiting thread's copies). 4-warp CTAs
+// pack an SM's registers and shared memory finely.
 template <int G, int K, int MODE>
 struct PathRing {
-  static constexpr int kThreads = (MODE == kLastTerm || (MODE == kTerm && K >= 16)) ? 128 : kPathThreads;
-  static constexpr int kMinBlocks = MODE == kLastTerm ? (K <= 8 ? 6 : 3)
-                                    : MODE == kTerm   ? (K <= 8 ? 4 : (K >= 16 ? 5 : 2))
-                                                      : (K <= 8 ? 3 : 2);
+  static constexpr int kThreads = 128;
+  static constexpr int kMinBlocks = K <= 8 ? 8 : 5;
   static constexpr int ND = 2 * G * K;
-  static constexpr int kStages = PathMode<MODE>::kStages;
-  static constexpr int kPlaneBytes = (32 / G) * PathMode<MODE>::kPlanes * ND;
-  static constexpr int kIntBytes = 32 * 4;
-  static constexpr int kStageBytes = kPlaneBytes + kIntBytes;
+  static constexpr int kPlanes = MODE == kAccumulate ? 3 : 1;
+  static constexpr int kStages = MODE == kTerm ? 8 : 4;
+  static constexpr int kPlaneBytes = (32 / G) * kPlanes * ND;
+  static constexpr int kStageBytes = kPlaneBytes + 32 * 4;
   static constexpr int kWarpBytes = kStages * kStageBytes;
   // Each warp's rings, then each warp's copy of its match's P2 table.
   static constexpr int kBlockBytes = (kThreads / 32) * (kWarpBytes + 512);
 };
 
-// CTAs per SM (PathRing): four 8-warp CTAs for the 8-word term passes (64
-// registers, no spills), two for the 12-word ones, five 4-warp CTAs for the
-// 16-word ones; six or three 4-warp CTAs for the byte-term last pass; three
-// or two 8-warp CTAs for the u16-sum passes.
-//
-// The step loop is unrolled by the ring depth NS so that ring slots and the
-// intensity queue are indexed statically; each chain keeps running pointers
-// (advanced by one pixel along the path per step) instead of recomputing
-// addresses. The first pixel needs no special case: with a zero predecessor
-// vector and a zero minimum, best = 0, so T = 0 and L = C there.
-//
-// One launch runs the passes of a PassSet: a single pass, or the seven term
-// passes of a segment at once (they only read the costs and each writes its
-// own term array, so their chain blocks can be taken in any order).
+// G lanes walk one chain, 2 K consecutive labels per lane (K / 8 units), 32 / G
+// chains per warp. The step loop is unrolled by the ring depth NS so that ring
+// slots are indexed statically; each chain keeps running pointers (advanced by
+// one pixel along the path per step). The first pixel needs no special case:
+// with a zero clamp, best = 0, so T = 0 and L = C there. FULL: every unit of
+// the group is inside the match's label count.
 template <int G, int K, int MODE, bool FULL>
 R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN((PathRing<G, K, MODE>::kThreads), (PathRing<G, K, MODE>::kMinBlocks))
     sgm_path_kernel(const SgmMatch* R3D_RESTRICT matches, const SgmPathJob* R3D_RESTRICT jobs, int njobs,
                     const PassSet ps, const uint8_t* R3D_RESTRICT cost, uint16_t* sum, uint8_t* terms,
-                    int64_t tstride, int4* R3D_RESTRICT info, uint32_t* rkeys, const uint16_t* R3D_RESTRICT ints,
-                    const int* cancel) {
+                    int64_t tstride, const uint16_t* R3D_RESTRICT ints, const int* cancel) {
   constexpr int CPW = 32 / G;  // chains per warp
-  constexpr int U = K / 4;     // units of 8 labels per lane
+  constexpr int NV = K / 8;    // units per lane
   constexpr int NS = PathRing<G, K, MODE>::kStages;
-  constexpr bool kReadsSum = MODE == kAccumulate || MODE == kLast;
-  constexpr bool kWta = MODE == kLast || MODE == kLastTerm;
-  // K a multiple of 8: a lane's 2 K labels are NV 16-byte aligned pieces of
-  // every byte plane (piece v = units 2 v, 2 v + 1, valid together since
-  // label counts are multiples of 16).
-  constexpr bool kVec = K % 8 == 0;
-  constexpr int NV = K / 8;
+  using Ring = PathRing<G, K, MODE>;
   R3D_DYNAMIC_SMEM(smem);
   const int lane = static_cast<int>(threadIdx.x & 31u);
   const int gi = lane / G, t = lane % G;
@@ -363,7 +406,6 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN((PathRing<G, K, MODE>::kThreads), (PathRin
   const int left_lane = (lane + 31) & 31, right_lane = (lane + 1) & 31;
   const int wpb = static_cast<int>(blockDim.x) >> 5;
   const int64_t nwarps = static_cast<int64_t>(gridDim.x) * wpb;
-  using Ring = PathRing<G, K, MODE>;
   unsigned char* const ring = smem + static_cast<size_t>(threadIdx.x >> 5) * Ring::kWarpBytes;
   // The warp's copy of the P2 table of the match it works on (256 u16),
   // reloaded when a chain block belongs to another match.
@@ -372,7 +414,6 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN((PathRing<G, K, MODE>::kThreads), (PathRin
   int lut_match = -1;
   unsigned char* const ring_cost = ring + gi * Ring::ND + e0;
   unsigned char* const ring_sum = ring + CPW * Ring::ND + gi * 2 * Ring::ND + 2 * e0;
-  unsigned char* const ring_term = ring + CPW * Ring::ND + gi * Ring::ND + e0;  // + r * CPW * ND
   unsigned char* const ring_int = ring + Ring::kPlaneBytes + lane * 4;
   const uint32_t one = ps.one;
   for (int64_t gblk = static_cast<int64_t>(blockIdx.x) * wpb + (threadIdx.x >> 5); gblk < ps.total;
@@ -397,19 +438,17 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN((PathRing<G, K, MODE>::kThreads), (PathRin
     int maxlen = len;
 #pragma unroll
     for (int o = G; o < 32; o <<= 1) maxlen = r3dsimt::imax(maxlen, static_cast<int>(r3dsimt::shfl_xor(maxlen, o)));
-    bool uvalid[U];
+    bool uvalid[NV];
 #pragma unroll
-    for (int u = 0; u < U; ++u) uvalid[u] = FULL || e0 + 8 * u < nd;
-    // Running offsets (cells, pixels) of the pixel being issued (NS - 1
-    // ahead) and of the pixel being computed.
+    for (int v = 0; v < NV; ++v) uvalid[v] = FULL || e0 + 16 * v < nd;
+    // Running pointers of the pixel being issued (NS - 1 ahead) and of the
+    // pixel being computed.
     const int64_t dcell = (static_cast<int64_t>(dy) * w + dx) * nd;
     const int64_t cell0 = job.cell_off + e0 + (static_cast<int64_t>(sy) * w + sx) * nd;
     const uint8_t* c_in = cost + cell0;
     const uint16_t* s_in = sum + cell0;
-    const uint8_t* t_in = terms + cell0;
     uint16_t* s_out = sum + cell0;
     uint8_t* t_out = terms + cell0 + static_cast<int64_t>(tslot) * tstride;
-    int64_t px_out = job.px_off + static_cast<int64_t>(sy) * w + sx;
     const int64_t dpx = static_cast<int64_t>(dy) * w + dx;
     // Intensity of the pixel being issued (each lane copies the aligned
     // 4-byte word holding it into the stage), and the parity of the
@@ -418,40 +457,17 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN((PathRing<G, K, MODE>::kThreads), (PathRin
     const uint16_t* i_iss = ints + job.px_off + static_cast<int64_t>(sy) * w + sx;
     const uint32_t par0 = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(i_iss) >> 1) & 1u;
     const uint32_t dpar = static_cast<uint32_t>(dpx) & 1u;
-    int x = sx, y = sy;
 
     auto issue = [&](int i, int st) {
       if (i < len) {
         unsigned char* rc = ring_cost + st * Ring::kStageBytes;
-        if constexpr (kVec) {
 #pragma unroll
-          for (int v = 0; v < NV; ++v) {
-            if (uvalid[2 * v]) {
-              r3dsimt::cp_async16(rc + 16 * v, c_in + 16 * v);
-              if constexpr (kReadsSum) {
-                r3dsimt::cp_async16(ring_sum + st * Ring::kStageBytes + 32 * v, s_in + 16 * v);
-                r3dsimt::cp_async16(ring_sum + st * Ring::kStageBytes + 32 * v + 16, s_in + 16 * v + 8);
-              }
-              if constexpr (MODE == kLastTerm) {
-#pragma unroll
-                for (int r = 0; r < kTermArrays; ++r)
-                  r3dsimt::cp_async16(ring_term + st * Ring::kStageBytes + r * CPW * Ring::ND + 16 * v,
-                                      t_in + r * tstride + 16 * v);
-              }
-            }
-          }
-        } else {
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            if (uvalid[u]) {
-              r3dsimt::cp_async8(rc + 8 * u, c_in + 8 * u);
-              if constexpr (kReadsSum) r3dsimt::cp_async16(ring_sum + st * Ring::kStageBytes + 16 * u, s_in + 8 * u);
-              if constexpr (MODE == kLastTerm) {
-#pragma unroll
-                for (int r = 0; r < kTermArrays; ++r)
-                  r3dsimt::cp_async8(ring_term + st * Ring::kStageBytes + r * CPW * Ring::ND + 8 * u,
-                                     t_in + r * tstride + 8 * u);
-              }
+        for (int v = 0; v < NV; ++v) {
+          if (uvalid[v]) {
+            r3dsimt::cp_async16(rc + 16 * v, c_in + 16 * v);
+            if constexpr (MODE == kAccumulate) {
+              r3dsimt::cp_async16(ring_sum + st * Ring::kStageBytes + 32 * v, s_in + 16 * v);
+              r3dsimt::cp_async16(ring_sum + st * Ring::kStageBytes + 32 * v + 16, s_in + 16 * v + 8);
             }
           }
         }
@@ -460,8 +476,7 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN((PathRing<G, K, MODE>::kThreads), (PathRin
       }
       r3dsimt::cp_async_commit();
       c_in += dcell;
-      if constexpr (kReadsSum) s_in += dcell;
-      if constexpr (MODE == kLastTerm) t_in += dcell;
+      if constexpr (MODE == kAccumulate) s_in += dcell;
       i_iss += dpx;
     };
 #pragma unroll
@@ -470,273 +485,74 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN((PathRing<G, K, MODE>::kThreads), (PathRin
 #pragma unroll
     for (int k = 0; k < K; ++k) prev[k] = 0;
     uint32_t pmin = 0;
-    // Intensities and P2. With four stages or more, the next pixel's stage
-    // has landed when this pixel is computed, so the P2 of the step into the
-    // next pixel is looked up one step ahead, off the step's critical path
-    // (iprev is then this pixel's intensity); with two stages the P2 of the
-    // step into this pixel is looked up in its step (iprev is the previous
-    // pixel's intensity). The first step's P2 is unused: its predecessor
-    // vector is zero.
-    constexpr bool kAheadP2 = NS >= 4;
-    int iprev = 0;
+    // The next pixel's stage has landed when this pixel is computed, so the
+    // P2 of the step into the next pixel is looked up one step ahead, off the
+    // step's critical path (iprev is then this pixel's intensity). The first
+    // step's P2 is 0, with pmin = 0 the zero clamp of the first pixel.
     uint32_t p2next = 0;
-    if constexpr (kAheadP2) {
-      r3dsimt::cp_async_wait<NS - 2>();  // the first of the NS - 1 stages in flight
-      const uint32_t iw0 = *reinterpret_cast<const uint32_t*>(ring_int);
-      iprev = static_cast<int>((iw0 >> (16u * par0)) & 0xFFFFu);
-    }
+    r3dsimt::cp_async_wait<NS - 2>();  // the first of the NS - 1 stages in flight
+    const uint32_t iw0 = *reinterpret_cast<const uint32_t*>(ring_int);
+    int iprev = static_cast<int>((iw0 >> (16u * par0)) & 0xFFFFu);
 
     auto step = [&](const int i, const int q) {
       const bool on = i < len;
-      constexpr int kNext = NS - 1;
-      issue(i + kNext, (q + kNext) % NS);
-      uint32_t pen;
-      if constexpr (kAheadP2) {
-        r3dsimt::cp_async_wait<NS - 2>();  // this pixel's stage and the next one's
-        const uint32_t iw = *reinterpret_cast<const uint32_t*>(ring_int + ((q + 1) % NS) * Ring::kStageBytes);
-        const int inext =
-            static_cast<int>((iw >> (16u * ((par0 ^ (static_cast<uint32_t>(i + 1) & dpar)) & 1u))) & 0xFFFFu);
-        pen = pmin + p2next;
-        const int dn = inext - iprev;
-        p2next = lut[(dn < 0 ? -dn : dn) >> 8];
-        iprev = inext;
-      } else {
-        r3dsimt::cp_async_wait<NS - 1>();
-        const uint32_t iw = *reinterpret_cast<const uint32_t*>(ring_int + q * Ring::kStageBytes);
-        const int icur =
-            static_cast<int>((iw >> (16u * ((par0 ^ (static_cast<uint32_t>(i) & dpar)) & 1u))) & 0xFFFFu);
-        const int dn = icur - iprev;
-        iprev = icur;
-        pen = pmin + lut[(dn < 0 ? -dn : dn) >> 8];
-      }
-      const unsigned char* sc = ring_cost + q * Ring::kStageBytes;
-      uint2 craw[U];
-      if constexpr (kVec) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-          const uint4 w4 = uvalid[2 * v] ? *reinterpret_cast<const uint4*>(sc + 16 * v) : make_uint4(0, 0, 0, 0);
-          craw[2 * v] = make_uint2(w4.x, w4.y);
-          craw[2 * v + 1] = make_uint2(w4.z, w4.w);
-        }
-      } else {
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-          craw[u] = uvalid[u] ? *reinterpret_cast<const uint2*>(sc + 8 * u) : make_uint2(0, 0);
-      }
-      uint32_t c2[K];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        c2[4 * u + 0] = r3dsimt::perm(craw[u].x, 0u, 0x4140u);
-        c2[4 * u + 1] = r3dsimt::perm(craw[u].x, 0u, 0x4342u);
-        c2[4 * u + 2] = r3dsimt::perm(craw[u].y, 0u, 0x4140u);
-        c2[4 * u + 3] = r3dsimt::perm(craw[u].y, 0u, 0x4342u);
-      }
-      // out = L_r = C + T_r with T_r = best - min L(q).
-      const uint32_t pen2 = pen * 0x10001u;
-      const uint32_t negmp = pmin * 0xFFFEFFFFu;  // -(pmin in both halves) modulo 2^32
+      issue(i + NS - 1, (q + NS - 1) % NS);
       const uint32_t hl = r3dsimt::shfl(prev[K - 1], left_lane);
       const uint32_t hr = r3dsimt::shfl(prev[0], right_lane);
-      uint32_t wv[K + 2];
-      wv[0] = t > 0 ? hl : kSent2;
+      r3dsimt::cp_async_wait<NS - 2>();  // this pixel's stage and the next one's
+      const uint32_t iw = *reinterpret_cast<const uint32_t*>(ring_int + ((q + 1) % NS) * Ring::kStageBytes);
+      const int inext =
+          static_cast<int>((iw >> (16u * ((par0 ^ (static_cast<uint32_t>(i + 1) & dpar)) & 1u))) & 0xFFFFu);
+      const uint32_t pen2 = (pmin + p2next) * 0x10001u;
+      const uint32_t negmp = pmin * 0xFFFEFFFFu;  // -(pmin in both halves) modulo 2^32
+      const int dn = inext - iprev;
+      p2next = lut[(dn < 0 ? -dn : dn) >> 8];
+      iprev = inext;
+      uint32_t cl[K], best[K], c2[K], out[K], tr[K];
 #pragma unroll
-      for (int k = 0; k < K; ++k) wv[1 + k] = prev[k];
-      wv[K + 1] = t + 1 < G ? hr : kSent2;
-      uint32_t out[K], tr[K];
-      uint32_t mprev = r3dsimt::perm(wv[0], wv[1], 0x5432u);
+      for (int k = 0; k < K; ++k) cl[k] = r3dsimt::vmin2(prev[k], pen2);
+      best_terms<K>(cl, t > 0 ? r3dsimt::vmin2(hl, pen2) : pen2, t + 1 < G ? r3dsimt::vmin2(hr, pen2) : pen2, one, p1x2,
+                    best);
+      const unsigned char* sc = ring_cost + q * Ring::kStageBytes;
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+        unpack_unit(uvalid[v] ? *reinterpret_cast<const uint4*>(sc + 16 * v) : make_uint4(0, 0, 0, 0), c2 + 8 * v);
+      // out = L_r = C + T_r with T_r = best - min L(q).
 #pragma unroll
       for (int k = 0; k < K; ++k) {
-        const uint32_t mnext = r3dsimt::perm(wv[k + 1], wv[k + 2], 0x5432u);
-        const uint32_t nb = r3dsimt::vmin2(mprev, mnext);
-        const uint32_t best = r3dsimt::vmin2(wv[k + 1], r3dsimt::vaddmin2(nb, p1x2, pen2));
-        tr[k] = fma_add(best, one, negmp);
+        tr[k] = fma_add(best[k], one, negmp);
         out[k] = fma_add(tr[k], one, c2[k]);
-        mprev = mnext;
+        if (!uvalid[k / 8]) out[k] = kSent2;
       }
-      // Minimum over the lane's labels (a tree), then over the chain's lanes.
-      uint32_t mm[K];
+      // Minimum over the lane's labels, then over the chain's lanes.
+      const uint32_t mm = min_words<K>(out);
+      pmin = group_umin<G>(r3dsimt::umin(mm & 0xFFFFu, mm >> 16));
+      if (on) {
 #pragma unroll
-      for (int k = 0; k < K; ++k) {
-        if (!uvalid[k / 4]) out[k] = kSent2;
-        mm[k] = out[k];
-      }
-#pragma unroll
-      for (int s = 1; s < K; s <<= 1) {
-#pragma unroll
-        for (int k = 0; k + s < K; k += 2 * s) mm[k] = r3dsimt::vmin2(mm[k], mm[k + s]);
-      }
-      pmin = group_umin<G>(r3dsimt::umin(mm[0] & 0xFFFFu, mm[0] >> 16));
-      uint32_t s[K];
-      if constexpr (MODE == kFirst) {
-        if (on) {
-#pragma unroll
-          for (int u = 0; u < U; ++u)
-            if (uvalid[u])
-              r3dsimt::st_stream(reinterpret_cast<uint4*>(s_out + 8 * u),
-                                 make_uint4(out[4 * u], out[4 * u + 1], out[4 * u + 2], out[4 * u + 3]));
-        }
-      } else if constexpr (MODE == kTerm) {
-        if (on) {
-          if constexpr (kVec) {
-#pragma unroll
-            for (int v = 0; v < NV; ++v)
-              if (uvalid[2 * v])
-                r3dsimt::st_stream(reinterpret_cast<uint4*>(t_out + 16 * v),
-                                   make_uint4(r3dsimt::perm(tr[8 * v], tr[8 * v + 1], 0x6420u),
-                                              r3dsimt::perm(tr[8 * v + 2], tr[8 * v + 3], 0x6420u),
-                                              r3dsimt::perm(tr[8 * v + 4], tr[8 * v + 5], 0x6420u),
-                                              r3dsimt::perm(tr[8 * v + 6], tr[8 * v + 7], 0x6420u)));
+        for (int v = 0; v < NV; ++v) {
+          if (!uvalid[v]) continue;
+          const uint32_t* o = out + 8 * v;
+          if constexpr (MODE == kTerm) {
+            r3dsimt::st_stream(reinterpret_cast<uint4*>(t_out + 16 * v), pack_unit(tr + 8 * v));
           } else {
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-              if (uvalid[u])
-                r3dsimt::st_stream8(reinterpret_cast<uint2*>(t_out + 8 * u),
-                                    make_uint2(r3dsimt::perm(tr[4 * u], tr[4 * u + 1], 0x6420u),
-                                               r3dsimt::perm(tr[4 * u + 2], tr[4 * u + 3], 0x6420u)));
-          }
-        }
-      } else if constexpr (MODE == kLastTerm) {
-        // S = L_8 + 7 C + sum of the seven byte terms (no halfword overflows).
-#pragma unroll
-        for (int k = 0; k < K; ++k) s[k] = out[k] + 7u * c2[k];
-        const unsigned char* stt = ring_term + q * Ring::kStageBytes;
-#pragma unroll
-        for (int r = 0; r < kTermArrays; ++r) {
-          uint2 tw[U];
-          if constexpr (kVec) {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-              const uint4 w4 = uvalid[2 * v] ? *reinterpret_cast<const uint4*>(stt + r * CPW * Ring::ND + 16 * v)
-                                             : make_uint4(0, 0, 0, 0);
-              tw[2 * v] = make_uint2(w4.x, w4.y);
-              tw[2 * v + 1] = make_uint2(w4.z, w4.w);
+            uint4 a = make_uint4(o[0], o[1], o[2], o[3]), b = make_uint4(o[4], o[5], o[6], o[7]);
+            if constexpr (MODE == kAccumulate) {
+              const uint4* ss = reinterpret_cast<const uint4*>(ring_sum + q * Ring::kStageBytes + 32 * v);
+              const uint4 x = ss[0], y = ss[1];
+              a = make_uint4(add2(x.x, a.x, no_carry), add2(x.y, a.y, no_carry), add2(x.z, a.z, no_carry),
+                             add2(x.w, a.w, no_carry));
+              b = make_uint4(add2(y.x, b.x, no_carry), add2(y.y, b.y, no_carry), add2(y.z, b.z, no_carry),
+                             add2(y.w, b.w, no_carry));
             }
-          } else {
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-              tw[u] = uvalid[u] ? *reinterpret_cast<const uint2*>(stt + r * CPW * Ring::ND + 8 * u) : make_uint2(0, 0);
-          }
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            s[4 * u + 0] = fma_add(r3dsimt::perm(tw[u].x, 0u, 0x4140u), one, s[4 * u + 0]);
-            s[4 * u + 1] = fma_add(r3dsimt::perm(tw[u].x, 0u, 0x4342u), one, s[4 * u + 1]);
-            s[4 * u + 2] = fma_add(r3dsimt::perm(tw[u].y, 0u, 0x4140u), one, s[4 * u + 2]);
-            s[4 * u + 3] = fma_add(r3dsimt::perm(tw[u].y, 0u, 0x4342u), one, s[4 * u + 3]);
-          }
-        }
-      } else {
-        const unsigned char* ss = ring_sum + q * Ring::kStageBytes;
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const uint4 sraw = uvalid[u] ? *reinterpret_cast<const uint4*>(ss + 16 * u) : make_uint4(0, 0, 0, 0);
-          s[4 * u + 0] = add2(sraw.x, out[4 * u + 0], no_carry);
-          s[4 * u + 1] = add2(sraw.y, out[4 * u + 1], no_carry);
-          s[4 * u + 2] = add2(sraw.z, out[4 * u + 2], no_carry);
-          s[4 * u + 3] = add2(sraw.w, out[4 * u + 3], no_carry);
-        }
-        if constexpr (MODE == kAccumulate) {
-          if (on) {
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-              if (uvalid[u])
-                r3dsimt::st_stream(reinterpret_cast<uint4*>(s_out + 8 * u),
-                                   make_uint4(s[4 * u], s[4 * u + 1], s[4 * u + 2], s[4 * u + 3]));
+            r3dsimt::st_stream(reinterpret_cast<uint4*>(s_out + 16 * v), a);
+            r3dsimt::st_stream(reinterpret_cast<uint4*>(s_out + 16 * v + 8), b);
           }
         }
       }
-      if constexpr (kWta) {
-        // Winner-takes-all over the total sums (sgm_kernels.cpp:332-358):
-        // the first minimum, the second best outside +-1, and S at kb -+ 1.
-        // Labels of units past nd count as 0xFFFF (they follow every valid
-        // label, so they never come first among equal minima); with byte
-        // terms their sum is the sentinel 0x7FFF, above every valid S (at
-        // most 8 (255 + 255)), which serves as well.
-        uint32_t sv[K];
-#pragma unroll
-        for (int k = 0; k < K; ++k) sv[k] = (MODE == kLastTerm || uvalid[k / 4]) ? s[k] : 0xFFFFFFFFu;
-        // The lane's minimum and its first label, as one key S << 16 | label
-        // whose minimum over the lane group is (bcost, kb).
-        uint32_t mv = sv[0];
-#pragma unroll
-        for (int k = 1; k < K; ++k) mv = r3dsimt::vmin2(mv, sv[k]);
-        const uint32_t lmin = r3dsimt::umin(mv & 0xFFFFu, mv >> 16);
-        // Per word min(S - lmin, 1) is 0 in the halves at the minimum (every
-        // half is >= lmin, so the subtraction borrows nothing).
-        const uint32_t l2 = lmin * 0x10001u;
-        uint32_t miss = 0;
-#pragma unroll
-        for (int k = 0; k < K; ++k) miss |= r3dsimt::vmin2(sv[k] - l2, 0x00010001u) << k;
-        const uint32_t hit = ~miss & (((1u << K) - 1u) * 0x10001u);
-        const uint32_t he = hit & 0xFFFFu, ho = hit >> 16;
-        const uint32_t fe = he != 0 ? static_cast<uint32_t>(2 * (r3dsimt::ffs(he) - 1)) : 0xFFFFu;
-        const uint32_t fo = ho != 0 ? static_cast<uint32_t>(2 * (r3dsimt::ffs(ho) - 1) + 1) : 0xFFFFu;
-        const uint32_t key = group_umin<G>((lmin << 16) | (r3dsimt::umin(fe, fo) + static_cast<uint32_t>(e0)));
-        const uint32_t bcost = key >> 16;
-        const int kb = static_cast<int>(key & 0xFFFFu);
-        // The second best outside kb -+ 1. Label kb - 1 lies in the lane's
-        // word wa = (kb - 1 - e0) >> 1 (arithmetic shift; out of [0, K) in
-        // other lanes): its high half only when kb - 1 - e0 is odd, then kb and
-        // kb + 1 fill word wa + 1; its both halves when even, then kb + 1 is the
-        // low half of word wa + 1.
-        const int wo = kb - 1 - e0;
-        const int wa = wo >> 1;
-        const uint32_t mask_a = (wo & 1) ? 0xFFFF0000u : 0xFFFFFFFFu;
-        const uint32_t mask_b = (wo & 1) ? 0xFFFFFFFFu : 0x0000FFFFu;
-        uint32_t sec2 = 0xFFFFFFFFu;
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-          const uint32_t m = (k == wa ? mask_a : 0u) | (k == wa + 1 ? mask_b : 0u);
-          sec2 = r3dsimt::vmin2(sec2, sv[k] | m);
-        }
-        const uint32_t sec = group_umin<G>(r3dsimt::umin(sec2 & 0xFFFFu, sec2 >> 16));
-        const int km = kb > 0 ? kb - 1 : 0, kp = kb + 1 < nd ? kb + 1 : nd - 1;
-        const int base_lane = gi * G;
-        uint32_t vm = pick<K>(s, (km % (2 * K)) >> 1);
-        uint32_t vp = pick<K>(s, (kp % (2 * K)) >> 1);
-        vm = r3dsimt::shfl(vm, (base_lane + km / (2 * K)) & 31);
-        vp = r3dsimt::shfl(vp, (base_lane + kp / (2 * K)) & 31);
-        const uint32_t sm = (km & 1) ? (vm >> 16) : (vm & 0xFFFFu);
-        const uint32_t sp = (kp & 1) ? (vp >> 16) : (vp & 0xFFFFu);
-        if (on) {
-          if (t == 0)
-            info[px_out] = make_int4(static_cast<int>(static_cast<uint32_t>(kb) | (bcost << 16)),
-                                     static_cast<int>(sec | (sm << 16)), static_cast<int>(sp), 0);
-          if (job.volume != nullptr) {
-            uint16_t* vb = job.volume + (static_cast<int64_t>(y) * w + x) * nd + e0;
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-              if (uvalid[u])
-                *reinterpret_cast<uint4*>(vb + 8 * u) = make_uint4(s[4 * u], s[4 * u + 1], s[4 * u + 2], s[4 * u + 3]);
-          }
-          if (m.diagonal_lr) {
-            // Right-view WTA along the diagonal (sgm_kernels.cpp:349-356): the
-            // smallest (S, x) key per right column.
-            const RowInterval lv = m.bv[job.y0 + y];
-            const int bx = job.x0 + x;
-            if (bx >= lv.first && bx <= lv.last) {
-              uint32_t* keys = rkeys + job.rk_off + static_cast<int64_t>(y) * (w + nd);
-              const int b0 = x + nd - 1;
-#pragma unroll
-              for (int k = 0; k < K; ++k) {
-                if (uvalid[k / 4]) {
-                  const int e = e0 + 2 * k;
-                  atomicMin(keys + (b0 - e), ((s[k] & 0xFFFFu) << 16) | static_cast<uint32_t>(x));
-                  atomicMin(keys + (b0 - e - 1), (s[k] & 0xFFFF0000u) | static_cast<uint32_t>(x));
-                }
-              }
-            }
-          }
-        }
-      }
-      (void)s;
 #pragma unroll
       for (int k = 0; k < K; ++k) prev[k] = out[k];
-      if constexpr (MODE == kFirst || MODE == kAccumulate) s_out += dcell;
       if constexpr (MODE == kTerm) t_out += dcell;
-      if constexpr (kWta) {
-        px_out += dpx;
-        x += dx;
-        y += dy;
-      }
+      else s_out += dcell;
     };
     for (int i0 = 0; i0 < maxlen; i0 += NS) {
 #pragma unroll
@@ -749,14 +565,14 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN((PathRing<G, K, MODE>::kThreads), (PathRin
 
 // ---------------------------------------------------------------- acceptance
 // stereo_matcher.cpp:474-523: validity, the rejection of a minimum on the edge
-// of a reduced range (:501-503), the diagonal left-right check (`shift` is the
-// row's key offset), uniqueness, subpixel fit and confidence of one pixel.
+// of a reduced range (:501-503), the diagonal left-right check (`keys` are the
+// row's right-view keys, `shift` their offset), uniqueness, subpixel fit and confidence of one pixel.
 struct Winner {
   int best;                    // label of the first minimum
   uint32_t bcost, sec, sm, sp;  // S there, second best, S at best -+ 1
 };
 R3D_DEVICE void accept_pixel(const SgmMatch& m, const SgmPathJob& job, int x, int y, int lo, int num, const Winner& v,
-                             const uint32_t* rkeys, int shift, float& d, float& cf) {
+                             const uint32_t* keys, int shift, float& d, float& cf) {
   const int bx = job.x0 + x, by = job.y0 + y;
   const RowInterval rv = m.pv[by];
   const int jb = v.best - lo;
@@ -764,7 +580,7 @@ R3D_DEVICE void accept_pixel(const SgmMatch& m, const SgmPathJob& job, int x, in
   bool ok = xr >= rv.first && xr <= rv.last;
   if ((jb == 0 && lo > 0) || (jb == num - 1 && lo + num < m.nd)) ok = false;
   if (ok && m.diagonal_lr) {
-    const uint32_t key = rkeys[job.rk_off + static_cast<int64_t>(y) * (job.w + m.nd) + (x - v.best + shift)];
+    const uint32_t key = keys[x - v.best + shift];
     const int rb = key == 0xFFFFFFFFu ? 0xFFFF : static_cast<int>(key & 0xFFFFu) - x + v.best;
     const int diff = rb - v.best;
     if ((diff < 0 ? -diff : diff) > m.lr_max_diff) ok = false;
@@ -791,37 +607,165 @@ R3D_DEVICE Winner unpack_winner(int4 in) {
                 static_cast<uint32_t>(in.y) >> 16, static_cast<uint32_t>(in.z)};
 }
 
-// Full range: lo = 0, num = nd for every pixel.
+
+// ---------------------------------------------------------------- winners
+// v[j] for a runtime j in [0, 8): selects on the bits of j (a register array
+// cannot be indexed at run time without local memory).
+R3D_DEVICE uint32_t pick8(const uint32_t (&v)[8], int j) {
+  const bool b0 = (j & 1) != 0, b1 = (j & 2) != 0, b2 = (j & 4) != 0;
+  const uint32_t a = b0 ? v[1] : v[0], b = b0 ? v[3] : v[2], c = b0 ? v[5] : v[4], d = b0 ? v[7] : v[6];
+  const uint32_t e = b1 ? b : a, f = b1 ? d : c;
+  return b2 ? f : e;
+}
+R3D_DEVICE uint32_t group_min_rt(uint32_t v, int g) {
+  for (int o = g >> 1; o > 0; o >>= 1) v = r3dsimt::umin(v, r3dsimt::shfl_xor(v, o));
+  return v;
+}
+
+// Full range (lo = 0, num = nd): total sums, winner-takes-all
+// (sgm_kernels.cpp:332-358: the first minimum, the second best outside +-1, S
+// at kb -+ 1) and acceptance of every pixel of a tile row, one warp per row. A
+// pixel's labels are spread over g lanes, one unit of 16 each (NU units for
+// more than 512 labels), 32 / g pixels at a time; every 32 pixels the lanes
+// take one pixel each for the acceptance.
+//
+// The sums form here and not in an eighth path pass: a pixel's nine byte
+// planes are independent of its neighbours', so the reads are wide, coalesced
+// and as many as the memory system takes (the path pass kept two pixels of
+// eight planes in flight per chain, 4.3 TB/s on a large pair and latency-bound
+// on a small one), and all eight directions run as one launch.
+//
+// The right-view winners of the diagonal check (sgm_kernels.cpp:349-356: the
+// smallest S << 16 | x per right column) live in shared memory for the row:
+// one shared-memory atomic per cell where the path pass had a global one.
+template <bool TERMS, int NU>
 R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
-    sgm_path_accept_kernel(const SgmMatch* R3D_RESTRICT matches, const SgmPathJob* R3D_RESTRICT jobs, int njobs,
-                           int64_t pixels, const int4* R3D_RESTRICT info, const uint32_t* R3D_RESTRICT rkeys) {
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < pixels; i += stride) {
-    const int j = find_job(jobs, njobs, i, [](const SgmPathJob& q) { return q.px_off; });
+    sgm_path_wta_kernel(const SgmMatch* R3D_RESTRICT matches, const SgmPathJob* R3D_RESTRICT jobs, int njobs,
+                        int64_t rows, const uint8_t* R3D_RESTRICT cost, const uint16_t* R3D_RESTRICT sum,
+                        const uint8_t* R3D_RESTRICT terms, int64_t tstride, int4* info, int key_words) {
+  R3D_DYNAMIC_SMEM(smem);
+  const int lane = static_cast<int>(threadIdx.x & 31u), warp = static_cast<int>(threadIdx.x >> 5);
+  const int wpb = static_cast<int>(blockDim.x) >> 5;
+  const int64_t nwarps = static_cast<int64_t>(gridDim.x) * wpb;
+  int4* const winners = reinterpret_cast<int4*>(smem) + warp * 32;
+  uint32_t* const keys = reinterpret_cast<uint32_t*>(smem + static_cast<size_t>(wpb) * 512) +
+                         static_cast<size_t>(warp) * key_words;
+  for (int64_t r = static_cast<int64_t>(blockIdx.x) * wpb + warp; r < rows; r += nwarps) {
+    const int j = find_job(jobs, njobs, r, [](const SgmPathJob& q) { return q.row_off; });
     const SgmPathJob& job = jobs[j];
     const SgmMatch& m = matches[job.match];
-    const int nd = m.nd, w = job.w;
-    const int p = static_cast<int>(i - job.px_off);
-    const int y = p / w, x = p - (p / w) * w;
+    const int nd = m.nd, w = job.w, nu = nd >> 4;
+    const int y = static_cast<int>(r - job.row_off);
+    const int64_t row_px = static_cast<int64_t>(y) * w;
     const RowInterval lv = m.bv[job.y0 + y];
-    float d = kInfF, cf = 0.0F;
-    if (job.x0 + x >= lv.first && job.x0 + x <= lv.last)
-      accept_pixel(m, job, x, y, 0, nd, unpack_winner(info[i]), rkeys, nd - 1, d, cf);
-    job.disp[p] = d;
-    if (job.conf != nullptr) job.conf[p] = cf;
-    if (p == 0) *job.cells = static_cast<unsigned long long>(w) * static_cast<unsigned long long>(job.h) * nd;
+    const bool diag = m.diagonal_lr != 0;
+    int g = 1;
+    while (g < nu && g < 32) g <<= 1;
+    const int per = 32 / g, gi = lane / g, t = lane & (g - 1);
+    const int64_t cell0 = job.cell_off + row_px * nd;
+    if (diag) {
+      for (int k = lane; k < w + nd; k += 32) keys[k] = 0xFFFFFFFFu;
+      r3dsimt::syncwarp();
+    }
+    if (y == 0 && lane == 0)
+      *job.cells = static_cast<unsigned long long>(w) * static_cast<unsigned long long>(job.h) * nd;
+    for (int xb = 0; xb < w; xb += 32) {
+      for (int s = 0; s < g && xb + s * per < w; ++s) {
+        const int x = xb + s * per + gi;
+        const bool inside = x < w && job.x0 + x >= lv.first && job.x0 + x <= lv.last;
+        const bool need = inside || (x < w && job.volume != nullptr);
+        const int64_t cell = cell0 + static_cast<int64_t>(x) * nd;
+        uint32_t wv[NU][8];
+        uint32_t kmin = 0xFFFFFFFFu;
+#pragma unroll
+        for (int n = 0; n < NU; ++n) {
+          const int u = t + 32 * n;
+          if (need && u < nu) {
+            sum_unit<TERMS>(cost + cell, terms + cell, tstride, sum + cell, u, wv[n]);
+            const uint32_t e = static_cast<uint32_t>(16 * u);
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              kmin = r3dsimt::umin(kmin, r3dsimt::umin((wv[n][k] << 16) | (e + k), (wv[n][k] & 0xFFFF0000u) | (e + k + 8)));
+            if (job.volume != nullptr) store_unit(job.volume + (row_px + x) * nd + 16 * u, wv[n]);
+          } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) wv[n][k] = 0xFFFFFFFFu;
+          }
+        }
+        kmin = group_min_rt(kmin, g);
+        const int kb = static_cast<int>(kmin & 0xFFFFu);
+        uint32_t sec2 = 0xFFFFFFFFu;
+#pragma unroll
+        for (int n = 0; n < NU; ++n) {
+          // Bit l: label l of the unit lies within kb -+ 1; its low and high
+          // byte in the two halves line up with the halves of word k >> k.
+          const int rel = kb - 1 - 16 * (t + 32 * n);
+          const uint32_t ex = rel >= 16 || rel < -2 ? 0u : (rel >= 0 ? 7u << rel : 7u >> -rel);
+          const uint32_t ex2 = (ex & 0xFFu) | ((ex & 0xFF00u) << 8);
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            sec2 = r3dsimt::vmin2(sec2, wv[n][k] | (((ex2 >> k) & 0x00010001u) * 0xFFFFu));
+        }
+        const uint32_t sec = group_min_rt(r3dsimt::umin(sec2 & 0xFFFFu, sec2 >> 16), g);
+        const int km = kb > 0 ? kb - 1 : 0, kp = kb + 1 < nd ? kb + 1 : nd - 1;
+        uint32_t vm = pick8(wv[0], km & 7), vp = pick8(wv[0], kp & 7);
+        if constexpr (NU > 1) {
+          if (km >= 512) vm = pick8(wv[NU - 1], km & 7);
+          if (kp >= 512) vp = pick8(wv[NU - 1], kp & 7);
+        }
+        vm = r3dsimt::shfl(vm, (gi * g + ((km >> 4) & (g - 1))) & 31);
+        vp = r3dsimt::shfl(vp, (gi * g + ((kp >> 4) & (g - 1))) & 31);
+        const Winner win{kb, kmin >> 16, sec, (km & 8) ? vm >> 16 : vm & 0xFFFFu, (kp & 8) ? vp >> 16 : vp & 0xFFFFu};
+        if (t == 0) winners[s * per + gi] = pack_winner(win);
+        if (diag && inside) {
+#pragma unroll
+          for (int n = 0; n < NU; ++n) {
+            const int u = t + 32 * n;
+            if (u < nu) {
+              uint32_t* kr = keys + x + nd - 1 - 16 * u;
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                atomicMin(kr - k, (wv[n][k] << 16) | static_cast<uint32_t>(x));
+                atomicMin(kr - k - 8, (wv[n][k] & 0xFFFF0000u) | static_cast<uint32_t>(x));
+              }
+            }
+          }
+        }
+      }
+      r3dsimt::syncwarp();
+      const int x = xb + lane;
+      if (x < w) {
+        const int64_t p = row_px + x;
+        if (diag) {
+          info[job.px_off + p] = winners[lane];
+        } else {
+          float d = kInfF, cf = 0.0F;
+          if (job.x0 + x >= lv.first && job.x0 + x <= lv.last)
+            accept_pixel(m, job, x, y, 0, nd, unpack_winner(winners[lane]), nullptr, 0, d, cf);
+          job.disp[p] = d;
+          if (job.conf != nullptr) job.conf[p] = cf;
+        }
+      }
+      r3dsimt::syncwarp();
+    }
+    if (diag) {  // the row's keys are complete
+      for (int x = lane; x < w; x += 32) {
+        const int64_t p = row_px + x;
+        float d = kInfF, cf = 0.0F;
+        if (job.x0 + x >= lv.first && job.x0 + x <= lv.last)
+          accept_pixel(m, job, x, y, 0, nd, unpack_winner(info[job.px_off + p]), keys, nd - 1, d, cf);
+        job.disp[p] = d;
+        if (job.conf != nullptr) job.conf[p] = cf;
+      }
+      r3dsimt::syncwarp();
+    }
   }
 }
 
 // ================================================================ ranged tiles
 // Per-pixel label ranges (lo, num; num a multiple of 16): the same passes on
 // costs, terms and sums packed per tile, pixel after pixel, in units of 16
-// labels. Within a unit the labels are interleaved so that a 32-bit word of
-// the passes holds labels k and k + 8: the neighbours d -+ 1 of word k are
-// then words k -+ 1, without byte permutes. Byte planes (costs, terms) store
-// the bytes of word j = 0..3 of a unit as labels 2 j, 2 j + 1, 2 j + 8, 2 j + 9
-// (one mask or permute unpacks a word, one multiply-add packs two); sums
-// store word k = 0..7 as the halves of labels k and k + 8.
+// labels.
 
 // Record of a pixel: x = cell offset / 16 within its tile | min(units, 31)
 // << 27 (a tile has fewer than 2^31 labels; 31 stands for 31 or more, looked
@@ -944,11 +888,10 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
           // Census XOR packed separately (each byte at most 32, no carries).
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            const int l[4] = {2 * k, 2 * k + 1, 2 * k + 8, 2 * k + 9};
             uint32_t a = 0, b = 0;
 #pragma unroll
             for (int i = 3; i >= 0; --i) {
-              const uint64_t d = cl ^ crow[xr0 - l[i]];
+              const uint64_t d = cl ^ crow[xr0 - unit_label(k, i)];
               a = a * 256u + static_cast<uint32_t>(r3dsimt::popc(static_cast<uint32_t>(d)));
               b = b * 256u + static_cast<uint32_t>(r3dsimt::popc(static_cast<uint32_t>(d >> 32)));
             }
@@ -1137,30 +1080,14 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
       const unsigned char* src = data + st * R::kStageBytes;
       uint32_t c2[K], tr[K];
 #pragma unroll
-      for (int u = 0; u < UF; ++u) {
-        const uint4 v = *reinterpret_cast<const uint4*>(src + u * 512);
-        const uint32_t cw[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          c2[8 * u + 2 * k] = cw[k] & 0x00FF00FFu;
-          c2[8 * u + 2 * k + 1] = r3dsimt::perm(cw[k], 0u, 0x4341u);
-        }
-      }
+      for (int u = 0; u < UF; ++u) unpack_unit(*reinterpret_cast<const uint4*>(src + u * 512), c2 + 8 * u);
 #pragma unroll
       for (int k = 0; k < K; ++k) {
         tr[k] = fma_add(best[k], one, negmp);
         out[k] = fma_add(tr[k], one, c2[k]);
         if (k >= 8 && !upper) out[k] = kSent2;
       }
-      {
-        constexpr int N3 = (K + 2) / 3;
-        uint32_t t3[N3];
-#pragma unroll
-        for (int k = 0; k < N3; ++k)
-          t3[k] = r3dsimt::vmin3(out[3 * k], out[3 * k + 1 < K ? 3 * k + 1 : 3 * k], out[3 * k + 2 < K ? 3 * k + 2 : 3 * k]);
-#pragma unroll
-        for (int k = 0; k < N3; k += 2) pm = r3dsimt::vmin3(pm, t3[k], t3[k + 1 < N3 ? k + 1 : k]);
-      }
+      pm = r3dsimt::vmin2(pm, min_words<K>(out));
       if (!on) return;
 #pragma unroll
       for (int u = 0; u < UF; ++u) {
@@ -1168,9 +1095,7 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
         const int64_t off = static_cast<int64_t>(at + u) * 16;
         const int q = 8 * u;
         if constexpr (MODE == kTerm) {
-          r3dsimt::st_stream(reinterpret_cast<uint4*>(tout + off),
-                             make_uint4(tr[q] + 256u * tr[q + 1], tr[q + 2] + 256u * tr[q + 3],
-                                        tr[q + 4] + 256u * tr[q + 5], tr[q + 6] + 256u * tr[q + 7]));
+          r3dsimt::st_stream(reinterpret_cast<uint4*>(tout + off), pack_unit(tr + q));
         } else {
           uint32_t v[8];
 #pragma unroll
@@ -1281,18 +1206,7 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
         uint32_t cl[K];
 #pragma unroll
         for (int k = 0; k < K; ++k) cl[k] = r3dsimt::vmin2(prev[k], pen2);
-#pragma unroll
-        for (int u = 0; u < UF; ++u) {
-          // Words -1 and 8 of the unit: labels (16 u - 1, 16 u + 7) and (16 u + 8, 16 u + 16).
-          uint32_t s[10];
-          s[0] = fma_add(r3dsimt::perm(u > 0 ? cl[8 * (u > 0 ? u - 1 : 0) + 7] : pen2, cl[8 * u + 7], 0x5432u), one, p1x2);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) s[1 + k] = fma_add(cl[8 * u + k], one, p1x2);
-          s[9] = fma_add(r3dsimt::perm(cl[8 * u], u + 1 < UF ? cl[8 * (u + 1 < UF ? u + 1 : 0)] : pen2, 0x5432u), one,
-                         p1x2);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) best[8 * u + k] = r3dsimt::vmin3(cl[8 * u + k], s[k], s[2 + k]);
-        }
+        best_terms<K>(cl, pen2, pen2, one, p1x2, best);
         finish(best, st, at, on, true);
         if (!fast_next) {
           make_clean();
@@ -1378,37 +1292,8 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
     const int64_t off = static_cast<int64_t>(rc.x & kRecOffset) * 16;
     const uint8_t* cp = cost + job.cell_off + off;
     const uint8_t* tp = terms + job.cell_off + off;
-    const uint4* sp4 = reinterpret_cast<const uint4*>(sum + job.cell_off + off);
-    // Word k of a unit holds labels k and k + 8.
-    auto unit = [&](int u, uint32_t (&wv)[8]) {
-      if constexpr (TERMS) {
-        uint4 t[1 + kRangedTerms];
-        t[0] = *reinterpret_cast<const uint4*>(cp + 16 * u);
-#pragma unroll
-        for (int r = 0; r < kRangedTerms; ++r)
-          t[1 + r] = r3dsimt::ld_stream(reinterpret_cast<const uint4*>(tp + r * tstride + 16 * u));
-#pragma unroll
-        for (int r = 0; r <= kRangedTerms; ++r) {
-          const uint32_t tw[4] = {t[r].x, t[r].y, t[r].z, t[r].w};
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const uint32_t a = tw[k] & 0x00FF00FFu, b = r3dsimt::perm(tw[k], 0u, 0x4341u);
-            wv[2 * k] = r == 0 ? 8u * a : wv[2 * k] + a;
-            wv[2 * k + 1] = r == 0 ? 8u * b : wv[2 * k + 1] + b;
-          }
-        }
-        return;
-      }
-      const uint4 a = sp4[2 * u], b = sp4[2 * u + 1];
-      wv[0] = a.x;
-      wv[1] = a.y;
-      wv[2] = a.z;
-      wv[3] = a.w;
-      wv[4] = b.x;
-      wv[5] = b.y;
-      wv[6] = b.z;
-      wv[7] = b.w;
-    };
+    const uint16_t* sp = sum + job.cell_off + off;
+    auto unit = [&](int u, uint32_t (&wv)[8]) { sum_unit<TERMS>(cp, tp, tstride, sp, u, wv); };
     uint32_t wv[8];
     uint32_t kmin = 0xFFFFFFFFu;
     for (int u = nu - 1; u >= 0; --u) {  // ends with unit 0 in wv: the only one of most pixels
@@ -1418,14 +1303,7 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
         const uint32_t e = static_cast<uint32_t>(16 * u + k);
         kmin = r3dsimt::umin(kmin, r3dsimt::umin((wv[k] << 16) | e, (wv[k] & 0xFFFF0000u) | (e + 8)));
       }
-      if (job.volume != nullptr) {
-        uint16_t* vol = job.volume + off + 16 * u;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          vol[k] = static_cast<uint16_t>(wv[k] & 0xFFFFu);
-          vol[k + 8] = static_cast<uint16_t>(wv[k] >> 16);
-        }
-      }
+      if (job.volume != nullptr) store_unit(job.volume + off + 16 * u, wv);
     }
     const int kb = static_cast<int>(kmin & 0xFFFFu);
     const int km = kb > 0 ? kb - 1 : 0;
@@ -1466,7 +1344,7 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
       continue;
     }
     float d = kInfF, cf = 0.0F;
-    if (inside) accept_pixel(m, job, x, y, lo, num, win, rkeys, 0, d, cf);
+    if (inside) accept_pixel(m, job, x, y, lo, num, win, nullptr, 0, d, cf);
     job.disp[p] = d;
     if (job.conf != nullptr) job.conf[p] = cf;
   }
@@ -1492,7 +1370,8 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
     if (job.x0 + x >= lv.first && job.x0 + x <= lv.last) {
       const uint2 rc = rec[i];
       accept_pixel(m, job, x, y, static_cast<int>(rc.y & 0xFFFFu), 16 * rec_units(rc, m, job, x, y),
-                   unpack_winner(info[i]), rkeys, rowshift[job.row_off + y], d, cf);
+                   unpack_winner(info[i]), rkeys + job.rk_off + static_cast<int64_t>(y) * (job.w + m.nd),
+                   rowshift[job.row_off + y], d, cf);
     }
     job.disp[p] = d;
     if (job.conf != nullptr) job.conf[p] = cf;
@@ -1500,12 +1379,14 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
 }
 
 // ---------------------------------------------------------------- launches
-// Pass order: the first pass writes the sums, the last takes the WTA.
+// The path directions; the long chains (rows, columns) before the diagonals, so
+// that a tile, and a launch, ends on short blocks.
 struct Pass {
   int cls, dx, dy;
 };
-constexpr Pass kPasses[8] = {{0, 1, 0},  {1, 0, 1},   {2, 1, 1},  {2, -1, 1},
-                             {1, 0, -1}, {2, -1, -1}, {2, 1, -1}, {0, -1, 0}};
+constexpr Pass kPasses[kMaxPasses] = {{0, 1, 0}, {0, -1, 0}, {1, 0, 1},   {1, 0, -1},
+                                      {2, 1, 1}, {2, -1, 1}, {2, -1, -1}, {2, 1, -1}};
+constexpr int kAllPasses[kMaxPasses] = {0, 1, 2, 3, 4, 5, 6, 7};
 
 template <class Kernel>
 int resident_grid(Kernel kernel, int sms, int64_t work_items, int per_block, size_t smem = 0,
@@ -1517,23 +1398,17 @@ int resident_grid(Kernel kernel, int sms, int64_t work_items, int per_block, siz
   return static_cast<int>(need < resident ? (need > 0 ? need : 1) : resident);
 }
 
-// Algorithmic HBM bytes of one pass over `cells` cells of `pixels` pixels:
-// costs read, sums read (not by the first pass) and written (not by the
-// full-range last pass, which writes the WTA records instead); byte terms:
-// one written per cell by passes 1..7, seven read by the last pass.
-uint64_t pass_bytes(int mode, bool ranged, const SgmPathSegment& g) {
-  const uint64_t c = static_cast<uint64_t>(g.cells), px = static_cast<uint64_t>(g.pixels);
-  if (mode == kFirst) return 3 * c;
-  if (mode == kTerm) return 2 * c;
-  if (mode == kLastTerm) return (1 + kTermArrays) * c + 16 * px;
-  if (mode == kLast && !ranged) return 3 * c + 16 * px;
-  return 5 * c;
+// Algorithmic HBM bytes of one pass over a segment's cells: costs read; terms
+// written; sums read (not by the first pass) and written.
+uint64_t pass_bytes(int mode, const SgmPathSegment& g) {
+  const uint64_t c = static_cast<uint64_t>(g.cells);
+  return (mode == kTerm ? 2 : (mode == kFirst ? 3 : 5)) * c;
 }
 
 template <int G, int K, int MODE, bool FULL = false>
 void launch_pass(const PassSet& ps, const SgmMatch* dm, const SgmPathJob* jobs, int njobs, const uint8_t* cost,
-                 uint16_t* sum, uint8_t* terms, int64_t tstride, int4* info, uint32_t* rkeys, const uint16_t* ints,
-                 int sms, cudaStream_t s, const SgmPathSegment& seg, const int* cancel) {
+                 uint16_t* sum, uint8_t* terms, int64_t tstride, const uint16_t* ints, int sms, cudaStream_t s,
+                 const SgmPathSegment& seg, const int* cancel) {
   const cudaEvent_t ev0 = profile_on() ? profile_mark(s) : nullptr;
   auto* k = sgm_path_kernel<G, K, MODE, FULL>;
   constexpr size_t smem = PathRing<G, K, MODE>::kBlockBytes;
@@ -1547,14 +1422,14 @@ void launch_pass(const PassSet& ps, const SgmMatch* dm, const SgmPathJob* jobs, 
   const int64_t nb = ps.total;
   constexpr int threads = PathRing<G, K, MODE>::kThreads;
   R3D_LAUNCH(k, dim3(resident_grid(k, sms, nb, threads / 32, smem, threads)), dim3(threads), smem, s, dm, jobs, njobs,
-             ps, cost, sum, terms, tstride, info, rkeys, ints, cancel);
+             ps, cost, sum, terms, tstride, ints, cancel);
   launched("sgm_path_kernel");
   if (ev0 != nullptr) {
     char shape[32];
     std::snprintf(shape, sizeof(shape), "%dx%d/mode%d", G, K, MODE);
     const uint64_t n = static_cast<uint64_t>(ps.n);
     profile_pass(ev0, profile_mark(s), "sgm_path_kernel", shape, n * static_cast<uint64_t>(seg.cells),
-                 n * static_cast<uint64_t>(seg.pixels), n * pass_bytes(MODE, false, seg));
+                 n * static_cast<uint64_t>(seg.pixels), n * pass_bytes(MODE, seg));
   }
 }
 
@@ -1578,41 +1453,27 @@ PassSet pass_set(const SgmPathSegment& g, const int* qs, int n, int* next) {
 
 template <int G, int K>
 void launch_passes(const SgmMatch* dm, const SgmPathJob* jobs, const SgmPathSegment& g, const uint8_t* cost,
-                   uint16_t* sum, uint8_t* terms, int64_t tstride, int4* info, uint32_t* rkeys, const uint16_t* ints,
-                   int sms, cudaStream_t s, const int* cancel, int* counters) {
-  for (int q = 0; q < 8; ++q)
+                   uint16_t* sum, uint8_t* terms, int64_t tstride, const uint16_t* ints, int sms, cudaStream_t s,
+                   const int* cancel, int* counters) {
+  for (int q = 0; q < kMaxPasses; ++q)
     if (g.blocks[kPasses[q].cls] <= 0) return;  // no pixels: every class has chains otherwise
   if (terms != nullptr) {
-    // The seven term passes in one launch, then the last pass, which finds
-    // all seven term arrays written.
-    const int qs[kTermArrays] = {0, 1, 2, 3, 4, 5, 6};
-    const int last = 7;
-    // Segments whose matches fill every label unit take the kernels without
-    // the per-unit validity selects.
-    if (g.full != 0) {
-      launch_pass<G, K, kTerm, true>(pass_set(g, qs, kTermArrays, counters), dm, jobs, g.count, cost, sum, terms, tstride, info,
-                                     rkeys, ints, sms, s, g, cancel);
-      launch_pass<G, K, kLastTerm, true>(pass_set(g, &last, 1, counters + 1), dm, jobs, g.count, cost, sum, terms, tstride, info,
-                                         rkeys, ints, sms, s, g, cancel);
-    } else {
-      launch_pass<G, K, kTerm>(pass_set(g, qs, kTermArrays, counters), dm, jobs, g.count, cost, sum, terms, tstride, info,
-                               rkeys, ints, sms, s, g, cancel);
-      launch_pass<G, K, kLastTerm>(pass_set(g, &last, 1, counters + 1), dm, jobs, g.count, cost, sum, terms, tstride, info, rkeys,
-                                   ints, sms, s, g, cancel);
-    }
+    // The eight term passes in one launch (they only read the costs and each
+    // writes its own term array). Segments whose matches fill every unit take
+    // the kernel without the per-unit validity selects.
+    const PassSet ps = pass_set(g, kAllPasses, kTermArrays, counters);
+    if (g.full != 0)
+      launch_pass<G, K, kTerm, true>(ps, dm, jobs, g.count, cost, sum, terms, tstride, ints, sms, s, g, cancel);
+    else
+      launch_pass<G, K, kTerm>(ps, dm, jobs, g.count, cost, sum, terms, tstride, ints, sms, s, g, cancel);
     return;
   }
-  for (int q = 0; q < 8; ++q) {
-    const PassSet ps = pass_set(g, &q, 1, counters + q);
+  for (int q = 0; q < kMaxPasses; ++q) {
+    const PassSet ps = pass_set(g, kAllPasses + q, 1, counters + q);
     if (q == 0)
-      launch_pass<G, K, kFirst>(ps, dm, jobs, g.count, cost, sum, terms, tstride, info, rkeys, ints, sms, s, g,
-                                cancel);
-    else if (q < 7)
-      launch_pass<G, K, kAccumulate>(ps, dm, jobs, g.count, cost, sum, terms, tstride, info, rkeys, ints, sms, s, g,
-                                     cancel);
+      launch_pass<G, K, kFirst>(ps, dm, jobs, g.count, cost, sum, terms, tstride, ints, sms, s, g, cancel);
     else
-      launch_pass<G, K, kLast>(ps, dm, jobs, g.count, cost, sum, terms, tstride, info, rkeys, ints, sms, s, g,
-                               cancel);
+      launch_pass<G, K, kAccumulate>(ps, dm, jobs, g.count, cost, sum, terms, tstride, ints, sms, s, g, cancel);
   }
 }
 
@@ -1620,19 +1481,15 @@ void launch_passes(const SgmMatch* dm, const SgmPathJob* jobs, const SgmPathSegm
 #define R3D_PATH_SHAPES(X) \
   X(1, 8)                  \
   X(2, 8)                  \
-  X(2, 12)                 \
-  X(2, 16)                 \
   X(4, 8)                  \
-  X(4, 12)                 \
-  X(4, 16)                 \
   X(8, 8)                  \
-  X(8, 12)                 \
-  X(8, 16)                 \
   X(16, 8)                 \
-  X(16, 12)                \
-  X(16, 16)                \
   X(32, 8)                 \
-  X(32, 12)
+  X(2, 16)                 \
+  X(4, 16)                 \
+  X(8, 16)                 \
+  X(16, 16)                \
+  X(32, 16)
 
 }  // namespace
 
@@ -1653,9 +1510,13 @@ bool path_shape_compiled(int g, int k) {
 
 SgmPathShape sgm_path_shape(int nd) {
   // A compiled shape from R3DGPU_PATH_SHAPE ("G,K": any label count it
-  // covers) or the tuning table (an entry for exactly this label count),
-  // else the narrowest row of 8 or 12 label pairs per lane, ties to fewer
-  // lanes per chain.
+  // covers) or the tuning table (an entry for exactly this label count), else
+  // 8 label pairs per lane up to 64 labels, 16 above, with the fewest lanes.
+  // Whole pair, 2048x1536 (1536x1152 for 384 labels): 64 labels 3.57 ms with 8
+  // pairs per lane, 3.65 with 16; 96: 5.54 and 5.38; 128: 5.85 and 5.76; 256:
+  // 11.35 and 10.21; 384: 13.01 and 10.89. 24 pairs per lane, which fit 48,
+  // 96, 192 and 384 labels without idle lanes, took 3.84, 5.78, 10.2 and 11.4
+  // (longer steps, fewer chains in flight).
   if (const char* e = std::getenv("R3DGPU_PATH_SHAPE")) {
     int g = 0, k = 0;
     if (std::sscanf(e, "%d,%d", &g, &k) == 2 && path_shape_compiled(g, k) && 2 * g * k >= nd) return {g, k};
@@ -1664,14 +1525,17 @@ SgmPathShape sgm_path_shape(int nd) {
   if (it != tuning().path.end() && path_shape_compiled(it->second.g, it->second.k) &&
       2 * it->second.g * it->second.k >= nd)
     return {it->second.g, it->second.k};
+  const int k_want = nd <= 64 ? 8 : 16;
   SgmPathShape best{0, 0};
   int best_nd = 1 << 30;
-#define R3D_SHAPE(g, k)                                       \
-  if (k != 16 && 2 * g * k >= nd && 2 * g * k < best_nd) { \
-    best = SgmPathShape{g, k};                                \
-    best_nd = 2 * g * k;                                      \
+#define R3D_SHAPE(g, k)                                              \
+  if (k == k_want && 2 * g * k >= nd && 2 * g * k < best_nd) { \
+    best = SgmPathShape{g, k};                                       \
+    best_nd = 2 * g * k;                                             \
   }
-  R3D_PATH_SHAPES(R3D_SHAPE)
+  if (nd <= kPathMaxLabels) {
+    R3D_PATH_SHAPES(R3D_SHAPE)
+  }
 #undef R3D_SHAPE
   return best;
 }
@@ -1686,10 +1550,10 @@ SgmPathBuffers sgm_path_buffers(int64_t cells, int64_t pixels, int64_t keys, boo
   b.terms = b.sum;
   o += terms ? static_cast<size_t>(kTermArrays) * static_cast<size_t>(b.term_stride)
              : align256(static_cast<size_t>(cells) * 2);
+  // Winners of a tile row until its right-view keys are complete: only for
+  // matches with the diagonal check.
   b.info = o;
-  o += align256(static_cast<size_t>(pixels) * 16);
-  b.rkeys = o;
-  o += align256(static_cast<size_t>(keys) * 4);
+  if (keys > 0) o += align256(static_cast<size_t>(pixels) * 16);
   // The tiles' base intensities, pixel after pixel, and 16 bytes more: the
   // pass kernels copy the aligned 4-byte word holding a pixel's intensity.
   b.ints = o;
@@ -1707,11 +1571,9 @@ void launch_sgm_path_wave(const SgmMatch* dm, const SgmPathWave& wave, int sms, 
   uint16_t* sum = reinterpret_cast<uint16_t*>(wave.buffer + B.sum);
   uint8_t* terms = wave.terms != 0 ? wave.buffer + B.terms : nullptr;
   int4* info = reinterpret_cast<int4*>(wave.buffer + B.info);
-  uint32_t* rkeys = reinterpret_cast<uint32_t*>(wave.buffer + B.rkeys);
   uint16_t* ints = reinterpret_cast<uint16_t*>(wave.buffer + B.ints);
   int* counters = reinterpret_cast<int*>(wave.buffer + B.counters);
   if (8 * wave.nsegs > kPathCounters) fail(R3DGPU_EINVAL, "stereo: too many path kernel shapes in a wave");
-  if (wave.keys > 0) R3D_CUDA(cudaMemsetAsync(rkeys, 0xFF, static_cast<size_t>(wave.keys) * 4, s));
   {
     constexpr size_t max_smem = static_cast<size_t>(kPathThreads / 32) * kCostStage * 8;
     static thread_local int configured[64] = {};
@@ -1735,7 +1597,7 @@ void launch_sgm_path_wave(const SgmMatch* dm, const SgmPathWave& wave, int sms, 
     bool done = false;
 #define R3D_SHAPE(gg, kk)                                                                                     \
   if (!done && g.shape.g_ == gg && g.shape.k_ == kk) {                                                        \
-    launch_passes<gg, kk>(dm, jobs, g, cost, sum, terms, B.term_stride, info, rkeys, ints, sms, s, wave.cancel, \
+    launch_passes<gg, kk>(dm, jobs, g, cost, sum, terms, B.term_stride, ints, sms, s, wave.cancel,            \
                           counters + 8 * q);                                                                  \
     done = true;                                                                                              \
   }
@@ -1743,9 +1605,18 @@ void launch_sgm_path_wave(const SgmMatch* dm, const SgmPathWave& wave, int sms, 
 #undef R3D_SHAPE
     if (!done) fail(R3DGPU_EINVAL, "stereo: bad path kernel shape");
   }
-  R3D_LAUNCH(sgm_path_accept_kernel, dim3(resident_grid(sgm_path_accept_kernel, sms, wave.pixels, kPathThreads)),
-             dim3(kPathThreads), 0, s, dm, wave.jobs, wave.njobs, wave.pixels, info, rkeys);
-  launched("sgm_path_accept_kernel");
+  bool wide = false;  // more than 512 labels: two units per lane
+  for (int q = 0; q < wave.nsegs; ++q) wide = wide || 2 * wave.segs[q].shape.g_ * wave.segs[q].shape.k_ > 512;
+  auto* wta = terms != nullptr ? (wide ? sgm_path_wta_kernel<true, 2> : sgm_path_wta_kernel<true, 1>)
+                               : (wide ? sgm_path_wta_kernel<false, 2> : sgm_path_wta_kernel<false, 1>);
+  // A row's right-view keys: tile width + labels, at most kCostStage + 1.
+  const int key_words = wave.keys > 0 ? kCostStage + 4 : 0;
+  const size_t smem = static_cast<size_t>(kPathThreads / 32) * (512 + 4 * static_cast<size_t>(key_words));
+  if (wave.keys > 0)
+    R3D_CUDA(cudaFuncSetAttribute(wta, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  R3D_LAUNCH(wta, dim3(resident_grid(wta, sms, wave.rows, kPathThreads / 32, smem)), dim3(kPathThreads), smem, s, dm,
+             wave.jobs, wave.njobs, wave.rows, cost, sum, terms, B.term_stride, info, key_words);
+  launched("sgm_path_wta_kernel");
 }
 
 // ---------------------------------------------------------------- ranged launches
@@ -1780,13 +1651,9 @@ void launch_ranged_pass(const PassSet& ps, const SgmMatch* dm, const SgmPathJob*
     // Per pixel and pass also the 8-byte record (range and cell offset).
     const uint64_t n = static_cast<uint64_t>(ps.n);
     profile_pass(ev0, profile_mark(s), "sgm_path_ranged_kernel", shape, n * static_cast<uint64_t>(seg.cells),
-                 n * static_cast<uint64_t>(seg.pixels), n * (pass_bytes(MODE, true, seg) + 8 * static_cast<uint64_t>(seg.pixels)));
+                 n * static_cast<uint64_t>(seg.pixels), n * (pass_bytes(MODE, seg) + 8 * static_cast<uint64_t>(seg.pixels)));
   }
 }
-
-// The ranged passes' order: the long chains (rows, columns) before the
-// diagonals of the same tile, so that a launch ends on short blocks.
-constexpr int kRangedOrder[8] = {0, 7, 1, 4, 2, 3, 5, 6};
 
 template <int K>
 void launch_ranged_passes(const SgmMatch* dm, const SgmPathJob* jobs, const SgmPathSegment& g, const uint2* rec,
@@ -1796,12 +1663,12 @@ void launch_ranged_passes(const SgmMatch* dm, const SgmPathJob* jobs, const SgmP
     if (g.blocks[kPasses[q].cls] <= 0) return;  // no pixels: every class has chains otherwise
   if (terms != nullptr) {
     // Byte terms: all eight directions in one launch.
-    launch_ranged_pass<K, kTerm>(pass_set(g, kRangedOrder, kRangedTerms, counters), dm, jobs, g.count, rec, cost, sum,
+    launch_ranged_pass<K, kTerm>(pass_set(g, kAllPasses, kTermArrays, counters), dm, jobs, g.count, rec, cost, sum,
                                  terms, tstride, ovf, ovf_words, sms, s, g, cancel);
     return;
   }
   for (int q = 0; q < 8; ++q) {
-    const PassSet ps = pass_set(g, kRangedOrder + q, 1, counters + q);
+    const PassSet ps = pass_set(g, kAllPasses + q, 1, counters + q);
     if (q == 0)
       launch_ranged_pass<K, kFirst>(ps, dm, jobs, g.count, rec, cost, sum, terms, tstride, ovf, ovf_words, sms, s, g,
                                     cancel);
@@ -1832,7 +1699,7 @@ SgmPathBuffers sgm_path_ranged_buffers(int64_t cells, int64_t pixels, int64_t ke
   // Eight byte-term arrays, or the u16 sums.
   b.sum = b.terms = o;
   b.term_stride = terms ? static_cast<int64_t>(align256(static_cast<size_t>(cells))) : 0;
-  o += terms ? static_cast<size_t>(kRangedTerms) * static_cast<size_t>(b.term_stride)
+  o += terms ? static_cast<size_t>(kTermArrays) * static_cast<size_t>(b.term_stride)
              : align256(static_cast<size_t>(cells) * 2);
   // Winners and right-view keys: only for matches with the diagonal check.
   b.info = o;
