@@ -19,32 +19,54 @@ R3D_DEVICE int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi
 // ------------------------------------------------------------------ census
 // 9x7 Census (census.cpp:20-35, 104-113): the 62 neighbours in raster order,
 // first in bit 61, bit = neighbour < centre; borders replicated.
+//
+// Two pixels per thread: their 10 x 7 neighbourhood comes from shared memory as
+// 5 words a row (35 loads for two pixels instead of 126), and a comparison is
+// one subtraction whose sign a funnel shift appends to the code. Bound by the
+// ALU pipe (about 160 operations a pixel against 10 bytes).
 constexpr int kCBX = 32, kCBY = 8;
+constexpr int kCTW = 2 * kCBX + 8;  // tile columns (x0 - 4 .. x0 + 2 kCBX + 3)
 
 R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kCBX* kCBY) census_kernel(const uint16_t* __restrict__ img, int64_t stride, int w,
                                                            int h, uint64_t* __restrict__ out, int64_t ostride) {
   R3D_DYNAMIC_SMEM(smem_raw);
-  auto tile = reinterpret_cast<uint16_t(*)[kCBX + 8]>(smem_raw);
-  const int x0 = blockIdx.x * kCBX, y0 = blockIdx.y * kCBY;
-  for (int i = threadIdx.y * kCBX + threadIdx.x; i < (kCBY + 6) * (kCBX + 8); i += kCBX * kCBY) {
-    const int ty = i / (kCBX + 8), tx = i % (kCBX + 8);
+  auto tile = reinterpret_cast<uint16_t(*)[kCTW]>(smem_raw);
+  const int x0 = blockIdx.x * (2 * kCBX), y0 = blockIdx.y * kCBY;
+  for (int i = threadIdx.y * kCBX + threadIdx.x; i < (kCBY + 6) * kCTW; i += kCBX * kCBY) {
+    const int ty = i / kCTW, tx = i % kCTW;
     const int gx = clampi(x0 + tx - 4, 0, w - 1), gy = clampi(y0 + ty - 3, 0, h - 1);
     tile[ty][tx] = img[static_cast<int64_t>(gy) * stride + gx];
   }
   r3dsimt::syncthreads();
-  const int x = x0 + threadIdx.x, y = y0 + threadIdx.y;
+  const int lx = 2 * static_cast<int>(threadIdx.x), ly = static_cast<int>(threadIdx.y);
+  const int x = x0 + lx, y = y0 + ly;
   if (x >= w || y >= h) return;
-  const uint16_t c = tile[threadIdx.y + 3][threadIdx.x + 4];
-  uint64_t bits = 0;
+  // Centres of the two pixels (columns lx + 4 and lx + 5 of the tile).
+  const uint32_t cw = *reinterpret_cast<const uint32_t*>(&tile[ly + 3][lx + 4]);
+  const uint32_t ca = cw & 0xFFFFu, cb = cw >> 16;
+  uint32_t a[2] = {0, 0}, b[2] = {0, 0};  // codes: bits 61..32, bits 31..0
+  int n = 0;
 #pragma unroll
   for (int j = 0; j < 7; ++j) {
+    uint32_t v[10];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      const uint32_t t = *reinterpret_cast<const uint32_t*>(&tile[ly + j][lx + 2 * k]);
+      v[2 * k] = t & 0xFFFFu;
+      v[2 * k + 1] = t >> 16;
+    }
 #pragma unroll
     for (int i = 0; i < 9; ++i) {
       if (j == 3 && i == 4) continue;
-      bits = (bits << 1) | static_cast<uint64_t>(tile[threadIdx.y + j][threadIdx.x + i] < c);
+      const int q = n < 30 ? 0 : 1;
+      ++n;
+      a[q] = r3dsimt::funnel_l(v[i] - ca, a[q], 1);  // the sign bit: neighbour < centre
+      b[q] = r3dsimt::funnel_l(v[i + 1] - cb, b[q], 1);
     }
   }
-  out[static_cast<int64_t>(y) * ostride + x] = bits;
+  uint64_t* o = out + static_cast<int64_t>(y) * ostride + x;
+  o[0] = (static_cast<uint64_t>(a[0]) << 32) | a[1];
+  if (x + 1 < w) o[1] = (static_cast<uint64_t>(b[0]) << 32) | b[1];
 }
 
 // ------------------------------------------------------------------ pyramid
@@ -117,24 +139,20 @@ R3D_GLOBAL void intervals_kernel(const uint8_t* __restrict__ mask, int64_t strid
 // ------------------------------------------------------------------ left-right check
 // stereo_matcher.cpp:777-805: xo = lround(x + sign * d); mismatch if the other
 // map is invalid there or differs by more than max_diff.
-R3D_GLOBAL void lr_check_kernel(const float* __restrict__ map, const float* __restrict__ other, int w, int h, int wo,
-                                int sign, int max_diff, uint8_t* __restrict__ bad) {
+// out = map with the mismatches +inf (out may be map itself: a pixel reads
+// only itself in it).
+R3D_GLOBAL void lr_check_kernel(const float* map, const float* __restrict__ other, int w, int h, int wo, int sign,
+                                int max_diff, float* out) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= w || y >= h) return;
-  const float d = map[static_cast<int64_t>(y) * w + x];
-  uint8_t b = 0;
+  float d = map[static_cast<int64_t>(y) * w + x];
   if (r3dsimt::finitef(d)) {
     const float pos = __fadd_rn(static_cast<float>(x), __fmul_rn(static_cast<float>(sign), d));
     const long xo = lroundf(pos);
     const float dother = xo >= 0 && xo < wo ? other[static_cast<int64_t>(y) * wo + xo] : kInf;
-    b = (!r3dsimt::finitef(dother) || fabsf(__fsub_rn(d, dother)) > static_cast<float>(max_diff)) ? 1 : 0;
+    if (!r3dsimt::finitef(dother) || fabsf(__fsub_rn(d, dother)) > static_cast<float>(max_diff)) d = kInf;
   }
-  bad[static_cast<int64_t>(y) * w + x] = b;
-}
-
-R3D_GLOBAL void apply_bad_kernel(float* __restrict__ map, const uint8_t* __restrict__ bad, int64_t n) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n && bad[i]) map[i] = kInf;
+  out[static_cast<int64_t>(y) * w + x] = d;
 }
 
 // ------------------------------------------------------------------ speckles
@@ -199,40 +217,63 @@ R3D_DEVICE void uf_unite_local(int* par, int a, int b) {
 }
 
 // Per tile: local union, then parent[p] = global index of p's local root and
-// size[p] = 0 for every pixel of the tile.
+// size[p] = the valid pixels of p's part of the segment at local roots, 0
+// elsewhere. A warp labels a row's runs of connected pixels with two ballots
+// and no union; only where two rows' runs first touch do they unite (a union
+// per pixel pair, each walking contended root chains, took 310 us for 2048 x
+// 1536 pixels).
 R3D_GLOBAL void uf_tile_kernel(const float* __restrict__ d, int w, int h, float max_diff, int* parent, int* size) {
   R3D_DYNAMIC_SMEM(smem);
   int* par = reinterpret_cast<int*>(smem);
   float* dv = reinterpret_cast<float*>(smem + sizeof(int) * kUfTile * kUfTile);
+  int* cnt = reinterpret_cast<int*>(smem + 2 * sizeof(int) * kUfTile * kUfTile);
+  uint32_t* starts = reinterpret_cast<uint32_t*>(smem + 3 * sizeof(int) * kUfTile * kUfTile);  // run starts per row
   const int tx0 = static_cast<int>(blockIdx.x) * kUfTile, ty0 = static_cast<int>(blockIdx.y) * kUfTile;
   const int tw = r3dsimt::imin(kUfTile, w - tx0), th = r3dsimt::imin(kUfTile, h - ty0);
-  const int nt = static_cast<int>(blockDim.x);
-  for (int i = static_cast<int>(threadIdx.x); i < kUfTile * kUfTile; i += nt) {
-    const int lx = i % kUfTile, ly = i / kUfTile;
-    par[i] = i;
-    dv[i] = (lx < tw && ly < th) ? d[static_cast<int64_t>(ty0 + ly) * w + tx0 + lx] : kInf;
+  const int lane = static_cast<int>(threadIdx.x & 31u), nw = static_cast<int>(blockDim.x >> 5);
+  for (int ly = static_cast<int>(threadIdx.x >> 5); ly < kUfTile; ly += nw) {
+    const int i = ly * kUfTile + lane;
+    const float v = (lane < tw && ly < th) ? d[static_cast<int64_t>(ty0 + ly) * w + tx0 + lane] : kInf;
+    dv[i] = v;
+    cnt[i] = 0;
+    r3dsimt::syncwarp();
+    const float left = lane > 0 ? dv[i - 1] : kInf;
+    const bool joined = lane > 0 && lane < tw && r3dsimt::finitef(left) && fabsf(__fsub_rn(v, left)) <= max_diff;
+    const uint32_t st = ~r3dsimt::ballot(joined);
+    par[i] = ly * kUfTile + 31 - r3dsimt::clz(st & (0xFFFFFFFFu >> (31 - lane)));  // lane 0 always starts a run
+    if (lane == 0) starts[ly] = st;
   }
   r3dsimt::syncthreads();
-  for (int i = static_cast<int>(threadIdx.x); i < kUfTile * kUfTile; i += nt) {
-    const int lx = i % kUfTile, ly = i / kUfTile;
-    const float v = dv[i];
-    if (lx >= tw || ly >= th || !r3dsimt::finitef(v)) continue;
-    if (lx + 1 < tw && fabsf(__fsub_rn(dv[i + 1], v)) <= max_diff) uf_unite_local(par, i, i + 1);
-    if (ly + 1 < th && fabsf(__fsub_rn(dv[i + kUfTile], v)) <= max_diff) uf_unite_local(par, i, i + kUfTile);
+  for (int ly = static_cast<int>(threadIdx.x >> 5); ly < kUfTile; ly += nw) {
+    const int i = ly * kUfTile + lane;
+    const bool down = lane < tw && ly + 1 < th && r3dsimt::finitef(dv[i]) &&
+                      fabsf(__fsub_rn(dv[i + (ly + 1 < kUfTile ? kUfTile : 0)], dv[i])) <= max_diff;
+    const uint32_t dm = r3dsimt::ballot(down);
+    // The pair to the left joins the same two runs already.
+    const uint32_t both = ly + 1 < kUfTile ? ~(starts[ly] | starts[ly + 1]) : 0u;
+    const bool done = lane > 0 && ((dm >> (lane - 1)) & 1u) != 0 && ((both >> lane) & 1u) != 0;
+    if (down && !done) uf_unite_local(par, i, i + kUfTile);
   }
   r3dsimt::syncthreads();
-  for (int i = static_cast<int>(threadIdx.x); i < kUfTile * kUfTile; i += nt) {
-    const int lx = i % kUfTile, ly = i / kUfTile;
-    if (lx >= tw || ly >= th) continue;
+  for (int ly = static_cast<int>(threadIdx.x >> 5); ly < kUfTile; ly += nw) {
+    const int i = ly * kUfTile + lane;
     const int r = uf_root_local(par, i);
-    const int64_t g = static_cast<int64_t>(ty0 + ly) * w + tx0 + lx;
-    parent[g] = (ty0 + r / kUfTile) * w + tx0 + r % kUfTile;
-    size[g] = 0;
+    dv[i] = r3dsimt::finitef(dv[i]) ? 1.0F : 0.0F;
+    // One addition per run part of the warp's row that shares a root.
+    const uint32_t peers = r3dsimt::match_any(static_cast<uint32_t>(r));
+    const uint32_t valid = peers & r3dsimt::ballot(dv[i] != 0.0F);
+    if (lane == r3dsimt::ffs(peers) - 1 && valid != 0) atomicAdd(cnt + r, r3dsimt::popc(valid));
+    if (lane < tw && ly < th)
+      parent[static_cast<int64_t>(ty0 + ly) * w + tx0 + lane] = (ty0 + r / kUfTile) * w + tx0 + r % kUfTile;
   }
+  r3dsimt::syncthreads();
+  for (int ly = static_cast<int>(threadIdx.x >> 5); ly < th; ly += nw)
+    if (lane < tw) size[static_cast<int64_t>(ty0 + ly) * w + tx0 + lane] = cnt[ly * kUfTile + lane];
 }
 
 // Unions across tile borders: the pixel pairs straddling a vertical tile
-// boundary, then those straddling a horizontal one.
+// boundary, then those straddling a horizontal one. A pair whose two segments
+// are those of the pair in the lane before it leaves the union to that lane.
 R3D_GLOBAL void uf_border_kernel(const float* __restrict__ d, int w, int h, float max_diff, int* parent) {
   const int64_t nvx = static_cast<int64_t>((w - 1) / kUfTile) * h;  // vertical boundaries x all rows
   const int64_t nhy = static_cast<int64_t>((h - 1) / kUfTile) * w;  // horizontal boundaries x all columns
@@ -249,25 +290,30 @@ R3D_GLOBAL void uf_border_kernel(const float* __restrict__ d, int w, int h, floa
     const int y = (k + 1) * kUfTile - 1;
     a = y * w + x;
     b = a + w;
-  } else {
-    return;
   }
-  const float u = d[a], v = d[b];
-  if (r3dsimt::finitef(u) && fabsf(__fsub_rn(v, u)) <= max_diff) uf_unite(parent, a, b);
+  bool join = false;
+  if (a >= 0) {
+    const float u = d[a], v = d[b];
+    join = r3dsimt::finitef(u) && fabsf(__fsub_rn(v, u)) <= max_diff;
+  }
+  const int pa = join ? __ldcg(parent + a) : -1, pb = join ? __ldcg(parent + b) : -1;
+  const int lane = static_cast<int>(r3dsimt::lane_id()), before = lane > 0 ? lane - 1 : 0;
+  const int qa = static_cast<int>(r3dsimt::shfl(static_cast<uint32_t>(pa), before));
+  const int qb = static_cast<int>(r3dsimt::shfl(static_cast<uint32_t>(pb), before));
+  if (join && !(lane > 0 && pa == qa && pb == qb)) uf_unite(parent, a, b);
 }
 
-// Segment sizes: the lanes of a warp whose pixels share a root add their
-// count with one atomic; every pixel's parent becomes its root.
+// Segment sizes: the local roots' counts are added to their global roots
+// (which hold their own part already); every valid pixel's parent becomes its
+// root.
 R3D_GLOBAL void uf_count_kernel(const float* __restrict__ d, int64_t n, int* parent, int* size) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const bool ok = i < n && r3dsimt::finitef(d[i]);
-  const int r = ok ? uf_root(parent, static_cast<int>(i)) : -1;
-  const uint32_t peers = r3dsimt::match_any(static_cast<uint32_t>(r));
-  if (ok) {
-    parent[i] = r;
-    if (static_cast<int>(r3dsimt::lane_id()) == r3dsimt::ffs(peers) - 1)
-      atomicAdd(size + r, r3dsimt::popc64(peers));
-  }
+  if (i >= n) return;
+  const int r = uf_root(parent, static_cast<int>(i));
+  if (r == static_cast<int>(i)) return;
+  if (r3dsimt::finitef(d[i])) parent[i] = r;
+  const int c = size[i];  // nonzero at local roots only; nothing is added to one that is not a global root
+  if (c != 0) atomicAdd(size + r, c);
 }
 
 R3D_GLOBAL void uf_filter_kernel(float* __restrict__ d, int64_t n, const int* parent, const int* size, int min_size) {
@@ -280,46 +326,48 @@ R3D_GLOBAL void uf_filter_kernel(float* __restrict__ d, int64_t n, const int* pa
 // ------------------------------------------------------------------ median
 // stereo_matcher.cpp:972-1021: median of the valid values of the 3x3
 // neighbourhood; an even count averages the two middle values.
-R3D_GLOBAL void median_kernel(const float* __restrict__ in, int w, int h, float* __restrict__ out) {
+// Invalid neighbours enter as +inf, so that they sort behind the valid ones: a
+// fixed sorting network of 25 exchanges in registers (an insertion sort of the
+// valid ones needs a run-time indexed array in local memory: 64 us for 2048 x
+// 1536 pixels).
+R3D_GLOBAL void median_kernel(const float* __restrict__ in, int w, int h, float* __restrict__ out, int64_t ostride) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= w || y >= h) return;
+  float* o = out + static_cast<int64_t>(y) * ostride + x;
   const float c = in[static_cast<int64_t>(y) * w + x];
   if (!r3dsimt::finitef(c)) {
-    out[static_cast<int64_t>(y) * w + x] = c;
+    *o = c;
     return;
   }
   float v[9];
   int n = 0;
 #pragma unroll
-  for (int dy = -1; dy <= 1; ++dy) {
+  for (int k = 0; k < 9; ++k) {
+    const int qx = x + k % 3 - 1, qy = y + k / 3 - 1;
+    float q = kInf;
+    if (qx >= 0 && qy >= 0 && qx < w && qy < h) q = in[static_cast<int64_t>(qy) * w + qx];
+    const bool ok = r3dsimt::finitef(q);
+    v[k] = ok ? q : kInf;
+    n += ok ? 1 : 0;
+  }
+  constexpr int kNet[25][2] = {{0, 3}, {1, 7}, {2, 5}, {4, 8}, {0, 7}, {2, 4}, {3, 8}, {5, 6}, {0, 2},
+                               {1, 3}, {4, 5}, {7, 8}, {1, 4}, {3, 6}, {5, 7}, {0, 1}, {2, 4}, {3, 5},
+                               {6, 8}, {2, 3}, {4, 5}, {6, 7}, {1, 2}, {3, 4}, {5, 6}};
 #pragma unroll
-    for (int dx = -1; dx <= 1; ++dx) {
-      const int qx = x + dx, qy = y + dy;
-      if (qx >= 0 && qy >= 0 && qx < w && qy < h) {
-        const float q = in[static_cast<int64_t>(qy) * w + qx];
-        if (r3dsimt::finitef(q)) v[n++] = q;
-      }
+  for (int k = 0; k < 25; ++k) {
+    const float a = v[kNet[k][0]], b = v[kNet[k][1]];
+    v[kNet[k][0]] = a < b ? a : b;
+    v[kNet[k][1]] = a < b ? b : a;
+  }
+  float m = v[0], below = v[0];  // v[n / 2] and v[n / 2 - 1], 1 <= n <= 9
+#pragma unroll
+  for (int k = 1; k <= 4; ++k) {
+    if (n / 2 >= k) {
+      below = m;
+      m = v[k];
     }
   }
-  for (int a = 1; a < n; ++a) {
-    const float key = v[a];
-    int b = a - 1;
-    while (b >= 0 && v[b] > key) {
-      v[b + 1] = v[b];
-      --b;
-    }
-    v[b + 1] = key;
-  }
-  float m = v[n / 2];
-  if ((n & 1) == 0) m = __fmul_rn(0.5F, __fadd_rn(m, v[n / 2 - 1]));
-  out[static_cast<int64_t>(y) * w + x] = m;
-}
-
-R3D_GLOBAL void unmirror_offset_kernel(const float* __restrict__ in, int w, int h, float offset,
-                                       float* __restrict__ out) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= w || y >= h) return;
-  out[static_cast<int64_t>(y) * w + x] = __fsub_rn(in[static_cast<int64_t>(y) * w + (w - 1 - x)], offset);
+  *o = (n & 1) == 0 ? __fmul_rn(0.5F, __fadd_rn(m, below)) : m;
 }
 
 R3D_GLOBAL void copy2d_kernel(const float* __restrict__ in, int64_t istride, int w, int h, float* __restrict__ out,
@@ -466,18 +514,43 @@ R3D_DEVICE float axis_weight(int v, int c0, int c1, int size, int blend_px) {
 // accumulated in tile-index order; valid if the valid weight is at least half
 // of all weight; the dominant tile wins when the mean is more than 1 px away.
 R3D_GLOBAL void blend_kernel(const BlendTile* __restrict__ tiles, int ntiles, int tiles_x, int w, int h, int blend,
-                             int mirror_out, float offset, float* __restrict__ out_disp, float* __restrict__ out_conf,
-                             int64_t ostride) {
+                             int mirror_out, float offset, float* __restrict__ out_disp, int64_t dstride,
+                             float* __restrict__ out_conf, int64_t cstride) {
+  // The tile rows and columns that reach into the block (tiles are sorted by
+  // x0 and by x0 + w, so they are contiguous): a pixel of a 13 x 9 tile image
+  // looks at one to four tiles instead of 117.
+  R3D_DYNAMIC_SMEM(smem);
+  int* range = reinterpret_cast<int*>(smem);  // first and last column, first and last row
+  const int tid = static_cast<int>(threadIdx.y * blockDim.x + threadIdx.x);
+  const int nt = static_cast<int>(blockDim.x * blockDim.y);
+  const int tiles_y = ntiles / tiles_x;
+  if (tid < 4) range[tid] = (tid & 1) != 0 ? -1 : 0x7FFFFFFF;
+  r3dsimt::syncthreads();
+  {
+    const int bx0 = blockIdx.x * blockDim.x, by0 = blockIdx.y * blockDim.y;
+    const int bx1 = bx0 + static_cast<int>(blockDim.x), by1 = by0 + static_cast<int>(blockDim.y);
+    for (int i = tid; i < tiles_x; i += nt)
+      if (tiles[i].x0 < bx1 && tiles[i].x0 + tiles[i].w > bx0) {
+        atomicMin(range, i);
+        atomicMax(range + 1, i);
+      }
+    for (int j = tid; j < tiles_y; j += nt)
+      if (tiles[j * tiles_x].y0 < by1 && tiles[j * tiles_x].y0 + tiles[j * tiles_x].h > by0) {
+        atomicMin(range + 2, j);
+        atomicMax(range + 3, j);
+      }
+  }
+  r3dsimt::syncthreads();
+  const int i0 = range[0], i1 = range[1], j0 = range[2], j1 = range[3];
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= w || y >= h) return;
   float wsum = 0.0F, wall = 0.0F, dsum = 0.0F, csum = 0.0F, wbest = 0.0F, dbest = kInf;
-  const int tiles_y = ntiles / tiles_x;
-  for (int j = 0; j < tiles_y; ++j) {
+  for (int j = j0; j <= j1; ++j) {
     const BlendTile& t0 = tiles[j * tiles_x];
     if (y < t0.y0 || y >= t0.y0 + t0.h) continue;
     const float wy = axis_weight(y, t0.c0y, t0.c1y, h, blend);
     if (wy <= 0.0F) continue;
-    for (int i = 0; i < tiles_x; ++i) {
+    for (int i = i0; i <= i1; ++i) {
       const BlendTile& t = tiles[j * tiles_x + i];
       if (x < t.x0 || x >= t.x0 + t.w) continue;
       const float wg = __fmul_rn(wy, axis_weight(x, t.c0x, t.c1x, w, blend));
@@ -503,8 +576,8 @@ R3D_GLOBAL void blend_kernel(const BlendTile* __restrict__ tiles, int ntiles, in
     if (out_conf != nullptr) cv = __fdiv_rn(csum, wsum);
   }
   const int xo = mirror_out ? w - 1 - x : x;
-  out_disp[static_cast<int64_t>(y) * ostride + xo] = __fsub_rn(dv, offset);
-  if (out_conf != nullptr) out_conf[static_cast<int64_t>(y) * ostride + xo] = cv;
+  out_disp[static_cast<int64_t>(y) * dstride + xo] = __fsub_rn(dv, offset);
+  if (out_conf != nullptr) out_conf[static_cast<int64_t>(y) * cstride + xo] = cv;
 }
 
 // ------------------------------------------------------------------ tile cells
@@ -573,7 +646,8 @@ std::atomic<uint64_t>& launch_counter() {
 
 void launch_census(const uint16_t* img, int64_t stride, int w, int h, uint64_t* out, int64_t ostride, cudaStream_t s) {
   if (w <= 0 || h <= 0) return;
-  R3D_LAUNCH(census_kernel, dim3(ceil_div(w, kCBX), ceil_div(h, kCBY)), dim3(kCBX, kCBY), (kCBY + 6) * (kCBX + 8) * sizeof(uint16_t), s, img, stride, w, h, out, ostride);
+  R3D_LAUNCH(census_kernel, dim3(ceil_div(w, 2 * kCBX), ceil_div(h, kCBY)), dim3(kCBX, kCBY),
+             (kCBY + 6) * kCTW * sizeof(uint16_t), s, img, stride, w, h, out, ostride);
   launched("census_kernel");
 }
 
@@ -599,6 +673,12 @@ void launch_mirror_u16(const uint16_t* in, int64_t istride, int w, int h, uint16
   launched("mirror_kernel<u16>");
 }
 
+void launch_mirror_u64(const uint64_t* in, int w, int h, uint64_t* out, cudaStream_t s) {
+  const dim3 b(32, 8);
+  R3D_LAUNCH(mirror_kernel<uint64_t>, grid2d(w, h, b), b, 0, s, in, w, w, h, out);
+  launched("mirror_kernel<u64>");
+}
+
 void launch_mirror_u8(const uint8_t* in, int64_t istride, int w, int h, uint8_t* out, cudaStream_t s) {
   const dim3 b(32, 8);
   R3D_LAUNCH(mirror_kernel<uint8_t>, grid2d(w, h, b), b, 0, s, in, istride, w, h, out);
@@ -610,22 +690,18 @@ void launch_intervals(const uint8_t* mask, int64_t stride, int w, int h, RowInte
   launched("intervals_kernel");
 }
 
-void launch_lr_check(const float* map, const float* other, int w, int h, int wo, int sign, int max_diff, uint8_t* bad,
+void launch_lr_check(const float* map, const float* other, int w, int h, int wo, int sign, int max_diff, float* out,
                      cudaStream_t s) {
   const dim3 b(32, 8);
-  R3D_LAUNCH(lr_check_kernel, grid2d(w, h, b), b, 0, s, map, other, w, h, wo, sign, max_diff, bad);
+  R3D_LAUNCH(lr_check_kernel, grid2d(w, h, b), b, 0, s, map, other, w, h, wo, sign, max_diff, out);
   launched("lr_check_kernel");
-}
-
-void launch_apply_bad(float* map, const uint8_t* bad, int64_t n, cudaStream_t s) {
-  R3D_LAUNCH(apply_bad_kernel, static_cast<unsigned>(ceil_div64(n, 256)), 256, 0, s, map, bad, n);
-  launched("apply_bad_kernel");
 }
 
 void launch_segments(const float* d, int w, int h, float max_diff, int* parent, int* size, cudaStream_t s) {
   const int64_t n = static_cast<int64_t>(w) * h;
   const dim3 tiles(static_cast<unsigned>(ceil_div64(w, kUfTile)), static_cast<unsigned>(ceil_div64(h, kUfTile)));
-  R3D_LAUNCH(uf_tile_kernel, tiles, 256, 2 * sizeof(int) * kUfTile * kUfTile, s, d, w, h, max_diff, parent, size);
+  R3D_LAUNCH(uf_tile_kernel, tiles, 256, 3 * sizeof(int) * kUfTile * kUfTile + 4 * kUfTile, s, d, w, h, max_diff, parent,
+             size);
   launched("uf_tile_kernel");
   const int64_t nb = static_cast<int64_t>((w - 1) / kUfTile) * h + static_cast<int64_t>((h - 1) / kUfTile) * w;
   if (nb > 0) {
@@ -648,16 +724,10 @@ void launch_remove_speckles(float* d, int w, int h, int min_size, float max_diff
   launched("uf_filter_kernel");
 }
 
-void launch_median3x3(const float* in, int w, int h, float* out, cudaStream_t s) {
+void launch_median3x3(const float* in, int w, int h, float* out, int64_t ostride, cudaStream_t s) {
   const dim3 b(32, 8);
-  R3D_LAUNCH(median_kernel, grid2d(w, h, b), b, 0, s, in, w, h, out);
+  R3D_LAUNCH(median_kernel, grid2d(w, h, b), b, 0, s, in, w, h, out, ostride);
   launched("median_kernel");
-}
-
-void launch_unmirror_offset(const float* in, int w, int h, float offset, float* out, cudaStream_t s) {
-  const dim3 b(32, 8);
-  R3D_LAUNCH(unmirror_offset_kernel, grid2d(w, h, b), b, 0, s, in, w, h, offset, out);
-  launched("unmirror_offset_kernel");
 }
 
 void launch_copy2d_f32(const float* in, int64_t istride, int w, int h, float* out, int64_t ostride, cudaStream_t s) {
@@ -726,12 +796,11 @@ void launch_ranges_from_coarse(const float* coarse, int wc, int hc, int w, int h
   launched("range_final_kernel");
 }
 
-void launch_blend(const BlendTile* tiles, int ntiles, int tiles_x, const int* /*bx*/, const int* /*by*/, int w, int h,
-                  int blend, int mirror_out, float offset, float* out_disp, float* out_conf, int64_t ostride,
-                  cudaStream_t s) {
+void launch_blend(const BlendTile* tiles, int ntiles, int tiles_x, int w, int h, int blend, int mirror_out,
+                  float offset, float* out_disp, int64_t dstride, float* out_conf, int64_t cstride, cudaStream_t s) {
   const dim3 b(32, 8);
-  R3D_LAUNCH(blend_kernel, grid2d(w, h, b), b, 0, s, tiles, ntiles, tiles_x, w, h, blend, mirror_out, offset, out_disp,
-                                             out_conf, ostride);
+  R3D_LAUNCH(blend_kernel, grid2d(w, h, b), b, 16, s, tiles, ntiles, tiles_x, w, h, blend, mirror_out, offset, out_disp,
+             dstride, out_conf, cstride);
   launched("blend_kernel");
 }
 

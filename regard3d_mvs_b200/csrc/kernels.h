@@ -23,13 +23,14 @@ void launch_pyramid_u16(const uint16_t* in, int64_t istride, int w, int h, uint1
 void launch_reduce_mask(const uint8_t* in, int64_t istride, int w, int h, uint8_t* out, int64_t ostride,
                         cudaStream_t s);
 void launch_mirror_u16(const uint16_t* in, int64_t istride, int w, int h, uint16_t* out, cudaStream_t s);
+void launch_mirror_u64(const uint64_t* in, int w, int h, uint64_t* out, cudaStream_t s);  // contiguous
 void launch_mirror_u8(const uint8_t* in, int64_t istride, int w, int h, uint8_t* out, cudaStream_t s);
 // mask == nullptr: every row is [0, w - 1].
 void launch_intervals(const uint8_t* mask, int64_t stride, int w, int h, RowInterval* out, cudaStream_t s);
-// map[i] = +inf where bad[i] != 0.
-void launch_lr_check(const float* map, const float* other, int w, int h, int wo, int sign, int max_diff,
-                     uint8_t* bad, cudaStream_t s);
-void launch_apply_bad(float* map, const uint8_t* bad, int64_t n, cudaStream_t s);
+// Left-right check of map (w x h) against other (wo x h): out = map with the
+// mismatches +inf (out may be map).
+void launch_lr_check(const float* map, const float* other, int w, int h, int wo, int sign, int max_diff, float* out,
+                     cudaStream_t s);
 // Segments of 4-neighbours of the contiguous map d (w x h, invalid = +inf)
 // whose values differ by at most max_diff: afterwards parent[i] is the root
 // (smallest index) of valid pixel i's segment and size[root] its pixel count.
@@ -39,9 +40,7 @@ void launch_remove_speckles(float* d, int w, int h, int min_size, float max_diff
 // Same filter with the scratch in a static device array (noalloc.cu); the
 // map is device memory of `device`, contiguous, and the work is enqueued on `s`.
 void remove_speckles_static_scratch(int device, float* d, int w, int h, int min_size, float max_diff, cudaStream_t s);
-void launch_median3x3(const float* in, int w, int h, float* out, cudaStream_t s);
-// out[y][x] = in[y][w - 1 - x] - offset.
-void launch_unmirror_offset(const float* in, int w, int h, float offset, float* out, cudaStream_t s);
+void launch_median3x3(const float* in, int w, int h, float* out, int64_t ostride, cudaStream_t s);
 void launch_copy2d_f32(const float* in, int64_t istride, int w, int h, float* out, int64_t ostride, cudaStream_t s);
 
 struct RangeParams {
@@ -66,11 +65,10 @@ struct BlendTile {
 };
 
 // Blends the tiles of one match (stereo_matcher.cpp:700-766). Output at
-// (x, y) goes to out_disp[y * ostride + (mirror_out ? w - 1 - x : x)] minus
-// `offset`; conf_out may be null.
-void launch_blend(const BlendTile* tiles, int ntiles, int tiles_x, const int* bx, const int* by, int w, int h,
-                  int blend, int mirror_out, float offset, float* out_disp, float* out_conf, int64_t ostride,
-                  cudaStream_t s);
+// (x, y) goes to out_disp[y * dstride + (mirror_out ? w - 1 - x : x)] minus
+// `offset`; out_conf (row stride cstride) may be null.
+void launch_blend(const BlendTile* tiles, int ntiles, int tiles_x, int w, int h, int blend, int mirror_out,
+                  float offset, float* out_disp, int64_t dstride, float* out_conf, int64_t cstride, cudaStream_t s);
 
 // Per-tile label statistics: stats[0] = largest num, stats[1 + i] = pixels
 // with num above tile_stat_width(i) (32, 64, 128, 192, 256, 384, 512).

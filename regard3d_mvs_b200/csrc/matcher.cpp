@@ -459,7 +459,7 @@ struct PairRun {
   Match left, right;
   bool has_right = false;
   RowInterval *int_l = nullptr, *int_r = nullptr;
-  float *disp_l = nullptr, *conf_l = nullptr, *disp_r = nullptr;
+  float *disp_l = nullptr, *disp_r = nullptr;
   uint64_t cells = 0;
   std::vector<unsigned long long*> cell_arrays;  // device, summed at the end
   std::vector<int> cell_counts;
@@ -611,14 +611,16 @@ void prepare_level(PairRun& P, Arena& A, Pinned& H, cudaStream_t s) {
     lnum = nu;
   }
   fill_match(P.left.m, o, in.left, cl, cr, wr, P.int_l, P.int_r, llo, lnum, in.dmin, in.nd,
-             P.check_lr && !P.lr_full, true);
+             P.check_lr && !P.lr_full, l == 0 && P.req->out.confidence != nullptr);
   P.has_right = P.check_lr && P.lr_full;
   if (P.has_right) {
-    uint16_t* ml = A.alloc<uint16_t>(static_cast<size_t>(wl) * h);
+    // The mirrored right image's intensities set the penalties. Its Census and
+    // the left one's: a mirrored image's codes are the image's with the bits
+    // of every window row reversed, in both images alike, so Hamming costs
+    // are the same with the plain codes mirrored.
     uint16_t* mr = A.alloc<uint16_t>(static_cast<size_t>(wr) * h);
-    launch_mirror_u16(in.left.p, in.left.stride, wl, h, ml, s);
     launch_mirror_u16(in.right.p, in.right.stride, wr, h, mr, s);
-    const DView<uint16_t> vml{ml, wl, h, wl}, vmr{mr, wr, h, wr};
+    const DView<uint16_t> vmr{mr, wr, h, wr};
     DView<uint8_t> mlm, mrm;
     if (!in.lmask.empty()) {
       uint8_t* p = A.alloc<uint8_t>(static_cast<size_t>(wl) * h);
@@ -630,8 +632,13 @@ void prepare_level(PairRun& P, Arena& A, Pinned& H, cudaStream_t s) {
       launch_mirror_u8(in.rmask.p, in.rmask.stride, wr, h, p, s);
       mrm = {p, wr, h, wr};
     }
-    const uint64_t* cml = census(vml);
-    const uint64_t* cmr = census(vmr);
+    auto mirrored = [&](const uint64_t* c, int w) {
+      uint64_t* o = A.alloc<uint64_t>(static_cast<size_t>(w) * h);
+      launch_mirror_u64(c, w, h, o, s);
+      return o;
+    };
+    const uint64_t* cml = mirrored(cl, wl);
+    const uint64_t* cmr = mirrored(cr, wr);
     RowInterval* iml = intervals(mlm, wl);
     RowInterval* imr = intervals(mrm, wr);
     if (ranged) {
@@ -733,7 +740,10 @@ void finish_level(PairRun& P, Arena& A, Pinned& H, cudaStream_t s) {
   const LevelIn& in = P.lv[l];
   const r3dgpu_stereo_options& o = P.o;
   const int wl = in.left.w, wr = in.right.w, h = in.left.h;
-  auto blend = [&](Match& M, int W, bool mirror_out, float offset, float* disp, float* conf) {
+  // At level 0 the last stage writes the caller's map: the blend its
+  // confidence, the median (or a copy) its disparity.
+  const r3dgpu_disparity_map& res = P.req->out;
+  auto blend = [&](Match& M, int W, bool mirror_out, float offset, float* disp, float* conf, int64_t cstride) {
     const int n = static_cast<int>(M.layout.tiles.size());
     BlendTile* bt = H.alloc<BlendTile>(n);
     for (int i = 0; i < n; ++i) {
@@ -743,43 +753,45 @@ void finish_level(PairRun& P, Arena& A, Pinned& H, cudaStream_t s) {
     }
     BlendTile* d = A.alloc<BlendTile>(n);
     R3D_CUDA(cudaMemcpyAsync(d, bt, sizeof(BlendTile) * n, cudaMemcpyHostToDevice, s));
-    launch_blend(d, n, M.layout.tiles_x, nullptr, nullptr, W, h, o.tile_blend, mirror_out ? 1 : 0, offset, disp, conf,
-                 W, s);
+    launch_blend(d, n, M.layout.tiles_x, W, h, o.tile_blend, mirror_out ? 1 : 0, offset, disp, W, conf, cstride, s);
   };
   P.disp_l = A.alloc<float>(static_cast<size_t>(wl) * h);
-  P.conf_l = A.alloc<float>(static_cast<size_t>(wl) * h);
-  blend(P.left, wl, false, 0.0F, P.disp_l, P.conf_l);
+  blend(P.left, wl, false, 0.0F, P.disp_l, l == 0 ? res.confidence : nullptr, res.stride);
   const bool need_right = P.lr_full && l > 0;
   const int speckle = o.speckle_size >> (2 * l);
   int* uf = nullptr;
-  auto post_filter = [&](float*& d, int W) {
+  // Speckle filter in place, then the median (or a plain copy) into `to`, or
+  // into a buffer of its own.
+  auto post_filter = [&](float*& d, int W, float* to, int64_t stride) {
     if (speckle > 1) {
       if (!uf) uf = A.alloc<int>(2 * static_cast<size_t>(std::max(wl, wr)) * h);
       launch_remove_speckles(d, W, h, speckle, o.speckle_diff, uf, s);
     }
     if (o.median) {
-      float* m = A.alloc<float>(static_cast<size_t>(W) * h);
-      launch_median3x3(d, W, h, m, s);
+      float* m = to != nullptr ? to : A.alloc<float>(static_cast<size_t>(W) * h);
+      launch_median3x3(d, W, h, m, to != nullptr ? stride : W, s);
       d = m;
+    } else if (to != nullptr) {
+      launch_copy2d_f32(d, W, W, h, to, stride, s);
     }
   };
   if (P.has_right) {
     P.disp_r = A.alloc<float>(static_cast<size_t>(wr) * h);
-    blend(P.right, wr, true, static_cast<float>(wr - wl), P.disp_r, nullptr);
-    uint8_t* bad_l = A.alloc<uint8_t>(static_cast<size_t>(wl) * h);
+    blend(P.right, wr, true, static_cast<float>(wr - wl), P.disp_r, nullptr, 0);
     if (need_right) {
-      uint8_t* bad_r = A.alloc<uint8_t>(static_cast<size_t>(wr) * h);
-      launch_lr_check(P.disp_r, P.disp_l, wr, h, wl, +1, o.lr_max_diff, bad_r, s);
-      launch_lr_check(P.disp_l, P.disp_r, wl, h, wr, -1, o.lr_max_diff, bad_l, s);
-      launch_apply_bad(P.disp_l, bad_l, static_cast<int64_t>(wl) * h, s);
-      launch_apply_bad(P.disp_r, bad_r, static_cast<int64_t>(wr) * h, s);
-      post_filter(P.disp_r, wr);
+      // Both checks read the unchecked maps.
+      float* checked_l = A.alloc<float>(static_cast<size_t>(wl) * h);
+      float* checked_r = A.alloc<float>(static_cast<size_t>(wr) * h);
+      launch_lr_check(P.disp_r, P.disp_l, wr, h, wl, +1, o.lr_max_diff, checked_r, s);
+      launch_lr_check(P.disp_l, P.disp_r, wl, h, wr, -1, o.lr_max_diff, checked_l, s);
+      P.disp_l = checked_l;
+      P.disp_r = checked_r;
+      post_filter(P.disp_r, wr, nullptr, 0);
     } else {
-      launch_lr_check(P.disp_l, P.disp_r, wl, h, wr, -1, o.lr_max_diff, bad_l, s);
-      launch_apply_bad(P.disp_l, bad_l, static_cast<int64_t>(wl) * h, s);
+      launch_lr_check(P.disp_l, P.disp_r, wl, h, wr, -1, o.lr_max_diff, P.disp_l, s);
     }
   }
-  post_filter(P.disp_l, wl);
+  post_filter(P.disp_l, wl, l == 0 ? res.disparity : nullptr, res.stride);
   P.coarse_left = P.disp_l;
   P.coarse_wl = wl;
   P.coarse_h = h;
@@ -1279,12 +1291,8 @@ BatchRun enqueue_batch(r3dgpu_pair* pairs, int count, cudaStream_t s, int slot) 
       finish_level(*P, A, H, s);
     }
   }
-  // Outputs and cell counts.
+  // Cell counts.
   for (auto& P : runs) {
-    r3dgpu_disparity_map& out = const_cast<r3dgpu_pair*>(P.req)->out;
-    const int wl = P.lv[0].left.w, h = P.lv[0].left.h;
-    launch_copy2d_f32(P.coarse_left, wl, wl, h, out.disparity, out.stride, s);
-    if (out.confidence) launch_copy2d_f32(P.conf_l, wl, wl, h, out.confidence, out.stride, s);
     for (size_t k = 0; k < P.cell_arrays.size(); ++k) {
       unsigned long long* hc = H.alloc<unsigned long long>(P.cell_counts[k]);
       R3D_CUDA(cudaMemcpyAsync(hc, P.cell_arrays[k], sizeof(unsigned long long) * P.cell_counts[k],
@@ -2048,7 +2056,7 @@ r3dgpu_status r3dgpu_median_filter_3x3_host(const float* disparity, int32_t widt
     cudaStream_t s = nullptr;
     const float* d = upload(A, disparity, width, height, width, s);
     float* m = A.alloc<float>(static_cast<size_t>(width) * height);
-    launch_median3x3(d, width, height, m, s);
+    launch_median3x3(d, width, height, m, width, s);
     R3D_CUDA(cudaMemcpyAsync(out, m, sizeof(float) * width * height, cudaMemcpyDeviceToHost, s));
     R3D_CUDA(cudaStreamSynchronize(s));
   });

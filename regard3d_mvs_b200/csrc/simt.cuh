@@ -62,6 +62,9 @@ R3D_DEVICE uint32_t vaddmin2(uint32_t a, uint32_t b, uint32_t c) { return vmin2(
 R3D_DEVICE uint32_t perm(uint32_t a, uint32_t b, uint32_t s) { return __byte_perm(a, b, s); }
 // Low word of (hi:lo) >> s, s in [0, 31].
 R3D_DEVICE uint32_t funnel_r(uint32_t lo, uint32_t hi, uint32_t s) { return __funnelshift_r(lo, hi, s); }
+// High word of (hi:lo) << s, s in [0, 31].
+R3D_DEVICE uint32_t funnel_l(uint32_t lo, uint32_t hi, uint32_t s) { return __funnelshift_l(lo, hi, s); }
+R3D_DEVICE int clz(uint32_t v) { return __clz(static_cast<int>(v)); }
 R3D_DEVICE int popc(uint32_t v) { return __popc(v); }
 R3D_DEVICE int popc64(uint64_t v) { return __popcll(v); }
 // Streaming (evict-first) 16-byte load and store.
@@ -196,6 +199,10 @@ inline uint32_t perm(uint32_t a, uint32_t b, uint32_t s) {
 inline uint32_t funnel_r(uint32_t lo, uint32_t hi, uint32_t s) {
   return static_cast<uint32_t>(((static_cast<uint64_t>(hi) << 32) | lo) >> (s & 31u));
 }
+inline uint32_t funnel_l(uint32_t lo, uint32_t hi, uint32_t s) {
+  return static_cast<uint32_t>((((static_cast<uint64_t>(hi) << 32) | lo) << (s & 31u)) >> 32);
+}
+inline int clz(uint32_t v) { return v != 0 ? __builtin_clz(v) : 32; }
 inline int popc(uint32_t v) { return __builtin_popcount(v); }
 inline int popc64(uint64_t v) { return __builtin_popcountll(v); }
 inline uint4 ld_stream(const uint4* p) { return *p; }
@@ -232,6 +239,7 @@ inline unsigned long long atomicAdd(unsigned long long* p, unsigned long long v)
   return o;
 }
 inline unsigned atomicMin(unsigned* p, unsigned v) { const unsigned o = *p; if (v < o) *p = v; return o; }
+inline int atomicMin(int* p, int v) { const int o = *p; if (v < o) *p = v; return o; }
 inline int atomicMax(int* p, int v) { const int o = *p; if (v > o) *p = v; return o; }
 inline int atomicCAS(int* p, int cmp, int v) { const int o = *p; if (o == cmp) *p = v; return o; }
 template <class T>
