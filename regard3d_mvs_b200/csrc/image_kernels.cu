@@ -482,6 +482,10 @@ R3D_GLOBAL void range_final_kernel(const float* __restrict__ cmin, const float* 
 }
 
 // ------------------------------------------------------------------ blend
+// a / b clamped to [0, 1], b > 0: the division only where the clamp does not
+// decide (a >= b rounds to at least 1, a <= 0 to at most 0).
+R3D_DEVICE float clamped_ratio(float a, float b) { return a >= b ? 1.0F : (a > 0.0F ? fminf(__fdiv_rn(a, b), 1.0F) : 0.0F); }
+
 // stereo_matcher.cpp:530-543
 R3D_DEVICE float axis_weight(int v, int c0, int c1, int size, int blend_px) {
   const float blend = static_cast<float>(blend_px);
@@ -490,8 +494,7 @@ R3D_DEVICE float axis_weight(int v, int c0, int c1, int size, int blend_px) {
   if (c0 > 0) {
     float t;
     if (blend_px > 0) {
-      t = __fdiv_rn(__fadd_rn(__fsub_rn(pos, static_cast<float>(c0)), __fmul_rn(0.5F, blend)), blend);
-      t = fminf(fmaxf(t, 0.0F), 1.0F);
+      t = clamped_ratio(__fadd_rn(__fsub_rn(pos, static_cast<float>(c0)), __fmul_rn(0.5F, blend)), blend);
     } else {
       t = v >= c0 ? 1.0F : 0.0F;
     }
@@ -500,8 +503,7 @@ R3D_DEVICE float axis_weight(int v, int c0, int c1, int size, int blend_px) {
   if (c1 < size) {
     float t;
     if (blend_px > 0) {
-      t = __fdiv_rn(__fsub_rn(__fadd_rn(static_cast<float>(c1), __fmul_rn(0.5F, blend)), pos), blend);
-      t = fminf(fmaxf(t, 0.0F), 1.0F);
+      t = clamped_ratio(__fsub_rn(__fadd_rn(static_cast<float>(c1), __fmul_rn(0.5F, blend)), pos), blend);
     } else {
       t = v < c1 ? 1.0F : 0.0F;
     }
@@ -544,6 +546,18 @@ R3D_GLOBAL void blend_kernel(const BlendTile* __restrict__ tiles, int ntiles, in
   const int i0 = range[0], i1 = range[1], j0 = range[2], j1 = range[3];
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= w || y >= h) return;
+  if (i0 == i1 && j0 == j1) {
+    // One tile: where both its axis weights are 1 the mean is the value itself.
+    const BlendTile& t = tiles[j0 * tiles_x + i0];
+    if (axis_weight(y, t.c0y, t.c1y, h, blend) == 1.0F && axis_weight(x, t.c0x, t.c1x, w, blend) == 1.0F) {
+      const int64_t ti = static_cast<int64_t>(y - t.y0) * t.w + (x - t.x0);
+      const float dv = t.disp[ti];
+      const int xo = mirror_out ? w - 1 - x : x;
+      out_disp[static_cast<int64_t>(y) * dstride + xo] = __fsub_rn(dv, offset);
+      if (out_conf != nullptr) out_conf[static_cast<int64_t>(y) * cstride + xo] = r3dsimt::finitef(dv) ? t.conf[ti] : 0.0F;
+      return;
+    }
+  }
   float wsum = 0.0F, wall = 0.0F, dsum = 0.0F, csum = 0.0F, wbest = 0.0F, dbest = kInf;
   for (int j = j0; j <= j1; ++j) {
     const BlendTile& t0 = tiles[j * tiles_x];

@@ -862,9 +862,26 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
     const int safe = rv.first > 0 ? rv.first : 0;
     const uint32_t inv = static_cast<uint32_t>(m.invalid_cost);
     int run = rowstart[r] >> 4;
+    // The inputs of the next 32 pixels are loaded while the present ones are
+    // worked on.
+    int lo_n = 0, nu_n = 0;
+    uint32_t iv_n = 0;
+    uint64_t cl_n = 0;
+    auto load = [&](int x) {
+      if (x >= w) return;
+      const int bx = job.x0 + x;
+      lo_n = lorow[bx];
+      nu_n = numrow[bx] >> 4;
+      iv_n = irow[bx];
+      cl_n = lrow[bx];
+    };
+    load(lane);
     for (int xb = 0; xb < w; xb += 32) {
       const int x = xb + lane, bx = job.x0 + x;
-      const int lo = x < w ? lorow[bx] : 0, nu = x < w ? numrow[bx] >> 4 : 0;
+      const int lo = lo_n, nu = x < w ? nu_n : 0;
+      const uint32_t iv = iv_n;
+      const uint64_t cl = cl_n;
+      load(x + 32);
       int incl = nu;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -876,9 +893,8 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
       if (x < w)
         rec[job.px_off + static_cast<int64_t>(y) * w + x] =
             make_uint2(static_cast<uint32_t>(off) | (r3dsimt::umin(static_cast<uint32_t>(nu), kRecWide) << kRecShift),
-                       static_cast<uint32_t>(lo) | (static_cast<uint32_t>(irow[bx]) << 16));
+                       static_cast<uint32_t>(lo) | (iv << 16));
       const bool inside = x < w && bx >= lv.first && bx <= lv.last;
-      const uint64_t cl = inside ? lrow[bx] : 0;
       uint8_t* out = cost + job.cell_off + static_cast<int64_t>(off) * 16;
       for (int u = 0; u < nu; ++u) {
         uint32_t q[4] = {0, 0, 0, 0};
@@ -925,7 +941,10 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
 // label order into their own buffers (up to kVecLabels labels in shared
 // memory, wider ones in global memory that the L1 holds), and the step reads
 // its predecessor labels at its range's shift there, sentinels around them.
-// Everything is private to a lane: no barrier, no warp-wide minimum.
+// Everything is private to a lane: no barrier, no warp-wide minimum. A step
+// takes about 250 instructions of 32 pixels (K = 8), 370 (K = 16), a quarter
+// of the steps realigned; issue and shared-memory latency bound it (0.47 of the
+// issue slots, DRAM 24 %).
 //
 // One lane per chain against the lane group of the full-range passes: most
 // ranges are one or two units, so a group would idle on the narrow pixels and
@@ -947,9 +966,8 @@ struct RangedRing {
   static constexpr int kData = D * kStageBytes;
   static constexpr int kRec = NR * 32 * 8;
   static constexpr int kVecLabels = 32;          // labels of a vector in shared memory
-  static constexpr int kPadWords = (CH + 2) / 2;  // sentinels before and after a vector
-  static constexpr int kVecStep = kVecLabels / 2 + kPadWords;  // from buffer 0 to buffer 1
-  static constexpr int kVecStride = (2 * kVecStep + kPadWords + 1) | 1;
+  static constexpr int kVecStep = kVecLabels / 2 + 1;  // words of a buffer: a vector and a sentinel after it
+  static constexpr int kVecStride = (2 * kVecStep) | 1;
   static constexpr int kVec = 32 * kVecStride * 4;
   static constexpr int kWarpBytes = kData + kRec + kVec + 512;
   static constexpr int kBlockBytes = (kRangedThreads / 32) * kWarpBytes;
@@ -964,7 +982,7 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
   // Modes: kFirst / kAccumulate write or add u16 sums; kTerm writes the
   // pass's byte terms (all eight directions in one launch).
   using R = RangedRing<K, MODE>;
-  constexpr int CH = R::CH, UF = R::UF, D = R::D, NR = R::NR, NS = R::kVecLabels, PAD = R::kPadWords;
+  constexpr int CH = R::CH, UF = R::UF, D = R::D, NR = R::NR, NS = R::kVecLabels;
   R3D_DYNAMIC_SMEM(smem);
   const int lane = static_cast<int>(threadIdx.x & 31u), warp = static_cast<int>(threadIdx.x >> 5);
   const int wpb = static_cast<int>(blockDim.x) >> 5;
@@ -972,19 +990,13 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
   unsigned char* const wb = smem + static_cast<size_t>(warp) * R::kWarpBytes;
   unsigned char* const data = wb + lane * 16;
   uint2* const recs = reinterpret_cast<uint2*>(wb + R::kData) + lane;  // slot q at recs[32 q]
-  // Buffer b of the lane: words -PAD .. NS / 2 + PAD - 1 around vec + b * kVecStep.
-  uint32_t* const vec = reinterpret_cast<uint32_t*>(wb + R::kData + R::kRec) + lane * R::kVecStride + PAD;
+  // The lane's buffer b at vec + b * kVecStep: the words of a vector, then one
+  // of sentinels. Reads clamp their word index to it as an unsigned number, so
+  // that words before the vector come from there too.
+  uint32_t* const vec = reinterpret_cast<uint32_t*>(wb + R::kData + R::kRec) + lane * R::kVecStride;
   uint16_t* const lut = reinterpret_cast<uint16_t*>(wb + R::kData + R::kRec + R::kVec);
-  // The lane's buffers of wide vectors: word q (from -PAD on) of buffer b at
-  // wide[(b * ovf_words + q) * 32].
-  uint32_t* const wide =
-      ovf + ((static_cast<int64_t>(blockIdx.x) * wpb + warp) * 2 * ovf_words + PAD) * 32 + lane;
-  if (ovf_words > 0) {
-    for (int k = 1; k <= PAD; ++k) {
-      wide[-32 * k] = kSent2;
-      wide[(ovf_words - k) * 32] = kSent2;
-    }
-  }
+  // The lane's buffers of wide vectors: word q of buffer b at wide[(b * ovf_words + q) * 32].
+  uint32_t* const wide = ovf + (static_cast<int64_t>(blockIdx.x) * wpb + warp) * 2 * ovf_words * 32 + lane;
   int lut_match = -1;
   const uint32_t one = ps.one;
   for (int64_t gblk = static_cast<int64_t>(blockIdx.x) * wpb + warp; gblk < ps.total;
@@ -1004,16 +1016,37 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
     const int w = job.w;
     const uint32_t p1x2 = static_cast<uint32_t>(m.p1) * 0x10001u;
     const bool no_carry = m.sum_no_carry != 0;
-    int sx, sy, len;
-    chain_geometry(cls, dx, dy, w, job.h, blk * 32 + lane, sx, sy, len);
-    int maxlen = len;
+    // The lane's chain: pixel (sx, sy) + i (dx, dy) at step i, t0 <= i < t1.
+    // Diagonals run in step by row (a lane waits t0 steps for its chain's first
+    // row), so that the 32 lanes are on adjacent pixels of one row; chains that
+    // start down the tile's side, each from its own first pixel, would put
+    // every lane on a row of its own, 32 cache lines per load.
+    int sx, sy, t0 = 0, t1;
+    if (cls == 2) {
+      const int c = static_cast<int>(blk) * 32 + lane - (job.h - 1);  // column at step 0, along dx
+      sx = dx > 0 ? c : w - 1 - c;
+      sy = dy > 0 ? 0 : job.h - 1;
+      t0 = c < 0 ? -c : 0;
+      t1 = c < w ? r3dsimt::imin(job.h, w - c) : 0;
+      int first = t1 > t0 ? t0 : job.h;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) maxlen = r3dsimt::imax(maxlen, static_cast<int>(r3dsimt::shfl_xor(maxlen, o)));
+      for (int o = 1; o < 32; o <<= 1) first = r3dsimt::imin(first, static_cast<int>(r3dsimt::shfl_xor(static_cast<uint32_t>(first), o)));
+      t0 -= first;
+      t1 -= first;
+      sx += first * dx;
+      sy += first * dy;
+    } else {
+      chain_geometry(cls, dx, dy, w, job.h, blk * 32 + lane, sx, sy, t1);
+    }
+    int maxlen = t1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) maxlen = r3dsimt::imax(maxlen, static_cast<int>(r3dsimt::shfl_xor(static_cast<uint32_t>(maxlen), o)));
+    auto has = [&](int i) { return i >= t0 && i < t1; };
     const uint8_t* const cbase = cost + job.cell_off;
     uint16_t* const sbase = sum + job.cell_off;
     uint8_t* const tout = terms + job.cell_off + tslot * tstride;
     const int dpx = dy * w + dx;
-    const uint2* rp = rec + job.px_off + static_cast<int64_t>(sy) * w + sx;  // record of the next pixel to request
+    const uint2* rp = rec + job.px_off + static_cast<int64_t>(sy) * w + sx;  // record of the next step to request
     auto units_of = [&](const uint2& r, int i) { return rec_units(r, m, job, sx + i * dx, sy + i * dy); };
     // Chunk of the pixel with `left` units from unit `at` on into ring slot st.
     auto issue_chunk = [&](int st, int at, int left) {
@@ -1033,29 +1066,29 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
     // Pixel i + D - 1's first chunk into slot st, pixel i + 2 D - 1's record;
     // one group. (Records: requested D steps before the data, so landed.)
     auto issue = [&](int i, int st) {
-      if (i + D - 1 < len) {
+      if (has(i + D - 1)) {
         const uint2 r = recs[((i + D - 1) & (NR - 1)) * 32];
         issue_chunk(st, static_cast<int>(r.x & kRecOffset), static_cast<int>(r.x >> kRecShift));
       }
-      if (i + 2 * D - 1 < len) r3dsimt::cp_async8(&recs[((i + 2 * D - 1) & (NR - 1)) * 32], rp);
+      if (has(i + 2 * D - 1)) r3dsimt::cp_async8(&recs[((i + 2 * D - 1) & (NR - 1)) * 32], rp);
       rp += dpx;
       r3dsimt::cp_async_commit();
     };
 #pragma unroll
     for (int k = 0; k < 2 * D - 1; ++k) {
-      if (k < len) recs[k * 32] = *rp;
+      if (has(k)) recs[k * 32] = *rp;
       rp += dpx;
     }
 #pragma unroll
     for (int k = 0; k < D - 1; ++k) {
-      if (k < len) {
+      if (has(k)) {
         const uint2 r = recs[k * 32];
         issue_chunk(k, static_cast<int>(r.x & kRecOffset), static_cast<int>(r.x >> kRecShift));
       }
       r3dsimt::cp_async_commit();
     }
     uint2 rc = make_uint2(0, 0);  // this pixel's record
-    if (len > 0) rc = recs[0];
+    if (has(0)) rc = recs[0];
     // The predecessor's range, its minimum over labels in both halves,
     // negated, and the clamp min L(q) + P2. A zero clamp makes the first
     // pixel's best term 0 whatever the predecessor words hold: T = 0, L = C.
@@ -1065,14 +1098,7 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
 #pragma unroll
     for (int k = 0; k < K; ++k) prev[k] = 0;
     bool single = static_cast<int>(rc.x >> kRecShift) == UF;  // this pixel is one full chunk
-    bool fast = r3dsimt::ballot(len > 0 && !single) == 0;
-    bool clean = false;  // the buffers hold sentinels outside what this chain wrote
-    int high = 0;        // labels of the longest vector written
-    auto make_clean = [&]() {
-      if (clean) return;
-      for (int k = -PAD; k < R::kVecStride - PAD; ++k) vec[k] = kSent2;
-      clean = true;
-    };
+    bool fast = r3dsimt::ballot(has(0) && !single) == 0;
     // From the best terms of a chunk (its bytes in ring slot st, its cells
     // from unit `at` on): T = best - min L(q), L = C + T, and the outputs.
     uint32_t out[K], pm;
@@ -1133,23 +1159,13 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
         uint32_t* v = vec + (i & 1) * R::kVecStep + c * K;
 #pragma unroll
         for (int k = 0; k < K; ++k) v[k] = nat[k];
-        if (last) {
-          // Sentinels after the vector where a longer one was written before.
-          if (n < high) {
-#pragma unroll
-            for (int k = 0; k < PAD; ++k) v[end + k] = kSent2;
-          }
-          high = r3dsimt::imax(high, n);
-        }
+        if (last) v[end] = kSent2;
       } else {
         uint32_t* v = wide + ((i & 1) * ovf_words + c * K) * 32;
 #pragma unroll
         for (int k = 0; k < K; ++k)
           if (k < 8 || upper) v[k * 32] = nat[k];
-        if (last) {
-#pragma unroll
-          for (int k = 0; k < PAD; ++k) v[(end + k) * 32] = kSent2;
-        }
+        if (last) v[end * 32] = kSent2;
       }
     };
     // best = min(L(q, d), L(q, d -+ 1) + P1, min L(q) + P2); clamping first
@@ -1157,20 +1173,20 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
     // 1, for the labels of chunk c at lo.
     auto best_from_memory = [&](uint32_t (&best)[K], int i, int c, int lo) {
       // Predecessor labels b - 1 .. b + CH (its own indexing).
-      int b = c * CH + lo - lo_q;
-      b = r3dsimt::imax(r3dsimt::imin(b, num_q + 1), -(CH + 1));
+      const int b = c * CH + lo - lo_q;
       // pr[k]: labels b - 1 + 2 k, b + 2 k, from the words holding them.
       const int f = (b - 1) >> 1;
       const uint32_t par = 16u * (static_cast<uint32_t>(b - 1) & 1u);
+      const uint32_t end = static_cast<uint32_t>(num_q >> 1);
       uint32_t wd[K + 2], pr[K + 1];
       if (num_q <= NS) {
-        const uint32_t* vq = vec + ((i & 1) ^ 1) * R::kVecStep + f;
+        const uint32_t* vq = vec + ((i & 1) ^ 1) * R::kVecStep;
 #pragma unroll
-        for (int k = 0; k < K + 2; ++k) wd[k] = vq[k];
+        for (int k = 0; k < K + 2; ++k) wd[k] = vq[r3dsimt::umin(static_cast<uint32_t>(f + k), end)];
       } else {
-        const uint32_t* oq = wide + (((i & 1) ^ 1) * ovf_words + f) * 32;
+        const uint32_t* oq = wide + ((i & 1) ^ 1) * ovf_words * 32;
 #pragma unroll
-        for (int k = 0; k < K + 2; ++k) wd[k] = oq[k * 32];
+        for (int k = 0; k < K + 2; ++k) wd[k] = oq[r3dsimt::umin(static_cast<uint32_t>(f + k), end) * 32];
       }
 #pragma unroll
       for (int k = 0; k < K + 1; ++k) pr[k] = r3dsimt::funnel_r(wd[k], wd[k + 1], par);
@@ -1189,13 +1205,13 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
     };
     for (int i = 0; i < maxlen; ++i) {
       const int st = i & (D - 1), st_in = (i + D - 1) & (D - 1);  // slots of this pixel and of the one issued now
-      const bool on = i < len;
+      const bool on = has(i), on_n = has(i + 1);
       const int at = static_cast<int>(rc.x & kRecOffset);
       const int lo = static_cast<int>(rc.y & 0xFFFFu);
       uint2 rn = rc;  // the next pixel's record
-      if (i + 1 < len) rn = recs[((i + 1) & (NR - 1)) * 32];
+      if (on_n) rn = recs[((i + 1) & (NR - 1)) * 32];
       const bool single_n = static_cast<int>(rn.x >> kRecShift) == UF;
-      const bool okn = i + 1 >= len || (single && single_n && ((rn.y ^ rc.y) & 0xFFFFu) == 0);
+      const bool okn = !on_n || (single_n && (!on || (single && ((rn.y ^ rc.y) & 0xFFFFu) == 0)));
       const bool fast_next = r3dsimt::ballot(!okn) == 0;
       pm = kSent2;
       uint32_t best[K];
@@ -1208,12 +1224,8 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
         for (int k = 0; k < K; ++k) cl[k] = r3dsimt::vmin2(prev[k], pen2);
         best_terms<K>(cl, pen2, pen2, one, p1x2, best);
         finish(best, st, at, on, true);
-        if (!fast_next) {
-          make_clean();
-          if (on) store_vec(i, 0, n, true);
-        }
+        if (!fast_next && on) store_vec(i, 0, n, true);
       } else {
-        make_clean();
         n = on ? units_of(rc, i) : 1;
         const bool multi = r3dsimt::ballot(n > UF) != 0;
         if (!multi) {
@@ -1253,8 +1265,9 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
       {
         const uint32_t mp = r3dsimt::vmin2(pm, r3dsimt::perm(pm, pm, 0x1032u));
         const int dn = static_cast<int>(rn.y >> 16) - static_cast<int>(rc.y >> 16);
-        pen2 = mp + lut[(dn < 0 ? -dn : dn) >> 8] * 0x10001u;
-        negmp = 0u - mp;
+        // A chain that starts at the next step keeps the zero clamp.
+        pen2 = on ? mp + lut[(dn < 0 ? -dn : dn) >> 8] * 0x10001u : 0u;
+        negmp = on ? 0u - mp : 0u;
       }
       lo_q = lo;
       num_q = 16 * n;
@@ -1274,79 +1287,118 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
 // as short as the others (in one launch with them: the chains of one direction
 // alone leave most of the SMs idle on a single pair) and saves the stored sum:
 // 11 bytes per cell against 12.
+//
+// One warp per tile row, a lane per pixel, the next 32 records loaded while the
+// present pixels are worked on (a search for the tile and a record per pixel
+// before its planes are known left the loads waiting on each other). The first
+// two units of a pixel stay in registers.
 template <bool TERMS>
 R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
     sgm_path_ranged_wta_kernel(const SgmMatch* R3D_RESTRICT matches, const SgmPathJob* R3D_RESTRICT jobs, int njobs,
-                               int64_t pixels, const uint2* R3D_RESTRICT rec, const uint8_t* R3D_RESTRICT cost,
+                               int64_t rows, const uint2* R3D_RESTRICT rec, const uint8_t* R3D_RESTRICT cost,
                                const uint16_t* R3D_RESTRICT sum, const uint8_t* R3D_RESTRICT terms, int64_t tstride,
                                const int* R3D_RESTRICT rowshift, int4* R3D_RESTRICT info, uint32_t* rkeys) {
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < pixels; i += stride) {
-    const int j = find_job(jobs, njobs, i, [](const SgmPathJob& q) { return q.px_off; });
+  const int lane = static_cast<int>(threadIdx.x & 31u);
+  const int wpb = static_cast<int>(blockDim.x) >> 5;
+  const int64_t nwarps = static_cast<int64_t>(gridDim.x) * wpb;
+  for (int64_t r = static_cast<int64_t>(blockIdx.x) * wpb + (threadIdx.x >> 5); r < rows; r += nwarps) {
+    const int j = find_job(jobs, njobs, r, [](const SgmPathJob& q) { return q.row_off; });
     const SgmPathJob& job = jobs[j];
     const SgmMatch& m = matches[job.match];
-    const int p = static_cast<int>(i - job.px_off);
-    const int y = p / job.w, x = p - y * job.w;
-    const uint2 rc = rec[i];
-    const int lo = static_cast<int>(rc.y & 0xFFFFu), nu = rec_units(rc, m, job, x, y), num = 16 * nu;
-    const int64_t off = static_cast<int64_t>(rc.x & kRecOffset) * 16;
-    const uint8_t* cp = cost + job.cell_off + off;
-    const uint8_t* tp = terms + job.cell_off + off;
-    const uint16_t* sp = sum + job.cell_off + off;
-    auto unit = [&](int u, uint32_t (&wv)[8]) { sum_unit<TERMS>(cp, tp, tstride, sp, u, wv); };
-    uint32_t wv[8];
-    uint32_t kmin = 0xFFFFFFFFu;
-    for (int u = nu - 1; u >= 0; --u) {  // ends with unit 0 in wv: the only one of most pixels
-      unit(u, wv);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const uint32_t e = static_cast<uint32_t>(16 * u + k);
-        kmin = r3dsimt::umin(kmin, r3dsimt::umin((wv[k] << 16) | e, (wv[k] & 0xFFFF0000u) | (e + 8)));
-      }
-      if (job.volume != nullptr) store_unit(job.volume + off + 16 * u, wv);
-    }
-    const int kb = static_cast<int>(kmin & 0xFFFFu);
-    const int km = kb > 0 ? kb - 1 : 0;
-    const int kp = kb + 1 < num ? kb + 1 : (num > 0 ? num - 1 : 0);
-    uint32_t sec = 0xFFFFu, sm = 0, spv = 0;
-    for (int u = 0; u < nu; ++u) {
-      if (u > 0) unit(u, wv);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          const int e = 16 * u + k + 8 * hf;
-          const uint32_t v = hf != 0 ? wv[k] >> 16 : wv[k] & 0xFFFFu;
-          if (e + 1 < kb || e > kb + 1) sec = r3dsimt::umin(sec, v);
-          if (e == km) sm = v;
-          if (e == kp) spv = v;
-        }
-      }
-    }
-    const Winner win{lo + kb, kmin >> 16, sec, sm, spv};
+    const int w = job.w, y = static_cast<int>(r - job.row_off);
+    const int64_t row_px = static_cast<int64_t>(y) * w;
     const RowInterval lv = m.bv[job.y0 + y];
-    const bool inside = job.x0 + x >= lv.first && job.x0 + x <= lv.last;
-    if (m.diagonal_lr) {
-      info[i] = pack_winner(win);
-      if (inside) {
-        uint32_t* keys = rkeys + job.rk_off + static_cast<int64_t>(y) * (job.w + m.nd);
-        const int base = x - lo + rowshift[job.row_off + y];
-        for (int u = 0; u < nu; ++u) {
-          unit(u, wv);
+    uint2 rn = make_uint2(0, 0);
+    if (lane < w) rn = rec[job.px_off + row_px + lane];
+    for (int x = lane; x < w; x += 32) {
+      const uint2 rc = rn;
+      if (x + 32 < w) rn = rec[job.px_off + row_px + x + 32];
+      const int64_t p = row_px + x;
+      const bool inside = job.x0 + x >= lv.first && job.x0 + x <= lv.last;
+      if (!inside && job.volume == nullptr) {
+        job.disp[p] = kInfF;
+        if (job.conf != nullptr) job.conf[p] = 0.0F;
+        continue;
+      }
+      const int lo = static_cast<int>(rc.y & 0xFFFFu), nu = rec_units(rc, m, job, x, y), num = 16 * nu;
+      const int64_t off = static_cast<int64_t>(rc.x & kRecOffset) * 16;
+      const uint8_t* cp = cost + job.cell_off + off;
+      const uint8_t* tp = terms + job.cell_off + off;
+      const uint16_t* sp = sum + job.cell_off + off;
+      uint32_t w0[8], w1[8], wx[8];
+      sum_unit<TERMS>(cp, tp, tstride, sp, 0, w0);
+      if (nu > 1) sum_unit<TERMS>(cp, tp, tstride, sp, 1, w1);
+      uint32_t kmin = 0xFFFFFFFFu;
+      auto least = [&](int u, const uint32_t (&wv)[8]) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const int e = 16 * u + k;
-            atomicMin(keys + (base - e), (wv[k] << 16) | static_cast<uint32_t>(x));
-            atomicMin(keys + (base - e - 8), (wv[k] & 0xFFFF0000u) | static_cast<uint32_t>(x));
+        for (int k = 0; k < 8; ++k) {
+          const uint32_t e = static_cast<uint32_t>(16 * u + k);
+          kmin = r3dsimt::umin(kmin, r3dsimt::umin((wv[k] << 16) | e, (wv[k] & 0xFFFF0000u) | (e + 8)));
+        }
+        if (job.volume != nullptr) store_unit(job.volume + off + 16 * u, wv);
+      };
+      least(0, w0);
+      if (nu > 1) least(1, w1);
+      for (int u = 2; u < nu; ++u) {
+        sum_unit<TERMS>(cp, tp, tstride, sp, u, wx);
+        least(u, wx);
+      }
+      const int kb = static_cast<int>(kmin & 0xFFFFu);
+      const int km = kb > 0 ? kb - 1 : 0;
+      const int kp = kb + 1 < num ? kb + 1 : num - 1;
+      uint32_t sec2 = 0xFFFFFFFFu, sm = 0, spv = 0;
+      auto second = [&](int u, const uint32_t (&wv)[8]) {
+        // Bit l: label l of the unit lies within kb -+ 1; its low and high
+        // byte in the two halves line up with the halves of word k >> k.
+        const int rel = kb - 1 - 16 * u;
+        const uint32_t ex = rel >= 16 || rel < -2 ? 0u : (rel >= 0 ? 7u << rel : 7u >> -rel);
+        const uint32_t ex2 = (ex & 0xFFu) | ((ex & 0xFF00u) << 8);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          sec2 = r3dsimt::vmin2(sec2, wv[k] | (((ex2 >> k) & 0x00010001u) * 0xFFFFu));
+        if ((km >> 4) == u) {
+          const uint32_t v = pick8(wv, km & 7);
+          sm = (km & 8) ? v >> 16 : v & 0xFFFFu;
+        }
+        if ((kp >> 4) == u) {
+          const uint32_t v = pick8(wv, kp & 7);
+          spv = (kp & 8) ? v >> 16 : v & 0xFFFFu;
+        }
+      };
+      second(0, w0);
+      if (nu > 1) second(1, w1);
+      for (int u = 2; u < nu; ++u) {
+        sum_unit<TERMS>(cp, tp, tstride, sp, u, wx);
+        second(u, wx);
+      }
+      const Winner win{lo + kb, kmin >> 16, r3dsimt::umin(sec2 & 0xFFFFu, sec2 >> 16), sm, spv};
+      if (m.diagonal_lr) {
+        info[job.px_off + p] = pack_winner(win);
+        if (inside) {
+          uint32_t* keys = rkeys + job.rk_off + static_cast<int64_t>(y) * (w + m.nd);
+          const int base = x - lo + rowshift[r];
+          auto post = [&](int u, const uint32_t (&wv)[8]) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const int e = 16 * u + k;
+              atomicMin(keys + (base - e), (wv[k] << 16) | static_cast<uint32_t>(x));
+              atomicMin(keys + (base - e - 8), (wv[k] & 0xFFFF0000u) | static_cast<uint32_t>(x));
+            }
+          };
+          post(0, w0);
+          if (nu > 1) post(1, w1);
+          for (int u = 2; u < nu; ++u) {
+            sum_unit<TERMS>(cp, tp, tstride, sp, u, wx);
+            post(u, wx);
           }
         }
+        continue;
       }
-      continue;
+      float d = kInfF, cf = 0.0F;
+      if (inside) accept_pixel(m, job, x, y, lo, num, win, nullptr, 0, d, cf);
+      job.disp[p] = d;
+      if (job.conf != nullptr) job.conf[p] = cf;
     }
-    float d = kInfF, cf = 0.0F;
-    if (inside) accept_pixel(m, job, x, y, lo, num, win, nullptr, 0, d, cf);
-    job.disp[p] = d;
-    if (job.conf != nullptr) job.conf[p] = cf;
   }
 }
 
@@ -1622,9 +1674,12 @@ void launch_sgm_path_wave(const SgmMatch* dm, const SgmPathWave& wave, int sms, 
 // ---------------------------------------------------------------- ranged launches
 namespace {
 
-// Largest number of resident CTAs per SM any ranged pass kernel is launched
-// with (the overflow has one slot per resident warp).
-constexpr int kRangedMaxPerSm = 24;
+// Resident one-warp CTAs per SM of a ranged pass launch (the overflow has one
+// slot per resident warp). Registers and shared memory allow 20 to 25; more
+// than 12 put more tiles in flight than the L2 holds the costs of (6048x4032:
+// 30.8 ms with 12, 31.5 with 16, 32.3 with 25; 33.5 with 6), smaller pairs do
+// not care.
+constexpr int kRangedMaxPerSm = 12;
 
 template <int K, int MODE>
 void launch_ranged_pass(const PassSet& ps, const SgmMatch* dm, const SgmPathJob* jobs, int njobs, const uint2* rec,
@@ -1716,9 +1771,9 @@ SgmPathBuffers sgm_path_ranged_buffers(int64_t cells, int64_t pixels, int64_t ke
   o += align256(static_cast<size_t>(rows) * 4);
   b.rowshift = o;
   o += align256(static_cast<size_t>(rows) * 4);
-  // Words of a wide vector's buffer (none where every vector fits shared
-  // memory), with the sentinels around it, for both item sizes.
-  b.overflow_words = maxnum > RangedRing<8, kTerm>::kVecLabels ? maxnum / 2 + 2 * RangedRing<16, kTerm>::kPadWords + 2 : 0;
+  // Words of a wide vector's buffer: the vector and a word of sentinels (none
+  // where every vector fits shared memory).
+  b.overflow_words = maxnum > RangedRing<8, kTerm>::kVecLabels ? maxnum / 2 + 1 : 0;
   b.overflow = o;
   // One slot (two buffers for each of 32 lanes) per resident warp.
   const int64_t slots = static_cast<int64_t>(sms) * kRangedMaxPerSm * (kRangedThreads / 32);
@@ -1768,8 +1823,8 @@ void launch_sgm_path_ranged_wave(const SgmMatch* dm, const SgmPathRangedWave& wa
       fail(R3DGPU_EINVAL, "stereo: bad ranged path kernel shape");
   }
   auto* wta = terms != nullptr ? sgm_path_ranged_wta_kernel<true> : sgm_path_ranged_wta_kernel<false>;
-  R3D_LAUNCH(wta, dim3(resident_grid(wta, sms, wave.pixels, kPathThreads)), dim3(kPathThreads), 0, s, dm, wave.jobs,
-             wave.njobs, wave.pixels, rec, cost, sum, terms, B.term_stride, rowshift, info, rkeys);
+  R3D_LAUNCH(wta, dim3(resident_grid(wta, sms, wave.rows, kPathThreads / 32)), dim3(kPathThreads), 0, s, dm, wave.jobs,
+             wave.njobs, wave.rows, rec, cost, sum, terms, B.term_stride, rowshift, info, rkeys);
   launched("sgm_path_ranged_wta_kernel");
   if (wave.keys > 0) {  // matches with the diagonal left-right check
     R3D_LAUNCH(sgm_path_ranged_accept_kernel,
