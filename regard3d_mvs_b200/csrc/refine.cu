@@ -1,21 +1,29 @@
 // Patch-based depth refinement (r3dgpu_refine_depth_map) and its input images
 // (r3dgpu_make_refinement_image), the reference's src/r3d/mvs/refinement.cpp.
 //
-// One warp per depth-map pixel. The window samples (25 for the default 9 x 9
-// window at step 2, 49 for a 7 x 7 window at step 1, at most 225) are spread
-// over the lanes: each lane warps, samples and normalises its samples, and
-// every sum of the NCC and of the Gauss-Newton terms is an xor-butterfly
-// reduction. After a butterfly every lane holds the same bits (the partial
-// sums meet in mirrored order, and IEEE addition commutes), so the per-pixel
-// control flow — view selection, the damped Gauss-Newton loop with step
-// shrinking, the acceptance test — is uniform over the warp and runs in every
-// lane, with no shared memory and no barriers. The window terms compute in
-// double precision as the reference does; with fp32 = 1 the Gauss-Newton
-// terms (Jacobian, J^T J, J^T e: the bulk of the work) are float while the
-// objective that decides which steps are taken (sampled values, window
-// normalisation, NCC) and the 3 x 3 LDL^T solve stay double. Sums run in a different order than the
-// reference's sequential loops, so results agree with a double-precision CPU
-// restatement to rounding, not bit for bit.
+// Four depth-map pixels per warp, 8 lanes each. The lanes of a pixel split into
+// one group per view (two lanes each for 4 views); a lane warps, samples and
+// normalises every second (or so) of its view's window samples (25 for the
+// default 9 x 9 window at step 2, 49 for a 7 x 7 window at step 1, at most
+// 225), and every sum of the NCC and of the Gauss-Newton terms is an
+// xor-butterfly over the pixel's lanes. After a butterfly these hold the same
+// bits (the partial sums meet in mirrored order, and IEEE addition commutes),
+// so the per-pixel decisions — view selection, the damped Gauss-Newton loop
+// with step shrinking, the acceptance test — are the same in all of them. The
+// four pixels run in step: a pixel that is done idles until the last is.
+//
+// Four pixels per warp against one: the warp-wide set-up of a view's warp, the
+// 3 x 3 solve and the butterflies, half of the instructions of a warp per
+// pixel, serve four pixels at once (786,432 pixels of 49 samples in 4 views:
+// 12.5 G warp instructions with one pixel per warp).
+//
+// The window terms compute in double precision as the reference does; with
+// fp32 = 1 the Gauss-Newton terms (Jacobian, J^T J, J^T e: the bulk of the
+// work) are float while the objective that decides which steps are taken
+// (sampled values, window normalisation, NCC) and the 3 x 3 LDL^T solve stay
+// double. Sums run in a different order than the reference's sequential loops,
+// so results agree with a double-precision CPU restatement to rounding, not
+// bit for bit.
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -34,13 +42,57 @@ constexpr int kMaxSamples = 225;  // refinement.cpp:21
 constexpr int kMaxViews = 8;      // refinement.cpp:22
 constexpr double kDiscontinuity = 0.05;
 enum : int { kInput, kRefined, kUnconfirmed, kCounters };
+constexpr int kSlots = 128, kSlotStride = 4;  // copies of the counters (one address takes an addition at a time)
+constexpr int kPixels = 4;                    // pixels per warp
+constexpr int kLanes = 32 / kPixels;          // lanes per pixel (at least one per view)
+constexpr int kRefineThreads = 128;
+static_assert(kLanes >= kMaxViews, "a lane per view");
+
+// A view's pixel as the kernels read it: intensity and derivatives, the
+// intensity already in double (a conversion runs at a quarter of the double
+// rate, and a sample has four): 16 bytes with float derivatives, 32 with double
+// ones.
+template <class T>
+struct Texels;
+template <>
+struct Texels<float> {
+  static constexpr int kWords = 1;  // float4 words per pixel
+  static R3D_DEVICE void load(const float4* p, double& v, float& gx, float& gy) {
+    const float4 a = __ldg(p);
+    memcpy(&v, &a, 8);
+    gx = a.z;
+    gy = a.w;
+  }
+  static R3D_DEVICE void store(float4* p, float v, float gx, float gy) {
+    const double d = v;
+    float4 a;
+    memcpy(&a, &d, 8);
+    a.z = gx;
+    a.w = gy;
+    *p = a;
+  }
+};
+template <>
+struct Texels<double> {
+  static constexpr int kWords = 2;
+  static R3D_DEVICE void load(const float4* p, double& v, double& gx, double& gy) {
+    const float4 a = __ldg(p), b = __ldg(p + 1);
+    memcpy(&v, &a, 8);
+    memcpy(&gx, reinterpret_cast<const char*>(&a) + 8, 8);
+    memcpy(&gy, &b, 8);
+  }
+  static R3D_DEVICE void store(float4* p, float v, float gx, float gy) {
+    const double d[4] = {v, gx, gy, 0.0};
+    memcpy(p, d, 32);
+  }
+};
 
 // Plane-induced warp into a view (refinement.cpp:24-30): h = m (qx, qy, 1) + b w(q).
 struct ViewGeo {
   double m[9];  // K_j R_j R_0^T K_0^-1, row-major
   double b[3];  // K_j R_j (C_0 - C_j)
-  const float4* data;  // (intensity, d/dx, d/dy, 0) per pixel, repacked from the 3-channel image
-  int64_t stride;      // in pixels
+  const float4* data;  // the view's texels (repack_kernel)
+  int64_t stride;      // texels per row
   int width, height;
 };
 
@@ -71,30 +123,22 @@ R3D_DEVICE T shfl_t(T v, int src) {
   return v;
 }
 
-// Butterfly sums of K values over aligned groups of `width` lanes (masks
-// below width), and from there across the groups (masks width .. 16). After
-// each, all lanes of a group (or of the warp) hold the same bits: the partial
-// sums meet in mirrored order and IEEE addition commutes.
+// Butterfly sums of K values over aligned groups of `to / from` lanes: masks
+// from .. to / 2 (below a view's lane count: over its lanes; from there on: over
+// the pixel's views). After them all lanes of a group hold the same bits: the
+// partial sums meet in mirrored order and IEEE addition commutes.
 template <class T, int K>
-R3D_DEVICE void sums_below(T (&v)[K], int width) {
-  for (int m = 1; m < width; m <<= 1) {
-#pragma unroll
-    for (int i = 0; i < K; ++i) v[i] += shfl_xor_t(v[i], m);
-  }
-}
-
-template <class T, int K>
-R3D_DEVICE void sums_from(T (&v)[K], int width) {
-  for (int m = width; m < 32; m <<= 1) {
+R3D_DEVICE void sums(T (&v)[K], int from, int to) {
+  for (int m = from; m < to; m <<= 1) {
 #pragma unroll
     for (int i = 0; i < K; ++i) v[i] += shfl_xor_t(v[i], m);
   }
 }
 
 template <class T>
-R3D_DEVICE T warp_sum(T v) {
+R3D_DEVICE T pixel_sum(T v) {
   T a[1] = {v};
-  sums_below(a, 32);
+  sums(a, 1, kLanes);
   return a[0];
 }
 
@@ -105,9 +149,27 @@ R3D_DEVICE bool finite_d(double v) { return v - v == 0.0; }
 // Smallest power of two >= m (m in 1..8): the number of lane groups.
 R3D_DEVICE int groups_for(int m) { return m <= 1 ? 1 : (m <= 2 ? 2 : (m <= 4 ? 4 : 8)); }
 
-// Per warp in shared memory: the normalised base window n0[s] and the
-// window coordinates (offset / radius) of each window column.
-constexpr int kWarpTableDoubles = kMaxSamples + 16;
+// In shared memory, per pixel the normalised base window n0[s] (kMaxSamples
+// doubles at most, p.n used) and per warp the window coordinates (offset /
+// radius) of each window column, kept as doubles.
+constexpr int kMaxSide = 16;
+
+// floor(q) of |q| < 2^22 as float and as int, without the conversion unit:
+// adding 1.5 * 2^23 rounds to a whole number that the sum's low bits hold.
+R3D_DEVICE float floor_small(float q, int& i) {
+  const float magic = 12582912.0F;
+  const float t = __fadd_rn(q, magic);
+  float r = __fsub_rn(t, magic);
+  int bits, mbits;
+  memcpy(&bits, &t, 4);
+  memcpy(&mbits, &magic, 4);
+  i = bits - mbits;
+  if (r > q) {
+    r = __fsub_rn(r, 1.0F);
+    --i;
+  }
+  return r;
+}
 
 // One view's terms at plane theta (refinement.cpp:46-152), computed by the
 // `gsize` lanes of a group: lane `gl` of the group takes the window samples
@@ -127,8 +189,8 @@ constexpr int kWarpTableDoubles = kMaxSamples + 16;
 // variance well conditioned); the Jacobian moments are T.
 template <class T, bool JAC>
 R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y, const double* theta,
-                               const Params& p, const double* table, double shift, int gl, int gsize, bool& valid,
-                               double& ncc_out, double* hh, double* gg) {
+                               const Params& p, const double* n0s, const double* coord, double shift, int gl,
+                               int gsize, bool& valid, double& ncc_out, double* hh, double* gg) {
   double ob[3] = {0.0, 0.0, 0.0};
   T jm[15];
 #pragma unroll
@@ -140,8 +202,6 @@ R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y
             m4 = static_cast<T>(g.m[4]), m6 = static_cast<T>(g.m[6]), m7 = static_cast<T>(g.m[7]);
     const T max_x = static_cast<T>(g.width - 1), max_y = static_cast<T>(g.height - 1);
     const T th0 = static_cast<T>(theta[0]), th1 = static_cast<T>(theta[1]), th2 = static_cast<T>(theta[2]);
-    const T hc0 = static_cast<T>(row3(g.m, 0, x, y, 1.0)), hc1 = static_cast<T>(row3(g.m, 1, x, y, 1.0)),
-            hc2 = static_cast<T>(row3(g.m, 2, x, y, 1.0));
     // In float, pixel positions of a few thousand carry about 1e-4 px of
     // rounding. The float path therefore projects the window centre at the
     // current depth in double once and each sample as a small float offset:
@@ -149,7 +209,7 @@ R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y
     const bool rel = sizeof(T) == 4;
     double hz = 0.0;
     int ic0 = 0, ic1 = 0;
-    T fc0 = 0, fc1 = 0, cf0 = 0, cf1 = 0, hzf = 0;
+    T fc0 = 0, fc1 = 0, cf0 = 0, cf1 = 0, hzf = 0, ft0 = 0, ft1 = 0, hc0 = 0, hc1 = 0, hc2 = 0;
     if (rel) {
       const double H0 = row3(g.m, 0, x, y, 1.0) + g.b[0] * theta[0];
       const double H1 = row3(g.m, 1, x, y, 1.0) + g.b[1] * theta[0];
@@ -165,14 +225,19 @@ R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y
           cf0 = static_cast<T>(c0);
           cf1 = static_cast<T>(c1);
           hzf = static_cast<T>(hz);
+          ft0 = static_cast<T>(f0);
+          ft1 = static_cast<T>(f1);
         } else {
           hz = 0.0;
         }
       }
     }
     const bool offsets = rel && hz > 0.0;
-    const double* n0s = table;
-    const double* coord = table + kMaxSamples;  // offset / radius of window column c
+    if (!offsets) {
+      hc0 = static_cast<T>(row3(g.m, 0, x, y, 1.0));
+      hc1 = static_cast<T>(row3(g.m, 1, x, y, 1.0));
+      hc2 = static_cast<T>(row3(g.m, 2, x, y, 1.0));
+    }
     // Window column and row of sample s, advanced by gsize per step.
     int col = gl % p.side, row = gl / p.side;
     const int dcol = gsize % p.side, drow = gsize / p.side;
@@ -203,13 +268,15 @@ R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y
           bad = true;
           break;
         }
-        const T fl0 = floor(q0), fl1 = floor(q1);
-        ix = ic0 + static_cast<int>(fl0);
-        iy = ic1 + static_cast<int>(fl1);
+        int k0, k1;
+        const T fl0 = floor_small(static_cast<float>(q0), k0), fl1 = floor_small(static_cast<float>(q1), k1);
+        ix = ic0 + k0;
+        iy = ic1 + k1;
         fx = q0 - fl0;
         fy = q1 - fl1;
-        px = static_cast<T>(ix) + fx;
-        py = static_cast<T>(iy) + fy;
+        // ix and iy as floats: exact wherever they are inside an image.
+        px = (ft0 + fl0) + fx;
+        py = (ft1 + fl1) + fy;
         // px in [0, width - 1) and py in [0, height - 1), as below.
         if (!(ix >= 0 && iy >= 0 && ix <= g.width - 2 && iy <= g.height - 2)) {
           bad = true;
@@ -236,20 +303,26 @@ R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y
         fx = px - static_cast<T>(ix);
         fy = py - static_cast<T>(iy);
       }
-      const float4* r0 = g.data + static_cast<int64_t>(iy) * g.stride + ix;
-      const float4 c00 = __ldg(r0), c01 = __ldg(r0 + 1), c10 = __ldg(r0 + g.stride), c11 = __ldg(r0 + g.stride + 1);
+      constexpr int TW = Texels<T>::kWords;
+      const float4* r0 = g.data + (static_cast<int64_t>(iy) * g.stride + ix) * TW;
+      const float4* r1 = r0 + g.stride * TW;
+      double v00, v01, v10, v11;
+      T x00, x01, x10, x11, y00, y01, y10, y11;
+      Texels<T>::load(r0, v00, x00, y00);
+      Texels<T>::load(r0 + TW, v01, x01, y01);
+      Texels<T>::load(r1, v10, x10, y10);
+      Texels<T>::load(r1 + TW, v11, x11, y11);
       const double fxd = fx, fyd = fy;
-      const double raw = ((1.0 - fyd) * ((1.0 - fxd) * static_cast<double>(c00.x) + fxd * static_cast<double>(c01.x)) +
-                          fyd * ((1.0 - fxd) * static_cast<double>(c10.x) + fxd * static_cast<double>(c11.x))) -
-                         shift;
+      const double raw =
+          ((1.0 - fyd) * ((1.0 - fxd) * v00 + fxd * v01) + fyd * ((1.0 - fxd) * v10 + fxd * v11)) - shift;
       const double n0 = n0s[s];
       ob[0] += raw;
       ob[1] += raw * raw;
       ob[2] += raw * n0;
       if (JAC) {
         const T ax = T(1) - fx, ay = T(1) - fy;
-        const T gx = ay * (ax * c00.y + fx * c01.y) + fy * (ax * c10.y + fx * c11.y);
-        const T gy = ay * (ax * c00.z + fx * c01.z) + fy * (ax * c10.z + fx * c11.z);
+        const T gx = ay * (ax * x00 + fx * x01) + fy * (ax * x10 + fx * x11);
+        const T gy = ay * (ax * y00 + fx * y01) + fy * (ax * y10 + fx * y11);
         const T dpx = (b0 - px * b2) * inv_z, dpy = (b1 - py * b2) * inv_z;
         const T dv = gx * dpx + gy * dpy;
         const T a0 = dv, a1 = dv * sx, a2 = dv * sy;
@@ -276,8 +349,8 @@ R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y
   const uint32_t lane = r3dsimt::lane_id();
   const uint32_t gmask = (gsize == 32 ? 0xFFFFFFFFu : ((1u << gsize) - 1u) << (lane & ~static_cast<uint32_t>(gsize - 1)));
   const bool group_bad = (r3dsimt::ballot(bad) & gmask) != 0;
-  sums_below(ob, gsize);
-  if (JAC) sums_below(jm, gsize);
+  sums(ob, 1, gsize);
+  if (JAC) sums(jm, 1, gsize);
   for (int i = 0; i < 6; ++i) hh[i] = 0.0;
   for (int i = 0; i < 3; ++i) gg[i] = 0.0;
   ncc_out = 0.0;
@@ -389,153 +462,154 @@ R3D_DEVICE void solve_damped(const double* hh, const double* gg, double* delta) 
   for (int i = 0; i < 3; ++i) delta[perm[i]] = -y[i];
 }
 
-// One warp per depth-map pixel; per warp a table of kWarpTableDoubles
-// doubles in dynamic shared memory.
+// Dynamic shared memory: per pixel of the block p.n doubles, then per warp
+// kMaxSide doubles.
 template <class T>
-R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN(256, 2)
+R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN(kRefineThreads, 4)
     refine_kernel(const float* R3D_RESTRICT input, float* depth, float* conf, int64_t stride,
                   const float* R3D_RESTRICT base, int64_t bstride, const ViewGeo* R3D_RESTRICT views, Params p,
                   unsigned long long* counters) {
   R3D_DYNAMIC_SMEM(smem);
-  const int64_t pix = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  if (pix >= static_cast<int64_t>(p.width) * p.height) return;  // whole warp
-  const int lane = static_cast<int>(r3dsimt::lane_id());
-  const bool lead = lane == 0;
-  double* table = reinterpret_cast<double*>(smem) + (threadIdx.x >> 5) * kWarpTableDoubles;
+  const int lane = static_cast<int>(r3dsimt::lane_id()), warp = static_cast<int>(threadIdx.x >> 5);
+  const int sub = lane / kLanes, wl = lane % kLanes;  // the pixel of the warp, the lane of the pixel
+  const bool lead = wl == 0;
+  const int64_t total = static_cast<int64_t>(p.width) * p.height;
+  const int64_t first = ((static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * kPixels;
+  if (first >= total) return;  // whole warp
+  const int64_t pix = first + sub < total ? first + sub : first;
   const int y = static_cast<int>(pix / p.width), x = static_cast<int>(pix - static_cast<int64_t>(y) * p.width);
   const float z0 = input[pix];
-  if (!(z0 > 0.0F)) return;
+  const bool valid_px = first + sub < total && z0 > 0.0F;
   const int64_t at = static_cast<int64_t>(y) * stride + x;
-  if (lead) {
-    atomicAdd(counters + kInput, 1ULL);
-    conf[at] = 0.0F;
-  }
+  unsigned long long* const slot = counters + (blockIdx.x % kSlots) * kSlotStride;
+  auto count = [&](int counter, bool pred) {  // pixels of the warp with pred (one vote each)
+    const uint32_t b = r3dsimt::ballot(pred && lead);
+    if (lane == 0 && b != 0) atomicAdd(slot + counter, static_cast<unsigned long long>(r3dsimt::popc(b)));
+  };
+  count(kInput, valid_px);
+  if (valid_px && lead) conf[at] = 0.0F;
   const int r = p.radius;
-  if (p.num_views == 0 || x < r || y < r || x >= p.width - r || y >= p.height - r) return;
+  bool live = valid_px && p.num_views > 0 && x >= r && y >= r && x < p.width - r && y < p.height - r;
+  if (r3dsimt::ballot(live) == 0) return;
 
-  // The normalised base window (sample s = lane + 32 k) into the table.
-  double nb[kMaxSamples / 32 + 1];
+  // The normalised base window into the pixel's table.
+  double* const n0s = reinterpret_cast<double*>(smem) + static_cast<size_t>(warp * kPixels + sub) * p.n;
+  double* const coord =
+      reinterpret_cast<double*>(smem) + static_cast<size_t>(blockDim.x / 32 * kPixels) * p.n + warp * kMaxSide;
   double sum = 0.0;
-#pragma unroll
-  for (int k = 0; k < kMaxSamples / 32 + 1; ++k) {
-    const int s = lane + 32 * k;
-    nb[k] = 0.0;
-    if (s < p.n) {
-      const int dx = (s % p.side) * p.step - r, dy = (s / p.side) * p.step - r;
-      nb[k] = base[static_cast<int64_t>(y + dy) * bstride + 3 * (x + dx)];
-      sum += nb[k];
-    }
+  for (int s = wl; s < p.n; s += kLanes) {
+    const int dx = (s % p.side) * p.step - r, dy = (s / p.side) * p.step - r;
+    const double v = live ? base[static_cast<int64_t>(y + dy) * bstride + 3 * (x + dx)] : 0.0;
+    n0s[s] = v;
+    sum += v;
   }
-  const double mean = warp_sum(sum) / p.n;
+  const double mean = pixel_sum(sum) / p.n;
   double norm2 = 0.0;
-#pragma unroll
-  for (int k = 0; k < kMaxSamples / 32 + 1; ++k)
-    if (lane + 32 * k < p.n) {
-      nb[k] -= mean;
-      norm2 += nb[k] * nb[k];
-    }
-  norm2 = warp_sum(norm2);
-  if (norm2 < p.min_texture2n) return;
+  for (int s = wl; s < p.n; s += kLanes) {
+    const double v = n0s[s] - mean;
+    n0s[s] = v;
+    norm2 += v * v;
+  }
+  norm2 = pixel_sum(norm2);
+  live = live && !(norm2 < p.min_texture2n);
   const double inv_norm = 1.0 / sqrt(norm2);
-#pragma unroll
-  for (int k = 0; k < kMaxSamples / 32 + 1; ++k)
-    if (lane + 32 * k < p.n) table[lane + 32 * k] = nb[k] * inv_norm;
-  if (lane < p.side) table[kMaxSamples + lane] = static_cast<double>(lane * p.step - r) / r;
+  for (int s = wl; s < p.n; s += kLanes) n0s[s] *= inv_norm;
+  if (lane < p.side) coord[lane] = static_cast<double>(lane * p.step - r) / r;
   r3dsimt::syncwarp();
+  if (r3dsimt::ballot(live) == 0) return;
 
   const double w0 = 1.0 / z0;
-  const double theta0[3] = {w0, r * initial_slope(input, p.width, p.height, x, y, 1, 0),
-                            r * initial_slope(input, p.width, p.height, x, y, 0, 1)};
+  const double theta0[3] = {w0, live ? r * initial_slope(input, p.width, p.height, x, y, 1, 0) : 0.0,
+                            live ? r * initial_slope(input, p.width, p.height, x, y, 0, 1) : 0.0};
   const double xd = x, yd = y;
-  double hh_v[6], gg_v[3];
 
-  // Local view selection at the initial plane: all views at once, one lane
-  // group per view.
-  int used[kMaxViews];
+  // The lane's view: gsize lanes each, the same for all pixels of the launch.
+  const int gsize = kLanes / groups_for(p.num_views);
+  const int my_t = wl / gsize, gl = wl % gsize;
+  const ViewGeo& my_view = views[my_t < p.num_views ? my_t : 0];
+  const uint32_t px_mask = (1u << kLanes) - 1u;
+
+  // Local view selection at the initial plane.
+  double hh_v[6], gg_v[3];
+  bool use = live && my_t < p.num_views;  // the lane's view is used by its pixel
   int m = 0;
   double s0 = 0.0;
   {
-    const int gsize = 32 / groups_for(p.num_views);
-    const int t = lane / gsize;
-    const bool active = t < p.num_views;
     bool valid;
     double ncc;
-    evaluate_group<T, false>(views[active ? t : 0], active, xd, yd, theta0, p, table, mean, lane % gsize, gsize,
-                             valid, ncc, hh_v, gg_v);
-    const uint32_t ok = r3dsimt::ballot(active && valid && ncc >= p.min_ncc);
+    evaluate_group<T, false>(my_view, use, xd, yd, theta0, p, n0s, coord, mean, gl, gsize, valid, ncc, hh_v, gg_v);
+    use = use && valid && ncc >= p.min_ncc;
+    const uint32_t ok = (r3dsimt::ballot(use) >> (sub * kLanes)) & px_mask;
     for (int j = 0; j < p.num_views; ++j) {
-      const double nj = shfl_t(ncc, j * gsize);  // group j's value
+      const double nj = shfl_t(ncc, sub * kLanes + j * gsize);  // group j's value
       if ((ok >> (j * gsize)) & 1u) {
-        used[m++] = j;
+        ++m;
         s0 += nj;
       }
     }
   }
-  if (m == 0) {
-    if (p.drop_unconfirmed && lead) {
-      depth[at] = 0.0F;
-      atomicAdd(counters + kUnconfirmed, 1ULL);
-    }
-    return;
-  }
-  s0 /= m;
-  if (lead) conf[at] = static_cast<float>(s0);
-  double max_motion = 0.0;
-  for (int t = 0; t < m; ++t) max_motion = fmax(max_motion, centre_motion(views[used[t]], xd, yd, w0));
+  const bool unconfirmed = live && m == 0 && p.drop_unconfirmed != 0;
+  count(kUnconfirmed, unconfirmed);
+  if (unconfirmed && lead) depth[at] = 0.0F;
+  live = live && m > 0;
+  if (r3dsimt::ballot(live) == 0) return;
+  const int views_used = m > 0 ? m : 1;
+  s0 /= views_used;
+  if (live && lead) conf[at] = static_cast<float>(s0);
+  double max_motion = use ? centre_motion(my_view, xd, yd, w0) : 0.0;
+  for (int o = gsize; o < kLanes; o <<= 1) max_motion = fmax(max_motion, shfl_xor_t(max_motion, o));
 
-  // Mean NCC and Gauss-Newton terms over the used views (one lane group
-  // each); -inf if a view drops out.
-  const int gsize = 32 / groups_for(m);
-  const int my_t = lane / gsize;
-  const bool my_active = my_t < m;
-  const ViewGeo& my_view = views[used[my_active ? my_t : 0]];
-  auto evaluate = [&](const double* theta, double* hh, double* gg) {
+  // Mean NCC and Gauss-Newton terms over the used views; -inf if a view drops out.
+  auto evaluate = [&](const double* theta, bool active, double* hh, double* gg) {
     bool valid;
     double ncc;
-    evaluate_group<T, true>(my_view, my_active, xd, yd, theta, p, table, mean, lane % gsize, gsize, valid, ncc,
-                            hh_v, gg_v);
-    if (r3dsimt::ballot(!valid) != 0) return -__builtin_huge_val();
+    evaluate_group<T, true>(my_view, active && use, xd, yd, theta, p, n0s, coord, mean, gl, gsize, valid, ncc, hh_v,
+                            gg_v);
+    const bool dropped = ((r3dsimt::ballot(!valid) >> (sub * kLanes)) & px_mask) != 0;
     double tot[10] = {ncc, hh_v[0], hh_v[1], hh_v[2], hh_v[3], hh_v[4], hh_v[5], gg_v[0], gg_v[1], gg_v[2]};
-    sums_from(tot, gsize);
+    sums(tot, gsize, kLanes);
     for (int i = 0; i < 6; ++i) hh[i] = tot[1 + i];
     for (int i = 0; i < 3; ++i) gg[i] = tot[7 + i];
-    return tot[0] / m;
+    return dropped ? -__builtin_huge_val() : tot[0] / views_used;
   };
 
   double hh[6], gg[3];
   double best[3] = {theta0[0], theta0[1], theta0[2]};
-  double best_score = evaluate(best, hh, gg);
-  if (!finite_d(best_score)) return;
+  double best_score = evaluate(best, live, hh, gg);
+  live = live && finite_d(best_score);
   double scale = 1.0;
-  for (int it = 0; it < p.iterations; ++it) {
+  bool stepping = live;
+  for (int it = 0; it < p.iterations && r3dsimt::ballot(stepping) != 0; ++it) {
     double delta[3];
     solve_damped(hh, gg, delta);
-    if (!(finite_d(delta[0]) && finite_d(delta[1]) && finite_d(delta[2]))) break;
+    stepping = stepping && finite_d(delta[0]) && finite_d(delta[1]) && finite_d(delta[2]);
     // At most one pixel of motion per step at the window border.
     const double motion = max_motion * ((fabs(delta[0]) + fabs(delta[1])) + fabs(delta[2]));
     if (motion > 1.0)
       for (int i = 0; i < 3; ++i) delta[i] /= motion;
     for (int i = 0; i < 3; ++i) delta[i] *= scale;
-    if (max_motion * ((fabs(delta[0]) + fabs(delta[1])) + fabs(delta[2])) < 1e-3) break;
+    if (max_motion * ((fabs(delta[0]) + fabs(delta[1])) + fabs(delta[2])) < 1e-3) stepping = false;
     double h2[6], g2[3];
     const double cand[3] = {best[0] + delta[0], best[1] + delta[1], best[2] + delta[2]};
-    const double score = evaluate(cand, h2, g2);
-    if (score > best_score) {
-      for (int i = 0; i < 3; ++i) best[i] = cand[i];
-      best_score = score;
-      for (int i = 0; i < 6; ++i) hh[i] = h2[i];
-      for (int i = 0; i < 3; ++i) gg[i] = g2[i];
-      scale = 1.0;
-    } else {
-      scale *= 0.25;
+    const double score = evaluate(cand, stepping, h2, g2);
+    if (stepping) {
+      if (score > best_score) {
+        for (int i = 0; i < 3; ++i) best[i] = cand[i];
+        best_score = score;
+        for (int i = 0; i < 6; ++i) hh[i] = h2[i];
+        for (int i = 0; i < 3; ++i) gg[i] = g2[i];
+        scale = 1.0;
+      } else {
+        scale *= 0.25;
+      }
     }
   }
-  if (best_score > s0 + p.min_gain && best[0] > 0.0 && max_motion * fabs(best[0] - w0) <= p.max_shift_px) {
-    if (lead) {
-      depth[at] = static_cast<float>(1.0 / best[0]);
-      conf[at] = static_cast<float>(best_score);
-      atomicAdd(counters + kRefined, 1ULL);
-    }
+  const bool taken =
+      live && best_score > s0 + p.min_gain && best[0] > 0.0 && max_motion * fabs(best[0] - w0) <= p.max_shift_px;
+  count(kRefined, taken);
+  if (taken && lead) {
+    depth[at] = static_cast<float>(1.0 / best[0]);
+    conf[at] = static_cast<float>(best_score);
   }
 }
 
@@ -580,13 +654,13 @@ R3D_GLOBAL void gradient_kernel(const float* gray, int64_t gstride, int w, int h
   o[2] = __fmul_rn(__fsub_rn(down[x], up[x]), h > 1 ? sy : 0.0F);
 }
 
-// A view's 3-channel refinement image as one float4 per pixel (one 16-byte
-// load per bilinear corner in the refinement kernel).
+// A view's 3-channel refinement image as texels.
+template <class T>
 R3D_GLOBAL void repack_kernel(const float* in, int64_t istride, int w, int h, float4* out) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= w || y >= h) return;
   const float* p = in + static_cast<int64_t>(y) * istride + 3 * x;
-  out[static_cast<int64_t>(y) * w + x] = make_float4(p[0], p[1], p[2], 0.0F);
+  Texels<T>::store(out + (static_cast<int64_t>(y) * w + x) * Texels<T>::kWords, p[0], p[1], p[2]);
 }
 
 // ------------------------------------------------------------------ host side
@@ -599,7 +673,7 @@ struct Scratch {
 
 Scratch& scratch() {
   thread_local Scratch s;
-  s.counters.reserve(kCounters);
+  s.counters.reserve(kSlots * kSlotStride);
   s.views.reserve(kMaxViews);
   return s;
 }
@@ -643,11 +717,11 @@ template <class T>
 void launch_refine(const float* input, float* depth, float* conf, int64_t stride, const float* base,
                    int64_t bstride, const ViewGeo* views, const Params& p, unsigned long long* counters,
                    cudaStream_t s) {
-  const int64_t warps = static_cast<int64_t>(p.width) * p.height;
-  const size_t smem = sizeof(double) * kWarpTableDoubles * 8;
+  constexpr int per_block = kRefineThreads / 32 * kPixels;
+  const size_t smem = sizeof(double) * (static_cast<size_t>(per_block) * p.n + kRefineThreads / 32 * kMaxSide);
   auto kernel = refine_kernel<T>;
-  R3D_LAUNCH(kernel, static_cast<unsigned>(ceil_div64(warps, 8)), 256, smem, s, input, depth, conf, stride, base,
-             bstride, views, p, counters);
+  R3D_LAUNCH(kernel, static_cast<unsigned>(ceil_div64(static_cast<int64_t>(p.width) * p.height, per_block)),
+             kRefineThreads, smem, s, input, depth, conf, stride, base, bstride, views, p, counters);
   launched(sizeof(T) == 8 ? "refine_kernel<f64>" : "refine_kernel<f32>");
 }
 
@@ -677,22 +751,24 @@ void refine(float* depth, float* conf, int64_t stride, const r3dgpu_pinhole_came
       fail(R3DGPU_EINVAL, "refinement: view " + std::to_string(j) + " has no image");
     geo[j] = view_geometry(cam, v);
   }
-  R3D_CUDA(cudaMemsetAsync(sc.counters.get(), 0, sizeof(unsigned long long) * kCounters, s));
+  R3D_CUDA(cudaMemsetAsync(sc.counters.get(), 0, sizeof(unsigned long long) * kSlots * kSlotStride, s));
   if (w > 0 && h > 0) {
-    // The views' images as one float4 per pixel.
+    // The views' images as texels.
+    const size_t words = o.fp32 ? Texels<float>::kWords : Texels<double>::kWords;
     size_t total = 0;
     for (int j = 0; j < nv; ++j)
-      total += static_cast<size_t>(views[j].camera.intrinsics.width) * views[j].camera.intrinsics.height;
+      total += words * static_cast<size_t>(views[j].camera.intrinsics.width) * views[j].camera.intrinsics.height;
     sc.packed.reserve(total > 0 ? total : 1);
     size_t off = 0;
     for (int j = 0; j < nv; ++j) {
       const int vw = views[j].camera.intrinsics.width, vh = views[j].camera.intrinsics.height;
       float4* dst = sc.packed.get() + off;
       const dim3 b(32, 8), g(static_cast<unsigned>(ceil_div(vw, 32)), static_cast<unsigned>(ceil_div(vh, 8)));
-      R3D_LAUNCH(repack_kernel, g, b, 0, s, views[j].data, views[j].stride, vw, vh, dst);
+      auto repack = o.fp32 ? repack_kernel<float> : repack_kernel<double>;
+      R3D_LAUNCH(repack, g, b, 0, s, views[j].data, views[j].stride, vw, vh, dst);
       launched("repack_kernel");
       geo[j].data = dst;
-      off += static_cast<size_t>(vw) * vh;
+      off += words * static_cast<size_t>(vw) * vh;
     }
     if (nv > 0)
       R3D_CUDA(cudaMemcpyAsync(sc.views.get(), geo, sizeof(ViewGeo) * nv, cudaMemcpyHostToDevice, s));
@@ -708,9 +784,11 @@ void refine(float* depth, float* conf, int64_t stride, const r3dgpu_pinhole_came
       launch_refine<double>(sc.input.get(), depth, conf, stride, base.data, base.stride, sc.views.get(), p,
                             sc.counters.get(), s);
   }
-  unsigned long long c[kCounters];
-  R3D_CUDA(cudaMemcpyAsync(c, sc.counters.get(), sizeof(c), cudaMemcpyDeviceToHost, s));
+  unsigned long long slots[kSlots * kSlotStride], c[kCounters] = {};
+  R3D_CUDA(cudaMemcpyAsync(slots, sc.counters.get(), sizeof(slots), cudaMemcpyDeviceToHost, s));
   R3D_CUDA(cudaStreamSynchronize(s));
+  for (int k = 0; k < kSlots; ++k)
+    for (int i = 0; i < kCounters; ++i) c[i] += slots[k * kSlotStride + i];
   if (stats != nullptr) *stats = r3dgpu_refinement_stats{c[kInput], c[kRefined], c[kInput] - c[kRefined] - c[kUnconfirmed],
                                                          c[kUnconfirmed]};
 }
