@@ -48,50 +48,28 @@ constexpr int kLanes = 32 / kPixels;          // lanes per pixel (at least one p
 constexpr int kRefineThreads = 128;
 static_assert(kLanes >= kMaxViews, "a lane per view");
 
-// A view's pixel as the kernels read it: intensity and derivatives, the
-// intensity already in double (a conversion runs at a quarter of the double
-// rate, and a sample has four): 16 bytes with float derivatives, 32 with double
-// ones.
+// A view's pixel as the kernels read it, 16 bytes: the intensity already in
+// double (a sample has four, and a conversion runs at a quarter of the double
+// rate), and the derivatives in float. (32 bytes with double derivatives made
+// the double path wait on its loads.)
+R3D_DEVICE void load_texel(const float4* p, double& v, float& gx, float& gy) {
+  const float4 a = __ldg(p);
+  memcpy(&v, &a, 8);
+  gx = a.z;
+  gy = a.w;
+}
+
+// A window sample: its pixel offset and offset / radius.
 template <class T>
-struct Texels;
-template <>
-struct Texels<float> {
-  static constexpr int kWords = 1;  // float4 words per pixel
-  static R3D_DEVICE void load(const float4* p, double& v, float& gx, float& gy) {
-    const float4 a = __ldg(p);
-    memcpy(&v, &a, 8);
-    gx = a.z;
-    gy = a.w;
-  }
-  static R3D_DEVICE void store(float4* p, float v, float gx, float gy) {
-    const double d = v;
-    float4 a;
-    memcpy(&a, &d, 8);
-    a.z = gx;
-    a.w = gy;
-    *p = a;
-  }
-};
-template <>
-struct Texels<double> {
-  static constexpr int kWords = 2;
-  static R3D_DEVICE void load(const float4* p, double& v, double& gx, double& gy) {
-    const float4 a = __ldg(p), b = __ldg(p + 1);
-    memcpy(&v, &a, 8);
-    memcpy(&gx, reinterpret_cast<const char*>(&a) + 8, 8);
-    memcpy(&gy, &b, 8);
-  }
-  static R3D_DEVICE void store(float4* p, float v, float gx, float gy) {
-    const double d[4] = {v, gx, gy, 0.0};
-    memcpy(p, d, 32);
-  }
+struct alignas(4 * sizeof(T)) Sample {
+  T dx, dy, sx, sy;
 };
 
 // Plane-induced warp into a view (refinement.cpp:24-30): h = m (qx, qy, 1) + b w(q).
 struct ViewGeo {
   double m[9];  // K_j R_j R_0^T K_0^-1, row-major
   double b[3];  // K_j R_j (C_0 - C_j)
-  const float4* data;  // the view's texels (repack_kernel)
+  const float4* data;  // the view's texels
   int64_t stride;      // texels per row
   int width, height;
 };
@@ -149,11 +127,6 @@ R3D_DEVICE bool finite_d(double v) { return v - v == 0.0; }
 // Smallest power of two >= m (m in 1..8): the number of lane groups.
 R3D_DEVICE int groups_for(int m) { return m <= 1 ? 1 : (m <= 2 ? 2 : (m <= 4 ? 4 : 8)); }
 
-// In shared memory, per pixel the normalised base window n0[s] (kMaxSamples
-// doubles at most, p.n used) and per warp the window coordinates (offset /
-// radius) of each window column, kept as doubles.
-constexpr int kMaxSide = 16;
-
 // floor(q) of |q| < 2^22 as float and as int, without the conversion unit:
 // adding 1.5 * 2^23 rounds to a whole number that the sum's low bits hold.
 R3D_DEVICE float floor_small(float q, int& i) {
@@ -174,7 +147,7 @@ R3D_DEVICE float floor_small(float q, int& i) {
 // One view's terms at plane theta (refinement.cpp:46-152), computed by the
 // `gsize` lanes of a group: lane `gl` of the group takes the window samples
 // gl, gl + gsize, ... NCC of the warped window with the normalised base
-// window and, with JAC, J^T J (xx xy xz yy yz zz) and J^T e of
+// window, J^T J (xx xy xz yy yz zz) and J^T e of
 // sum (n_q - n0_q)^2 in (w, a, b). `valid` is false if a sample leaves the
 // image or the window has no texture. All lanes of the group return the same
 // values; `active` false (a group without a view) returns zeros and valid.
@@ -187,9 +160,9 @@ R3D_DEVICE float floor_small(float q, int& i) {
 // J^T e = (p ncc - sum a n0) / |raw - mean|. The objective moments are double
 // (intensities shifted by `shift`, the base window's mean, to keep the
 // variance well conditioned); the Jacobian moments are T.
-template <class T, bool JAC>
+template <class T>
 R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y, const double* theta,
-                               const Params& p, const double* n0s, const double* coord, double shift, int gl,
+                               const Params& p, const Sample<T>* samples, const double* n0s, double shift, int gl,
                                int gsize, bool& valid, double& ncc_out, double* hh, double* gg) {
   double ob[3] = {0.0, 0.0, 0.0};
   T jm[15];
@@ -238,18 +211,9 @@ R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y
       hc1 = static_cast<T>(row3(g.m, 1, x, y, 1.0));
       hc2 = static_cast<T>(row3(g.m, 2, x, y, 1.0));
     }
-    // Window column and row of sample s, advanced by gsize per step.
-    int col = gl % p.side, row = gl / p.side;
-    const int dcol = gsize % p.side, drow = gsize / p.side;
     for (int s = gl; s < p.n; s += gsize) {
-      const T dx = static_cast<T>(col * p.step - p.radius), dy = static_cast<T>(row * p.step - p.radius);
-      const T sx = static_cast<T>(coord[col]), sy = static_cast<T>(coord[row]);
-      col += dcol;
-      row += drow;
-      if (col >= p.side) {
-        col -= p.side;
-        ++row;
-      }
+      const Sample<T> q = samples[s];
+      const T dx = q.dx, dy = q.dy, sx = q.sx, sy = q.sy;
       T inv_z, px, py, fx, fy;
       int ix, iy;
       if (offsets) {
@@ -258,16 +222,8 @@ R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y
         const T d1 = (m3 * dx + m4 * dy) + b1 * ws;
         const T d2 = (m6 * dx + m7 * dy) + b2 * ws;
         const T h2 = hzf + d2;
-        if (!(h2 > T(0))) {
-          bad = true;
-          break;
-        }
         inv_z = T(1) / h2;
         const T q0 = fc0 + (d0 - cf0 * d2) * inv_z, q1 = fc1 + (d1 - cf1 * d2) * inv_z;
-        if (!(fabs(q0) < T(1e6) && fabs(q1) < T(1e6))) {
-          bad = true;
-          break;
-        }
         int k0, k1;
         const T fl0 = floor_small(static_cast<float>(q0), k0), fl1 = floor_small(static_cast<float>(q1), k1);
         ix = ic0 + k0;
@@ -277,8 +233,9 @@ R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y
         // ix and iy as floats: exact wherever they are inside an image.
         px = (ft0 + fl0) + fx;
         py = (ft1 + fl1) + fy;
-        // px in [0, width - 1) and py in [0, height - 1), as below.
-        if (!(ix >= 0 && iy >= 0 && ix <= g.width - 2 && iy <= g.height - 2)) {
+        // In front of the camera, px in [0, width - 1) and py in [0, height - 1), as below.
+        if (!(h2 > T(0) && fabs(q0) < T(1e6) && fabs(q1) < T(1e6) && ix >= 0 && iy >= 0 && ix <= g.width - 2 &&
+              iy <= g.height - 2)) {
           bad = true;
           break;
         }
@@ -303,15 +260,14 @@ R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y
         fx = px - static_cast<T>(ix);
         fy = py - static_cast<T>(iy);
       }
-      constexpr int TW = Texels<T>::kWords;
-      const float4* r0 = g.data + (static_cast<int64_t>(iy) * g.stride + ix) * TW;
-      const float4* r1 = r0 + g.stride * TW;
+      const float4* r0 = g.data + static_cast<int64_t>(iy) * g.stride + ix;
+      const float4* r1 = r0 + g.stride;
       double v00, v01, v10, v11;
-      T x00, x01, x10, x11, y00, y01, y10, y11;
-      Texels<T>::load(r0, v00, x00, y00);
-      Texels<T>::load(r0 + TW, v01, x01, y01);
-      Texels<T>::load(r1, v10, x10, y10);
-      Texels<T>::load(r1 + TW, v11, x11, y11);
+      float x00, x01, x10, x11, y00, y01, y10, y11;
+      load_texel(r0, v00, x00, y00);
+      load_texel(r0 + 1, v01, x01, y01);
+      load_texel(r1, v10, x10, y10);
+      load_texel(r1 + 1, v11, x11, y11);
       const double fxd = fx, fyd = fy;
       const double raw =
           ((1.0 - fyd) * ((1.0 - fxd) * v00 + fxd * v01) + fyd * ((1.0 - fxd) * v10 + fxd * v11)) - shift;
@@ -319,7 +275,7 @@ R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y
       ob[0] += raw;
       ob[1] += raw * raw;
       ob[2] += raw * n0;
-      if (JAC) {
+      {
         const T ax = T(1) - fx, ay = T(1) - fy;
         const T gx = ay * (ax * x00 + fx * x01) + fy * (ax * x10 + fx * x11);
         const T gy = ay * (ax * y00 + fx * y01) + fy * (ax * y10 + fx * y11);
@@ -350,7 +306,7 @@ R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y
   const uint32_t gmask = (gsize == 32 ? 0xFFFFFFFFu : ((1u << gsize) - 1u) << (lane & ~static_cast<uint32_t>(gsize - 1)));
   const bool group_bad = (r3dsimt::ballot(bad) & gmask) != 0;
   sums(ob, 1, gsize);
-  if (JAC) sums(jm, 1, gsize);
+  sums(jm, 1, gsize);
   for (int i = 0; i < 6; ++i) hh[i] = 0.0;
   for (int i = 0; i < 3; ++i) gg[i] = 0.0;
   ncc_out = 0.0;
@@ -366,7 +322,6 @@ R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y
   const double inv_norm = 1.0 / sqrt(norm2);
   const double ncc = ob[2] * inv_norm;
   ncc_out = ncc;
-  if (!JAC) return;
   const T inv = static_cast<T>(inv_norm), n = static_cast<T>(p.n), meanf = static_cast<T>(mean);
   const T dm[3] = {jm[0] / n, jm[1] / n, jm[2] / n};
   const T pr[3] = {inv * (jm[3] - meanf * jm[0]), inv * (jm[4] - meanf * jm[1]), inv * (jm[5] - meanf * jm[2])};
@@ -462,8 +417,8 @@ R3D_DEVICE void solve_damped(const double* hh, const double* gg, double* delta) 
   for (int i = 0; i < 3; ++i) delta[perm[i]] = -y[i];
 }
 
-// Dynamic shared memory: per pixel of the block p.n doubles, then per warp
-// kMaxSide doubles.
+// Dynamic shared memory: the window's p.n samples, then per pixel of the block
+// its p.n normalised base window values.
 template <class T>
 R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN(kRefineThreads, 4)
     refine_kernel(const float* R3D_RESTRICT input, float* depth, float* conf, int64_t stride,
@@ -475,6 +430,14 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN(kRefineThreads, 4)
   const bool lead = wl == 0;
   const int64_t total = static_cast<int64_t>(p.width) * p.height;
   const int64_t first = ((static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * kPixels;
+  const int r = p.radius;
+  Sample<T>* const samples = reinterpret_cast<Sample<T>*>(smem);
+  for (int s = static_cast<int>(threadIdx.x); s < p.n; s += static_cast<int>(blockDim.x)) {
+    const int ox = (s % p.side) * p.step - r, oy = (s / p.side) * p.step - r;
+    samples[s] = Sample<T>{static_cast<T>(ox), static_cast<T>(oy), static_cast<T>(static_cast<double>(ox) / r),
+                           static_cast<T>(static_cast<double>(oy) / r)};
+  }
+  r3dsimt::syncthreads();
   if (first >= total) return;  // whole warp
   const int64_t pix = first + sub < total ? first + sub : first;
   const int y = static_cast<int>(pix / p.width), x = static_cast<int>(pix - static_cast<int64_t>(y) * p.width);
@@ -488,14 +451,11 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN(kRefineThreads, 4)
   };
   count(kInput, valid_px);
   if (valid_px && lead) conf[at] = 0.0F;
-  const int r = p.radius;
   bool live = valid_px && p.num_views > 0 && x >= r && y >= r && x < p.width - r && y < p.height - r;
   if (r3dsimt::ballot(live) == 0) return;
 
   // The normalised base window into the pixel's table.
-  double* const n0s = reinterpret_cast<double*>(smem) + static_cast<size_t>(warp * kPixels + sub) * p.n;
-  double* const coord =
-      reinterpret_cast<double*>(smem) + static_cast<size_t>(blockDim.x / 32 * kPixels) * p.n + warp * kMaxSide;
+  double* const n0s = reinterpret_cast<double*>(samples + p.n) + static_cast<size_t>(warp * kPixels + sub) * p.n;
   double sum = 0.0;
   for (int s = wl; s < p.n; s += kLanes) {
     const int dx = (s % p.side) * p.step - r, dy = (s / p.side) * p.step - r;
@@ -514,7 +474,6 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN(kRefineThreads, 4)
   live = live && !(norm2 < p.min_texture2n);
   const double inv_norm = 1.0 / sqrt(norm2);
   for (int s = wl; s < p.n; s += kLanes) n0s[s] *= inv_norm;
-  if (lane < p.side) coord[lane] = static_cast<double>(lane * p.step - r) / r;
   r3dsimt::syncwarp();
   if (r3dsimt::ballot(live) == 0) return;
 
@@ -529,15 +488,15 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN(kRefineThreads, 4)
   const ViewGeo& my_view = views[my_t < p.num_views ? my_t : 0];
   const uint32_t px_mask = (1u << kLanes) - 1u;
 
-  // Local view selection at the initial plane.
-  double hh_v[6], gg_v[3];
+  // Local view selection at the initial plane; the selected views' terms there
+  // are those of the first Gauss-Newton step.
+  double ncc, hh_v[6], gg_v[3];
   bool use = live && my_t < p.num_views;  // the lane's view is used by its pixel
   int m = 0;
   double s0 = 0.0;
   {
     bool valid;
-    double ncc;
-    evaluate_group<T, false>(my_view, use, xd, yd, theta0, p, n0s, coord, mean, gl, gsize, valid, ncc, hh_v, gg_v);
+    evaluate_group<T>(my_view, use, xd, yd, theta0, p, samples, n0s, mean, gl, gsize, valid, ncc, hh_v, gg_v);
     use = use && valid && ncc >= p.min_ncc;
     const uint32_t ok = (r3dsimt::ballot(use) >> (sub * kLanes)) & px_mask;
     for (int j = 0; j < p.num_views; ++j) {
@@ -559,23 +518,28 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN(kRefineThreads, 4)
   double max_motion = use ? centre_motion(my_view, xd, yd, w0) : 0.0;
   for (int o = gsize; o < kLanes; o <<= 1) max_motion = fmax(max_motion, shfl_xor_t(max_motion, o));
 
-  // Mean NCC and Gauss-Newton terms over the used views; -inf if a view drops out.
-  auto evaluate = [&](const double* theta, bool active, double* hh, double* gg) {
-    bool valid;
-    double ncc;
-    evaluate_group<T, true>(my_view, active && use, xd, yd, theta, p, n0s, coord, mean, gl, gsize, valid, ncc, hh_v,
-                            gg_v);
-    const bool dropped = ((r3dsimt::ballot(!valid) >> (sub * kLanes)) & px_mask) != 0;
+  // Mean NCC and Gauss-Newton terms over the used views, from each lane's view's.
+  auto total_terms = [&](double* hh, double* gg) {
     double tot[10] = {ncc, hh_v[0], hh_v[1], hh_v[2], hh_v[3], hh_v[4], hh_v[5], gg_v[0], gg_v[1], gg_v[2]};
+    if (!use)
+      for (int i = 0; i < 10; ++i) tot[i] = 0.0;
     sums(tot, gsize, kLanes);
     for (int i = 0; i < 6; ++i) hh[i] = tot[1 + i];
     for (int i = 0; i < 3; ++i) gg[i] = tot[7 + i];
-    return dropped ? -__builtin_huge_val() : tot[0] / views_used;
+    return tot[0] / views_used;
+  };
+  // The same at plane theta; -inf if a view drops out.
+  auto evaluate = [&](const double* theta, bool active, double* hh, double* gg) {
+    bool valid;
+    evaluate_group<T>(my_view, active && use, xd, yd, theta, p, samples, n0s, mean, gl, gsize, valid, ncc, hh_v, gg_v);
+    const bool dropped = ((r3dsimt::ballot(!valid) >> (sub * kLanes)) & px_mask) != 0;
+    const double score = total_terms(hh, gg);
+    return dropped ? -__builtin_huge_val() : score;
   };
 
   double hh[6], gg[3];
   double best[3] = {theta0[0], theta0[1], theta0[2]};
-  double best_score = evaluate(best, live, hh, gg);
+  double best_score = total_terms(hh, gg);
   live = live && finite_d(best_score);
   double scale = 1.0;
   bool stepping = live;
@@ -655,12 +619,16 @@ R3D_GLOBAL void gradient_kernel(const float* gray, int64_t gstride, int w, int h
 }
 
 // A view's 3-channel refinement image as texels.
-template <class T>
 R3D_GLOBAL void repack_kernel(const float* in, int64_t istride, int w, int h, float4* out) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= w || y >= h) return;
   const float* p = in + static_cast<int64_t>(y) * istride + 3 * x;
-  Texels<T>::store(out + (static_cast<int64_t>(y) * w + x) * Texels<T>::kWords, p[0], p[1], p[2]);
+  const double v = p[0];
+  float4 a;
+  memcpy(&a, &v, 8);
+  a.z = p[1];
+  a.w = p[2];
+  out[static_cast<int64_t>(y) * w + x] = a;
 }
 
 // ------------------------------------------------------------------ host side
@@ -718,7 +686,7 @@ void launch_refine(const float* input, float* depth, float* conf, int64_t stride
                    int64_t bstride, const ViewGeo* views, const Params& p, unsigned long long* counters,
                    cudaStream_t s) {
   constexpr int per_block = kRefineThreads / 32 * kPixels;
-  const size_t smem = sizeof(double) * (static_cast<size_t>(per_block) * p.n + kRefineThreads / 32 * kMaxSide);
+  const size_t smem = (sizeof(Sample<T>) + sizeof(double) * per_block) * static_cast<size_t>(p.n);
   auto kernel = refine_kernel<T>;
   R3D_LAUNCH(kernel, static_cast<unsigned>(ceil_div64(static_cast<int64_t>(p.width) * p.height, per_block)),
              kRefineThreads, smem, s, input, depth, conf, stride, base, bstride, views, p, counters);
@@ -754,21 +722,19 @@ void refine(float* depth, float* conf, int64_t stride, const r3dgpu_pinhole_came
   R3D_CUDA(cudaMemsetAsync(sc.counters.get(), 0, sizeof(unsigned long long) * kSlots * kSlotStride, s));
   if (w > 0 && h > 0) {
     // The views' images as texels.
-    const size_t words = o.fp32 ? Texels<float>::kWords : Texels<double>::kWords;
     size_t total = 0;
     for (int j = 0; j < nv; ++j)
-      total += words * static_cast<size_t>(views[j].camera.intrinsics.width) * views[j].camera.intrinsics.height;
+      total += static_cast<size_t>(views[j].camera.intrinsics.width) * views[j].camera.intrinsics.height;
     sc.packed.reserve(total > 0 ? total : 1);
     size_t off = 0;
     for (int j = 0; j < nv; ++j) {
       const int vw = views[j].camera.intrinsics.width, vh = views[j].camera.intrinsics.height;
       float4* dst = sc.packed.get() + off;
       const dim3 b(32, 8), g(static_cast<unsigned>(ceil_div(vw, 32)), static_cast<unsigned>(ceil_div(vh, 8)));
-      auto repack = o.fp32 ? repack_kernel<float> : repack_kernel<double>;
-      R3D_LAUNCH(repack, g, b, 0, s, views[j].data, views[j].stride, vw, vh, dst);
+      R3D_LAUNCH(repack_kernel, g, b, 0, s, views[j].data, views[j].stride, vw, vh, dst);
       launched("repack_kernel");
       geo[j].data = dst;
-      off += words * static_cast<size_t>(vw) * vh;
+      off += static_cast<size_t>(vw) * vh;
     }
     if (nv > 0)
       R3D_CUDA(cudaMemcpyAsync(sc.views.get(), geo, sizeof(ViewGeo) * nv, cudaMemcpyHostToDevice, s));
