@@ -123,6 +123,7 @@ R3D_DEVICE T pixel_sum(T v) {
 // Finite (neither infinite nor NaN): v - v is 0 exactly then, NaN otherwise.
 R3D_DEVICE bool finite_d(double v) { return v - v == 0.0; }
 
+using r3dsimt::fmadd;
 
 // Smallest power of two >= m (m in 1..8): the number of lane groups.
 R3D_DEVICE int groups_for(int m) { return m <= 1 ? 1 : (m <= 2 ? 2 : (m <= 4 ? 4 : 8)); }
@@ -159,7 +160,9 @@ R3D_DEVICE float floor_small(float q, int& i) {
 // J^T J = (sum d d^T - p p^T) / |raw - mean|^2 and
 // J^T e = (p ncc - sum a n0) / |raw - mean|. The objective moments are double
 // (intensities shifted by `shift`, the base window's mean, to keep the
-// variance well conditioned); the Jacobian moments are T.
+// variance well conditioned); the Jacobian moments are T. Products and sums of
+// a sample are contracted (fmadd): a rounding less each, and a fifth of the
+// instructions.
 template <class T>
 R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y, const double* theta,
                                const Params& p, const Sample<T>* samples, const double* n0s, double shift, int gl,
@@ -217,13 +220,13 @@ R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y
       T inv_z, px, py, fx, fy;
       int ix, iy;
       if (offsets) {
-        const T ws = th1 * sx + th2 * sy;  // w(q) - w at the window centre
-        const T d0 = (m0 * dx + m1 * dy) + b0 * ws;
-        const T d1 = (m3 * dx + m4 * dy) + b1 * ws;
-        const T d2 = (m6 * dx + m7 * dy) + b2 * ws;
+        const T ws = fmadd(th1, sx, th2 * sy);  // w(q) - w at the window centre
+        const T d0 = fmadd(b0, ws, fmadd(m0, dx, m1 * dy));
+        const T d1 = fmadd(b1, ws, fmadd(m3, dx, m4 * dy));
+        const T d2 = fmadd(b2, ws, fmadd(m6, dx, m7 * dy));
         const T h2 = hzf + d2;
         inv_z = T(1) / h2;
-        const T q0 = fc0 + (d0 - cf0 * d2) * inv_z, q1 = fc1 + (d1 - cf1 * d2) * inv_z;
+        const T q0 = fmadd(fmadd(-cf0, d2, d0), inv_z, fc0), q1 = fmadd(fmadd(-cf1, d2, d1), inv_z, fc1);
         int k0, k1;
         const T fl0 = floor_small(static_cast<float>(q0), k0), fl1 = floor_small(static_cast<float>(q1), k1);
         ix = ic0 + k0;
@@ -240,10 +243,10 @@ R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y
           break;
         }
       } else {
-        const T wq = (th0 + th1 * sx) + th2 * sy;
-        const T h0 = ((hc0 + m0 * dx) + m1 * dy) + b0 * wq;
-        const T h1 = ((hc1 + m3 * dx) + m4 * dy) + b1 * wq;
-        const T h2 = ((hc2 + m6 * dx) + m7 * dy) + b2 * wq;
+        const T wq = fmadd(th2, sy, fmadd(th1, sx, th0));
+        const T h0 = fmadd(b0, wq, fmadd(m1, dy, fmadd(m0, dx, hc0)));
+        const T h1 = fmadd(b1, wq, fmadd(m4, dy, fmadd(m3, dx, hc1)));
+        const T h2 = fmadd(b2, wq, fmadd(m7, dy, fmadd(m6, dx, hc2)));
         if (!(h2 > T(0))) {
           bad = true;
           break;
@@ -269,35 +272,36 @@ R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y
       load_texel(r1, v10, x10, y10);
       load_texel(r1 + 1, v11, x11, y11);
       const double fxd = fx, fyd = fy;
-      const double raw =
-          ((1.0 - fyd) * ((1.0 - fxd) * v00 + fxd * v01) + fyd * ((1.0 - fxd) * v10 + fxd * v11)) - shift;
+      const double ux = 1.0 - fxd, uy = 1.0 - fyd;
+      const double raw = fmadd(uy, fmadd(ux, v00, fxd * v01), fyd * fmadd(ux, v10, fxd * v11)) - shift;
       const double n0 = n0s[s];
       ob[0] += raw;
-      ob[1] += raw * raw;
-      ob[2] += raw * n0;
+      ob[1] = fmadd(raw, raw, ob[1]);
+      ob[2] = fmadd(raw, n0, ob[2]);
       {
         const T ax = T(1) - fx, ay = T(1) - fy;
-        const T gx = ay * (ax * x00 + fx * x01) + fy * (ax * x10 + fx * x11);
-        const T gy = ay * (ax * y00 + fx * y01) + fy * (ax * y10 + fx * y11);
-        const T dpx = (b0 - px * b2) * inv_z, dpy = (b1 - py * b2) * inv_z;
-        const T dv = gx * dpx + gy * dpy;
+        const T tx00 = x00, tx01 = x01, tx10 = x10, tx11 = x11, ty00 = y00, ty01 = y01, ty10 = y10, ty11 = y11;
+        const T gx = fmadd(ay, fmadd(ax, tx00, fx * tx01), fy * fmadd(ax, tx10, fx * tx11));
+        const T gy = fmadd(ay, fmadd(ax, ty00, fx * ty01), fy * fmadd(ax, ty10, fx * ty11));
+        const T dpx = fmadd(-px, b2, b0) * inv_z, dpy = fmadd(-py, b2, b1) * inv_z;
+        const T dv = fmadd(gx, dpx, gy * dpy);
         const T a0 = dv, a1 = dv * sx, a2 = dv * sy;
         const T rf = static_cast<T>(raw), nf = static_cast<T>(n0);
         jm[0] += a0;
         jm[1] += a1;
         jm[2] += a2;
-        jm[3] += rf * a0;
-        jm[4] += rf * a1;
-        jm[5] += rf * a2;
-        jm[6] += a0 * a0;
-        jm[7] += a0 * a1;
-        jm[8] += a0 * a2;
-        jm[9] += a1 * a1;
-        jm[10] += a1 * a2;
-        jm[11] += a2 * a2;
-        jm[12] += nf * a0;
-        jm[13] += nf * a1;
-        jm[14] += nf * a2;
+        jm[3] = fmadd(rf, a0, jm[3]);
+        jm[4] = fmadd(rf, a1, jm[4]);
+        jm[5] = fmadd(rf, a2, jm[5]);
+        jm[6] = fmadd(a0, a0, jm[6]);
+        jm[7] = fmadd(a0, a1, jm[7]);
+        jm[8] = fmadd(a0, a2, jm[8]);
+        jm[9] = fmadd(a1, a1, jm[9]);
+        jm[10] = fmadd(a1, a2, jm[10]);
+        jm[11] = fmadd(a2, a2, jm[11]);
+        jm[12] = fmadd(nf, a0, jm[12]);
+        jm[13] = fmadd(nf, a1, jm[13]);
+        jm[14] = fmadd(nf, a2, jm[14]);
       }
     }
   }

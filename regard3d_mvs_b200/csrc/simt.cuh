@@ -29,6 +29,9 @@
 namespace r3dsimt {
 
 R3D_DEVICE bool finitef(float v) { return isfinite(v); }
+// a * b + c rounded once.
+R3D_DEVICE float fmadd(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+R3D_DEVICE double fmadd(double a, double b, double c) { return __fma_rn(a, b, c); }
 R3D_DEVICE int imin(int a, int b) { return min(a, b); }
 R3D_DEVICE int imax(int a, int b) { return max(a, b); }
 R3D_DEVICE uint32_t umin(uint32_t a, uint32_t b) { return min(a, b); }
@@ -158,6 +161,8 @@ unsigned char* dynamic_smem();
 void launch(dim3 grid, dim3 block, size_t smem, const std::function<void()>& body);
 
 inline bool finitef(float v) { return std::isfinite(v); }
+inline float fmadd(float a, float b, float c) { return std::fma(a, b, c); }
+inline double fmadd(double a, double b, double c) { return std::fma(a, b, c); }
 inline int imin(int a, int b) { return a < b ? a : b; }
 inline int imax(int a, int b) { return a > b ? a : b; }
 inline uint32_t umin(uint32_t a, uint32_t b) { return a < b ? a : b; }
