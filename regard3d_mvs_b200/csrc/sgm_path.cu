@@ -1041,7 +1041,8 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
     int maxlen = t1;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) maxlen = r3dsimt::imax(maxlen, static_cast<int>(r3dsimt::shfl_xor(static_cast<uint32_t>(maxlen), o)));
-    auto has = [&](int i) { return i >= t0 && i < t1; };
+    const uint32_t chain_len = t1 > t0 ? static_cast<uint32_t>(t1 - t0) : 0u;
+    auto has = [&](int i) { return static_cast<uint32_t>(i - t0) < chain_len; };
     const uint8_t* const cbase = cost + job.cell_off;
     uint16_t* const sbase = sum + job.cell_off;
     uint8_t* const tout = terms + job.cell_off + tslot * tstride;
@@ -1063,13 +1064,14 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
         }
       }
     };
+    // Records read ahead of their use (a step's first decisions and addresses
+    // depend on them): this pixel's, the next one's, and that of the pixel
+    // whose first chunk is issued in this step.
+    uint2 rc = make_uint2(0, 0), rn = rc, ri = rc;
     // Pixel i + D - 1's first chunk into slot st, pixel i + 2 D - 1's record;
-    // one group. (Records: requested D steps before the data, so landed.)
+    // one group.
     auto issue = [&](int i, int st) {
-      if (has(i + D - 1)) {
-        const uint2 r = recs[((i + D - 1) & (NR - 1)) * 32];
-        issue_chunk(st, static_cast<int>(r.x & kRecOffset), static_cast<int>(r.x >> kRecShift));
-      }
+      if (has(i + D - 1)) issue_chunk(st, static_cast<int>(ri.x & kRecOffset), static_cast<int>(ri.x >> kRecShift));
       if (has(i + 2 * D - 1)) r3dsimt::cp_async8(&recs[((i + 2 * D - 1) & (NR - 1)) * 32], rp);
       rp += dpx;
       r3dsimt::cp_async_commit();
@@ -1087,8 +1089,10 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
       }
       r3dsimt::cp_async_commit();
     }
-    uint2 rc = make_uint2(0, 0);  // this pixel's record
     if (has(0)) rc = recs[0];
+    rn = rc;
+    if (has(1)) rn = recs[32];
+    if (has(D - 1)) ri = recs[(D - 1) * 32];
     // The predecessor's range, its minimum over labels in both halves,
     // negated, and the clamp min L(q) + P2. A zero clamp makes the first
     // pixel's best term 0 whatever the predecessor words hold: T = 0, L = C.
@@ -1208,17 +1212,25 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
       const bool on = has(i), on_n = has(i + 1);
       const int at = static_cast<int>(rc.x & kRecOffset);
       const int lo = static_cast<int>(rc.y & 0xFFFFu);
-      uint2 rn = rc;  // the next pixel's record
-      if (on_n) rn = recs[((i + 1) & (NR - 1)) * 32];
       const bool single_n = static_cast<int>(rn.x >> kRecShift) == UF;
       const bool okn = !on_n || (single_n && (!on || (single && ((rn.y ^ rc.y) & 0xFFFFu) == 0)));
       const bool fast_next = r3dsimt::ballot(!okn) == 0;
+      const int dn = static_cast<int>(rn.y >> 16) - static_cast<int>(rc.y >> 16);
+      const uint32_t p2 = lut[(dn < 0 ? -dn : dn) >> 8];  // of the step into the next pixel
       pm = kSent2;
       uint32_t best[K];
       int n = UF;
+      uint2 rn2 = rn, ri2 = ri;
+      // The records of the next step; they landed with the group just waited
+      // for (requested D - 1 steps ago or before).
+      auto look_ahead = [&]() {
+        if (has(i + 2)) rn2 = recs[((i + 2) & (NR - 1)) * 32];
+        if (has(i + D)) ri2 = recs[((i + D) & (NR - 1)) * 32];
+      };
       if (fast) {
         issue(i, st_in);
         r3dsimt::cp_async_wait<D - 1>();
+        look_ahead();
         uint32_t cl[K];
 #pragma unroll
         for (int k = 0; k < K; ++k) cl[k] = r3dsimt::vmin2(prev[k], pen2);
@@ -1231,6 +1243,7 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
         if (!multi) {
           issue(i, st_in);
           r3dsimt::cp_async_wait<D - 1>();
+          look_ahead();
           best_from_memory(best, i, 0, lo);
           finish(best, st, at, on, n > 1);
           if (!fast_next && on) store_vec(i, 0, n, n > 1);
@@ -1242,6 +1255,7 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
           if (n > UF) issue_chunk(sb, at + UF, n - UF);
           r3dsimt::cp_async_commit();
           r3dsimt::cp_async_wait<D - 1>();
+          look_ahead();
           for (int c = 0; r3dsimt::ballot(c * UF < n) != 0; ++c) {
             const bool have = c * UF < n, upper = n - c * UF > 1;
             if (have) {
@@ -1264,14 +1278,15 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
       for (int k = 0; k < K; ++k) prev[k] = out[k];
       {
         const uint32_t mp = r3dsimt::vmin2(pm, r3dsimt::perm(pm, pm, 0x1032u));
-        const int dn = static_cast<int>(rn.y >> 16) - static_cast<int>(rc.y >> 16);
         // A chain that starts at the next step keeps the zero clamp.
-        pen2 = on ? mp + lut[(dn < 0 ? -dn : dn) >> 8] * 0x10001u : 0u;
+        pen2 = on ? mp + p2 * 0x10001u : 0u;
         negmp = on ? 0u - mp : 0u;
       }
       lo_q = lo;
       num_q = 16 * n;
       rc = rn;
+      rn = rn2;
+      ri = ri2;
       single = single_n;
       fast = fast_next;
     }
