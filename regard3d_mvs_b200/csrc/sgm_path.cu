@@ -638,8 +638,12 @@ R3D_DEVICE uint32_t group_min_rt(uint32_t v, int g) {
 // The right-view winners of the diagonal check (sgm_kernels.cpp:349-356: the
 // smallest S << 16 | x per right column) live in shared memory for the row:
 // one shared-memory atomic per cell where the path pass had a global one.
+//
+// The grid's second dimension cuts a row into parts (one with the diagonal
+// check, whose keys need the row in one warp): a 640x480 pair has 1,920 tile
+// rows for 3,552 resident warps.
 template <bool TERMS, int NU>
-R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
+R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN(kPathThreads, (NU == 1 ? 3 : 2))
     sgm_path_wta_kernel(const SgmMatch* R3D_RESTRICT matches, const SgmPathJob* R3D_RESTRICT jobs, int njobs,
                         int64_t rows, const uint8_t* R3D_RESTRICT cost, const uint16_t* R3D_RESTRICT sum,
                         const uint8_t* R3D_RESTRICT terms, int64_t tstride, int4* info, int key_words) {
@@ -650,6 +654,7 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
   int4* const winners = reinterpret_cast<int4*>(smem) + warp * 32;
   uint32_t* const keys = reinterpret_cast<uint32_t*>(smem + static_cast<size_t>(wpb) * 512) +
                          static_cast<size_t>(warp) * key_words;
+  const int part = static_cast<int>(blockIdx.y), parts = static_cast<int>(gridDim.y);
   for (int64_t r = static_cast<int64_t>(blockIdx.x) * wpb + warp; r < rows; r += nwarps) {
     const int j = find_job(jobs, njobs, r, [](const SgmPathJob& q) { return q.row_off; });
     const SgmPathJob& job = jobs[j];
@@ -663,13 +668,17 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
     while (g < nu && g < 32) g <<= 1;
     const int per = 32 / g, gi = lane / g, t = lane & (g - 1);
     const int64_t cell0 = job.cell_off + row_px * nd;
+    // The item's columns, whole groups of 32.
+    const int groups = (w + 31) / 32;
+    const int xfirst = 32 * (groups * part / parts);
+    const int xend = r3dsimt::imin(w, 32 * (groups * (part + 1) / parts));
     if (diag) {
       for (int k = lane; k < w + nd; k += 32) keys[k] = 0xFFFFFFFFu;
       r3dsimt::syncwarp();
     }
-    if (y == 0 && lane == 0)
+    if (y == 0 && xfirst == 0 && lane == 0)
       *job.cells = static_cast<unsigned long long>(w) * static_cast<unsigned long long>(job.h) * nd;
-    for (int xb = 0; xb < w; xb += 32) {
+    for (int xb = xfirst; xb < xend; xb += 32) {
       for (int s = 0; s < g && xb + s * per < w; ++s) {
         const int x = xb + s * per + gi;
         const bool inside = x < w && job.x0 + x >= lv.first && job.x0 + x <= lv.last;
@@ -1681,8 +1690,14 @@ void launch_sgm_path_wave(const SgmMatch* dm, const SgmPathWave& wave, int sms, 
   const size_t smem = static_cast<size_t>(kPathThreads / 32) * (512 + 4 * static_cast<size_t>(key_words));
   if (wave.keys > 0)
     R3D_CUDA(cudaFuncSetAttribute(wta, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  R3D_LAUNCH(wta, dim3(resident_grid(wta, sms, wave.rows, kPathThreads / 32, smem)), dim3(kPathThreads), smem, s, dm,
-             wave.jobs, wave.njobs, wave.rows, cost, sum, terms, B.term_stride, info, key_words);
+  // Parts of a row, at most 8, while the rows alone give a resident warp (24 per
+  // SM) less than two items (640x480: 0.727 ms a pair with four parts, 0.770
+  // with one or two).
+  const int64_t resident = static_cast<int64_t>(sms) * 48;
+  const int64_t want = wave.keys > 0 || wave.rows <= 0 ? 1 : (resident + wave.rows - 1) / wave.rows;
+  const int parts = static_cast<int>(want > 8 ? 8 : want);
+  R3D_LAUNCH(wta, dim3(resident_grid(wta, sms, wave.rows, kPathThreads / 32, smem), parts), dim3(kPathThreads), smem, s,
+             dm, wave.jobs, wave.njobs, wave.rows, cost, sum, terms, B.term_stride, info, key_words);
   launched("sgm_path_wta_kernel");
 }
 
