@@ -186,8 +186,7 @@ def measured_peaks():
     return 6650.0, "fallback"
 
 
-PASS_MODES = {0: "first pass (u16 sums)", 1: "accumulate pass (u16 sums)", 2: "last pass (u16 sums, WTA)",
-              3: "term pass (byte terms)", 4: "last pass (byte terms, WTA)"}
+PASS_MODES = {0: "first pass (u16 sums)", 1: "accumulate pass (u16 sums)", 3: "term pass (byte terms)"}
 
 
 def pass_traffic_per_cell():
@@ -203,8 +202,8 @@ def pass_traffic_per_cell():
 
 def pass_roofline(launch_log, peak, peak_kind):
     """Roofline of the dominant kernel, the chain pass (sgm_path_kernel):
-    algorithmic bytes of its launches (costs read, sums or byte terms read and
-    written, WTA records) over their CUDA-event durations on the launching
+    algorithmic bytes of its launches (costs read, byte terms written or sums
+    read and written) over their CUDA-event durations on the launching
     stream; per pass mode as well."""
     passes = [e for e in launch_log if e.get("pass") and e["kernel"] == "sgm_path_kernel"]
     rpasses = [e for e in launch_log if e.get("pass") and e["kernel"] == "sgm_path_ranged_kernel"]
@@ -230,12 +229,11 @@ def pass_roofline(launch_log, peak, peak_kind):
     traffic = None
     if tpc and all(m in tpc for m in by_mode):
         traffic = sum(tpc[m] * b["cells"] for m, b in by_mode.items()) / len(passes)
-    out = {"bound": "hbm", "kernel": "sgm_path_kernel (chain passes of full-range tiles; a launch runs one pass, or the seven term passes of a tile group)", "achieved": achieved,
+    out = {"bound": "hbm", "kernel": "sgm_path_kernel (chain passes of full-range tiles; a launch runs one pass, or the eight term passes of a tile group)", "achieved": achieved,
            "peak": peak, "peak_kind": f"{peak_kind} copy bandwidth", "unit": "GB/s", "frac": achieved / peak,
            "traffic": traffic, "traffic_source": "profiles/sgm_path_traffic.json (ncu DRAM bytes per cell by mode)",
            "launches": len(passes), "avg_launch_ms": ms / len(passes), "alg_bytes_per_launch": nbytes / len(passes),
-           "alg_bytes_per_cell": {"first pass": 3, "accumulate pass": 5, "last pass": "3 + 16 per pixel",
-                                  "term pass": 2, "last pass (byte terms)": "8 + 16 per pixel"},
+           "alg_bytes_per_cell": {"first pass": 3, "accumulate pass": 5, "term pass": 2},
            "cells_per_launch": cells / len(passes),
            "by_mode": {str(k): v for k, v in sorted(by_mode.items())}}
     if rpasses:
@@ -244,7 +242,7 @@ def pass_roofline(launch_log, peak, peak_kind):
         out["ranged_pass"] = {"kernel": "sgm_path_ranged_kernel", "achieved": rb / (rms * 1e-3) / 1e9 if rms else 0.0,
                               "frac": (rb / (rms * 1e-3) / 1e9) / peak if rms else 0.0, "launches": len(rpasses),
                               "avg_launch_ms": rms / len(rpasses),
-                              "alg_bytes_per_cell": "3 (first) or 5, + 16 per pixel (range record)"}
+                              "alg_bytes_per_cell": "2 (terms), 3 (first) or 5, + 8 per pixel (range record)"}
     return out
 
 

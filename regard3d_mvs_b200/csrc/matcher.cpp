@@ -840,6 +840,12 @@ void plan_path_waves(const std::vector<std::pair<int, int>>& tiles, const std::v
     const char* rt = std::getenv("R3DGPU_RANGED_TERMS");
     if (rt != nullptr && *rt != '\0') terms = std::atoi(rt) == 1;
   }
+  // A tile whose terms alone would pass the wave's share of the scratch (9 bytes
+  // per label against 3) keeps its group on u16 sums.
+  for (const Entry& e : es)
+    if (terms)
+      terms = (ranged ? sgm_path_ranged_buffers(e.cells, e.px, e.keys, e.rows, e.maxnum, sms, true).total
+                      : sgm_path_buffers(e.cells, e.px, e.keys, true).total) <= cap_bytes;
   auto bytes = [&](int64_t cells, int64_t px, int64_t keys, int64_t rows, int maxnum) -> size_t {
     return ranged ? sgm_path_ranged_buffers(cells, px, keys, rows, maxnum, sms, terms).total
                   : sgm_path_buffers(cells, px, keys, terms).total;
