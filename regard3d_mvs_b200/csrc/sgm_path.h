@@ -1,9 +1,9 @@
-// Full-range SGM as eight chain passes (sgm_path.cu): the tiles of a wave are
-// aggregated one path direction at a time, every path split into its
-// independent 1-D chains (tile rows, columns or diagonals), many chains in
-// flight per SM. Costs (u8) are computed once per wave; each pass adds its
-// path to the wave's sum volume (u16 per cell), and the last pass also runs
-// the winner-takes-all. The acceptance rules follow in a per-pixel kernel.
+// SGM as eight chain passes (sgm_path.cu): the tiles of a wave are aggregated
+// one path direction at a time, every path split into its independent 1-D
+// chains (tile rows, columns or diagonals), many chains in flight per SM. Costs
+// (u8) are computed once per wave; each pass writes its path's byte terms (or
+// adds to the wave's u16 sums), and a per-pixel kernel forms the total sums,
+// takes the winners and applies the acceptance rules.
 #pragma once
 
 #include <cstddef>
@@ -40,7 +40,7 @@ struct SgmPathShape {
   int k_;
 };
 
-// Narrowest compiled shape for nd labels ({0, 0}: more labels than the path
+// The shape for nd labels ({0, 0}: more labels than the path
 // kernels take, or a tile too wide for the cost kernel's staged partner row:
 // tile width + nd - 1 must stay within 2048).
 SgmPathShape sgm_path_shape(int nd);
