@@ -850,8 +850,12 @@ void plan_path_waves(const std::vector<std::pair<int, int>>& tiles, const std::v
     return ranged ? sgm_path_ranged_buffers(cells, px, keys, rows, maxnum, sms, terms).total
                   : sgm_path_buffers(cells, px, keys, terms).total;
   };
-  std::stable_sort(es.begin(), es.end(),
-                   [](const Entry& a, const Entry& b) { return a.sh.g_ * a.sh.k_ < b.sh.g_ * b.sh.k_; });
+  // By width, then by shape: a segment per shape (a tuning table can give two
+  // label counts shapes of one width), at most as many as compiled shapes.
+  std::stable_sort(es.begin(), es.end(), [](const Entry& a, const Entry& b) {
+    const int wa = a.sh.g_ * a.sh.k_, wb = b.sh.g_ * b.sh.k_;
+    return wa != wb ? wa < wb : a.sh.g_ < b.sh.g_;
+  });
   max_bytes = 0;
   cells_sum = 0;
   px_sum = 0;

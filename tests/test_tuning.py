@@ -86,3 +86,22 @@ def test_path_shape_from_table(simt_matcher, monkeypatch):
     got, launches = _launches(simt_matcher, lambda: simt_matcher.match_stereo_batch(pairs))
     assert shapes(launches) == {"8x8"}
     assert np.array_equal(np.nan_to_num(got[0].disparity, posinf=-1), np.nan_to_num(ref[0].disparity, posinf=-1))
+
+
+def test_shapes_of_one_width_in_a_batch(simt_matcher, monkeypatch):
+    """Two shapes of the same label width (8x16 for 256 labels, 16x8 from the
+    table for 192) in turn over a batch of more pairs than a wave has block
+    counters for: tiles are grouped by the shape itself, one term launch each,
+    and the maps are those of the built-in shapes."""
+    pairs = []
+    for i in range(34):
+        left, right, _ = render_pair(Texture(63 + i), 18, 4, lambda x, y: 5.0 + 0.1 * x)
+        pairs.append(dict(left=left, right=right, disparity_min=0, num_disparities=192 if i % 2 else 256,
+                          options=StereoOptions(levels=0, lr_full_match=False)))
+    monkeypatch.setenv("R3DGPU_TUNING", "#")
+    ref = simt_matcher.match_stereo_batch(pairs)
+    monkeypatch.setenv("R3DGPU_TUNING", "path 192 16 8")
+    got, launches = _launches(simt_matcher, lambda: simt_matcher.match_stereo_batch(pairs))
+    assert sorted(e["shape"].split("/")[0] for e in launches if e.get("pass")) == ["16x8", "8x16"]
+    for a, b in zip(got, ref):
+        assert np.array_equal(a.disparity, b.disparity) and np.array_equal(a.confidence, b.confidence)
