@@ -1904,6 +1904,7 @@ r3dgpu_status r3dgpu_sgm_cost_volume_host(const r3dgpu_view_u16* left, const r3d
       launch_sgm_path_wave(dm, wv, W.sms, s);
       R3D_CUDA(cudaMemcpyAsync(out, vol, sizeof(uint16_t) * cells, cudaMemcpyDeviceToHost, s));
       R3D_CUDA(cudaStreamSynchronize(s));
+      profile_collect();
       return;
     }
     if (ranges_lo && ranges_num && sgm_path_ranged_enabled()) {
@@ -1940,6 +1941,7 @@ r3dgpu_status r3dgpu_sgm_cost_volume_host(const r3dgpu_view_u16* left, const r3d
       launch_sgm_path_ranged_wave(dm, wv, W.sms, s);
       R3D_CUDA(cudaMemcpyAsync(out, vol, sizeof(uint16_t) * cells, cudaMemcpyDeviceToHost, s));
       R3D_CUDA(cudaStreamSynchronize(s));
+      profile_collect();
       return;
     }
     const SgmFullPlan plan = (ranges_lo && ranges_num) ? SgmFullPlan{{0, 0}, 0} : sgm_full_plan(nd, W.smem_optin);

@@ -15,6 +15,7 @@ import pytest
 
 from images import Rng, Texture, mismatch_report, random_image, render_pair, same_disparities, to_u16
 from regard3d_mvs_b200.types import LabelRanges, StereoOptions, SubpixelMethod
+from test_tuning import pass_shapes
 
 pytestmark = pytest.mark.gpu
 
@@ -31,20 +32,23 @@ def _assert_same_map(a, b):
     assert a.num_disparities == b.num_disparities
 
 
-@pytest.mark.parametrize("shape,nd", [("1,8", 16), ("2,8", 32), ("2,16", 48), ("4,8", 64), ("4,12", 96),
-                                      ("4,16", 128), ("8,8", 112), ("8,12", 192), ("8,16", 208), ("16,8", 256),
-                                      ("16,12", 384), ("16,16", 512), ("32,8", 512), ("32,12", 768)])
+@pytest.mark.parametrize("shape,nd", [("1,8", 16), ("2,8", 32), ("2,16", 48), ("4,8", 64), ("4,16", 96),
+                                      ("4,16", 128), ("8,8", 112), ("8,16", 192), ("8,16", 208), ("16,8", 256),
+                                      ("16,16", 384), ("16,16", 512), ("32,8", 512), ("32,16", 768)])
 @pytest.mark.parametrize("p2", [120, 8000])
 def test_volume_chain_shapes(gpu_matcher, oracle, monkeypatch, shape, nd, p2):
-    """Every compiled chain-pass shape (lanes per chain, label pairs per lane)
-    against the textbook volume, with byte terms (P2 <= 255, intensity-adapted
-    penalties) and with u16 sums (P2 = 8000: sums that wrap)."""
+    """Every compiled chain-pass shape (lanes per chain, label pairs per lane;
+    the launches' profile names it) against the textbook volume, with byte
+    terms (P2 <= 255, intensity-adapted penalties) and with u16 sums (P2 =
+    8000: sums that wrap)."""
     monkeypatch.setenv("R3DGPU_PATH_SHAPE", shape)
     tex = Texture(19)
     left, right, _ = render_pair(tex, 70, 37, lambda x, y: 7.0 + 0.2 * x)
     o = StereoOptions(p1=20, p2=p2, p2_adapt=0 if p2 > 255 else 6, invalid_cost=40)
-    assert np.array_equal(gpu_matcher.sgm_cost_volume(left, right, -1, nd, o),
-                          oracle.sgm_cost_volume(left, right, -1, nd, o))
+    got, shapes = pass_shapes(gpu_matcher, lambda: gpu_matcher.sgm_cost_volume(left, right, -1, nd, o))
+    name = shape.replace(",", "x")
+    assert shapes == ({f"{name}/mode3"} if p2 <= 255 else {f"{name}/mode0", f"{name}/mode1"})
+    assert np.array_equal(got, oracle.sgm_cost_volume(left, right, -1, nd, o))
 
 
 @pytest.mark.parametrize("terms", ["0", "1"])

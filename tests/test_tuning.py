@@ -28,6 +28,12 @@ def _launches(m, run):
     return out, [e for e in json.loads(buf.value.decode() or "[]") if e["kernel"] != "sgm_round"]
 
 
+def pass_shapes(m, run):
+    """The result of run() and the shapes ("GxK/modeM") of its chain passes."""
+    out, launches = _launches(m, run)
+    return out, {e["shape"] for e in launches if e.get("pass")}
+
+
 def test_default_kernels_are_the_chain_passes(simt_matcher):
     """Full-range and ranged tiles go to the chain-pass kernels by default."""
     tex = Texture(61)
