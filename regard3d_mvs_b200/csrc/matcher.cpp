@@ -803,6 +803,12 @@ void finish_level(PairRun& P, Arena& A, Pinned& H, cudaStream_t s) {
   }
 }
 
+// R3DGPU_RANGED_TERMS=0 keeps u16 sums on ranged tiles (tests of that mode).
+bool ranged_terms_allowed() {
+  const char* e = std::getenv("R3DGPU_RANGED_TERMS");
+  return e == nullptr || *e == '\0' || std::atoi(e) == 1;
+}
+
 // Waves of the tiles of a round for the chain passes (full-range tiles, or
 // with `ranged` the tiles with per-pixel ranges): tiles in order of kernel
 // shape, a new wave whenever the next tile would take the wave's buffers past
@@ -832,14 +838,9 @@ void plan_path_waves(const std::vector<std::pair<int, int>>& tiles, const std::v
                        M.tile_maxnum[mt.second]});
   }
   // Waves keep byte terms when every match of the group allows them (all
-  // P2 <= 255); otherwise u16 sums. R3DGPU_RANGED_TERMS=0 keeps u16 sums on
-  // ranged groups (tests of that mode).
-  bool terms = true;
+  // P2 <= 255); otherwise u16 sums.
+  bool terms = !ranged || ranged_terms_allowed();
   for (const auto& mt : tiles) terms = terms && matches[mt.first]->m.term_u8 != 0;
-  if (ranged && terms) {
-    const char* rt = std::getenv("R3DGPU_RANGED_TERMS");
-    if (rt != nullptr && *rt != '\0') terms = std::atoi(rt) == 1;
-  }
   // A tile whose terms alone would pass the wave's share of the scratch (9 bytes
   // per label against 3) keeps its group on u16 sums.
   for (const Entry& e : es)
@@ -1935,7 +1936,7 @@ r3dgpu_status r3dgpu_sgm_cost_volume_host(const r3dgpu_view_u16* left, const r3d
       wv.keys = 0;
       wv.rows = h;
       wv.maxnum = max_num;
-      wv.terms = hm->term_u8;
+      wv.terms = hm->term_u8 != 0 && ranged_terms_allowed() ? 1 : 0;
       W.scratch.reserve(sgm_path_ranged_buffers(wv.cells, px, 0, h, max_num, W.sms, wv.terms != 0).total);
       wv.buffer = W.scratch.get();
       launch_sgm_path_ranged_wave(dm, wv, W.sms, s);

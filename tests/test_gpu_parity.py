@@ -63,8 +63,9 @@ def test_ranged_term_modes(gpu_matcher, oracle, monkeypatch, terms):
     num = np.array([[16 * r.uniform_int(1, 5) for _ in range(w)] for _ in range(h)], np.uint16)
     lo = np.array([[r.uniform_int(0, nd - int(n)) for n in row] for row in num], np.uint16)
     o = StereoOptions(p2=140, p2_adapt=5)
-    assert np.array_equal(gpu_matcher.sgm_cost_volume(left, right, 1, nd, o, LabelRanges(lo, num)),
-                          oracle.sgm_cost_volume(left, right, 1, nd, o, (lo, num)))
+    got, shapes = pass_shapes(gpu_matcher, lambda: gpu_matcher.sgm_cost_volume(left, right, 1, nd, o, LabelRanges(lo, num)))
+    assert {q.split("/")[1] for q in shapes} == ({"mode3"} if terms == "1" else {"mode0", "mode1"})
+    assert np.array_equal(got, oracle.sgm_cost_volume(left, right, 1, nd, o, (lo, num)))
     left, right, _ = render_pair(tex, 240, 128, lambda x, y: np.where(x < 100, 9.0, 21.0))
     o = StereoOptions(levels=2, tile_size=96, tile_margin=8, tile_blend=8, range_radius=1)
     _assert_same_map(gpu_matcher.match_stereo(left, right, None, None, 0, 48, o),

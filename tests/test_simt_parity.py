@@ -59,9 +59,9 @@ def test_volume_chain_shapes(simt_matcher, oracle, monkeypatch, shape, nd, p2):
 
 @pytest.mark.parametrize("terms", ["0", "1"])
 def test_ranged_term_modes(simt_matcher, oracle, monkeypatch, terms):
-    """Per-pixel ranges through the chain passes with u16 sums (the default)
-    and with byte terms (R3DGPU_RANGED_TERMS=1): volume and a hierarchical
-    match against the oracle."""
+    """Per-pixel ranges through the chain passes with u16 sums
+    (R3DGPU_RANGED_TERMS=0) and with byte terms (the default): volume and a
+    hierarchical match against the oracle."""
     monkeypatch.setenv("R3DGPU_RANGED_TERMS", terms)
     tex = Texture(29)
     w, h, nd = 33, 21, 112
@@ -70,8 +70,9 @@ def test_ranged_term_modes(simt_matcher, oracle, monkeypatch, terms):
     num = np.array([[16 * r.uniform_int(1, 5) for _ in range(w)] for _ in range(h)], np.uint16)
     lo = np.array([[r.uniform_int(0, nd - int(n)) for n in row] for row in num], np.uint16)
     o = StereoOptions(p2=140, p2_adapt=5)
-    assert np.array_equal(simt_matcher.sgm_cost_volume(left, right, 1, nd, o, LabelRanges(lo, num)),
-                          oracle.sgm_cost_volume(left, right, 1, nd, o, (lo, num)))
+    got, shapes = pass_shapes(simt_matcher, lambda: simt_matcher.sgm_cost_volume(left, right, 1, nd, o, LabelRanges(lo, num)))
+    assert {q.split("/")[1] for q in shapes} == ({"mode3"} if terms == "1" else {"mode0", "mode1"})
+    assert np.array_equal(got, oracle.sgm_cost_volume(left, right, 1, nd, o, (lo, num)))
     left, right, _ = render_pair(tex, 120, 64, lambda x, y: np.where(x < 50, 9.0, 21.0))
     o = StereoOptions(levels=2, tile_size=48, tile_margin=8, tile_blend=8, range_radius=1)
     a = simt_matcher.match_stereo(left, right, None, None, 0, 48, o)
