@@ -1882,7 +1882,7 @@ r3dgpu_status r3dgpu_sgm_cost_volume_host(const r3dgpu_view_u16* left, const r3d
       hj->w = wl;
       hj->h = h;
       const SgmPathShape sh = sgm_path_shape(nd);
-      SgmPathSegment seg{sh, 0, 1, {0, 0, 0}, static_cast<int64_t>(cells), px};
+      SgmPathSegment seg{sh, 0, 1, {0, 0, 0}, static_cast<int64_t>(cells), px, nd == 2 * sh.g_ * sh.k_ ? 1 : 0};
       for (int c = 0; c < kPathClasses; ++c) seg.blocks[c] = (sgm_path_chains(c, wl, h) + 32 / sh.g_ - 1) / (32 / sh.g_);
       hj->disp = A.alloc<float>(static_cast<size_t>(px));
       hj->cells = A.alloc<unsigned long long>(1);
