@@ -128,23 +128,6 @@ using r3dsimt::fmadd;
 // Smallest power of two >= m (m in 1..8): the number of lane groups.
 R3D_DEVICE int groups_for(int m) { return m <= 1 ? 1 : (m <= 2 ? 2 : (m <= 4 ? 4 : 8)); }
 
-// floor(q) of |q| < 2^22 as float and as int, without the conversion unit:
-// adding 1.5 * 2^23 rounds to a whole number that the sum's low bits hold.
-R3D_DEVICE float floor_small(float q, int& i) {
-  const float magic = 12582912.0F;
-  const float t = __fadd_rn(q, magic);
-  float r = __fsub_rn(t, magic);
-  int bits, mbits;
-  memcpy(&bits, &t, 4);
-  memcpy(&mbits, &magic, 4);
-  i = bits - mbits;
-  if (r > q) {
-    r = __fsub_rn(r, 1.0F);
-    --i;
-  }
-  return r;
-}
-
 // One view's terms at plane theta (refinement.cpp:46-152), computed by the
 // `gsize` lanes of a group: lane `gl` of the group takes the window samples
 // gl, gl + gsize, ... NCC of the warped window with the normalised base
@@ -227,10 +210,7 @@ R3D_DEVICE void evaluate_group(const ViewGeo& g, bool active, double x, double y
         const T h2 = hzf + d2;
         inv_z = T(1) / h2;
         const T q0 = fmadd(fmadd(-cf0, d2, d0), inv_z, fc0), q1 = fmadd(fmadd(-cf1, d2, d1), inv_z, fc1);
-        int k0, k1;
-        const T fl0 = floor_small(static_cast<float>(q0), k0), fl1 = floor_small(static_cast<float>(q1), k1);
-        ix = ic0 + k0;
-        iy = ic1 + k1;
+        const T fl0 = floor_small(static_cast<float>(q0), ic0, ix), fl1 = floor_small(static_cast<float>(q1), ic1, iy);
         fx = q0 - fl0;
         fy = q1 - fl1;
         // ix and iy as floats: exact wherever they are inside an image.

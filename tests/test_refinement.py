@@ -12,6 +12,9 @@ within 1e-5 relative of the double oracle.
 
 from __future__ import annotations
 
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
@@ -178,3 +181,40 @@ def test_depth_stage_in_one_call_equals_the_steps(simt_matcher):
     for x, y in zip(a, b):
         assert np.array_equal(x["depth"], y["depth"]) and np.array_equal(x["support"], y["support"])
         assert np.array_equal(x["confidence"], y["confidence"])
+
+
+FLOOR_PROGRAM = r"""
+#include <cmath>
+#include <cstdio>
+#include "geom.cuh"
+int main() {
+  int bad = 0, i = 0;
+  // Inside its range: the floor, exactly, as float and added to the base.
+  for (float q : {0.0F, -0.0F, 0.25F, -0.25F, 1.0F, -1.0F, 1023.75F, -1024.5F, 999999.5F, -999999.5F, 4194303.0F,
+                  -4194303.0F}) {
+    const float f = r3dgpu::floor_small(q, 100, i);
+    bad += f != std::floor(q) || i != 100 + static_cast<int>(std::floor(q));
+  }
+  // Outside it (samples at the camera plane): any value, no undefined arithmetic.
+  for (float q : {-12582912.0F, -12582913.0F, -1.3e7F, -2.0e7F, -2.6e7F, -1e9F, -1e30F, 1e9F, 1e30F, INFINITY, -INFINITY,
+                  NAN})
+    for (int base : {-99999999, 0, 99999999}) r3dgpu::floor_small(q, base, i);
+  std::printf("%d\n", bad);
+  return bad;
+}
+"""
+
+
+def test_floor_of_sample_positions(tmp_path):
+    """The float path's floor of sample positions: exact in its range, and free
+    of signed overflow for the positions that the range test after it rejects
+    (compiled with the overflow check, which ends the program)."""
+    src = tmp_path / "floor.cpp"
+    src.write_text(FLOOR_PROGRAM)
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "regard3d_mvs_b200", "csrc")
+    exe = str(tmp_path / "floor")
+    subprocess.run(["/usr/bin/g++", "-std=c++17", "-O0", "-DR3DGPU_SIMT_EMULATION", "-ffp-contract=off",
+                    "-fsanitize=signed-integer-overflow", "-fno-sanitize-recover=all", "-I", csrc, "-I",
+                    os.path.join(os.path.dirname(os.path.abspath(__file__)), "simt"), str(src), "-o", exe], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
