@@ -810,50 +810,53 @@ bool ranged_terms_allowed() {
 }
 
 // Waves of the tiles of a round for the chain passes (full-range tiles, or
-// with `ranged` the tiles with per-pixel ranges): tiles in order of kernel
-// shape, a new wave whenever the next tile would take the wave's buffers past
-// `cap_bytes` (a tile larger than that gets a wave of its own). The job
-// tables are copied to the device on s; `max_bytes` receives the largest
-// wave's buffer size.
+// with `ranged` the tiles with per-pixel ranges): tiles with byte terms, then
+// those with u16 sums, each in order of kernel shape, a new wave whenever the
+// next tile would take the wave's buffers past `cap_bytes` (a tile larger than
+// that gets a wave of its own). The job tables are copied to the device on s;
+// `max_bytes` receives the largest wave's buffer size.
+//
+// A tile keeps byte terms (9 bytes a label against 3) when its match allows
+// them (all P2 <= 255) and its buffers stay within `tile_cap`, the round's
+// scratch that this group may take. Both are decided tile by tile: another
+// pair's penalties or size do not change a pair's mode.
 void plan_path_waves(const std::vector<std::pair<int, int>>& tiles, const std::vector<Match*>& matches, bool ranged,
-                     size_t cap_bytes, int sms, Arena& A, Pinned& H, cudaStream_t s,
+                     size_t cap_bytes, size_t tile_cap, int sms, Arena& A, Pinned& H, cudaStream_t s,
                      std::vector<SgmPathRangedWave>& waves, std::vector<std::vector<SgmPathSegment>>& segs,
                      size_t& max_bytes, uint64_t& cells_sum, uint64_t& px_sum) {
   struct Entry {
     int i, t;
+    bool terms;
     SgmPathShape sh;
     int64_t cells, px, keys, rows;
     int maxnum;
+  };
+  auto bytes = [&](bool terms, int64_t cells, int64_t px, int64_t keys, int64_t rows, int maxnum) -> size_t {
+    return ranged ? sgm_path_ranged_buffers(cells, px, keys, rows, maxnum, sms, terms).total
+                  : sgm_path_buffers(cells, px, keys, terms).total;
   };
   std::vector<Entry> es;
   es.reserve(tiles.size());
   for (const auto& mt : tiles) {
     const Match& M = *matches[mt.first];
     const Tile& T = M.layout.tiles[mt.second];
-    const int64_t px = static_cast<int64_t>(T.w) * T.h;
-    const SgmPathShape sh = ranged ? sgm_path_ranged_shape(static_cast<int64_t>(M.tile_cells[mt.second]), px)
-                                   : sgm_path_shape(M.m.nd);
-    es.push_back(Entry{mt.first, mt.second, sh, static_cast<int64_t>(M.tile_cells[mt.second]), px,
-                       M.m.diagonal_lr ? static_cast<int64_t>(T.h) * (T.w + M.m.nd) : 0, T.h,
-                       M.tile_maxnum[mt.second]});
+    Entry e{};
+    e.i = mt.first;
+    e.t = mt.second;
+    e.cells = static_cast<int64_t>(M.tile_cells[mt.second]);
+    e.px = static_cast<int64_t>(T.w) * T.h;
+    e.keys = M.m.diagonal_lr ? static_cast<int64_t>(T.h) * (T.w + M.m.nd) : 0;
+    e.rows = T.h;
+    e.maxnum = M.tile_maxnum[mt.second];
+    e.terms = M.m.term_u8 != 0 && (!ranged || ranged_terms_allowed()) &&
+              bytes(true, e.cells, e.px, e.keys, e.rows, e.maxnum) <= tile_cap;
+    e.sh = ranged ? sgm_path_ranged_shape(e.cells, e.px) : sgm_path_shape(M.m.nd);
+    es.push_back(e);
   }
-  // Waves keep byte terms when every match of the group allows them (all
-  // P2 <= 255); otherwise u16 sums.
-  bool terms = !ranged || ranged_terms_allowed();
-  for (const auto& mt : tiles) terms = terms && matches[mt.first]->m.term_u8 != 0;
-  // A tile whose terms alone would pass the wave's share of the scratch (9 bytes
-  // per label against 3) keeps its group on u16 sums.
-  for (const Entry& e : es)
-    if (terms)
-      terms = (ranged ? sgm_path_ranged_buffers(e.cells, e.px, e.keys, e.rows, e.maxnum, sms, true).total
-                      : sgm_path_buffers(e.cells, e.px, e.keys, true).total) <= cap_bytes;
-  auto bytes = [&](int64_t cells, int64_t px, int64_t keys, int64_t rows, int maxnum) -> size_t {
-    return ranged ? sgm_path_ranged_buffers(cells, px, keys, rows, maxnum, sms, terms).total
-                  : sgm_path_buffers(cells, px, keys, terms).total;
-  };
-  // By width, then by shape: a segment per shape (a tuning table can give two
-  // label counts shapes of one width), at most as many as compiled shapes.
+  // By mode, width, then shape: a segment per shape (a tuning table can give
+  // two label counts shapes of one width), at most as many as compiled shapes.
   std::stable_sort(es.begin(), es.end(), [](const Entry& a, const Entry& b) {
+    if (a.terms != b.terms) return a.terms;
     const int wa = a.sh.g_ * a.sh.k_, wb = b.sh.g_ * b.sh.k_;
     return wa != wb ? wa < wb : a.sh.g_ < b.sh.g_;
   });
@@ -866,11 +869,13 @@ void plan_path_waves(const std::vector<std::pair<int, int>>& tiles, const std::v
   while (begin < es.size()) {
     int64_t cells = 0, px = 0, keys = 0, rows = 0;
     int maxnum = 16, span = 0;
+    const bool terms = es[begin].terms;
     size_t end = begin;
     while (end < es.size()) {
       const Entry& e = es[end];
       if (end > begin &&
-          bytes(cells + e.cells, px + e.px, keys + e.keys, rows + e.rows, std::max(maxnum, e.maxnum)) > cap_bytes)
+          (e.terms != terms || bytes(terms, cells + e.cells, px + e.px, keys + e.keys, rows + e.rows,
+                                     std::max(maxnum, e.maxnum)) > cap_bytes))
         break;
       cells += e.cells;
       px += e.px;
@@ -934,7 +939,7 @@ void plan_path_waves(const std::vector<std::pair<int, int>>& tiles, const std::v
     wv.max_span = span;
     waves.push_back(wv);
     segs.push_back(std::move(sg));
-    max_bytes = std::max(max_bytes, bytes(co, po, ko, ro, maxnum));
+    max_bytes = std::max(max_bytes, bytes(terms, co, po, ko, ro, maxnum));
     cells_sum += static_cast<uint64_t>(co);
     px_sum += static_cast<uint64_t>(po);
     begin = end;
@@ -1102,8 +1107,10 @@ BatchRun enqueue_batch(r3dgpu_pair* pairs, int count, cudaStream_t s, int slot) 
       L.g = &g;
       if (g.kind == kPath || g.kind == kPathRanged) {
         // Waves up to half the budget (fewer, longer pass launches with more
-        // chains in flight); a round has at most one group of each kind.
-        plan_path_waves(g.tiles, matches, g.kind == kPathRanged, round_budget / 2, W.sms, A, H, s, L.waves, L.segs,
+        // chains in flight); a round has at most one group of each kind. A
+        // group alone in its round may take all of it for a large tile.
+        plan_path_waves(g.tiles, matches, g.kind == kPathRanged, round_budget / 2,
+                        groups.size() == 1 ? round_budget : round_budget / 2, W.sms, A, H, s, L.waves, L.segs,
                         L.slot_bytes, L.cells_sum, L.px_sum);
         L.njobs = static_cast<int>(g.tiles.size());
         L.grid = 1;

@@ -111,3 +111,40 @@ def test_shapes_of_one_width_in_a_batch(simt_matcher, monkeypatch):
     assert sorted(e["shape"].split("/")[0] for e in launches if e.get("pass")) == ["16x8", "8x16"]
     for a, b in zip(got, ref):
         assert np.array_equal(a.disparity, b.disparity) and np.array_equal(a.confidence, b.confidence)
+
+
+def _scratch_budget(m, n):
+    """Sets the SGM scratch budget of this thread, as a server worker does (0: the default)."""
+    m.lib._ZN6r3dgpu25set_thread_scratch_budgetEm(ctypes.c_size_t(n))
+
+
+def test_pass_mode_by_tile(simt_matcher):
+    """The pass mode is each tile's own: a tile whose byte terms (9 bytes a
+    label) pass the scratch budget takes u16 sums (3 bytes), as a pair with a
+    P2 above 255 does, and the batch's other pairs keep byte terms."""
+    def pair(seed, w, h, nd, **kw):
+        left, right, _ = render_pair(Texture(seed), w, h, lambda x, y: 5.0 + 0.1 * x)
+        return dict(left=left, right=right, disparity_min=0, num_disparities=nd, options=StereoOptions(**kw))
+
+    def modes(pairs, budget):
+        _scratch_budget(simt_matcher, budget)
+        try:
+            return pass_shapes(simt_matcher, lambda: simt_matcher.match_stereo_batch(pairs))
+        finally:
+            _scratch_budget(simt_matcher, 0)
+
+    # 60 x 24 x 64 labels: 829 kB with terms, 276 kB without.
+    pairs = [pair(71, 60, 24, 64, levels=0), pair(72, 24, 12, 32, levels=0), pair(73, 20, 10, 16, levels=0, p2=400)]
+    ref, shapes = modes(pairs, 0)
+    assert shapes == {"4x8/mode3", "2x8/mode3", "1x8/mode0", "1x8/mode1"}
+    got, shapes = modes(pairs, 500_000)
+    assert shapes == {"4x8/mode0", "4x8/mode1", "2x8/mode3", "1x8/mode0", "1x8/mode1"}
+    for a, b in zip(got, ref):
+        assert np.array_equal(a.disparity, b.disparity) and np.array_equal(a.confidence, b.confidence)
+    # Ranged tiles: the finer level of a hierarchy (its coarser one, full range, is smaller).
+    pairs = [pair(74, 72, 40, 48, levels=1, range_radius=0, range_margin=2, range_fill=0)]
+    ref, shapes = modes(pairs, 0)
+    assert {q.split("/")[1] for q in shapes if q.startswith("1x")} == {"mode3"}
+    got, shapes = modes(pairs, 300_000)
+    assert {q.split("/")[1] for q in shapes if q.startswith("1x")} == {"mode0", "mode1"}
+    assert np.array_equal(got[0].disparity, ref[0].disparity)
