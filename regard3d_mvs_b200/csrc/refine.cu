@@ -1,8 +1,15 @@
 // Patch-based depth refinement (r3dgpu_refine_depth_map) and its input images
 // (r3dgpu_make_refinement_image), the reference's src/r3d/mvs/refinement.cpp.
 //
-// Four depth-map pixels per warp, 8 lanes each. The lanes of a pixel split into
-// one group per view (two lanes each for 4 views); a lane warps, samples and
+// A first kernel lists the pixels to refine (a depth, the window inside the
+// image); the refinement runs over that list, so that a sparse map costs what
+// its depths cost: four neighbours of which one has a depth would keep a warp
+// as long as four depths (1024 x 768 pixels, one in ten with a depth, float
+// terms: 4.8 ms with four neighbours per warp, 1.1 from the list; all with a
+// depth: 9.5 and 9.0).
+//
+// Four pixels per warp, 8 lanes each. The lanes of a pixel split into one
+// group per view (two lanes each for 4 views); a lane warps, samples and
 // normalises every second (or so) of its view's window samples (25 for the
 // default 9 x 9 window at step 2, 49 for a 7 x 7 window at step 1, at most
 // 225), and every sum of the NCC and of the Gauss-Newton terms is an
@@ -41,7 +48,7 @@ namespace {
 constexpr int kMaxSamples = 225;  // refinement.cpp:21
 constexpr int kMaxViews = 8;      // refinement.cpp:22
 constexpr double kDiscontinuity = 0.05;
-enum : int { kInput, kRefined, kUnconfirmed, kCounters };
+enum : int { kInput, kRefined, kUnconfirmed, kCounters, kListed = kCounters };  // kListed: slot 0 only
 constexpr int kSlots = 128, kSlotStride = 4;  // copies of the counters (one address takes an addition at a time)
 constexpr int kPixels = 4;                    // pixels per warp
 constexpr int kLanes = 32 / kPixels;          // lanes per pixel (at least one per view)
@@ -401,19 +408,68 @@ R3D_DEVICE void solve_damped(const double* hh, const double* gg, double* delta) 
   for (int i = 0; i < 3; ++i) delta[perm[i]] = -y[i];
 }
 
+// The pixels to refine, runs of kListRun pixels in the order their blocks come
+// to it (a run's pixels in image order): those with a depth whose window lies
+// inside the image, if there are views. Every pixel with a depth is counted
+// and its confidence zeroed.
+constexpr int kListThreads = 256, kListRun = 4 * kListThreads;
+R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kListThreads)
+    list_kernel(const float* R3D_RESTRICT input, float* conf, int64_t stride, Params p, int64_t* R3D_RESTRICT list,
+                unsigned long long* counters) {
+  constexpr int kWarps = kListThreads / 32, kParts = kListRun / 32;
+  R3D_DYNAMIC_SMEM(smem);
+  int64_t* const start = reinterpret_cast<int64_t*>(smem);  // of the run's 32-pixel parts in the list
+  const int lane = static_cast<int>(r3dsimt::lane_id()), warp = static_cast<int>(threadIdx.x >> 5);
+  const int64_t total = static_cast<int64_t>(p.width) * p.height;
+  const int64_t first = static_cast<int64_t>(blockIdx.x) * kListRun;
+  unsigned long long* const slot = counters + (blockIdx.x % kSlots) * kSlotStride;
+  uint32_t mine[kListRun / kListThreads];
+#pragma unroll
+  for (int k = 0; k < kListRun / kListThreads; ++k) {
+    const int part = k * kWarps + warp;
+    const int64_t pix = first + part * 32 + lane;
+    const bool valid = pix < total && input[pix] > 0.0F;
+    const int y = static_cast<int>(pix / p.width), x = static_cast<int>(pix - static_cast<int64_t>(y) * p.width);
+    if (valid) conf[static_cast<int64_t>(y) * stride + x] = 0.0F;
+    const uint32_t v = r3dsimt::ballot(valid);
+    if (lane == 0 && v != 0) atomicAdd(slot + kInput, static_cast<unsigned long long>(r3dsimt::popc(v)));
+    mine[k] = r3dsimt::ballot(valid && p.num_views > 0 && x >= p.radius && y >= p.radius && x < p.width - p.radius &&
+                              y < p.height - p.radius);
+    if (lane == 0) start[part] = r3dsimt::popc(mine[k]);
+  }
+  r3dsimt::syncthreads();
+  if (threadIdx.x == 0) {
+    int64_t n = 0;
+    for (int i = 0; i < kParts; ++i) {
+      const int64_t c = start[i];
+      start[i] = n;
+      n += c;
+    }
+    start[kParts] = n > 0 ? static_cast<int64_t>(atomicAdd(counters + kListed, static_cast<unsigned long long>(n))) : 0;
+  }
+  r3dsimt::syncthreads();
+#pragma unroll
+  for (int k = 0; k < kListRun / kListThreads; ++k) {
+    const int part = k * kWarps + warp;
+    if ((mine[k] >> lane) & 1u)
+      list[start[kParts] + start[part] + r3dsimt::popc(mine[k] & ((1u << lane) - 1u))] = first + part * 32 + lane;
+  }
+}
+
 // Dynamic shared memory: the window's p.n samples, then per pixel of the block
 // its p.n normalised base window values.
 template <class T>
 R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN(kRefineThreads, 4)
     refine_kernel(const float* R3D_RESTRICT input, float* depth, float* conf, int64_t stride,
                   const float* R3D_RESTRICT base, int64_t bstride, const ViewGeo* R3D_RESTRICT views, Params p,
-                  unsigned long long* counters) {
+                  const int64_t* R3D_RESTRICT list, unsigned long long* counters) {
   R3D_DYNAMIC_SMEM(smem);
   const int lane = static_cast<int>(r3dsimt::lane_id()), warp = static_cast<int>(threadIdx.x >> 5);
   const int sub = lane / kLanes, wl = lane % kLanes;  // the pixel of the warp, the lane of the pixel
   const bool lead = wl == 0;
-  const int64_t total = static_cast<int64_t>(p.width) * p.height;
+  const int64_t listed = static_cast<int64_t>(counters[kListed]);  // complete: written by the launch before
   const int64_t first = ((static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * kPixels;
+  if (first - warp * kPixels >= listed) return;  // whole block
   const int r = p.radius;
   Sample<T>* const samples = reinterpret_cast<Sample<T>*>(smem);
   for (int s = static_cast<int>(threadIdx.x); s < p.n; s += static_cast<int>(blockDim.x)) {
@@ -422,21 +478,17 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN(kRefineThreads, 4)
                            static_cast<T>(static_cast<double>(oy) / r)};
   }
   r3dsimt::syncthreads();
-  if (first >= total) return;  // whole warp
-  const int64_t pix = first + sub < total ? first + sub : first;
+  if (first >= listed) return;  // whole warp
+  bool live = first + sub < listed;
+  const int64_t pix = list[live ? first + sub : first];
   const int y = static_cast<int>(pix / p.width), x = static_cast<int>(pix - static_cast<int64_t>(y) * p.width);
   const float z0 = input[pix];
-  const bool valid_px = first + sub < total && z0 > 0.0F;
   const int64_t at = static_cast<int64_t>(y) * stride + x;
   unsigned long long* const slot = counters + (blockIdx.x % kSlots) * kSlotStride;
   auto count = [&](int counter, bool pred) {  // pixels of the warp with pred (one vote each)
     const uint32_t b = r3dsimt::ballot(pred && lead);
     if (lane == 0 && b != 0) atomicAdd(slot + counter, static_cast<unsigned long long>(r3dsimt::popc(b)));
   };
-  count(kInput, valid_px);
-  if (valid_px && lead) conf[at] = 0.0F;
-  bool live = valid_px && p.num_views > 0 && x >= r && y >= r && x < p.width - r && y < p.height - r;
-  if (r3dsimt::ballot(live) == 0) return;
 
   // The normalised base window into the pixel's table.
   double* const n0s = reinterpret_cast<double*>(samples + p.n) + static_cast<size_t>(warp * kPixels + sub) * p.n;
@@ -619,6 +671,7 @@ R3D_GLOBAL void repack_kernel(const float* in, int64_t istride, int w, int h, fl
 struct Scratch {
   DeviceBuffer<unsigned long long> counters;
   DeviceBuffer<float> input, blur_tmp, blur_out, taps;
+  DeviceBuffer<int64_t> list;  // the pixels to refine
   DeviceBuffer<ViewGeo> views;
   DeviceBuffer<float4> packed;  // the views' repacked images
 };
@@ -667,13 +720,18 @@ r3dgpu_refinement_options options_or_default(const r3dgpu_refinement_options* o)
 
 template <class T>
 void launch_refine(const float* input, float* depth, float* conf, int64_t stride, const float* base,
-                   int64_t bstride, const ViewGeo* views, const Params& p, unsigned long long* counters,
+                   int64_t bstride, const ViewGeo* views, const Params& p, int64_t* list, unsigned long long* counters,
                    cudaStream_t s) {
+  const int64_t total = static_cast<int64_t>(p.width) * p.height;
+  R3D_LAUNCH(list_kernel, static_cast<unsigned>(ceil_div64(total, kListRun)), kListThreads,
+             sizeof(int64_t) * (kListRun / 32 + 1), s, input, conf, stride, p, list, counters);
+  launched("list_kernel");
+  // Blocks for a full list; those past its end return at once.
   constexpr int per_block = kRefineThreads / 32 * kPixels;
   const size_t smem = (sizeof(Sample<T>) + sizeof(double) * per_block) * static_cast<size_t>(p.n);
   auto kernel = refine_kernel<T>;
-  R3D_LAUNCH(kernel, static_cast<unsigned>(ceil_div64(static_cast<int64_t>(p.width) * p.height, per_block)),
-             kRefineThreads, smem, s, input, depth, conf, stride, base, bstride, views, p, counters);
+  R3D_LAUNCH(kernel, static_cast<unsigned>(ceil_div64(total, per_block)), kRefineThreads, smem, s, input, depth, conf,
+             stride, base, bstride, views, p, list, counters);
   launched(sizeof(T) == 8 ? "refine_kernel<f64>" : "refine_kernel<f32>");
 }
 
@@ -722,6 +780,7 @@ void refine(float* depth, float* conf, int64_t stride, const r3dgpu_pinhole_came
     }
     if (nv > 0)
       R3D_CUDA(cudaMemcpyAsync(sc.views.get(), geo, sizeof(ViewGeo) * nv, cudaMemcpyHostToDevice, s));
+    sc.list.reserve(static_cast<size_t>(w) * h);
     sc.input.reserve(static_cast<size_t>(w) * h);
     R3D_CUDA(cudaMemcpy2DAsync(sc.input.get(), sizeof(float) * w, depth, sizeof(float) * stride, sizeof(float) * w,
                                h, cudaMemcpyDeviceToDevice, s));
@@ -729,10 +788,10 @@ void refine(float* depth, float* conf, int64_t stride, const r3dgpu_pinhole_came
              o.min_texture * o.min_texture * n, o.drop_unconfirmed};
     if (o.fp32)
       launch_refine<float>(sc.input.get(), depth, conf, stride, base.data, base.stride, sc.views.get(), p,
-                           sc.counters.get(), s);
+                           sc.list.get(), sc.counters.get(), s);
     else
       launch_refine<double>(sc.input.get(), depth, conf, stride, base.data, base.stride, sc.views.get(), p,
-                            sc.counters.get(), s);
+                            sc.list.get(), sc.counters.get(), s);
   }
   unsigned long long slots[kSlots * kSlotStride], c[kCounters] = {};
   R3D_CUDA(cudaMemcpyAsync(slots, sc.counters.get(), sizeof(slots), cudaMemcpyDeviceToHost, s));

@@ -123,6 +123,36 @@ def test_kernel_unrelated_views_equal_oracle(simt_matcher, oracle, scene):
     compare(a, b, simt_matcher.refine_depth_map(a, base, wrong, opts), oracle.refine_depth_map(b, base, wrong, opts))
 
 
+@pytest.mark.parametrize("build", ["simt_matcher", pytest.param("gpu_matcher", marks=pytest.mark.gpu)])
+@pytest.mark.parametrize("kind", ["none", "border", "few", "last"])
+def test_listed_pixels(request, oracle, scene, build, kind):
+    """The list of pixels to refine: no depth at all, depths whose windows leave
+    the image (counted, not refined), fewer pixels than a warp takes on both
+    sides of a run of 1,024, and the image's last runs only."""
+    matcher = request.getfixturevalue(build)
+    m, _, base, views, _ = scene
+    h, w = m["depth"].shape
+    keep = np.zeros(h * w, bool)
+    if kind == "border":
+        grid = keep.reshape(h, w)
+        grid[:4, ::9] = grid[-4:, ::7] = grid[::5, :4] = grid[::3, -4:] = True
+    elif kind == "few":
+        for k in (6, 11, 12):  # (1024 k - 1) and 1024 k lie inside the borders
+            assert 4 <= (1024 * k - 1) % w < w - 4 and 4 <= 1024 * k % w < w - 4
+        keep[[6 * 1024 - 1, 6 * 1024, 11 * 1024, 12 * 1024 - 1, 12 * 1024]] = True
+    elif kind == "last":
+        keep.reshape(h, w)[-8:-4, -20:] = True
+    out = []
+    for f in (matcher, oracle):
+        a = copy_map(m)
+        a["depth"] = np.where(keep.reshape(h, w), m["depth"], 0).astype(np.float32)
+        a["confidence"] = np.full((h, w), 0.25, np.float32)  # zeroed at depths, else kept
+        out.append((a, f.refine_depth_map(a, base, views, RefinementOptions(min_gain=0.0))))
+    (a, ia), (b, ib) = out
+    compare(a, b, ia, ib) if kind != "none" else np.testing.assert_array_equal(a["confidence"], b["confidence"])
+    assert ia == ib and ia["input"] == keep.sum()
+
+
 def fp32_error(a, b):
     """Relative depth error of the float path against the double oracle."""
     valid = b["depth"] > 0
