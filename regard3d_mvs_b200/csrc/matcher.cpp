@@ -810,15 +810,16 @@ bool ranged_terms_allowed() {
 }
 
 // Waves of the tiles of a round for the chain passes (full-range tiles, or
-// with `ranged` the tiles with per-pixel ranges): tiles with byte terms, then
-// those with u16 sums, each in order of kernel shape, a new wave whenever the
-// next tile would take the wave's buffers past `cap_bytes` (a tile larger than
-// that gets a wave of its own). The job tables are copied to the device on s;
+// with `ranged` the tiles with per-pixel ranges): tiles in order of pass mode,
+// then of kernel shape, a new wave for each mode and whenever the next tile
+// would take the wave's buffers past `cap_bytes` (a tile larger than that gets
+// a wave of its own). The job tables are copied to the device on s;
 // `max_bytes` receives the largest wave's buffer size.
 //
-// A tile keeps byte terms (9 bytes a label against 3) when its match allows
-// them (all P2 <= 255) and its buffers stay within `tile_cap`, the round's
-// scratch that this group may take. Both are decided tile by tile: another
+// A tile takes the fastest mode whose buffers stay within `tile_cap`, the
+// round's scratch that this group may take: byte terms (9 bytes a label) when
+// its match allows them (all P2 <= 255), else u16 sums in two volumes (5,
+// full-range tiles) or in one (3). This is decided tile by tile: another
 // pair's penalties or size do not change a pair's mode.
 void plan_path_waves(const std::vector<std::pair<int, int>>& tiles, const std::vector<Match*>& matches, bool ranged,
                      size_t cap_bytes, size_t tile_cap, int sms, Arena& A, Pinned& H, cudaStream_t s,
@@ -826,14 +827,14 @@ void plan_path_waves(const std::vector<std::pair<int, int>>& tiles, const std::v
                      size_t& max_bytes, uint64_t& cells_sum, uint64_t& px_sum) {
   struct Entry {
     int i, t;
-    bool terms;
+    SgmPathMode mode;
     SgmPathShape sh;
     int64_t cells, px, keys, rows;
     int maxnum;
   };
-  auto bytes = [&](bool terms, int64_t cells, int64_t px, int64_t keys, int64_t rows, int maxnum) -> size_t {
-    return ranged ? sgm_path_ranged_buffers(cells, px, keys, rows, maxnum, sms, terms).total
-                  : sgm_path_buffers(cells, px, keys, terms).total;
+  auto bytes = [&](SgmPathMode mode, int64_t cells, int64_t px, int64_t keys, int64_t rows, int maxnum) -> size_t {
+    return ranged ? sgm_path_ranged_buffers(cells, px, keys, rows, maxnum, sms, mode).total
+                  : sgm_path_buffers(cells, px, keys, mode).total;
   };
   std::vector<Entry> es;
   es.reserve(tiles.size());
@@ -848,15 +849,19 @@ void plan_path_waves(const std::vector<std::pair<int, int>>& tiles, const std::v
     e.keys = M.m.diagonal_lr ? static_cast<int64_t>(T.h) * (T.w + M.m.nd) : 0;
     e.rows = T.h;
     e.maxnum = M.tile_maxnum[mt.second];
-    e.terms = M.m.term_u8 != 0 && (!ranged || ranged_terms_allowed()) &&
-              bytes(true, e.cells, e.px, e.keys, e.rows, e.maxnum) <= tile_cap;
-    e.sh = ranged ? sgm_path_ranged_shape(e.cells, e.px) : sgm_path_shape(M.m.nd);
+    auto fits = [&](SgmPathMode mode) {
+      return bytes(mode, e.cells, e.px, e.keys, e.rows, e.maxnum) <= tile_cap;
+    };
+    e.mode = M.m.term_u8 != 0 && (!ranged || ranged_terms_allowed()) && fits(kPathTerms) ? kPathTerms
+             : !ranged && fits(kPathTwoSums)                                             ? kPathTwoSums
+                                                                                         : kPathSum;
+    e.sh = ranged ? sgm_path_ranged_shape(e.cells, e.px) : sgm_path_shape(M.m.nd, e.mode == kPathTerms);
     es.push_back(e);
   }
   // By mode, width, then shape: a segment per shape (a tuning table can give
   // two label counts shapes of one width), at most as many as compiled shapes.
   std::stable_sort(es.begin(), es.end(), [](const Entry& a, const Entry& b) {
-    if (a.terms != b.terms) return a.terms;
+    if (a.mode != b.mode) return a.mode < b.mode;
     const int wa = a.sh.g_ * a.sh.k_, wb = b.sh.g_ * b.sh.k_;
     return wa != wb ? wa < wb : a.sh.g_ < b.sh.g_;
   });
@@ -869,13 +874,13 @@ void plan_path_waves(const std::vector<std::pair<int, int>>& tiles, const std::v
   while (begin < es.size()) {
     int64_t cells = 0, px = 0, keys = 0, rows = 0;
     int maxnum = 16, span = 0;
-    const bool terms = es[begin].terms;
+    const SgmPathMode mode = es[begin].mode;
     size_t end = begin;
     while (end < es.size()) {
       const Entry& e = es[end];
       if (end > begin &&
-          (e.terms != terms || bytes(terms, cells + e.cells, px + e.px, keys + e.keys, rows + e.rows,
-                                     std::max(maxnum, e.maxnum)) > cap_bytes))
+          (e.mode != mode || bytes(mode, cells + e.cells, px + e.px, keys + e.keys, rows + e.rows,
+                                   std::max(maxnum, e.maxnum)) > cap_bytes))
         break;
       cells += e.cells;
       px += e.px;
@@ -935,11 +940,11 @@ void plan_path_waves(const std::vector<std::pair<int, int>>& tiles, const std::v
     wv.keys = ko;
     wv.rows = ro;
     wv.maxnum = maxnum;
-    wv.terms = terms ? 1 : 0;
+    wv.mode = mode;
     wv.max_span = span;
     waves.push_back(wv);
     segs.push_back(std::move(sg));
-    max_bytes = std::max(max_bytes, bytes(terms, co, po, ko, ro, maxnum));
+    max_bytes = std::max(max_bytes, bytes(mode, co, po, ko, ro, maxnum));
     cells_sum += static_cast<uint64_t>(co);
     px_sum += static_cast<uint64_t>(po);
     begin = end;
@@ -1060,7 +1065,7 @@ BatchRun enqueue_batch(r3dgpu_pair* pairs, int count, cudaStream_t s, int slot) 
         // Full-range tiles of every label count: the chain passes, one group.
         bool fits = true;
         for (int t = 0; t < nt; ++t) fits = fits && sgm_path_fits(M.layout.tiles[t].w, M.m.nd);
-        if (sgm_path_enabled() && sgm_path_shape(M.m.nd).g_ != 0 && fits) {
+        if (sgm_path_enabled() && sgm_path_shape(M.m.nd, true).g_ != 0 && fits) {
           Group& g = group_for(kPath, 0, SgmFullPlan{{0, 0}, 0});
           for (int t = 0; t < nt; ++t) g.tiles.emplace_back(i, t);
           continue;
@@ -1248,7 +1253,7 @@ BatchRun enqueue_batch(r3dgpu_pair* pairs, int count, cudaStream_t s, int slot) 
           w.keys = rw.keys;
           w.rows = rw.rows;
           w.buffer = scratch;
-          w.terms = rw.terms;
+          w.mode = rw.mode;
           w.max_span = rw.max_span;
           launch_sgm_path_wave(dm, w, W.sms, gs);
         }
@@ -1879,7 +1884,7 @@ r3dgpu_status r3dgpu_sgm_cost_volume_host(const r3dgpu_view_u16* left, const r3d
     }
     SgmMatch* hm = W.pinned.alloc<SgmMatch>(1);
     fill_match(*hm, o, DView<uint16_t>{dl, wl, h, wl}, cl, cr, wr, il, ir, rlo, rnum, disparity_min, nd, false, false);
-    if (!(ranges_lo && ranges_num) && sgm_path_enabled() && sgm_path_shape(nd).g_ != 0 && sgm_path_fits(wl, nd)) {
+    if (!(ranges_lo && ranges_num) && sgm_path_enabled() && sgm_path_shape(nd, true).g_ != 0 && sgm_path_fits(wl, nd)) {
       // The whole image as one full-range tile through the chain passes.
       SgmMatch* dm = A.alloc<SgmMatch>(1);
       R3D_CUDA(cudaMemcpyAsync(dm, hm, sizeof(SgmMatch), cudaMemcpyHostToDevice, s));
@@ -1888,7 +1893,8 @@ r3dgpu_status r3dgpu_sgm_cost_volume_host(const r3dgpu_view_u16* left, const r3d
       *hj = SgmPathJob{};
       hj->w = wl;
       hj->h = h;
-      const SgmPathShape sh = sgm_path_shape(nd);
+      const SgmPathMode mode = hm->term_u8 != 0 ? kPathTerms : kPathTwoSums;
+      const SgmPathShape sh = sgm_path_shape(nd, mode == kPathTerms);
       SgmPathSegment seg{sh, 0, 1, {0, 0, 0}, static_cast<int64_t>(cells), px, nd == 2 * sh.g_ * sh.k_ ? 1 : 0};
       for (int c = 0; c < kPathClasses; ++c) seg.blocks[c] = (sgm_path_chains(c, wl, h) + 32 / sh.g_ - 1) / (32 / sh.g_);
       hj->disp = A.alloc<float>(static_cast<size_t>(px));
@@ -1906,8 +1912,8 @@ r3dgpu_status r3dgpu_sgm_cost_volume_host(const r3dgpu_view_u16* left, const r3d
       wv.pixels = px;
       wv.keys = 0;
       wv.rows = h;
-      wv.terms = hm->term_u8;
-      W.scratch.reserve(sgm_path_buffers(wv.cells, px, 0, wv.terms != 0).total);
+      wv.mode = mode;
+      W.scratch.reserve(sgm_path_buffers(wv.cells, px, 0, mode).total);
       wv.buffer = W.scratch.get();
       launch_sgm_path_wave(dm, wv, W.sms, s);
       R3D_CUDA(cudaMemcpyAsync(out, vol, sizeof(uint16_t) * cells, cudaMemcpyDeviceToHost, s));
@@ -1943,8 +1949,8 @@ r3dgpu_status r3dgpu_sgm_cost_volume_host(const r3dgpu_view_u16* left, const r3d
       wv.keys = 0;
       wv.rows = h;
       wv.maxnum = max_num;
-      wv.terms = hm->term_u8 != 0 && ranged_terms_allowed() ? 1 : 0;
-      W.scratch.reserve(sgm_path_ranged_buffers(wv.cells, px, 0, h, max_num, W.sms, wv.terms != 0).total);
+      wv.mode = hm->term_u8 != 0 && ranged_terms_allowed() ? kPathTerms : kPathSum;
+      W.scratch.reserve(sgm_path_ranged_buffers(wv.cells, px, 0, h, max_num, W.sms, wv.mode).total);
       wv.buffer = W.scratch.get();
       launch_sgm_path_ranged_wave(dm, wv, W.sms, s);
       R3D_CUDA(cudaMemcpyAsync(out, vol, sizeof(uint16_t) * cells, cudaMemcpyDeviceToHost, s));

@@ -203,7 +203,11 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
 // path's term T_r = L_r - C (in [0, P2]) as one byte per cell, and the
 // per-pixel kernel forms S = 8 C + sum T_r (at most 8 (255 + 255) < 2^16, so
 // the sum modulo 2^16 is the plain sum). With u16 sums (any penalties) the
-// first pass writes the sum volume and the next seven add to it.
+// first launch writes the sums and the next ones add to them; full-range waves
+// run two directions a launch, each with a volume of its own, where the scratch
+// holds two: more chains in flight, and two reads of a cost close together (P2
+// = 600, one volume and two: 640x480 pair, 128 labels 1.58 and 1.08 ms;
+// 1024x768, 512 labels 8.45 and 7.65; 2048x1536, 128 labels 9.2 and 8.4).
 enum PassMode { kFirst = 0, kAccumulate = 1, kTerm = 3 };
 constexpr int kTermArrays = 8;
 constexpr int kMaxPasses = 8;
@@ -325,7 +329,8 @@ R3D_DEVICE uint32_t min_words(const uint32_t (&v)[N]) {
 }
 
 // The eight words of unit u of a pixel's total sums, from its cost and term
-// bytes (TERMS) or its stored u16 sums.
+// bytes (TERMS) or its stored u16 sums (tstride: values to the next array, 0
+// with one sum volume).
 template <bool TERMS>
 R3D_DEVICE void sum_unit(const uint8_t* cp, const uint8_t* tp, int64_t tstride, const uint16_t* sp, int u,
                          uint32_t (&wv)[8]) {
@@ -343,16 +348,24 @@ R3D_DEVICE void sum_unit(const uint8_t* cp, const uint8_t* tp, int64_t tstride, 
       for (int k = 0; k < 8; ++k) wv[k] = r == 0 ? 8u * c2[k] : wv[k] + c2[k];
     }
   } else {
-    const uint4* sp4 = reinterpret_cast<const uint4*>(sp);
-    const uint4 a = sp4[2 * u], b = sp4[2 * u + 1];
-    wv[0] = a.x;
-    wv[1] = a.y;
-    wv[2] = a.z;
-    wv[3] = a.w;
-    wv[4] = b.x;
-    wv[5] = b.y;
-    wv[6] = b.z;
-    wv[7] = b.w;
+    auto load = [u](const uint16_t* v, uint32_t (&w)[8]) {
+      const uint4 a = reinterpret_cast<const uint4*>(v)[2 * u], b = reinterpret_cast<const uint4*>(v)[2 * u + 1];
+      w[0] = a.x;
+      w[1] = a.y;
+      w[2] = a.z;
+      w[3] = a.w;
+      w[4] = b.x;
+      w[5] = b.y;
+      w[6] = b.z;
+      w[7] = b.w;
+    };
+    load(sp, wv);
+    if (tstride != 0) {  // a second volume
+      uint32_t w2[8];
+      load(sp + tstride, w2);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) wv[k] = r3dsimt::vadd2(wv[k], w2[k]);
+    }
   }
 }
 // Unit u's sums in label order.
@@ -376,7 +389,9 @@ struct PathRing {
   static constexpr int kMinBlocks = K <= 8 ? 8 : 5;
   static constexpr int ND = 2 * G * K;
   static constexpr int kPlanes = MODE == kAccumulate ? 3 : 1;
-  static constexpr int kStages = MODE == kTerm ? 8 : 4;
+  // The u16 modes with 4, 5 and 6 stages: 640x480 pair, 128 labels 1.12, 1.08
+  // and 1.10 ms; 1024x768, 96 labels 2.07, 1.96 and 1.99; 256: 4.13, 4.13, 4.16.
+  static constexpr int kStages = MODE == kTerm ? 8 : 5;
   static constexpr int kPlaneBytes = (32 / G) * kPlanes * ND;
   static constexpr int kStageBytes = kPlaneBytes + 32 * 4;
   static constexpr int kWarpBytes = kStages * kStageBytes;
@@ -446,9 +461,10 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS_MIN((PathRing<G, K, MODE>::kThreads), (PathRin
     const int64_t dcell = (static_cast<int64_t>(dy) * w + dx) * nd;
     const int64_t cell0 = job.cell_off + e0 + (static_cast<int64_t>(sy) * w + sx) * nd;
     const uint8_t* c_in = cost + cell0;
-    const uint16_t* s_in = sum + cell0;
-    uint16_t* s_out = sum + cell0;
-    uint8_t* t_out = terms + cell0 + static_cast<int64_t>(tslot) * tstride;
+    const int64_t out0 = cell0 + static_cast<int64_t>(tslot) * tstride;
+    const uint16_t* s_in = sum + out0;
+    uint16_t* s_out = sum + out0;
+    uint8_t* t_out = terms + out0;
     const int64_t dpx = static_cast<int64_t>(dy) * w + dx;
     // Intensity of the pixel being issued (each lane copies the aligned
     // 4-byte word holding it into the stage), and the parity of the
@@ -1544,8 +1560,10 @@ void launch_passes(const SgmMatch* dm, const SgmPathJob* jobs, const SgmPathSegm
       launch_pass<G, K, kTerm>(ps, dm, jobs, g.count, cost, sum, terms, tstride, ints, sms, s, g, cancel);
     return;
   }
-  for (int q = 0; q < kMaxPasses; ++q) {
-    const PassSet ps = pass_set(g, kAllPasses + q, 1, counters + q);
+  // Two directions at a time, each into its own volume, or one.
+  const int per = tstride != 0 ? 2 : 1;
+  for (int q = 0; q < kMaxPasses; q += per) {
+    const PassSet ps = pass_set(g, kAllPasses + q, per, counters + q);
     if (q == 0)
       launch_pass<G, K, kFirst>(ps, dm, jobs, g.count, cost, sum, terms, tstride, ints, sms, s, g, cancel);
     else
@@ -1584,15 +1602,20 @@ bool path_shape_compiled(int g, int k) {
 }
 }  // namespace
 
-SgmPathShape sgm_path_shape(int nd) {
+SgmPathShape sgm_path_shape(int nd, bool terms) {
   // A compiled shape from R3DGPU_PATH_SHAPE ("G,K": any label count it
   // covers) or the tuning table (an entry for exactly this label count), else
-  // 8 label pairs per lane up to 64 labels, 16 above, with the fewest lanes.
-  // Whole pair, 2048x1536 (1536x1152 for 384 labels): 64 labels 3.57 ms with 8
-  // pairs per lane, 3.65 with 16; 96: 5.54 and 5.38; 128: 5.85 and 5.76; 256:
-  // 11.35 and 10.21; 384: 13.01 and 10.89. 24 pairs per lane, which fit 48,
-  // 96, 192 and 384 labels without idle lanes, took 3.84, 5.78, 10.2 and 11.4
-  // (longer steps, fewer chains in flight).
+  // with the fewest lanes of 8 label pairs per lane (up to 64 labels, and
+  // u16 sums up to 512) or of 16.
+  // Byte terms, whole pair, 2048x1536 (1536x1152 for 384 labels): 64 labels
+  // 3.57 ms with 8 pairs per lane, 3.65 with 16; 96: 5.54 and 5.38; 128: 5.85
+  // and 5.76; 256: 11.35 and 10.21; 384: 13.01 and 10.89. 24 pairs per lane,
+  // which fit 48, 96, 192 and 384 labels without idle lanes, took 3.84, 5.78,
+  // 10.2 and 11.4 (longer steps, fewer chains in flight).
+  // u16 sums run two directions at a time, so chains in flight count for more.
+  // 1024x768 pair, P2 = 600, 8 and 16 pairs per lane: 64 labels 1.44 and 1.74
+  // ms; 96: 1.96 and 2.58; 128: 2.33 and 2.67; 256: 4.13 and 4.47; 384: 6.34
+  // and 6.72; 512: 7.65 and 8.34. 2048x1536, 128 labels: 8.40 and 9.02.
   if (const char* e = std::getenv("R3DGPU_PATH_SHAPE")) {
     int g = 0, k = 0;
     if (std::sscanf(e, "%d,%d", &g, &k) == 2 && path_shape_compiled(g, k) && 2 * g * k >= nd) return {g, k};
@@ -1601,7 +1624,7 @@ SgmPathShape sgm_path_shape(int nd) {
   if (it != tuning().path.end() && path_shape_compiled(it->second.g, it->second.k) &&
       2 * it->second.g * it->second.k >= nd)
     return {it->second.g, it->second.k};
-  const int k_want = nd <= 64 ? 8 : 16;
+  const int k_want = nd <= (terms ? 64 : 512) ? 8 : 16;
   SgmPathShape best{0, 0};
   int best_nd = 1 << 30;
 #define R3D_SHAPE(g, k)                                              \
@@ -1616,16 +1639,24 @@ SgmPathShape sgm_path_shape(int nd) {
   return best;
 }
 
-SgmPathBuffers sgm_path_buffers(int64_t cells, int64_t pixels, int64_t keys, bool terms) {
+namespace {
+// The arrays of the mode: their size, and b.stride.
+size_t path_arrays(SgmPathBuffers& b, int64_t cells, SgmPathMode mode) {
+  const int arrays = mode == kPathTerms ? kTermArrays : (mode == kPathTwoSums ? 2 : 1);
+  const size_t value = mode == kPathTerms ? 1 : 2;
+  const size_t bytes = align256(static_cast<size_t>(cells) * value);
+  b.stride = static_cast<int64_t>(bytes / value);
+  return static_cast<size_t>(arrays) * bytes;
+}
+}  // namespace
+
+SgmPathBuffers sgm_path_buffers(int64_t cells, int64_t pixels, int64_t keys, SgmPathMode mode) {
   SgmPathBuffers b{};
   size_t o = 0;
   b.cost = o;
   o += align256(static_cast<size_t>(cells));
-  b.sum = o;
-  b.term_stride = terms ? static_cast<int64_t>(align256(static_cast<size_t>(cells))) : 0;
-  b.terms = b.sum;
-  o += terms ? static_cast<size_t>(kTermArrays) * static_cast<size_t>(b.term_stride)
-             : align256(static_cast<size_t>(cells) * 2);
+  b.paths = o;
+  o += path_arrays(b, cells, mode);
   // Winners of a tile row until its right-view keys are complete: only for
   // matches with the diagonal check.
   b.info = o;
@@ -1642,10 +1673,12 @@ SgmPathBuffers sgm_path_buffers(int64_t cells, int64_t pixels, int64_t keys, boo
 
 void launch_sgm_path_wave(const SgmMatch* dm, const SgmPathWave& wave, int sms, cudaStream_t s) {
   if (wave.njobs <= 0 || wave.cells <= 0) return;
-  const SgmPathBuffers B = sgm_path_buffers(wave.cells, wave.pixels, wave.keys, wave.terms != 0);
+  const SgmPathBuffers B = sgm_path_buffers(wave.cells, wave.pixels, wave.keys, wave.mode);
   uint8_t* cost = wave.buffer + B.cost;
-  uint16_t* sum = reinterpret_cast<uint16_t*>(wave.buffer + B.sum);
-  uint8_t* terms = wave.terms != 0 ? wave.buffer + B.terms : nullptr;
+  uint16_t* sum = reinterpret_cast<uint16_t*>(wave.buffer + B.paths);
+  uint8_t* terms = wave.mode == kPathTerms ? wave.buffer + B.paths : nullptr;
+  // From one array to the next; 0: one sum volume.
+  const int64_t stride = wave.mode == kPathSum ? 0 : B.stride;
   int4* info = reinterpret_cast<int4*>(wave.buffer + B.info);
   uint16_t* ints = reinterpret_cast<uint16_t*>(wave.buffer + B.ints);
   int* counters = reinterpret_cast<int*>(wave.buffer + B.counters);
@@ -1673,7 +1706,7 @@ void launch_sgm_path_wave(const SgmMatch* dm, const SgmPathWave& wave, int sms, 
     bool done = false;
 #define R3D_SHAPE(gg, kk)                                                                                     \
   if (!done && g.shape.g_ == gg && g.shape.k_ == kk) {                                                        \
-    launch_passes<gg, kk>(dm, jobs, g, cost, sum, terms, B.term_stride, ints, sms, s, wave.cancel,            \
+    launch_passes<gg, kk>(dm, jobs, g, cost, sum, terms, stride, ints, sms, s, wave.cancel,                   \
                           counters + 8 * q);                                                                  \
     done = true;                                                                                              \
   }
@@ -1697,7 +1730,7 @@ void launch_sgm_path_wave(const SgmMatch* dm, const SgmPathWave& wave, int sms, 
   const int64_t want = wave.keys > 0 || wave.rows <= 0 ? 1 : (resident + wave.rows - 1) / wave.rows;
   const int parts = static_cast<int>(want > 8 ? 8 : want);
   R3D_LAUNCH(wta, dim3(resident_grid(wta, sms, wave.rows, kPathThreads / 32, smem), parts), dim3(kPathThreads), smem, s,
-             dm, wave.jobs, wave.njobs, wave.rows, cost, sum, terms, B.term_stride, info, key_words);
+             dm, wave.jobs, wave.njobs, wave.rows, cost, sum, terms, stride, info, key_words);
   launched("sgm_path_wta_kernel");
 }
 
@@ -1776,16 +1809,13 @@ SgmPathShape sgm_path_ranged_shape(int64_t cells, int64_t pixels) {
 }
 
 SgmPathBuffers sgm_path_ranged_buffers(int64_t cells, int64_t pixels, int64_t keys, int64_t rows, int maxnum,
-                                       int sms, bool terms) {
+                                       int sms, SgmPathMode mode) {
   SgmPathBuffers b{};
   size_t o = 0;
   b.cost = o;
   o += align256(static_cast<size_t>(cells));
-  // Eight byte-term arrays, or the u16 sums.
-  b.sum = b.terms = o;
-  b.term_stride = terms ? static_cast<int64_t>(align256(static_cast<size_t>(cells))) : 0;
-  o += terms ? static_cast<size_t>(kTermArrays) * static_cast<size_t>(b.term_stride)
-             : align256(static_cast<size_t>(cells) * 2);
+  b.paths = o;
+  o += path_arrays(b, cells, mode);
   // Winners and right-view keys: only for matches with the diagonal check.
   b.info = o;
   if (keys > 0) o += align256(static_cast<size_t>(pixels) * 16);
@@ -1815,10 +1845,11 @@ SgmPathBuffers sgm_path_ranged_buffers(int64_t cells, int64_t pixels, int64_t ke
 void launch_sgm_path_ranged_wave(const SgmMatch* dm, const SgmPathRangedWave& wave, int sms, cudaStream_t s) {
   if (wave.njobs <= 0 || wave.pixels <= 0) return;
   const SgmPathBuffers B =
-      sgm_path_ranged_buffers(wave.cells, wave.pixels, wave.keys, wave.rows, wave.maxnum, sms, wave.terms != 0);
+      sgm_path_ranged_buffers(wave.cells, wave.pixels, wave.keys, wave.rows, wave.maxnum, sms, wave.mode);
   uint8_t* cost = wave.buffer + B.cost;
-  uint16_t* sum = reinterpret_cast<uint16_t*>(wave.buffer + B.sum);
-  uint8_t* terms = wave.terms != 0 ? wave.buffer + B.terms : nullptr;
+  uint16_t* sum = reinterpret_cast<uint16_t*>(wave.buffer + B.paths);
+  uint8_t* terms = wave.mode == kPathTerms ? wave.buffer + B.paths : nullptr;
+  const int64_t stride = wave.mode == kPathSum ? 0 : B.stride;
   int4* info = reinterpret_cast<int4*>(wave.buffer + B.info);
   uint32_t* rkeys = reinterpret_cast<uint32_t*>(wave.buffer + B.rkeys);
   uint2* rec = reinterpret_cast<uint2*>(wave.buffer + B.rec);
@@ -1844,17 +1875,17 @@ void launch_sgm_path_ranged_wave(const SgmMatch* dm, const SgmPathRangedWave& wa
     const SgmPathSegment& g = wave.segs[q];
     const SgmPathJob* jobs = wave.jobs + g.first;
     if (g.shape.k_ == 8)
-      launch_ranged_passes<8>(dm, jobs, g, rec, cost, sum, terms, B.term_stride, ovf, B.overflow_words, sms, s,
+      launch_ranged_passes<8>(dm, jobs, g, rec, cost, sum, terms, stride, ovf, B.overflow_words, sms, s,
                               wave.cancel, counters + 8 * q);
     else if (g.shape.k_ == 16)
-      launch_ranged_passes<16>(dm, jobs, g, rec, cost, sum, terms, B.term_stride, ovf, B.overflow_words, sms, s,
+      launch_ranged_passes<16>(dm, jobs, g, rec, cost, sum, terms, stride, ovf, B.overflow_words, sms, s,
                                wave.cancel, counters + 8 * q);
     else
       fail(R3DGPU_EINVAL, "stereo: bad ranged path kernel shape");
   }
   auto* wta = terms != nullptr ? sgm_path_ranged_wta_kernel<true> : sgm_path_ranged_wta_kernel<false>;
   R3D_LAUNCH(wta, dim3(resident_grid(wta, sms, wave.rows, kPathThreads / 32)), dim3(kPathThreads), 0, s, dm, wave.jobs,
-             wave.njobs, wave.rows, rec, cost, sum, terms, B.term_stride, rowshift, info, rkeys);
+             wave.njobs, wave.rows, rec, cost, sum, terms, stride, rowshift, info, rkeys);
   launched("sgm_path_ranged_wta_kernel");
   if (wave.keys > 0) {  // matches with the diagonal left-right check
     R3D_LAUNCH(sgm_path_ranged_accept_kernel,

@@ -25,9 +25,9 @@ struct SgmPathJob {
   int pad_;
   int64_t cell_off;           // first cell of the tile in the wave's cost and sum volumes
   int64_t px_off;             // first pixel of the tile in the wave's WTA records
-  int64_t rk_off;             // first right-WTA key of the tile (diagonal LR only)
+  int64_t rk_off;             // ranged waves with the diagonal check: first right-WTA key of the tile
   int64_t blk[kPathClasses];  // first chain block (32 / G chains) of the tile, per chain class
-  int64_t row_off;            // ranged waves: first row of the tile in the wave's per-row arrays
+  int64_t row_off;            // first row of the tile in the wave
   float* disp;
   float* conf;
   unsigned long long* cells;
@@ -40,25 +40,30 @@ struct SgmPathShape {
   int k_;
 };
 
-// The shape for nd labels ({0, 0}: more labels than the path
-// kernels take, or a tile too wide for the cost kernel's staged partner row:
-// tile width + nd - 1 must stay within 2048).
-SgmPathShape sgm_path_shape(int nd);
-// Whether a full-range tile of width w with nd labels fits the cost kernel.
+// The shape for nd labels with byte terms or u16 sums ({0, 0}: more labels
+// than the path kernels take, in either mode).
+SgmPathShape sgm_path_shape(int nd, bool terms);
+// Whether a full-range tile of width w with nd labels fits the cost kernel's
+// staged partner row.
 inline bool sgm_path_fits(int w, int nd) { return w + nd - 1 <= 2048; }
 inline int64_t sgm_path_chains(int cls, int w, int h) { return cls == 0 ? h : (cls == 1 ? w : w + h - 1); }
 
-// Device buffers of a wave (bytes, 256-byte aligned pieces). Byte terms, in
-// place of the u16 sum volume: arrays of term_stride bytes from `terms` on
-// (seven of full-range waves, eight of ranged ones).
+// What the passes of a wave leave in global memory: byte terms, an array per
+// direction (every P2 <= 255), or u16 sums, in one volume or (full-range
+// waves) in two, one of each two directions that run together. Bytes per
+// label with the cost: 9, 3 and 5.
+enum SgmPathMode : int { kPathTerms, kPathSum, kPathTwoSums };
+
+// Device buffers of a wave (bytes, 256-byte aligned pieces).
 struct SgmPathBuffers {
-  size_t cost, sum, terms, info, rkeys, ints, total;  // ints: full-range waves, the tiles' intensities
-  size_t counters;                                    // block counters of the pass launches
-  int64_t term_stride;
-  size_t rec, rowsum, rowstart, rowshift, overflow;  // ranged waves only
-  int overflow_words;                                // per wide vector's buffer
+  size_t cost, paths, info, total;
+  size_t counters;  // block counters of the pass launches
+  int64_t stride;   // values (bytes or u16) from one array of `paths` to the next
+  size_t ints;      // full-range waves: the tiles' intensities
+  size_t rkeys, rec, rowsum, rowstart, rowshift, overflow;  // ranged waves only
+  int overflow_words;                                       // per wide vector's buffer
 };
-SgmPathBuffers sgm_path_buffers(int64_t cells, int64_t pixels, int64_t keys, bool terms);
+SgmPathBuffers sgm_path_buffers(int64_t cells, int64_t pixels, int64_t keys, SgmPathMode mode);
 
 // A wave on the device: all jobs (device pointer), and per shape the range
 // of jobs with its chain-block counts.
@@ -83,9 +88,9 @@ struct SgmPathWave {
   const SgmPathSegment* segs;  // host array
   int nsegs;
   int64_t cells, pixels, keys, rows;
-  unsigned char* buffer;  // sgm_path_buffers(cells, pixels, keys, terms).total bytes
+  unsigned char* buffer;  // sgm_path_buffers(cells, pixels, keys, mode).total bytes
   const int* cancel;      // device view of the caller's cancellation flag, or null
-  int terms;              // 1: byte terms (every match of the wave has term_u8)
+  SgmPathMode mode;       // kPathTerms: every match of the wave has term_u8
   int max_span;           // largest tile width + labels - 1 of the wave (0: unknown)
 };
 
@@ -110,11 +115,11 @@ struct SgmPathRangedWave {
   int maxnum;  // largest label count of a pixel of the wave
   unsigned char* buffer;
   const int* cancel;  // device view of the caller's cancellation flag, or null
-  int terms;          // byte terms (every match of the wave has term_u8)
+  SgmPathMode mode;   // kPathTerms (every match of the wave has term_u8) or kPathSum
   int max_span;       // largest tile width + labels - 1 of the wave (0: unknown)
 };
 SgmPathBuffers sgm_path_ranged_buffers(int64_t cells, int64_t pixels, int64_t keys, int64_t rows, int maxnum,
-                                       int sms, bool terms);
+                                       int sms, SgmPathMode mode);
 void launch_sgm_path_ranged_wave(const SgmMatch* dm, const SgmPathRangedWave& wave, int sms, cudaStream_t s);
 bool sgm_path_ranged_enabled();
 

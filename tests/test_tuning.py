@@ -5,6 +5,7 @@ identical, and environment overrides take precedence."""
 
 from __future__ import annotations
 
+import collections
 import ctypes
 import json
 
@@ -113,6 +114,18 @@ def test_shapes_of_one_width_in_a_batch(simt_matcher, monkeypatch):
         assert np.array_equal(a.disparity, b.disparity) and np.array_equal(a.confidence, b.confidence)
 
 
+def test_default_shapes_by_mode(simt_matcher):
+    """Byte terms take 16 label pairs per lane above 64 labels; u16 sums, one
+    direction at a time, 8 up to 512 labels."""
+    left, right, _ = render_pair(Texture(75), 12, 4, lambda x, y: 4.0 + 0.1 * x)
+    for nd, terms, sums in ((64, "4x8", "4x8"), (80, "4x16", "8x8"), (128, "4x16", "8x8"), (256, "8x16", "16x8"),
+                            (272, "16x16", "32x8"), (512, "16x16", "32x8"), (528, "32x16", "32x16")):
+        for p2, want in ((200, {f"{terms}/mode3"}), (400, {f"{sums}/mode0", f"{sums}/mode1"})):
+            _, shapes = pass_shapes(simt_matcher,
+                                    lambda: simt_matcher.sgm_cost_volume(left, right, 0, nd, StereoOptions(p2=p2)))
+            assert shapes == want, (nd, p2)
+
+
 def _scratch_budget(m, n):
     """Sets the SGM scratch budget of this thread, as a server worker does (0: the default)."""
     m.lib._ZN6r3dgpu25set_thread_scratch_budgetEm(ctypes.c_size_t(n))
@@ -120,8 +133,9 @@ def _scratch_budget(m, n):
 
 def test_pass_mode_by_tile(simt_matcher):
     """The pass mode is each tile's own: a tile whose byte terms (9 bytes a
-    label) pass the scratch budget takes u16 sums (3 bytes), as a pair with a
-    P2 above 255 does, and the batch's other pairs keep byte terms."""
+    label) pass the scratch budget takes u16 sums (two volumes, 5 bytes, two
+    directions a launch, or one, 3 bytes), as a pair with a P2 above 255 does,
+    and the batch's other pairs keep byte terms."""
     def pair(seed, w, h, nd, **kw):
         left, right, _ = render_pair(Texture(seed), w, h, lambda x, y: 5.0 + 0.1 * x)
         return dict(left=left, right=right, disparity_min=0, num_disparities=nd, options=StereoOptions(**kw))
@@ -129,18 +143,21 @@ def test_pass_mode_by_tile(simt_matcher):
     def modes(pairs, budget):
         _scratch_budget(simt_matcher, budget)
         try:
-            return pass_shapes(simt_matcher, lambda: simt_matcher.match_stereo_batch(pairs))
+            out, launches = _launches(simt_matcher, lambda: simt_matcher.match_stereo_batch(pairs))
+            return out, collections.Counter(e["shape"] for e in launches if e.get("pass"))
         finally:
             _scratch_budget(simt_matcher, 0)
 
-    # 60 x 24 x 64 labels: 829 kB with terms, 276 kB without.
+    # 60 x 24 x 64 labels: 829 kB with terms, 461 and 276 kB with sums (a wave for each of its two matches).
     pairs = [pair(71, 60, 24, 64, levels=0), pair(72, 24, 12, 32, levels=0), pair(73, 20, 10, 16, levels=0, p2=400)]
     ref, shapes = modes(pairs, 0)
-    assert shapes == {"4x8/mode3", "2x8/mode3", "1x8/mode0", "1x8/mode1"}
-    got, shapes = modes(pairs, 500_000)
-    assert shapes == {"4x8/mode0", "4x8/mode1", "2x8/mode3", "1x8/mode0", "1x8/mode1"}
-    for a, b in zip(got, ref):
-        assert np.array_equal(a.disparity, b.disparity) and np.array_equal(a.confidence, b.confidence)
+    assert shapes == {"4x8/mode3": 1, "2x8/mode3": 1, "1x8/mode0": 1, "1x8/mode1": 3}
+    for budget, adding in ((500_000, 3), (300_000, 7)):
+        got, shapes = modes(pairs, budget)
+        assert set(shapes) == {"4x8/mode0", "4x8/mode1", "2x8/mode3", "1x8/mode0", "1x8/mode1"}
+        assert (shapes["4x8/mode0"], shapes["4x8/mode1"]) == (2, 2 * adding)
+        for a, b in zip(got, ref):
+            assert np.array_equal(a.disparity, b.disparity) and np.array_equal(a.confidence, b.confidence)
     # Ranged tiles: the finer level of a hierarchy (its coarser one, full range, is smaller).
     pairs = [pair(74, 72, 40, 48, levels=1, range_radius=0, range_margin=2, range_fill=0)]
     ref, shapes = modes(pairs, 0)
