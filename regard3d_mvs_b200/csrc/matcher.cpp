@@ -1960,7 +1960,8 @@ r3dgpu_status r3dgpu_sgm_cost_volume_host(const r3dgpu_view_u16* left, const r3d
     }
     const SgmFullPlan plan = (ranges_lo && ranges_num) ? SgmFullPlan{{0, 0}, 0} : sgm_full_plan(nd, W.smem_optin);
     const SgmFullShape sh = plan.shape;
-    const bool ranged = !sh.g_ && !general_ranged_kernel();
+    // Neither a full-range shape nor ranges (more than 768 labels): the general kernel.
+    const bool ranged = ranges_lo && ranges_num && !general_ranged_kernel();
     SgmRangedPlan rplan{{0, 0}, 0};
     if (ranged) {
       // The whole image is one tile: its label statistics from the host ranges.

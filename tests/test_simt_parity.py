@@ -99,6 +99,14 @@ def test_volume_ranges_and_wrap(simt_matcher, oracle):
                           oracle.sgm_cost_volume(left, right, -5, 144, o))
 
 
+def test_volume_of_more_labels_than_the_shapes(simt_matcher, oracle):
+    """More than 768 labels without ranges: the general kernel."""
+    left, right, _ = render_pair(Texture(3), 20, 5, lambda x, y: 4.0 + 0.1 * x)
+    o = StereoOptions()
+    assert np.array_equal(simt_matcher.sgm_cost_volume(left, right, 0, 784, o),
+                          oracle.sgm_cost_volume(left, right, 0, 784, o))
+
+
 @pytest.mark.parametrize("opts", [
     StereoOptions(tile_size=32, tile_margin=4, tile_blend=4, levels=0),
     StereoOptions(tile_size=32, tile_margin=4, tile_blend=4, levels=0, lr_full_match=False, uniqueness=0.1),
