@@ -15,7 +15,7 @@ import pytest
 
 from images import Rng, Texture, mismatch_report, random_image, render_pair, same_disparities, to_u16
 from regard3d_mvs_b200.types import LabelRanges, StereoOptions, SubpixelMethod
-from test_tuning import pass_shapes
+from test_tuning import match_kernels, pass_shapes
 
 pytestmark = pytest.mark.gpu
 
@@ -301,12 +301,14 @@ def test_ranged_volume_kernels(gpu_matcher, oracle, monkeypatch, kernel, shape, 
 @pytest.mark.parametrize("lr_full", [True, False])
 def test_ranged_kernel_hierarchy_shapes(gpu_matcher, oracle, monkeypatch, lr_full):
     """The hierarchy with the wide-range shape and short bands."""
+    monkeypatch.setenv("R3DGPU_RANGED_KERNEL", "ranged")
     monkeypatch.setenv("R3DGPU_RANGED_SHAPE", "8,4")
     monkeypatch.setenv("R3DGPU_RANGED_ROWS", "12")
     left, right = _synthetic_pair(500, 380, 192, 4)
     o = StereoOptions(levels=2, range_radius=0, range_margin=8, lr_full_match=lr_full, tile_size=256)
-    _assert_same_map(gpu_matcher.match_stereo(left, right, None, None, 0, 192, o),
-                     oracle.match_stereo(left, right, None, None, 0, 192, o))
+    a, kernels = match_kernels(gpu_matcher, lambda: gpu_matcher.match_stereo(left, right, None, None, 0, 192, o))
+    assert "sgm_ranged_kernel" in kernels and "sgm_path_ranged_kernel" not in kernels
+    _assert_same_map(a, oracle.match_stereo(left, right, None, None, 0, 192, o))
 
 
 def test_batch_equals_single(gpu_matcher):

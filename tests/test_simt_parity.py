@@ -14,7 +14,7 @@ import pytest
 
 from images import Rng, Texture, mismatch_report, random_image, render_pair, same_disparities, to_u16
 from regard3d_mvs_b200.types import LabelRanges, StereoOptions, SubpixelMethod
-from test_tuning import pass_shapes
+from test_tuning import match_kernels, pass_shapes
 
 
 def _same_map(a, b):
@@ -196,6 +196,7 @@ def _smooth_ranges(w, h, nd, seed, wide_frac=0.08):
 def test_ranged_kernel_volume(simt_matcher, oracle, monkeypatch, shape, rows):
     """Ranged kernel: aligned, shifted and bounds-checked predecessor reads,
     wide pixels, band seams (few rows per band), against the textbook volume."""
+    monkeypatch.setenv("R3DGPU_RANGED_KERNEL", "ranged")
     monkeypatch.setenv("R3DGPU_RANGED_SHAPE", shape)
     monkeypatch.setenv("R3DGPU_RANGED_ROWS", str(rows))
     tex = Texture(29)
@@ -210,13 +211,15 @@ def test_ranged_kernel_volume(simt_matcher, oracle, monkeypatch, shape, rows):
 @pytest.mark.parametrize("lr_full", [True, False])
 def test_ranged_kernel_hierarchy(simt_matcher, oracle, monkeypatch, lr_full):
     """The hierarchy through the ranged kernel with many bands per tile."""
+    monkeypatch.setenv("R3DGPU_RANGED_KERNEL", "ranged")
     monkeypatch.setenv("R3DGPU_RANGED_ROWS", "8")
     tex = Texture(31)
     left, right, _ = render_pair(tex, 72, 52, lambda x, y: np.where(x < 35, 6.0 + 0.05 * y, 17.5))
     o = StereoOptions(levels=2, tile_size=48, tile_margin=8, tile_blend=8, lr_full_match=lr_full, range_radius=1,
                       range_margin=4)
-    _same_map(simt_matcher.match_stereo(left, right, None, None, 0, 32, o),
-              oracle.match_stereo(left, right, None, None, 0, 32, o))
+    a, kernels = match_kernels(simt_matcher, lambda: simt_matcher.match_stereo(left, right, None, None, 0, 32, o))
+    assert "sgm_ranged_kernel" in kernels and "sgm_path_ranged_kernel" not in kernels
+    _same_map(a, oracle.match_stereo(left, right, None, None, 0, 32, o))
 
 
 @pytest.mark.parametrize("opts", [
@@ -228,11 +231,13 @@ def test_ranged_kernel_wide_pixels_wta(simt_matcher, oracle, monkeypatch, opts):
     """Large range margins make most pixels wider than a row's narrow width:
     the warp-cooperative wide path decides the winners, second bests,
     subpixel neighbours and diagonal LR keys."""
+    monkeypatch.setenv("R3DGPU_RANGED_KERNEL", "ranged")
     monkeypatch.setenv("R3DGPU_RANGED_ROWS", "8")
     tex = Texture(37)
     left, right, _ = render_pair(tex, 60, 34, lambda x, y: np.where(y < 15, 9.0 + 0.1 * x, 21.0))
-    _same_map(simt_matcher.match_stereo(left, right, None, None, 0, 48, opts),
-              oracle.match_stereo(left, right, None, None, 0, 48, opts))
+    a, kernels = match_kernels(simt_matcher, lambda: simt_matcher.match_stereo(left, right, None, None, 0, 48, opts))
+    assert "sgm_ranged_kernel" in kernels and "sgm_path_ranged_kernel" not in kernels
+    _same_map(a, oracle.match_stereo(left, right, None, None, 0, 48, opts))
 
 
 def test_speckles_across_union_tiles(simt_matcher, oracle):

@@ -35,6 +35,12 @@ def pass_shapes(m, run):
     return out, {e["shape"] for e in launches if e.get("pass")}
 
 
+def match_kernels(m, run):
+    """The result of run() and the names of its matches' SGM kernels."""
+    out, launches = _launches(m, run)
+    return out, {e["kernel"] for e in launches}
+
+
 def test_default_kernels_are_the_chain_passes(simt_matcher):
     """Full-range and ranged tiles go to the chain-pass kernels by default."""
     tex = Texture(61)
