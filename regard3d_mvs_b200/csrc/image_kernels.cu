@@ -327,9 +327,10 @@ R3D_GLOBAL void uf_filter_kernel(float* __restrict__ d, int64_t n, const int* pa
 // stereo_matcher.cpp:972-1021: median of the valid values of the 3x3
 // neighbourhood; an even count averages the two middle values.
 // Invalid neighbours enter as +inf, so that they sort behind the valid ones: a
-// fixed sorting network of 25 exchanges in registers (an insertion sort of the
-// valid ones needs a run-time indexed array in local memory: 64 us for 2048 x
-// 1536 pixels).
+// fixed sorting network of 25 exchanges in registers, the nine-input network of
+// Dobbelaere's published list of smallest known networks (an insertion sort of
+// the valid ones needs a run-time indexed array in local memory: 64 us for 2048
+// x 1536 pixels).
 R3D_GLOBAL void median_kernel(const float* __restrict__ in, int w, int h, float* __restrict__ out, int64_t ostride) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= w || y >= h) return;
