@@ -258,11 +258,14 @@ R3D_GLOBAL void uf_tile_kernel(const float* __restrict__ d, int w, int h, float 
   for (int ly = static_cast<int>(threadIdx.x >> 5); ly < kUfTile; ly += nw) {
     const int i = ly * kUfTile + lane;
     const int r = uf_root_local(par, i);
-    dv[i] = r3dsimt::finitef(dv[i]) ? 1.0F : 0.0F;
-    // One addition per run part of the warp's row that shares a root.
-    const uint32_t peers = r3dsimt::match_any(static_cast<uint32_t>(r));
-    const uint32_t valid = peers & r3dsimt::ballot(dv[i] != 0.0F);
-    if (lane == r3dsimt::ffs(peers) - 1 && valid != 0) atomicAdd(cnt + r, r3dsimt::popc(valid));
+    // One addition per run (its pixels share a root), by its first lane.
+    const uint32_t valid = r3dsimt::ballot(r3dsimt::finitef(dv[i])), st = starts[ly];
+    if ((st >> lane) & 1u) {
+      const uint32_t later = lane < 31 ? st >> (lane + 1) : 0u;
+      const int len = later != 0 ? r3dsimt::ffs(later) : 32 - lane;
+      const int n = r3dsimt::popc(valid & ((0xFFFFFFFFu >> (32 - len)) << lane));
+      if (n != 0) atomicAdd(cnt + r, n);
+    }
     if (lane < tw && ly < th)
       parent[static_cast<int64_t>(ty0 + ly) * w + tx0 + lane] = (ty0 + r / kUfTile) * w + tx0 + r % kUfTile;
   }

@@ -255,3 +255,17 @@ def test_speckles_across_union_tiles(simt_matcher, oracle):
     for size, diff in ((5, 0.5), (40, 1.0), (400, 1.0), (3000, 0.2)):
         assert same_disparities(simt_matcher.remove_speckles(d.copy(), size, diff),
                                 oracle.remove_speckles(d, size, diff)), (size, diff)
+
+
+@pytest.mark.parametrize("w", [1, 31, 32, 33, 75])
+def test_speckles_of_thin_runs(simt_matcher, oracle, w):
+    """Runs of one pixel, of a whole tile row and everything between, in tiles
+    of one column to three: segment sizes are counted run by run."""
+    h = 37
+    rng = np.random.default_rng(w)
+    yy, xx = np.mgrid[0:h, 0:w]
+    for d in (10.0 * (xx % 2), 10.0 * (yy % 2), 10.0 * ((xx + yy) % 3), 0.0 * xx + 3.0, 500.0 * rng.random((h, w)),
+              np.where(rng.random((h, w)) < 0.55, 0.001 * xx, np.inf), np.round(2.0 * rng.random((h, w)))):
+        d = d.astype(np.float32)
+        for size in (2, 7, 40):
+            assert same_disparities(simt_matcher.remove_speckles(d.copy(), size, 0.5), oracle.remove_speckles(d, size, 0.5))
