@@ -818,9 +818,9 @@ bool ranged_terms_allowed() {
 //
 // A tile takes the fastest mode whose buffers stay within `tile_cap`, the
 // round's scratch that this group may take: byte terms (9 bytes a label) when
-// its match allows them (all P2 <= 255), else u16 sums in two volumes (5,
-// full-range tiles) or in one (3). This is decided tile by tile: another
-// pair's penalties or size do not change a pair's mode.
+// its match allows them (all P2 <= 255), else u16 sums in two volumes (5) or in
+// one (3). This is decided tile by tile: another pair's penalties or size do
+// not change a pair's mode.
 void plan_path_waves(const std::vector<std::pair<int, int>>& tiles, const std::vector<Match*>& matches, bool ranged,
                      size_t cap_bytes, size_t tile_cap, int sms, Arena& A, Pinned& H, cudaStream_t s,
                      std::vector<SgmPathRangedWave>& waves, std::vector<std::vector<SgmPathSegment>>& segs,
@@ -853,7 +853,7 @@ void plan_path_waves(const std::vector<std::pair<int, int>>& tiles, const std::v
       return bytes(mode, e.cells, e.px, e.keys, e.rows, e.maxnum) <= tile_cap;
     };
     e.mode = M.m.term_u8 != 0 && (!ranged || ranged_terms_allowed()) && fits(kPathTerms) ? kPathTerms
-             : !ranged && fits(kPathTwoSums)                                             ? kPathTwoSums
+             : fits(kPathTwoSums)                                                        ? kPathTwoSums
                                                                                          : kPathSum;
     e.sh = ranged ? sgm_path_ranged_shape(e.cells, e.px) : sgm_path_shape(M.m.nd, e.mode == kPathTerms);
     es.push_back(e);
@@ -1949,7 +1949,7 @@ r3dgpu_status r3dgpu_sgm_cost_volume_host(const r3dgpu_view_u16* left, const r3d
       wv.keys = 0;
       wv.rows = h;
       wv.maxnum = max_num;
-      wv.mode = hm->term_u8 != 0 && ranged_terms_allowed() ? kPathTerms : kPathSum;
+      wv.mode = hm->term_u8 != 0 && ranged_terms_allowed() ? kPathTerms : kPathTwoSums;
       W.scratch.reserve(sgm_path_ranged_buffers(wv.cells, px, 0, h, max_num, W.sms, wv.mode).total);
       wv.buffer = W.scratch.get();
       launch_sgm_path_ranged_wave(dm, wv, W.sms, s);

@@ -204,11 +204,12 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
 // path's term T_r = L_r - C (in [0, P2]) as one byte per cell, and the
 // per-pixel kernel forms S = 8 C + sum T_r (at most 8 (255 + 255) < 2^16, so
 // the sum modulo 2^16 is the plain sum). With u16 sums (any penalties) the
-// first launch writes the sums and the next ones add to them; full-range waves
-// run two directions a launch, each with a volume of its own, where the scratch
-// holds two: more chains in flight, and two reads of a cost close together (P2
-// = 600, one volume and two: 640x480 pair, 128 labels 1.58 and 1.08 ms;
-// 1024x768, 512 labels 8.45 and 7.65; 2048x1536, 128 labels 9.2 and 8.4).
+// first launch writes the sums and the next ones add to them, two directions a
+// launch, each with a volume of its own, where the scratch holds two: more
+// chains in flight, and two reads of a cost close together (P2 = 600, one volume
+// and two: 640x480 pair, 128 labels 1.58 and 1.08 ms; 1024x768, 512 labels 8.45
+// and 7.65; 2048x1536, 128 labels 9.2 and 8.4; four
+// levels of a 3072x2048 pair 29.4 and 19.2).
 enum PassMode { kFirst = 0, kAccumulate = 1, kTerm = 3 };
 constexpr int kTermArrays = 8;
 constexpr int kMaxPasses = 8;
@@ -1072,7 +1073,7 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kRangedThreads)
     const uint32_t chain_len = t1 > t0 ? static_cast<uint32_t>(t1 - t0) : 0u;
     auto has = [&](int i) { return static_cast<uint32_t>(i - t0) < chain_len; };
     const uint8_t* const cbase = cost + job.cell_off;
-    uint16_t* const sbase = sum + job.cell_off;
+    uint16_t* const sbase = sum + job.cell_off + tslot * tstride;
     uint8_t* const tout = terms + job.cell_off + tslot * tstride;
     const int dpx = dy * w + dx;
     const uint2* rp = rec + job.px_off + static_cast<int64_t>(sy) * w + sx;  // record of the next step to request
@@ -1787,8 +1788,9 @@ void launch_ranged_passes(const SgmMatch* dm, const SgmPathJob* jobs, const SgmP
                                  terms, tstride, ovf, ovf_words, sms, s, g, cancel);
     return;
   }
-  for (int q = 0; q < 8; ++q) {
-    const PassSet ps = pass_set(g, kAllPasses + q, 1, counters + q);
+  const int per = tstride != 0 ? 2 : 1;  // directions a launch, as in the full-range passes
+  for (int q = 0; q < kMaxPasses; q += per) {
+    const PassSet ps = pass_set(g, kAllPasses + q, per, counters + q);
     if (q == 0)
       launch_ranged_pass<K, kFirst>(ps, dm, jobs, g.count, rec, cost, sum, terms, tstride, ovf, ovf_words, sms, s, g,
                                     cancel);

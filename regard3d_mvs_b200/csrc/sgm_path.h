@@ -49,9 +49,9 @@ inline bool sgm_path_fits(int w, int nd) { return w + nd - 1 <= 2048; }
 inline int64_t sgm_path_chains(int cls, int w, int h) { return cls == 0 ? h : (cls == 1 ? w : w + h - 1); }
 
 // What the passes of a wave leave in global memory: byte terms, an array per
-// direction (every P2 <= 255), or u16 sums, in one volume or (full-range
-// waves) in two, one of each two directions that run together. Bytes per
-// label with the cost: 9, 3 and 5.
+// direction (every P2 <= 255), or u16 sums, in one volume or in two, one for
+// each of two directions that run together. Bytes per label with the cost: 9,
+// 3 and 5.
 enum SgmPathMode : int { kPathTerms, kPathSum, kPathTwoSums };
 
 // Device buffers of a wave (bytes, 256-byte aligned pieces).
@@ -115,7 +115,7 @@ struct SgmPathRangedWave {
   int maxnum;  // largest label count of a pixel of the wave
   unsigned char* buffer;
   const int* cancel;  // device view of the caller's cancellation flag, or null
-  SgmPathMode mode;   // kPathTerms (every match of the wave has term_u8) or kPathSum
+  SgmPathMode mode;   // kPathTerms: every match of the wave has term_u8
   int max_span;       // largest tile width + labels - 1 of the wave (0: unknown)
 };
 SgmPathBuffers sgm_path_ranged_buffers(int64_t cells, int64_t pixels, int64_t keys, int64_t rows, int maxnum,

@@ -164,10 +164,13 @@ def test_pass_mode_by_tile(simt_matcher):
         assert (shapes["4x8/mode0"], shapes["4x8/mode1"]) == (2, 2 * adding)
         for a, b in zip(got, ref):
             assert np.array_equal(a.disparity, b.disparity) and np.array_equal(a.confidence, b.confidence)
-    # Ranged tiles: the finer level of a hierarchy (its coarser one, full range, is smaller).
-    pairs = [pair(74, 72, 40, 48, levels=1, range_radius=0, range_margin=2, range_fill=0)]
-    ref, shapes = modes(pairs, 0)
-    assert {q.split("/")[1] for q in shapes if q.startswith("1x")} == {"mode3"}
-    got, shapes = modes(pairs, 300_000)
-    assert {q.split("/")[1] for q in shapes if q.startswith("1x")} == {"mode0", "mode1"}
-    assert np.array_equal(got[0].disparity, ref[0].disparity)
+    # Ranged tiles, the finer level of a hierarchy: 46 k labels a match at 9, 5 or 3 bytes, 23 kB of records, and in
+    # one of the two matches 230 kB for the vectors of wide pixels.
+    for p2, budget, want in ((200, 0, {"1x8/mode3": 1}), (200, 600_000, {"1x8/mode3": 1, "1x8/mode0": 1, "1x8/mode1": 3}),
+                             (200, 250_000, {"1x8/mode0": 2, "1x8/mode1": 14}), (400, 0, {"1x8/mode0": 1, "1x8/mode1": 3})):
+        pairs = [pair(74, 72, 40, 48, levels=1, range_radius=0, range_margin=2, range_fill=0, p2=p2)]
+        got, shapes = modes(pairs, budget)
+        assert {q: n for q, n in shapes.items() if q.startswith("1x8/")} == want, (p2, budget)
+        if p2 == 200:
+            ref = got if budget == 0 else ref
+            assert np.array_equal(got[0].disparity, ref[0].disparity)
