@@ -206,10 +206,10 @@ R3D_GLOBAL void R3D_LAUNCH_BOUNDS(kPathThreads)
 // the sum modulo 2^16 is the plain sum). With u16 sums (any penalties) the
 // first launch writes the sums and the next ones add to them, two directions a
 // launch, each with a volume of its own, where the scratch holds two: more
-// chains in flight, and two reads of a cost close together (P2 = 600, one volume
-// and two: 640x480 pair, 128 labels 1.58 and 1.08 ms; 1024x768, 512 labels 8.45
-// and 7.65; 2048x1536, 128 labels 9.2 and 8.4; four
-// levels of a 3072x2048 pair 29.4 and 19.2).
+// chains in flight for the same bytes (P2 = 600, one volume and two: 640x480
+// pair, 128 labels 1.58 and 1.08 ms; 1024x768, 512 labels 8.45 and 7.65;
+// 2048x1536, 128 labels 9.2 and 8.4, where an adding launch runs at 0.88 of the
+// copy rate; four levels of a 3072x2048 pair 29.4 and 19.2).
 enum PassMode { kFirst = 0, kAccumulate = 1, kTerm = 3 };
 constexpr int kTermArrays = 8;
 constexpr int kMaxPasses = 8;
