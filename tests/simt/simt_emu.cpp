@@ -59,6 +59,7 @@ thread_local int t_block_arrived = 0;
 thread_local int t_nthreads = 0;
 thread_local std::vector<WarpState>* t_warps = nullptr;
 thread_local std::unique_ptr<unsigned char[]> t_smem;
+thread_local std::vector<std::unique_ptr<char[]>> t_stacks;  // of finished launches, for the next one
 thread_local size_t t_smem_size = 0;
 thread_local const std::function<void()>* t_body = nullptr;
 thread_local std::string t_error;
@@ -234,7 +235,14 @@ void cp_async_wait_n(int n) {
 void launch(dim3 grid, dim3 block, size_t smem, const std::function<void()>& body) {
   const int nthreads = static_cast<int>(block.x * block.y * block.z);
   std::vector<Fiber> fibers(nthreads);
-  for (Fiber& f : fibers) f.stack.reset(new char[kStack]);
+  for (Fiber& f : fibers) {
+    if (t_stacks.empty()) {
+      f.stack.reset(new char[kStack]);
+    } else {
+      f.stack = std::move(t_stacks.back());
+      t_stacks.pop_back();
+    }
+  }
   std::vector<WarpState> warps((nthreads + 31) / 32);
   t_fibers = &fibers;
   t_warps = &warps;
@@ -298,6 +306,9 @@ void launch(dim3 grid, dim3 block, size_t smem, const std::function<void()>& bod
           }
         }
       }
+#ifndef R3D_ASAN  // (a finished fiber's frames stay marked in its stack's shadow)
+  for (Fiber& f : fibers) t_stacks.push_back(std::move(f.stack));
+#endif
   t_fibers = nullptr;
   t_cur = nullptr;
 }
